@@ -9,6 +9,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -601,188 +602,106 @@ __global__ void k_prep_B2h(const double *__restrict__ t2, Dims d, int Op8, const
 // ---------------------------------------------------------------------------
 // FP64 contraction kernels (one GEMM problem per blockIdx.z)
 // ---------------------------------------------------------------------------
-template <typename StageT>
 struct GemmLaunch {
     Dims d;
     ChunkDesc ch;
-    int cum[7];      // prefix sums used to decode blockIdx.z
+    int cum[7];      // prefix sums over orderings of the GEMM problems (blockIdx.z)
+    int nmt, nslice; // M tiles and K slices of blockIdx.x
     const double *A1, *B1, *A2, *B2;
-    StageT *S;       // staging
+    double *S;       // staging, or Wbar
     double *G;       // gradient target
 };
 
-template <typename StageT>
-__device__ __forceinline__ int find_tau(const GemmLaunch<StageT> &L, int b) {
+// The five contractions of a chunk.  F1: S_tau[p][q][y][x][r][z] = W for all
+// (tau, y, q); the adjoint kinds with Wbar[y][p][x][q][r][z] in L.S:
+//   B1A  ovvv: G_A1[y][p][x][f] += sum_{q,r,z} Wbar B1[q][r][z][f]   problems (tau, y)
+//   B1B  t2:   G_B1[q][r][z][f] += sum_{y,p,x} Wbar A1[y][p][x][f]   problems (tau, q)
+//   B1C  ovoo: G_A2[q][p][x][m] -= sum_{y,r,z} Wbar B2[y][r][z][m]   problems (tau, q)
+//   B1D  t2:   G_B2[y][r][z][m] -= sum_{q,p,x} Wbar A2[q][p][x][m]   problems (tau, y)
+// Orderings that share a block write the same rows in B1B and B1C, and K may
+// be cut into slices, so the adjoint kinds add atomically.
+enum GemmKind { GK_F1 = 0, GK_B1A, GK_B1B, GK_B1C, GK_B1D };
+__host__ __device__ constexpr bool gemm_kfa(int kind) { return kind == GK_F1 || kind == GK_B1A || kind == GK_B1C; }
+__host__ __device__ constexpr bool gemm_kfb(int kind) { return kind == GK_F1; }
+
+__device__ __forceinline__ int find_tau(const GemmLaunch &L, int b) {
     int t = 0;
     while (t + 1 < L.ch.nperm && b >= L.cum[t + 1]) t++;
     return t;
 }
 
-// F1: S_tau[p][q][y][x][r][z] = W for all (tau, y, q)
-__global__ void __launch_bounds__(256) k_f1_fp64(GemmLaunch<double> L) {
-    __shared__ GemmSmem sm;
-    const int b = blockIdx.z;
-    const int t = find_tau(L, b);
+template <int KIND, int BM, int BN>
+__global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant__ GemmLaunch L) {
+    extern __shared__ __align__(16) double gemm_smem[];
+    const int t = find_tau(L, blockIdx.z);
     const PermBlock &pb = L.ch.pb[t];
     const Dims &d = L.d;
-    const int o = d.o, v = d.v, Kp = d.Kp;
-    const int rem = b - L.cum[t];
-    const int y = rem / o, q = rem % o;
-    const long long yg = pb.Y0 + y;
+    const int o = d.o, v = d.v, Kp = d.Kp, rem = blockIdx.z - L.cum[t];
     const long long oTz = (long long)o * pb.Tz;
+    // Wbar strides
+    const long long s_q = pb.rzp, s_x = (long long)o * pb.rzp, s_p = (long long)pb.Tx * s_x, s_y = (long long)o * s_p;
+    const long long ovK = (long long)o * v * Kp, vK = (long long)v * Kp, ovo = (long long)o * v * o, vo = (long long)v * o;
     GemmArgs g;
-    g.M = o * pb.Tx;
-    g.N = o * pb.Tz;
-    g.K = v;
-    g.K2 = o;
-    g.A = GOp{L.A1 + (yg * o * v + pb.X0) * Kp, map2(pb.Tx, Kp, (long long)v * Kp), map1(1), 1};
-    g.B = GOp{L.B1 + ((long long)q * o * v + pb.Z0) * Kp, map2(pb.Tz, Kp, (long long)v * Kp), map1(1), 1};
-    g.A2 = GOp{L.A2 + ((long long)q * o * v + pb.X0) * o, map2(pb.Tx, o, (long long)v * o), map1(1), 1};
-    g.B2 = GOp{L.B2 + (yg * o * v + pb.Z0) * o, map2(pb.Tz, o, (long long)v * o), map1(1), 1};
-    g.C = L.S + pb.soff + (long long)q * pb.Ty * pb.Tx * oTz + (long long)y * pb.Tx * oTz;
-    g.cm = map2(pb.Tx, oTz, (long long)o * pb.Ty * pb.Tx * oTz);
-    g.cn = map1(1);
-    g.alpha = 1.0;
-    g.alpha2 = -1.0;
-    g.accumulate = 0;
-    const int m0 = blockIdx.x * kGBM, n0 = blockIdx.y * kGBN;
-    if (m0 >= g.M || n0 >= g.N) return;
-    gemm_fp64_tile(g, m0, n0, sm);
-}
-
-// ovvv gradient: G_A1[y][p][x][f] += sum_{q,r,z} Wbar * B1[q][r][z][f]; z = (tau, y)
-template <typename StageT>
-__global__ void __launch_bounds__(256) k_b1a_fp64(GemmLaunch<StageT> L) {
-    __shared__ GemmSmem sm;
-    const int b = blockIdx.z;
-    const int t = find_tau(L, b);
-    const PermBlock &pb = L.ch.pb[t];
-    const Dims &d = L.d;
-    const int o = d.o, v = d.v, Kp = d.Kp;
-    const int y = b - L.cum[t];
-    const long long oTz = (long long)o * pb.Tz;
-    GemmArgsT<StageT> g;
-    g.M = o * pb.Tx;
-    g.N = v;
-    g.K = o * o * pb.Tz;
     g.K2 = 0;
-    const long long s_r = pb.Tz, s_q = pb.rzp, s_x = (long long)o * pb.rzp;
-    const long long s_p = (long long)pb.Tx * s_x, s_y = (long long)o * s_p;
-    (void)s_r;
-    g.A = GOpT<StageT>{L.S + pb.swoff + (long long)y * s_y, map2(pb.Tx, s_x, s_p), map2((int)oTz, 1, s_q), 1};
-    g.B = GOp{L.B1 + (long long)pb.Z0 * Kp, map1(1),
-              map3(pb.Tz, o, Kp, (long long)v * Kp, (long long)o * v * Kp), 0};
-    g.C = L.G + (((long long)pb.Y0 + y) * o * v + pb.X0) * Kp;
-    g.cm = map2(pb.Tx, Kp, (long long)v * Kp);
     g.cn = map1(1);
     g.alpha = 1.0;
     g.alpha2 = 0.0;
-    g.accumulate = 1;
-    const int m0 = blockIdx.x * kGBM, n0 = blockIdx.y * kGBN;
+    g.atomic = 1;
+    if (KIND == GK_F1) {
+        const int y = rem / o, q = rem % o;
+        const long long yg = pb.Y0 + y;
+        g.M = o * pb.Tx;
+        g.N = o * pb.Tz;
+        g.K = v;
+        g.K2 = o;
+        g.A = GOp{L.A1 + yg * ovK + (long long)pb.X0 * Kp, map2(pb.Tx, Kp, vK), map1(1)};
+        g.B = GOp{L.B1 + q * ovK + (long long)pb.Z0 * Kp, map2(pb.Tz, Kp, vK), map1(1)};
+        g.A2 = GOp{L.A2 + q * ovo + (long long)pb.X0 * o, map2(pb.Tx, o, vo), map1(1)};
+        g.B2 = GOp{L.B2 + yg * ovo + (long long)pb.Z0 * o, map2(pb.Tz, o, vo), map1(1)};
+        g.C = L.S + pb.soff + ((long long)q * pb.Ty + y) * pb.Tx * oTz;
+        g.cm = map2(pb.Tx, oTz, (long long)o * pb.Ty * pb.Tx * oTz);
+        g.alpha2 = -1.0;
+        g.atomic = 0;
+    } else if (KIND == GK_B1A) {
+        g.M = o * pb.Tx;
+        g.N = v;
+        g.K = o * o * pb.Tz;
+        g.A = GOp{L.S + pb.swoff + rem * s_y, map2(pb.Tx, s_x, s_p), map2((int)oTz, 1, s_q)};
+        g.B = GOp{L.B1 + (long long)pb.Z0 * Kp, map1(1), map3(pb.Tz, o, Kp, vK, ovK)};
+        g.C = L.G + ((long long)pb.Y0 + rem) * ovK + (long long)pb.X0 * Kp;
+        g.cm = map2(pb.Tx, Kp, vK);
+    } else if (KIND == GK_B1B) {
+        g.M = o * pb.Tz;
+        g.N = v;
+        g.K = pb.Ty * o * pb.Tx;
+        g.A = GOp{L.S + pb.swoff + rem * s_q, map1(1), map3(pb.Tx, o, s_x, s_p, s_y)};
+        g.B = GOp{L.A1 + (long long)pb.Y0 * ovK + (long long)pb.X0 * Kp, map1(1), map3(pb.Tx, o, Kp, vK, ovK)};
+        g.C = L.G + rem * ovK + (long long)pb.Z0 * Kp;
+        g.cm = map2(pb.Tz, Kp, vK);
+    } else if (KIND == GK_B1C) {
+        g.M = o * pb.Tx;
+        g.N = o;
+        g.K = pb.Ty * o * pb.Tz;
+        g.A = GOp{L.S + pb.swoff + rem * s_q, map2(pb.Tx, s_x, s_p), map2((int)oTz, 1, s_y)};
+        g.B = GOp{L.B2 + (long long)pb.Y0 * ovo + (long long)pb.Z0 * o, map1(1), map3(pb.Tz, o, o, vo, ovo)};
+        g.C = L.G + rem * ovo + (long long)pb.X0 * o;
+        g.cm = map2(pb.Tx, o, vo);
+        g.alpha = -1.0;
+    } else {
+        g.M = o * pb.Tz;
+        g.N = o;
+        g.K = o * o * pb.Tx;
+        g.A = GOp{L.S + pb.swoff + rem * s_y, map1(1), map3(pb.Tx, o, s_x, s_p, s_q)};
+        g.B = GOp{L.A2 + (long long)pb.X0 * o, map1(1), map3(pb.Tx, o, o, vo, ovo)};
+        g.C = L.G + ((long long)pb.Y0 + rem) * ovo + (long long)pb.Z0 * o;
+        g.cm = map2(pb.Tz, o, vo);
+        g.alpha = -1.0;
+    }
+    const int m0 = (blockIdx.x % L.nmt) * BM, n0 = blockIdx.y * BN;
     if (m0 >= g.M || n0 >= g.N) return;
-    gemm_fp64_tile(g, m0, n0, sm);
+    gemm_fp64_tile<BM, BN, gemm_kfa(KIND), gemm_kfb(KIND)>(g, m0, n0, blockIdx.x / L.nmt, L.nslice, gemm_smem);
 }
 
-// t2 gradient (ovvv term): G_B1[q][r][z][f] += sum_{y,p,x} Wbar * A1[y][p][x][f]; z = q
-template <typename StageT>
-__global__ void __launch_bounds__(256) k_b1b_fp64(GemmLaunch<StageT> L) {
-    __shared__ GemmSmem sm;
-    // grid.z = (ordering, q): all orderings of the chunk in one launch; orderings
-    // that share a block write the same gradient rows, hence the atomic adds
-    const int q = blockIdx.z % L.d.o;
-    const PermBlock &pb = L.ch.pb[blockIdx.z / L.d.o];
-    const Dims &d = L.d;
-    const int o = d.o, v = d.v, Kp = d.Kp;
-    GemmArgsT<StageT> g;
-    g.M = o * pb.Tz;
-    g.N = v;
-    g.K = pb.Ty * o * pb.Tx;
-    g.K2 = 0;
-    const long long s_r = pb.Tz, s_q = pb.rzp, s_x = (long long)o * pb.rzp;
-    const long long s_p = (long long)pb.Tx * s_x, s_y = (long long)o * s_p;
-    (void)s_r;
-    g.A = GOpT<StageT>{L.S + pb.swoff + (long long)q * s_q, map1(1), map3(pb.Tx, o, s_x, s_p, s_y), 0};
-    g.B = GOp{L.A1 + ((long long)pb.Y0 * o * v + pb.X0) * Kp, map1(1),
-              map3(pb.Tx, o, Kp, (long long)v * Kp, (long long)o * v * Kp), 0};
-    g.C = L.G + ((long long)q * o * v + pb.Z0) * Kp;
-    g.cm = map2(pb.Tz, Kp, (long long)v * Kp);
-    g.cn = map1(1);
-    g.alpha = 1.0;
-    g.alpha2 = 0.0;
-    g.accumulate = 2;
-    const int m0 = blockIdx.x * kGBM, n0 = blockIdx.y * kGBN;
-    if (m0 >= g.M || n0 >= g.N) return;
-    gemm_fp64_tile(g, m0, n0, sm);
-}
-
-// ovoo gradient: G_A2[q][p][x][m] -= sum_{y,r,z} Wbar * B2[y][r][z][m]; z = q
-template <typename StageT>
-__global__ void __launch_bounds__(256) k_b1c_fp64(GemmLaunch<StageT> L) {
-    __shared__ GemmSmem sm;
-    // grid.z = (ordering, q): all orderings of the chunk in one launch; orderings
-    // that share a block write the same gradient rows, hence the atomic adds
-    const int q = blockIdx.z % L.d.o;
-    const PermBlock &pb = L.ch.pb[blockIdx.z / L.d.o];
-    const Dims &d = L.d;
-    const int o = d.o, v = d.v;
-    const long long oTz = (long long)o * pb.Tz;
-    GemmArgsT<StageT> g;
-    g.M = o * pb.Tx;
-    g.N = o;
-    g.K = pb.Ty * o * pb.Tz;
-    g.K2 = 0;
-    const long long s_r = pb.Tz, s_q = pb.rzp, s_x = (long long)o * pb.rzp;
-    const long long s_p = (long long)pb.Tx * s_x, s_y = (long long)o * s_p;
-    (void)s_r;
-    g.A = GOpT<StageT>{L.S + pb.swoff + (long long)q * s_q, map2(pb.Tx, s_x, s_p), map2((int)oTz, 1, s_y), 1};
-    g.B = GOp{L.B2 + ((long long)pb.Y0 * o * v + pb.Z0) * o, map1(1),
-              map3(pb.Tz, o, o, (long long)v * o, (long long)o * v * o), 0};
-    g.C = L.G + ((long long)q * o * v + pb.X0) * o;
-    g.cm = map2(pb.Tx, o, (long long)v * o);
-    g.cn = map1(1);
-    g.alpha = -1.0;
-    g.alpha2 = 0.0;
-    g.accumulate = 2;
-    const int m0 = blockIdx.x * kGBM, n0 = blockIdx.y * kGBN;
-    if (m0 >= g.M || n0 >= g.N) return;
-    gemm_fp64_tile(g, m0, n0, sm);
-}
-
-// t2 gradient (ooov term): G_B2[y][r][z][m] -= sum_{q,p,x} Wbar * A2[q][p][x][m]; z = (tau, y)
-template <typename StageT>
-__global__ void __launch_bounds__(256) k_b1d_fp64(GemmLaunch<StageT> L) {
-    __shared__ GemmSmem sm;
-    const int b = blockIdx.z;
-    const int t = find_tau(L, b);
-    const PermBlock &pb = L.ch.pb[t];
-    const Dims &d = L.d;
-    const int o = d.o, v = d.v;
-    const int y = b - L.cum[t];
-    GemmArgsT<StageT> g;
-    g.M = o * pb.Tz;
-    g.N = o;
-    g.K = o * o * pb.Tx;
-    g.K2 = 0;
-    const long long s_r = pb.Tz, s_q = pb.rzp, s_x = (long long)o * pb.rzp;
-    const long long s_p = (long long)pb.Tx * s_x, s_y = (long long)o * s_p;
-    (void)s_r;
-    g.A = GOpT<StageT>{L.S + pb.swoff + (long long)y * s_y, map1(1), map3(pb.Tx, o, s_x, s_p, s_q), 0};
-    g.B = GOp{L.A2 + (long long)pb.X0 * o, map1(1),
-              map3(pb.Tx, o, o, (long long)v * o, (long long)o * v * o), 0};
-    g.C = L.G + (((long long)pb.Y0 + y) * o * v + pb.Z0) * o;
-    g.cm = map2(pb.Tz, o, (long long)v * o);
-    g.cn = map1(1);
-    g.alpha = -1.0;
-    g.alpha2 = 0.0;
-    g.accumulate = 1;
-    const int m0 = blockIdx.x * kGBM, n0 = blockIdx.y * kGBN;
-    if (m0 >= g.M || n0 >= g.N) return;
-    gemm_fp64_tile(g, m0, n0, sm);
-}
-
-// ---------------------------------------------------------------------------
-// V-term gradients from Vbar: ovov, t2 (row dots), t1, fvo (column sums)
-// ---------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
 // gradient fold back to the reference layouts
 // ---------------------------------------------------------------------------
@@ -855,38 +774,6 @@ __global__ void k_fold_ovoo(const double *__restrict__ GA2, Dims d, double *__re
 }
 
 __global__ void k_copy_scalar(const double *src, double *dst) { dst[0] = src[0]; }
-
-// plain FP64 GEMM through the multi-index tile (DF factor products)
-__global__ void __launch_bounds__(256) k_gemm_plain(GemmArgs g) {
-    __shared__ GemmSmem sm;
-    const int m0 = blockIdx.x * kGBM, n0 = blockIdx.y * kGBN;
-    if (m0 >= g.M || n0 >= g.N) return;
-    gemm_fp64_tile(g, m0, n0, sm);
-}
-
-// C[m*cms + n*cns] = sum_k A[m*ams + k*aks] B[n*bms + k*bks]
-int gemm_plain(cudaStream_t st, int M, int N, int K, const double *A, long long ams, long long aks,
-               const double *B, long long bms, long long bks, double *C, long long cms, long long cns) {
-    GemmArgs g;
-    g.M = M;
-    g.N = N;
-    g.K = K;
-    g.K2 = 0;
-    g.A = GOp{A, map1(ams), map1(aks), aks == 1 ? 1 : 0};
-    g.B = GOp{B, map1(bms), map1(bks), bks == 1 ? 1 : 0};
-    g.A2 = g.A;
-    g.B2 = g.B;
-    g.C = C;
-    g.cm = map1(cms);
-    g.cn = map1(cns);
-    g.alpha = 1.0;
-    g.alpha2 = 0.0;
-    g.accumulate = 0;
-    const dim3 grid((unsigned)((M + kGBM - 1) / kGBM), (unsigned)((N + kGBN - 1) / kGBN));
-    if (grid.y > 65535) return TRIPLES_ERR_UNSUPPORTED;
-    TB_KLAUNCH(P_PREP, k_gemm_plain<<<grid, 256, 0, st>>>(g));
-    return TRIPLES_OK;
-}
 
 // ---------------------------------------------------------------------------
 // driver
@@ -969,6 +856,133 @@ static int num_sms() {
         g_num_sms[dev].store(n, std::memory_order_relaxed);
     }
     return n;
+}
+
+// ---------------------------------------------------------------------------
+// FP64 GEMM launches: tile and K-slice choice
+// ---------------------------------------------------------------------------
+// Of the tile shapes a contraction is built for, the one with the least padded
+// area, the smaller ones charged for the operand traffic they add.  With too
+// few tiles for two per SM, K is cut into slices of at least four K tiles
+// (atomic adds only).
+struct GemmTile {
+    int bm, bn, nslice;
+};
+
+static GemmTile gemm_tile(long long M, long long N, long long K, long long batches, bool slices) {
+    static const struct { int bm, bn; double w; } shapes[] = {
+        {128, 128, 1.0}, {128, 64, 1.08}, {64, 64, 1.15}, {128, 48, 1.25}, {128, 32, 1.35}, {128, 16, 1.6}};
+    GemmTile best{128, 128, 1};
+    double cost = -1.0;
+    for (const auto &s : shapes) {
+        const double c = (double)((M + s.bm - 1) / s.bm * s.bm) * ((N + s.bn - 1) / s.bn * s.bn) * s.w;
+        if (cost < 0 || c < cost) {
+            cost = c;
+            best.bm = s.bm;
+            best.bn = s.bn;
+        }
+    }
+    const long long blocks = (M + best.bm - 1) / best.bm * ((N + best.bn - 1) / best.bn) * batches;
+    const long long want = 2 * num_sms(), most = (K + 4 * kGBK - 1) / (4 * kGBK);
+    if (slices && blocks < want) {
+        const long long n = (want + blocks - 1) / blocks;
+        best.nslice = (int)(n < most ? n : most);
+        if (best.nslice < 1) best.nslice = 1;
+    }
+    return best;
+}
+
+// f(BM, BN) as compile-time constants for a tile of gemm_tile
+template <typename F>
+static int gemm_dispatch(const GemmTile &t, F &&f) {
+    using std::integral_constant;
+    if (t.bn == 128) return f(integral_constant<int, 128>{}, integral_constant<int, 128>{});
+    if (t.bn == 64 && t.bm == 128) return f(integral_constant<int, 128>{}, integral_constant<int, 64>{});
+    if (t.bn == 64) return f(integral_constant<int, 64>{}, integral_constant<int, 64>{});
+    if (t.bn == 48) return f(integral_constant<int, 128>{}, integral_constant<int, 48>{});
+    if (t.bn == 32) return f(integral_constant<int, 128>{}, integral_constant<int, 32>{});
+    return f(integral_constant<int, 128>{}, integral_constant<int, 16>{});
+}
+
+template <typename K>
+static int gemm_smem_optin(K kernel, size_t bytes) {
+    // above the default 48 KB a kernel has to opt in, once per device; the
+    // attribute call is idempotent and cheap next to a launch
+    TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return TRIPLES_OK;
+}
+
+// Largest M, N and K over the orderings; nb: GEMM problems in L.cum.
+template <int KIND>
+static int chunk_gemm(cudaStream_t st, int cat, GemmLaunch &L) {
+    const long long o = L.d.o, v = L.d.v;
+    long long M = 0, N = 0, K = 0;
+    for (int t = 0; t < L.ch.nperm; t++) {
+        const PermBlock &pb = L.ch.pb[t];
+        const long long m = o * (KIND == GK_F1 || KIND == GK_B1A || KIND == GK_B1C ? pb.Tx : pb.Tz);
+        const long long n = KIND == GK_F1 ? o * pb.Tz : (KIND == GK_B1A || KIND == GK_B1B ? v : o);
+        const long long k = KIND == GK_F1 ? v
+                            : KIND == GK_B1A ? o * o * pb.Tz
+                            : KIND == GK_B1B ? o * pb.Ty * pb.Tx
+                            : KIND == GK_B1C ? o * pb.Ty * pb.Tz
+                                             : o * o * pb.Tx;
+        M = m > M ? m : M;
+        N = n > N ? n : N;
+        K = k > K ? k : K;
+    }
+    L.cum[0] = 0;
+    for (int t = 0; t < L.ch.nperm; t++)
+        L.cum[t + 1] = L.cum[t] + (KIND == GK_F1 ? L.ch.pb[t].Ty * L.d.o
+                                   : KIND == GK_B1A || KIND == GK_B1D ? L.ch.pb[t].Ty : L.d.o);
+    const GemmTile tile = gemm_tile(M, N, K, L.cum[L.ch.nperm], KIND != GK_F1);
+    return gemm_dispatch(tile, [&](auto bm, auto bn) -> int {
+        constexpr int BM = decltype(bm)::value, BN = decltype(bn)::value;
+        using C = GemmCfg<BM, BN, gemm_kfa(KIND), gemm_kfb(KIND)>;
+        const int rc = gemm_smem_optin(k_chunk_fp64<KIND, BM, BN>, C::SMEM);
+        if (rc != TRIPLES_OK) return rc;
+        L.nmt = (int)((M + BM - 1) / BM);
+        L.nslice = tile.nslice;
+        const dim3 grid((unsigned)(L.nmt * L.nslice), (unsigned)((N + BN - 1) / BN), (unsigned)L.cum[L.ch.nperm]);
+        TB_KLAUNCH(cat, (k_chunk_fp64<KIND, BM, BN><<<grid, kGThreads, C::SMEM, st>>>(L)));
+        return TRIPLES_OK;
+    });
+}
+
+// plain FP64 GEMM through the multi-index tile (DF factor products)
+template <int BM, int BN, bool KFA, bool KFB>
+__global__ void __launch_bounds__(kGThreads) k_gemm_plain(const __grid_constant__ GemmArgs g) {
+    extern __shared__ __align__(16) double gemm_smem[];
+    gemm_fp64_tile<BM, BN, KFA, KFB>(g, blockIdx.x * BM, blockIdx.y * BN, 0, 1, gemm_smem);
+}
+
+// C[m*cms + n*cns] = sum_k A[m*ams + k*aks] B[n*bms + k*bks]; KFA / KFB: the
+// operand is contiguous along k
+template <bool KFA, bool KFB>
+static int gemm_plain(cudaStream_t st, int M, int N, int K, const double *A, long long ams, long long aks,
+                      const double *B, long long bms, long long bks, double *C, long long cms, long long cns) {
+    GemmArgs g;
+    g.M = M;
+    g.N = N;
+    g.K = K;
+    g.K2 = 0;
+    g.A = GOp{A, map1(ams), map1(aks)};
+    g.B = GOp{B, map1(bms), map1(bks)};
+    g.A2 = g.A;
+    g.B2 = g.B;
+    g.C = C;
+    g.cm = map1(cms);
+    g.cn = map1(cns);
+    g.alpha = 1.0;
+    g.alpha2 = 0.0;
+    g.atomic = 0;
+    constexpr int BM = 128, BN = 128;
+    using Cfg = GemmCfg<BM, BN, KFA, KFB>;
+    const dim3 grid((unsigned)((M + BM - 1) / BM), (unsigned)((N + BN - 1) / BN));
+    if (grid.y > 65535) return TRIPLES_ERR_UNSUPPORTED;
+    const int rc = gemm_smem_optin(k_gemm_plain<BM, BN, KFA, KFB>, Cfg::SMEM);
+    if (rc != TRIPLES_OK) return rc;
+    TB_KLAUNCH(P_PREP, (k_gemm_plain<BM, BN, KFA, KFB><<<grid, kGThreads, Cfg::SMEM, st>>>(g)));
+    return TRIPLES_OK;
 }
 
 // One-time set-up per device and kind of work (shared-memory opt-ins and
@@ -1497,11 +1511,6 @@ static int run_impl(const Plan &P, cudaStream_t st, const TriplesIO &io) {
             for (int C = 0; C <= B; C++) {
                 ChunkDesc ch;
                 make_chunk(d, A, B, C, ch);
-                int maxTx = 0, maxTz = 0;
-                for (int t = 0; t < ch.nperm; t++) {
-                    if (ch.pb[t].Tx > maxTx) maxTx = ch.pb[t].Tx;
-                    if (ch.pb[t].Tz > maxTz) maxTz = ch.pb[t].Tz;
-                }
                 // F1: raw amplitudes
                 if (mixed) {
                     TcF1Params T;
@@ -1517,17 +1526,13 @@ static int run_impl(const Plan &P, cudaStream_t st, const TriplesIO &io) {
                         TB_KLAUNCH(P_F1, (k_f1_tc<256, false><<<grid, kF1Threads, TcCfg<256>::SMEM, st>>>(
                                              Mf1, T, nullptr, nullptr, 0)));
                 } else {
-                    GemmLaunch<double> L;
+                    GemmLaunch L;
                     L.d = d;
                     L.ch = ch;
                     L.A1 = A1; L.B1 = B1; L.A2 = A2; L.B2 = B2;
                     L.S = (double *)S;
                     L.G = nullptr;
-                    L.cum[0] = 0;
-                    for (int t = 0; t < ch.nperm; t++) L.cum[t + 1] = L.cum[t] + ch.pb[t].Ty * d.o;
-                    TB_KLAUNCH(P_F1, k_f1_fp64<<<dim3((d.o * maxTx + kGBM - 1) / kGBM, (d.o * maxTz + kGBN - 1) / kGBN,
-                                     L.cum[ch.nperm]),
-                                256, 0, st>>>(L));
+                    if ((prc = chunk_gemm<GK_F1>(st, P_F1, L)) != TRIPLES_OK) return prc;
                 }
                 if (P.lno) {
                     // projected energy: whole-chunk epilogue instead of the orbit tiles
@@ -1627,27 +1632,19 @@ static int run_impl(const Plan &P, cudaStream_t st, const TriplesIO &io) {
                         if (brc != TRIPLES_OK) return brc;
                     }
                 } else {
-                GemmLaunch<StageT> L;
-                L.d = d;
-                L.ch = ch;
-                L.A1 = A1; L.B1 = B1; L.A2 = A2; L.B2 = B2;
-                L.S = reinterpret_cast<StageT *>(SW);
-                L.cum[0] = 0;
-                for (int t = 0; t < ch.nperm; t++) L.cum[t + 1] = L.cum[t] + ch.pb[t].Ty;
-                L.G = GA1;
-                TB_KLAUNCH(P_B1A, k_b1a_fp64<StageT><<<dim3((d.o * maxTx + kGBM - 1) / kGBM, (d.v + kGBN - 1) / kGBN, L.cum[ch.nperm]),
-                                     256, 0, st>>>(L));
-                L.G = GB2;
-                TB_KLAUNCH(P_B1D, k_b1d_fp64<StageT><<<dim3((d.o * maxTz + kGBM - 1) / kGBM, (d.o + kGBN - 1) / kGBN, L.cum[ch.nperm]),
-                                     256, 0, st>>>(L));
-                L.G = GB1;
-                TB_KLAUNCH(P_B1B, k_b1b_fp64<StageT><<<dim3((d.o * maxTz + kGBM - 1) / kGBM, (d.v + kGBN - 1) / kGBN,
-                                                             (unsigned)(d.o * ch.nperm)),
-                                     256, 0, st>>>(L));
-                L.G = GA2;
-                TB_KLAUNCH(P_B1C, k_b1c_fp64<StageT><<<dim3((d.o * maxTx + kGBM - 1) / kGBM, (d.o + kGBN - 1) / kGBN,
-                                                             (unsigned)(d.o * ch.nperm)),
-                                     256, 0, st>>>(L));
+                    GemmLaunch L;
+                    L.d = d;
+                    L.ch = ch;
+                    L.A1 = A1; L.B1 = B1; L.A2 = A2; L.B2 = B2;
+                    L.S = (double *)SW;
+                    L.G = GA1;
+                    if ((prc = chunk_gemm<GK_B1A>(st, P_B1A, L)) != TRIPLES_OK) return prc;
+                    L.G = GB2;
+                    if ((prc = chunk_gemm<GK_B1D>(st, P_B1D, L)) != TRIPLES_OK) return prc;
+                    L.G = GB1;
+                    if ((prc = chunk_gemm<GK_B1B>(st, P_B1B, L)) != TRIPLES_OK) return prc;
+                    L.G = GA2;
+                    if ((prc = chunk_gemm<GK_B1C>(st, P_B1C, L)) != TRIPLES_OK) return prc;
                 }
             }
     }
@@ -2126,7 +2123,7 @@ static int triples_df_call(void *stream, int precision, int nocc, int nvir, int 
     double *ovvv = (double *)(ws + L.off_ovvv), *gvvv = (double *)(ws + L.off_gvvv);
     const long long nov = (long long)nocc * nvir, npair = (long long)nvir * (nvir + 1) / 2;
     // ovvv[px][pair] = sum_P Lov[P][px] Lvv[P][pair]
-    if ((rc = tb::gemm_plain(st, (int)nov, (int)npair, naux, Lov, 1, nov, Lvv, 1, npair, ovvv, npair, 1)) !=
+    if ((rc = tb::gemm_plain<false, false>(st, (int)nov, (int)npair, naux, Lov, 1, nov, Lvv, 1, npair, ovvv, npair, 1)) !=
         TRIPLES_OK)
         return rc;
     io.ovvv = ovvv;
@@ -2134,11 +2131,11 @@ static int triples_df_call(void *stream, int precision, int nocc, int nvir, int 
     if ((rc = tb::run_triples(L.P, st, io)) != TRIPLES_OK) return rc;
     if (!want_grad) return TRIPLES_OK;
     // Lov_bar[P][px] = sum_pair G[px][pair] Lvv[P][pair]
-    if ((rc = tb::gemm_plain(st, (int)nov, naux, (int)npair, gvvv, npair, 1, Lvv, npair, 1, Lov_bar, 1, nov)) !=
+    if ((rc = tb::gemm_plain<true, true>(st, (int)nov, naux, (int)npair, gvvv, npair, 1, Lvv, npair, 1, Lov_bar, 1, nov)) !=
         TRIPLES_OK)
         return rc;
     // Lvv_bar[P][pair] = sum_px G[px][pair] Lov[P][px]
-    return tb::gemm_plain(st, (int)npair, naux, (int)nov, gvvv, 1, npair, Lov, nov, 1, Lvv_bar, 1, npair);
+    return tb::gemm_plain<false, true>(st, (int)npair, naux, (int)nov, gvvv, 1, npair, Lov, nov, 1, Lvv_bar, 1, npair);
 }
 
 int triples_energy_df(void *stream, int precision, int nocc, int nvir, int naux, const double *mo_energy,
