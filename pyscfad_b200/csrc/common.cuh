@@ -133,4 +133,36 @@ __host__ __device__ constexpr inline int perm_compose(int s, int pi) {
     return perm_index(ps[pp[0]], ps[pp[1]]);
 }
 
+// Staging layout of the mixed epilogue: S_tau[p][q][r][y block][x block][z block]
+// and, inside a block of (ey, ex, ez) = (min(8, Ty), ...) values, [y][x][z];
+// rows of 64 values (ex = ez = 8) are stored with bit 2 of the slot x*8+z
+// exchanged by y's bit 0 and bit 4 by y's bit 1.  Block sizes are powers of
+// two up to 16, so a block of fewer than 8 is one block.
+__host__ __device__ inline int f2m_row_swizzle(int y) { return ((y & 1) << 2) | ((y & 2) << 3); }
+
+struct StageRow {         // the z run of one (p, q, y, x): offset of r, z = base + r rs + z part
+    long long base;
+    int rs, ez, es, slot, swz;   // stride of r, z extent and size of a block, slot of z = 0, exchange
+    __host__ __device__ int at(int z) const { return (z >> 3) * es + ((slot + (z & 7)) ^ swz); }
+};
+
+__host__ __device__ inline StageRow f2m_stage_row(const PermBlock &pb, int o, int p, int q, int y, int x) {
+    const int ex = pb.Tx < 8 ? pb.Tx : 8, ey = pb.Ty < 8 ? pb.Ty : 8, ez = pb.Tz < 8 ? pb.Tz : 8;
+    const int nx = pb.Tx > 8 ? 2 : 1, nz = pb.Tz > 8 ? 2 : 1;
+    StageRow R;
+    R.ez = ez;
+    R.es = ex * ey * ez;
+    R.rs = pb.Tx * pb.Ty * pb.Tz;
+    R.slot = (x & 7) * ez;
+    R.swz = (ex == 8 && ez == 8) ? f2m_row_swizzle(y & 7) : 0;
+    R.base = pb.soff + (long long)(p * o + q) * o * R.rs + ((y >> 3) * nx + (x >> 3)) * nz * R.es + (y & 7) * (ex * ez);
+    return R;
+}
+
+__host__ __device__ inline long long f2m_stage_offset(const PermBlock &pb, int o, int p, int q, int r, int y, int x,
+                                                      int z) {
+    const StageRow R = f2m_stage_row(pb, o, p, q, y, x);
+    return R.base + (long long)r * R.rs + R.at(z);
+}
+
 }  // namespace tb

@@ -1,4 +1,5 @@
-// Chunk epilogue: energy and adjoint of the raw triples amplitudes.
+// FP64 chunk epilogue: energy and adjoint of the raw triples amplitudes (the
+// mixed-precision modes use f2m.cuh).
 //
 // One CTA owns one occupied representative i >= j >= k and one triple of
 // virtual sub-ranges (a-sub >= b-sub >= c-sub, SB wide).  Every raw
@@ -30,9 +31,6 @@
 // to its item(s) through the (sub-range ordering, occupied ordering) pairs of
 // its region, which in degenerate cases (repeated indices) are several.
 #pragma once
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-
 #include "common.cuh"
 
 namespace tb {
@@ -41,9 +39,10 @@ struct F2Sub {
     int st[3];
     int len[3];
 };
-constexpr int kMaxSub = 64;
+constexpr int kMaxSub = 64;    // sub-range triples of a chunk: (16 / 4)^3
+constexpr int kF2SB = 4;       // sub-range width
+constexpr int kF2Threads = kF2SB * kF2SB * kF2SB;
 
-template <typename StageT>
 struct F2P {
     Dims d;
     ChunkDesc ch;
@@ -51,63 +50,31 @@ struct F2P {
     F2Sub sub[kMaxSub];
     const int *ijk;
     const double *mo_e, *t1, *t2, *ovov, *fvo;
-    const StageT *S;    // W per ordering tau: [p][q][y][x][r][z] at ch.pb[tau].soff
-    void *SW;           // Wbar out; per tau at 2*soff: [h][y][p][x][q][r][z] (split) or at soff: [y][p][x][q][r][z]
-    int split;          // 0: StageT, 1: fp16 hi/lo, 2: bf16 hi/lo
-    const double *wscale;
+    const double *S;    // W per ordering tau: [p][q][y][x][r][z] at ch.pb[tau].soff
+    double *SW;         // Wbar out, per tau at ch.pb[tau].swoff: [y][p][x][q][r][z]
     double ybar;
     int want_grad;
     double *e_part;     // energy partial of each CTA, at sub * n_ijk + rep
-    int rep0, sub0;     // first occupied representative / sub-range triple of this launch
-    int nsub_l;         // sub-range triples of this launch: block b -> sub0 + b % nsub_l, rep0 + b / nsub_l
     int n_ijk;          // occupied representatives (stride of e_part)
     double *mo_bar, *t1_bar, *fvo_bar, *ovov_bar, *t2_bar;
 };
 
 // Shared-memory region layout: element (y,x,z) at y*SY + x*SX + z.  The padded
 // strides keep the permuted gathers of a warp within 2-way bank conflicts.
-template <int SB>
 struct F2Smem {
+    static constexpr int SB = kF2SB;
     static constexpr int SX = SB;
-    static constexpr int SY = (SB == 8) ? 69 : SB * SB + 1;
+    static constexpr int SY = SB * SB + 1;
     static constexpr int REG = SY * SB;
-    // W tile (y, x, z) at y*SYW + x*SX + z: 8-byte aligned rows for the
-    // 8-byte cp.async copies of the FP32 staging (SB = 8); item results keep SY
-    static constexpr int SYW = (SB == 8) ? 70 : SY;
-    static constexpr int REGW = SYW * SB;
     static constexpr int NV = 3 * SB;
     static constexpr int NVP = NV + 1;
     static constexpr int TAB = 6 * NV * NVP;
     static constexpr int ITEMS = SB * SB * SB;
-    static constexpr int NT = (SB == 8) ? 256 : ITEMS;     // threads per CTA
-    static constexpr int IPT = ITEMS / NT;                  // items per thread
-    static_assert(12 * REG <= 36 * REGW, "item results overlay the W tile");
+    static_assert(ITEMS == kF2Threads, "one orbit item per thread");
 };
 
-template <typename StageT, int SB>
 __host__ __device__ constexpr size_t f2_smem_bytes() {
-    return sizeof(StageT) * (36 * F2Smem<SB>::REGW + 2 * F2Smem<SB>::TAB + 2 * 3 * F2Smem<SB>::NV);
-}
-
-// 4- and 8-byte asynchronous copies global -> shared (L1-allocating, L2
-// evict-first hint: the staging is streamed once); src_bytes < size
-// zero-fills the rest of the destination without reading past src_bytes.
-__device__ __forceinline__ uint64_t f2_policy_evict_first() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-__device__ __forceinline__ void f2_cp_async(void *smem_dst, const void *gsrc, int size, int src_bytes,
-                                            uint64_t pol) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-    if (size == 8)
-        asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 8, %2, %3;" ::"r"(d), "l"(gsrc),
-                     "r"(src_bytes), "l"(pol)
-                     : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 4, %2, %3;" ::"r"(d), "l"(gsrc),
-                     "r"(src_bytes), "l"(pol)
-                     : "memory");
+    return sizeof(double) * (36 * F2Smem::REG + 2 * F2Smem::TAB + 2 * 3 * F2Smem::NV);
 }
 
 __host__ __device__ constexpr inline int pair_index(int sp, int sq) { return 2 * sp + (sq > sp ? sq - 1 : sq); }
@@ -253,36 +220,18 @@ __device__ __forceinline__ T group_reduce_scatter(T (&v)[NV], int lane) {
     return r;
 }
 
-// BATCH = false: the CTAs of one launch segment (parameters P0).  BATCH =
-// true: the CTAs of njobs segments (chunks of different problems) numbered job
-// after job (job_start[j] = first CTA of job j), parameters in device memory.
-template <typename StageT, int SB, bool BATCH>
-__global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
-    k_f2t(const __grid_constant__ F2P<StageT> P0, const F2P<StageT> *__restrict__ jobs,
-          const int *__restrict__ job_start, int njobs) {
-    int blk = (int)blockIdx.x;
-    const F2P<StageT> *Pp = &P0;
-    if constexpr (BATCH) {
-        int lo = 0, hi = njobs - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (job_start[mid] <= blk) lo = mid;
-            else hi = mid - 1;
-        }
-        blk -= job_start[lo];
-        Pp = &jobs[lo];
-    }
-    const F2P<StageT> &P = *Pp;
-    using C = F2Smem<SB>;
-    constexpr int NT = C::NT, IPT = C::IPT;
+__global__ void __launch_bounds__(kF2Threads, 4) k_f2t(const __grid_constant__ F2P P) {
+    using StageT = double;
+    using C = F2Smem;
+    constexpr int SB = C::SB, NT = kF2Threads;
     constexpr int REG = C::REG, NV = C::NV, NVP = C::NVP;
     constexpr int SX = C::SX, SY = C::SY;
-    constexpr int REGW = C::REGW, SYW = C::SYW;
-    constexpr int NW = NT / 32;
+    constexpr int NW = NT / 32, IPT = C::ITEMS / NT;
+    const int blk = (int)blockIdx.x;
     extern __shared__ __align__(16) uint8_t f2_smem[];
     StageT *sW = reinterpret_cast<StageT *>(f2_smem);
     StageT *sG = sW;                      // item results [12][REG] (padded) once W is consumed
-    StageT *tOV = sW + 36 * REGW;
+    StageT *tOV = sW + 36 * REG;
     StageT *tT2 = tOV + C::TAB;
     StageT *tT1 = tT2 + C::TAB;
     StageT *tFV = tT1 + 3 * NV;
@@ -295,10 +244,8 @@ __global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
     const Dims &d = P.d;
     const int o = d.o, v = d.v;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // linear grid, sub-range triple fastest: the blocks of one representative
-    // run together, so the two 16-byte halves of each Wbar sector meet in L2
-    const int sub = P.sub0 + (int)((unsigned)blk % (unsigned)P.nsub_l);
-    const int rep = P.rep0 + (int)((unsigned)blk / (unsigned)P.nsub_l);
+    // linear grid, sub-range triple fastest: the blocks of one representative run together
+    const int sub = blk % P.nsub, rep = blk / P.nsub;
     const F2Sub &R = P.sub[sub];
     const int ijk[3] = {P.ijk[3 * rep], P.ijk[3 * rep + 1], P.ijk[3 * rep + 2]};
 
@@ -364,30 +311,7 @@ __global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
     //      LB runs are fetched before any is stored, so their latencies overlap ----
     // distinct sub-ranges: the tables need only the blocks of two different ranges
     const bool distinct_rng = (cs[1] == 1 && cs[2] == 2);
-    if constexpr (sizeof(StageT) == 4 && SB == 8) {
-        // FP32 staging: four lanes per 32-byte run, 8-byte cp.async (two 4-byte
-        // copies where the run is not 8-byte aligned), zero-filled past the run
-        const uint64_t pol = f2_policy_evict_first();
-        const int npiece = nreg * SB * SB * 4;
-        for (int e = tid; e < npiece; e += NT) {
-            const int run = e >> 2, c = e & 3;
-            const int reg = run / (SB * SB), yy = (run / SB) % SB, xx = run % SB;
-            const int *rd = s_rd[reg];
-            if (xx < rd[3] && yy < rd[4]) {
-                const int n = rd[5] - 2 * c;   // valid values of this 2-value piece (<= 0: none)
-                const StageT *run0 = P.S + s_gb[reg] + (long long)yy * s_gs[reg][0] + (long long)xx * s_gs[reg][1];
-                const StageT *src = n > 0 ? run0 + 2 * c : run0;   // nothing is read when n <= 0
-                StageT *dst = sW + reg * REGW + yy * SYW + xx * SX + 2 * c;
-                if (n >= 2 && (reinterpret_cast<uintptr_t>(src) & 7) == 0) {
-                    f2_cp_async(dst, src, 8, 8, pol);
-                } else {
-                    f2_cp_async(dst, src, 4, n >= 1 ? 4 : 0, pol);
-                    f2_cp_async(dst + 1, n >= 2 ? src + 1 : src, 4, n >= 2 ? 4 : 0, pol);
-                }
-            }
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-    } else {
+    {
         constexpr int LB = 3;
         const int nrun = nreg * SB * SB;
         for (int e0 = tid; e0 < nrun; e0 += LB * NT) {
@@ -406,7 +330,7 @@ __global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
                         lzs[u] = rd[5];
                         ld_run(b[u], P.S + s_gb[reg] + (long long)yy * s_gs[reg][0] + (long long)xx * s_gs[reg][1],
                                lzs[u]);
-                        dst[u] = sW + reg * REGW + yy * SYW + xx * SX;
+                        dst[u] = sW + reg * REG + yy * SY + xx * SX;
                     }
                 }
             }
@@ -496,7 +420,7 @@ __global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
                     int pp[3], pt[3];
                     perm_of(pi, pp);
                     perm_of(tau, pt);
-                    sw += (double)sW[pat.reg[pi * 6 + tau] * REGW + loc[pp[1]] * SYW + loc[pp[0]] * SX + loc[pp[2]]];
+                    sw += (double)sW[pat.reg[pi * 6 + tau] * REG + loc[pp[1]] * SY + loc[pp[0]] * SX + loc[pp[2]]];
                     const int pair = pair_index(pt[0], pt[1]);
                     const int xl = vl[pp[0]], yl = vl[pp[1]], zl = vl[pp[2]];
                     sv += tOV[(pair * NV + xl) * NVP + yl] * tT1[pt[2] * NV + zl] +
@@ -529,19 +453,12 @@ __global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
                     gres[it][s] = (StageT)(g0 * (Z[s] + RW[s]));
                     gres[it][6 + s] = (StageT)(g0 * 0.5 * RW[s]);
                 }
-                if (SB * SB < 32) atomicAdd(&s_ev[vl[0]], -ddi);
+                atomicAdd(&s_ev[vl[0]], -ddi);
                 atomicAdd(&s_ev[vl[1]], -ddi);
                 atomicAdd(&s_ev[vl[2]], -ddi);
             }
         }
         dd_loc += ddi;
-        // with SB^2 >= 32 the a-slot index (item / SB^2) is uniform across a warp: reduce first
-        if (SB * SB >= 32 && P.want_grad) {
-            double dsum = -ddi;
-            for (int off = 16; off > 0; off >>= 1) dsum += __shfl_down_sync(0xffffffffu, dsum, off);
-            const int la = item / (SB * SB);
-            if (lane == 0 && la < R.len[0] && dsum != 0.0) atomicAdd(&s_ev[cs[0] * SB + la], dsum);
-        }
     }
 
     // ---- block reductions: chunk energy partial, occupied-energy gradient ----
@@ -594,7 +511,6 @@ __global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
     constexpr int NG = NT / GL;                  // groups per CTA
     // every region holds one (pi, rho) pair and no ordering constraint applies
     const bool simple = (n_ijk == 6) && distinct_rng;
-    const float wscf = (P.split != 0) ? (float)*P.wscale : 1.0f;
     const int grp = tid / GL, gl = tid % GL;
     const int nround = (nreg + NG - 1) / NG;
     for (int rr = 0; rr < nround; rr++) {
@@ -613,7 +529,6 @@ __global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
         const int pair = pair_index(pt[0], pt[1]);
         const StageT *a1 = tT1 + pt[2] * NV + zl0, *f1 = tFV + pt[2] * NV + zl0;
         const PermBlock &pb = P.ch.pb[rd[2]];
-        const long long half = (long long)pb.Ty * o * pb.Tx * o * pb.rzp;
         // V-term partials in the staging precision (FP32 in the mixed modes: 8-term
         // row sums and the warp's 64-run column sums), added to the FP64 gradients
         StageT colv[2 * SB];
@@ -671,35 +586,10 @@ __global__ void __launch_bounds__(F2Smem<SB>::NT, (SB == 8) ? 2 : 4)
             }
             // Wbar out
             const long long wl = s_wb[reg] + (long long)yy * s_ws[reg][0] + (long long)xx * s_ws[reg][1];
-            if (P.split == 0) {
-                RunBuf<StageT, SB> bw;
+            RunBuf<StageT, SB> bw;
 #pragma unroll
-                for (int zz = 0; zz < SB; zz++) bw.e[zz] = (StageT)wb[zz];
-                st_run(reinterpret_cast<StageT *>(P.SW) + pb.swoff + wl, bw, lz);
-            } else if (P.split == 1) {
-                // exact power-of-two scaling, then a two-term 16-bit split in FP32
-                RunBuf<__half, SB> bh, bl;
-#pragma unroll
-                for (int zz = 0; zz < SB; zz++) {
-                    const float xs = (float)wb[zz] * wscf;
-                    bh.e[zz] = __float2half_rn(xs);
-                    bl.e[zz] = __float2half_rn(xs - __half2float(bh.e[zz]));
-                }
-                __half *dst = reinterpret_cast<__half *>(P.SW) + 2 * pb.swoff + wl;
-                st_run(dst, bh, lz);
-                st_run(dst + half, bl, lz);
-            } else {
-                RunBuf<__nv_bfloat16, SB> bh, bl;
-#pragma unroll
-                for (int zz = 0; zz < SB; zz++) {
-                    const float xs = (float)wb[zz] * wscf;
-                    bh.e[zz] = __float2bfloat16_rn(xs);
-                    bl.e[zz] = __float2bfloat16_rn(xs - __bfloat162float(bh.e[zz]));
-                }
-                __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(P.SW) + 2 * pb.swoff + wl;
-                st_run(dst, bh, lz);
-                st_run(dst + half, bl, lz);
-            }
+            for (int zz = 0; zz < SB; zz++) bw.e[zz] = wb[zz];
+            st_run(P.SW + pb.swoff + wl, bw, lz);
             // V-term gradients: v = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r]
             const int x = R.st[pp[0]] + xx, y = R.st[pp[1]] + yy;
             const int te = (pair * NV + cslot(pp[0]) * SB + xx) * NVP + cslot(pp[1]) * SB + yy;
@@ -740,8 +630,10 @@ __device__ __forceinline__ void energy_sum_body(const double *__restrict__ e_par
     if (threadIdx.x == 0) *e_acc += s[0];
 }
 
-__global__ void k_f2_energy_sum(const double *__restrict__ e_part, int n, double *e_acc) {
+// ticket (if any): the epilogue's item counter, back to zero for the next launch
+__global__ void k_f2_energy_sum(const double *__restrict__ e_part, int n, double *e_acc, unsigned *ticket) {
     energy_sum_body(e_part, n, e_acc);
+    if (threadIdx.x == 0 && ticket) *ticket = 0u;
 }
 
 }  // namespace tb

@@ -34,8 +34,10 @@ struct TcCfg {
 };
 
 struct TcF1Params {
-    CUtensorMap tmS[6];       // per ordering with full 16 x 16 (x, z) blocks: S_tau as
-                              // [p][q][y][x][r*16+z], box {32, 16, 1, 1, 2}, 128B swizzle
+    CUtensorMap tmS[6];       // per ordering with full 16 x 16 (x, z) blocks, one 32 x 32 piece of
+                              // an epilogue warp per store: S_tau as [p][q][y][x][r*16+z], box
+                              // {32, 16, 1, 1, 2}, 128B swizzle; or (blocked) as [p][q][r][block]
+                              // [y*64 + slot], box {64, 4, 2, 1, 2}: the four (x, z) blocks of a y
     int tmS_ok[6];            // 1 where tmS is valid (else plain stores)
     Dims d;
     ChunkDesc ch;
@@ -49,6 +51,7 @@ struct TcF1Params {
     int *err;
     int bf16;
     int kseg;                 // K blocks per TMEM accumulation segment
+    int blocked;              // staging in the epilogue's 8 x 8 x 8 blocks (f2m_stage_offset)
 };
 
 constexpr int kF1Threads = 320;   // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
@@ -348,7 +351,11 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                 // pieces per warp store.
                 float *box = sstore + (warp - 2) * 32 * 32;
                 const int p0 = T.mt * 8 + quarter * 2;
-#pragma unroll
+                // this lane's float4 slot ch of its row: 128B-swizzled row of 32, or
+                // [p][r][x block, z block][x][z] with the row exchange of f2m_row_swizzle
+                const int bsw = f2m_row_swizzle(T.y);
+                const int brow = (lane >> 4) * 512 + ((lane >> 3) & 1) * 128, bx = (lane & 7) * 8;
+                #pragma unroll
                 for (int c = 0; c < HC / 32; c++) {
                     if (c > 0) {
                         if (lane == 0) bulk_wait_read0();
@@ -363,18 +370,51 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                         w.w = accf[c * 32 + ch * 4 + 3] * sc;
                         if (vrow)
                             wmax = fmaxf(wmax, fmaxf(fmaxf(fabsf(w.x), fabsf(w.y)), fmaxf(fabsf(w.z), fabsf(w.w))));
-                        *reinterpret_cast<float4 *>(box + lane * 32 + 4 * (ch ^ (lane & 7))) = w;
+                        const int at = P.blocked ? brow + (ch >> 2) * 256 + ((ch >> 1) & 1) * 64 + ((bx + (ch & 1) * 4) ^ bsw)
+                                                 : lane * 32 + 4 * (ch ^ (lane & 7));
+                        *reinterpret_cast<float4 *>(box + at) = w;
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    const int rz0 = T.nt * BN + half * HC + c * 32;
-                    if (lane == 0 && p0 < o && rz0 < o * 16) {
-                        tma_store_5d(&P.tmS[T.tau], box, rz0, 0, T.y, T.q, p0);
+                    const int r0 = T.nt * C::RT + half * (HC / 16) + c * 2;
+                    if (lane == 0 && p0 < o && r0 < o) {
+                        if (P.blocked) tma_store_5d(&P.tmS[T.tau], box, (T.y & 7) * 64, (T.y >> 3) * 4, r0, T.q, p0);
+                        else tma_store_5d(&P.tmS[T.tau], box, r0 * 16, 0, T.y, T.q, p0);
                         bulk_commit();
                     }
                 }
                 if (lane == 0) bulk_wait_read0();
                 __syncwarp();
+            } else if (vrow && P.blocked) {
+                const StageRow R = f2m_stage_row(pb, o, p, T.q, T.y, x);
+#pragma unroll
+                for (int h = 0; h < HC / 16; h++) {
+                    const int r = T.nt * C::RT + half * (HC / 16) + h;
+                    if (r >= o) continue;
+                    float *d = P.S + R.base + (long long)r * R.rs;
+                    if (R.ez == 8) {
+#pragma unroll
+                        for (int z4 = 0; z4 < 4; z4++) {
+                            if (4 * z4 >= pb.Tz) continue;
+                            float4 w;
+                            w.x = accf[h * 16 + z4 * 4 + 0] * sc;
+                            w.y = accf[h * 16 + z4 * 4 + 1] * sc;
+                            w.z = accf[h * 16 + z4 * 4 + 2] * sc;
+                            w.w = accf[h * 16 + z4 * 4 + 3] * sc;
+                            wmax = fmaxf(wmax, fmaxf(fmaxf(fabsf(w.x), fabsf(w.y)), fmaxf(fabsf(w.z), fabsf(w.w))));
+                            *reinterpret_cast<float4 *>(d + R.at(4 * z4)) = w;   // the exchange moves whole groups of four z
+                        }
+                    } else {
+#pragma unroll
+                        for (int z = 0; z < 4; z++) {
+                            if (z < pb.Tz) {
+                                const float w1 = accf[h * 16 + z] * sc;
+                                wmax = fmaxf(wmax, fabsf(w1));
+                                d[R.slot + z] = w1;
+                            }
+                        }
+                    }
+                }
             } else if (vrow) {
 #pragma unroll
                 for (int h = 0; h < HC / 16; h++) {

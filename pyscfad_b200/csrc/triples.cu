@@ -19,7 +19,7 @@
 #include "gemm_fp64.cuh"
 #include "tc_f1.cuh"
 #include "f2.cuh"
-#include "f2p.cuh"
+#include "f2m.cuh"
 #include "tc_b1.cuh"
 #include "lno.cuh"
 #include "pyscfad_b200.h"
@@ -152,7 +152,7 @@ static long long chunk_stage_elems(const ChunkDesc &ch, const Dims &d) {
 }
 
 int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, int lno,
-              const triples_options *opt) {
+              const triples_options *opt, bool vtables) {
     if (nocc < 1 || nvir < 1 || nocc > kMaxCols || nvir > 32767) return TRIPLES_ERR_INVALID_ARGUMENT;
     if (precision < TRIPLES_PRECISION_FP64 || precision > TRIPLES_PRECISION_MIXED_BF16)
         return TRIPLES_ERR_INVALID_ARGUMENT;
@@ -245,6 +245,13 @@ int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan
         P.off_GB1 = take(o * o * v * Kp * el);
         P.off_GA2 = take(o * o * v * o * el);
         P.off_GB2 = take(v * o * v * o * el);
+    }
+    // FP32 V-term tables of the mixed epilogue; without them it gathers the entries
+    P.vtables = vtables && mixed && !lno;
+    if (P.vtables) {
+        const size_t nb8 = (v + 7) / 8;
+        P.off_ot = take(o * o * nb8 * nb8 * 64 * sizeof(float2));
+        P.off_tf = take(o * nb8 * 8 * sizeof(float2));
     }
     P.off_ijk = take((size_t)P.n_ijk * 3 * sizeof(int));
     P.off_epart = take((size_t)P.n_ijk * P.f2_gy * el);
@@ -467,6 +474,7 @@ __global__ void k_chunk_scale_batch(const ChunkAux *__restrict__ aux, int scaled
 __global__ void k_energy_sum_batch(const ChunkAux *__restrict__ aux) {
     const ChunkAux &A = aux[blockIdx.x];
     energy_sum_body(A.e_part, A.n_part, &A.ctrl->e_acc);
+    if (threadIdx.x == 0) A.ctrl->ticket = 0u;   // for the next step's epilogue
 }
 
 template <typename H>
@@ -826,19 +834,24 @@ static int make_tmap5(CUtensorMap *tm, void *base, bool bf16, const uint64_t dim
     return r == CUDA_SUCCESS ? TRIPLES_OK : TRIPLES_ERR_CUDA;
 }
 
-// 5-D map over S_tau, an FP32 [p][q][y][x][rz] array (rz innermost, o*16 values),
-// used by the W-contraction epilogue to store 32 x 32 pieces; 128B swizzle.
-static int make_tmap_stage(CUtensorMap *tm, float *base, int o, int Tx, int Ty) {
+// 5-D map over S_tau (FP32), used by the W-contraction epilogue to store 32 x 32
+// pieces of full (x, z) blocks: [p][q][y][x][rz] (rz innermost, o*16 values,
+// 128B swizzle), or blocked, [p][q][r][y block, x block, z block][y][64].
+static int make_tmap_stage(CUtensorMap *tm, float *base, int o, int Tx, int Ty, bool blocked) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return TRIPLES_ERR_UNSUPPORTED;
-    const cuuint64_t gdim[5] = {(cuuint64_t)o * 16, (cuuint64_t)Tx, (cuuint64_t)Ty, (cuuint64_t)o, (cuuint64_t)o};
+    const int ey = Ty < 8 ? Ty : 8;
+    const cuuint64_t gdim_rows[5] = {(cuuint64_t)o * 16, (cuuint64_t)Tx, (cuuint64_t)Ty, (cuuint64_t)o, (cuuint64_t)o};
+    const cuuint64_t gdim_blk[5] = {(cuuint64_t)ey * 64, (cuuint64_t)(Ty / ey) * 4, (cuuint64_t)o, (cuuint64_t)o,
+                                    (cuuint64_t)o};
+    const cuuint64_t *gdim = blocked ? gdim_blk : gdim_rows;
     cuuint64_t gstr[4];
     gstr[0] = gdim[0] * sizeof(float);
     for (int i = 1; i < 4; i++) gstr[i] = gstr[i - 1] * gdim[i];
-    const cuuint32_t box[5] = {32, 16, 1, 1, 2}, es[5] = {1, 1, 1, 1, 1};
-    CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, gdim, gstr, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint32_t box_rows[5] = {32, 16, 1, 1, 2}, box_blk[5] = {64, 4, 2, 1, 2}, es[5] = {1, 1, 1, 1, 1};
+    CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, gdim, gstr, blocked ? box_blk : box_rows, es,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, blocked ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? TRIPLES_OK : TRIPLES_ERR_CUDA;
 }
 
@@ -1092,7 +1105,7 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     const dim3 gproj(clampw((maxcols / d.o + kLnoTile - 1) / kLnoTile), (unsigned)ch.nperm);
     TB_KLAUNCH(P_LNO, k_lno_tile_fwd<StageT><<<gtile, kLnoThreads, lno_tile_smem(), st>>>(A));
     TB_KLAUNCH(P_LNO_PROJ, k_lno_proj<<<gproj, kLnoThreads, lno_proj_smem(d.o), st>>>(A));
-    TB_KLAUNCH(P_PREP, k_f2_energy_sum<<<1, 256, 0, st>>>(A.part, (int)(gproj.x * gproj.y), &ctrl->e_acc));
+    TB_KLAUNCH(P_PREP, k_f2_energy_sum<<<1, 256, 0, st>>>(A.part, (int)(gproj.x * gproj.y), &ctrl->e_acc, nullptr));
     if (!P.want_grad) return TRIPLES_OK;
     if (split != 0)   // fp16: power-of-two scale of the split Wbar; bf16: scale 1 (both read by the contractions)
         TB_KLAUNCH(P_PREP, k_chunk_scale<<<1, 32, 0, st>>>(ctrl, io.mo_energy, d.o, ch.base[0], ch.nabc[0], ch.base[1],
@@ -1127,24 +1140,19 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
 // one-time device set-up and the mixed-precision kernel parameters of a call
 // and of one chunk, shared by the single-problem and the batched drivers
 // ---------------------------------------------------------------------------
-template <typename StageT>
-static int setup_epilogue() {
-    constexpr int kSB = sizeof(StageT) == 4 ? 8 : 4;
-    // once per device and element type: shared-memory opt-in and the
-    // constant tables of the epilogue's region patterns
-    return once_per_device(sizeof(StageT) == 4 ? INIT_F2_F32 : INIT_F2_F64, [&]() -> int {
-        TB_CUDA(cudaFuncSetAttribute(k_f2t<StageT, kSB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)f2_smem_bytes<StageT, kSB>()));
-        TB_CUDA(cudaFuncSetAttribute(k_f2t<StageT, kSB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)f2_smem_bytes<StageT, kSB>()));
-        if (sizeof(StageT) == 4) {
-            TB_CUDA(cudaFuncSetAttribute(k_f2p<1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F2pSmem::BYTES));
-            TB_CUDA(cudaFuncSetAttribute(k_f2p<2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F2pSmem::BYTES));
-            TB_CUDA(cudaFuncSetAttribute(k_f2p<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F2pSmem::BYTES));
-            TB_CUDA(cudaFuncSetAttribute(k_f2p<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F2pSmem::BYTES));
-            TB_CUDA(cudaFuncSetAttribute(k_f2p<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F2pSmem::BYTES));
-            TB_CUDA(cudaFuncSetAttribute(k_f2p<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F2pSmem::BYTES));
+// once per device and precision: shared-memory opt-ins and the constant tables
+// of the FP64 epilogue's region patterns
+static int setup_epilogue(bool mixed) {
+    return once_per_device(mixed ? INIT_F2_F32 : INIT_F2_F64, [&]() -> int {
+        if (mixed) {
+            const int bytes = (int)F2mSmem::BYTES;
+            TB_CUDA(cudaFuncSetAttribute(k_f2m<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            TB_CUDA(cudaFuncSetAttribute(k_f2m<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            TB_CUDA(cudaFuncSetAttribute(k_f2m<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            TB_CUDA(cudaFuncSetAttribute(k_f2m<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            return TRIPLES_OK;
         }
+        TB_CUDA(cudaFuncSetAttribute(k_f2t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f2_smem_bytes()));
         F2Pattern pats[kF2Patterns];
         f2_build_patterns(pats);
         TB_CUDA(cudaMemcpyToSymbol(c_f2pat, pats, sizeof(pats)));
@@ -1238,11 +1246,12 @@ static int f1_params(const Plan &P, const ChunkDesc &ch, char *ws, TcF1Params &T
     T.err = &ctrl->err;
     T.bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16 ? 1 : 0;
     T.kseg = P.kseg;
+    T.blocked = P.lno ? 0 : 1;
     for (int t = 0; t < 6; t++) T.tmS_ok[t] = 0;
     for (int t = 0; t < ch.nperm; t++) {
         const PermBlock &pb = ch.pb[t];
         if (pb.Tx == 16 && pb.Tz == 16 && d.o >= 2) {
-            const int trc = make_tmap_stage(&T.tmS[t], S + pb.soff, d.o, pb.Tx, pb.Ty);
+            const int trc = make_tmap_stage(&T.tmS[t], S + pb.soff, d.o, pb.Tx, pb.Ty, T.blocked != 0);
             if (trc != TRIPLES_OK) return trc;
             T.tmS_ok[t] = 1;
         }
@@ -1250,58 +1259,111 @@ static int f1_params(const Plan &P, const ChunkDesc &ch, char *ws, TcF1Params &T
     return TRIPLES_OK;
 }
 
-// Epilogue parameters of one chunk: every sub-range triple, those of three
-// distinct full 8-wide sub-ranges first (mixed precision; the persistent
-// kernel k_f2p takes them with every occupied representative but i == j == k).
-// Returns the number of those leading sub-range triples.
-template <typename StageT>
-static int f2_params(const Plan &P, const ChunkDesc &ch, char *ws, const TriplesIO &io, F2P<StageT> &F) {
-    constexpr int kSB = sizeof(StageT) == 4 ? 8 : 4;
-    const bool mixed = P.prec != TRIPLES_PRECISION_FP64;
-    Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
+// Sub-range triples of a chunk (edge sb), one per orbit of orderings: f(start, length).
+template <typename F>
+static void for_sub_ranges(const ChunkDesc &ch, int sb, F &&f) {
+    int n[3];
+    for (int t = 0; t < 3; t++) n[t] = (ch.nabc[t] + sb - 1) / sb;
+    for (int ia = 0; ia < n[0]; ia++)
+        for (int ib = 0; ib < n[1]; ib++) {
+            if (ch.blk[0] == ch.blk[1] && ib > ia) continue;
+            for (int ic = 0; ic < n[2]; ic++) {
+                if (ch.blk[1] == ch.blk[2] && ic > ib) continue;
+                const int idx[3] = {ia, ib, ic};
+                int st[3], len[3];
+                for (int t = 0; t < 3; t++) {
+                    st[t] = ch.base[t] + idx[t] * sb;
+                    len[t] = ch.nabc[t] - idx[t] * sb < sb ? ch.nabc[t] - idx[t] * sb : sb;
+                }
+                f(st, len);
+            }
+        }
+}
+
+// FP64 epilogue parameters of one chunk.
+static void f2_params(const Plan &P, const ChunkDesc &ch, char *ws, const TriplesIO &io, F2P &F) {
     F.d = P.d;
     F.ch = ch;
     F.nsub = 0;
-    int nsb[3];
-    for (int t = 0; t < 3; t++) nsb[t] = (ch.nabc[t] + kSB - 1) / kSB;
-    F2Sub rest[kMaxSub];
-    int nrest = 0;
-    for (int sa = 0; sa < nsb[0]; sa++)
-        for (int sb = 0; sb < nsb[1]; sb++) {
-            if (ch.blk[0] == ch.blk[1] && sb > sa) continue;
-            for (int sc = 0; sc < nsb[2]; sc++) {
-                if (ch.blk[1] == ch.blk[2] && sc > sb) continue;
-                F2Sub u;
-                const int si[3] = {sa, sb, sc};
-                for (int t = 0; t < 3; t++) {
-                    u.st[t] = ch.base[t] + si[t] * kSB;
-                    int len = ch.nabc[t] - si[t] * kSB;
-                    u.len[t] = len < kSB ? len : kSB;
-                }
-                const bool simple = mixed && u.len[0] == 8 && u.len[1] == 8 && u.len[2] == 8 &&
-                                    u.st[0] != u.st[1] && u.st[1] != u.st[2] && u.st[0] != u.st[2];
-                if (simple) F.sub[F.nsub++] = u;
-                else rest[nrest++] = u;
-            }
+    for_sub_ranges(ch, kF2SB, [&](const int *st, const int *len) {
+        F2Sub &u = F.sub[F.nsub++];
+        for (int t = 0; t < 3; t++) {
+            u.st[t] = st[t];
+            u.len[t] = len[t];
         }
-    const int n_simple_sub = F.nsub;
-    for (int t = 0; t < nrest; t++) F.sub[F.nsub++] = rest[t];
+    });
     F.ijk = (int *)(ws + P.off_ijk);
     F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
-    F.S = (StageT *)(ws + P.off_S);
-    F.SW = P.want_grad ? (void *)(ws + P.off_SW) : nullptr;
-    F.split = mixed ? (P.prec == TRIPLES_PRECISION_MIXED_BF16 ? 2 : 1) : 0;
-    F.wscale = &ctrl->wscale;
+    F.S = (const double *)(ws + P.off_S);
+    F.SW = P.want_grad ? (double *)(ws + P.off_SW) : nullptr;
     F.ybar = io.ybar;
     F.want_grad = P.want_grad;
     F.e_part = (double *)(ws + P.off_epart);
     F.n_ijk = P.n_ijk;
     F.mo_bar = io.mo_energy_bar;
     F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
-    F.rep0 = 0;
-    F.sub0 = 0;
-    F.nsub_l = F.nsub;
-    return n_simple_sub;
+}
+
+// Mixed-precision epilogue parameters of one chunk.
+static void f2m_params(const Plan &P, const ChunkDesc &ch, char *ws, const TriplesIO &io, bool whole, F2M &F) {
+    Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
+    const int o = P.d.o;
+    F.o = o;
+    F.v = P.d.v;
+    F.nb8 = (P.d.v + 7) / 8;
+    F.nsub = 0;
+    F.n_ijk = P.n_ijk;
+    F.whole = whole ? 1 : 0;
+    for_sub_ranges(ch, 8, [&](const int *st, const int *len) {
+        F2mSub &u = F.sub[F.nsub++];
+        u.full = 1;
+        for (int t = 0; t < 3; t++) {
+            u.st[t] = st[t];
+            u.len[t] = len[t];
+            if (len[t] != 8) u.full = 0;
+        }
+        u.pat = st[0] == st[2] ? 3 : (st[0] == st[1] ? 1 : (st[1] == st[2] ? 2 : 0));
+        u.bulk = u.bulk_bytes = 0;
+        for (int pi = 0; pi < 6; pi++) {
+            int pp[3];
+            perm_of(pi, pp);
+            int t = 0;
+            while (t + 1 < ch.nperm && !(ch.pb[t].bx == ch.blk[pp[0]] && ch.pb[t].by == ch.blk[pp[1]] &&
+                                         ch.pb[t].bz == ch.blk[pp[2]]))
+                t++;
+            const PermBlock &pb = ch.pb[t];
+            const int xs = st[pp[0]] - pb.X0, ys = st[pp[1]] - pb.Y0, zs = st[pp[2]] - pb.Z0;
+            F2mPi &D = u.pi[pi];
+            D.s0 = f2m_stage_offset(pb, o, 0, 0, 0, ys, xs, zs);   // (y, x, z) at a block's origin: no exchange
+            D.rs = pb.Tx * pb.Ty * pb.Tz;
+            D.wx = o * pb.rzp;
+            D.wp = pb.Tx * D.wx;
+            D.wy = o * D.wp;
+            D.rzp = pb.rzp;
+            D.tz = pb.Tz;
+            D.w0 = 2 * pb.swoff + (long long)ys * D.wy + (long long)xs * D.wx + zs;
+            D.half = (long long)pb.Ty * D.wy;
+            D.bytes = 4 * len[0] * len[1] * len[2];
+            if (D.bytes % 16 == 0) {
+                u.bulk |= 1 << pi;
+                u.bulk_bytes += D.bytes;
+            }
+        }
+    });
+    F.ijk = (int *)(ws + P.off_ijk);
+    F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
+    F.ot = P.vtables ? (const float2 *)(ws + P.off_ot) : nullptr;
+    F.tf = P.vtables ? (const float2 *)(ws + P.off_tf) : nullptr;
+    F.S = (const float *)(ws + P.off_S);
+    F.SW = P.want_grad ? (uint16_t *)(ws + P.off_SW) : nullptr;
+    F.wscale = &ctrl->wscale;
+    F.ybar = io.ybar;
+    F.want_grad = P.want_grad;
+    F.e_part = (double *)(ws + P.off_epart);
+    F.mo_bar = io.mo_energy_bar;
+    F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
+    F.err = &ctrl->err;
+    F.ticket = &ctrl->ticket;
 }
 
 // Adjoint-contraction parameters of one chunk and kind (0: ovvv_bar, 1: t2_bar
@@ -1441,6 +1503,11 @@ static int prep_launches(const Plan &P, cudaStream_t st, const TriplesIO &io) {
             TB_KLAUNCH(P_PREP, k_prep_B2h<__half><<<grid1d((long long)v * o * v * P.Op8, 256), 256, 0, st>>>(
                 io.t2, d, P.Op8, ctrl, (__half *)(ws + P.off_B2h)));
         }
+        if (P.vtables) {
+            const int nb8 = (d.v + 7) / 8;
+            TB_KLAUNCH(P_PREP, k_prep_vtables<<<grid1d((long long)o * o * nb8 * nb8 * 64, 256), 256, 0, st>>>(
+                io.ovov, io.t2, io.t1, io.fvo, d.o, d.v, nb8, (float2 *)(ws + P.off_ot), (float2 *)(ws + P.off_tf)));
+        }
         TB_LAUNCH_CHECK();
         if (P.want_grad) TB_CUDA(cudaMemsetAsync(SW, 0, P.wbar_elems * 4, st));
     }
@@ -1474,15 +1541,11 @@ static int fold_launches(const Plan &P, cudaStream_t st, const TriplesIO &io) {
 
 template <typename StageT>
 static int run_impl(const Plan &P, cudaStream_t st, const TriplesIO &io) {
-    constexpr int kSB = sizeof(StageT) == 4 ? 8 : 4;   // epilogue sub-block edge
-    {
-        const int rc = setup_epilogue<StageT>();
-        if (rc != TRIPLES_OK) return rc;
-    }
-    int prc = prep_launches<StageT>(P, st, io);
-    if (prc != TRIPLES_OK) return prc;
-    const Dims d = P.d;
     const bool mixed = P.prec != TRIPLES_PRECISION_FP64;
+    int prc = setup_epilogue(mixed);
+    if (prc != TRIPLES_OK) return prc;
+    if ((prc = prep_launches<StageT>(P, st, io)) != TRIPLES_OK) return prc;
+    const Dims d = P.d;
     const bool bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16;
     char *ws = (char *)io.workspace;
     Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
@@ -1538,64 +1601,26 @@ static int run_impl(const Plan &P, cudaStream_t st, const TriplesIO &io) {
                     // projected energy: whole-chunk epilogue instead of the orbit tiles
                     const int rc = lno_chunk<StageT>(P, ch, st, io, ws, ctrl, S, SW, ijk, mixed ? (bf16 ? 2 : 1) : 0);
                     if (rc != TRIPLES_OK) return rc;
-                } else {
-                    // F2: energy (+ adjoint of the raw amplitudes).  Sub-range
-                    // triples of three distinct full 8-wide sub-ranges come first;
-                    // in the mixed modes they go to the persistent kernel k_f2p with
-                    // the all-distinct occupied representatives (the first
-                    // n_distinct_ijk of the table) and, in a second launch, with the
-                    // representatives i = j > k and i > j = k that follow them; every
-                    // other item (i = j = k, the remaining sub-range triples) to k_f2t.
-                    F2P<StageT> F;
-                    const int n_simple_sub = f2_params<StageT>(P, ch, ws, io, F);
-                    if (mixed && P.want_grad)
+                } else if (mixed) {
+                    // F2: energy (+ adjoint of the raw amplitudes), every item of the chunk in one launch
+                    F2M F;
+                    f2m_params(P, ch, ws, io, false, F);
+                    if (P.want_grad)
                         TB_KLAUNCH(P_PREP, k_chunk_scale<<<1, 32, 0, st>>>(ctrl, io.mo_energy, d.o, ch.base[0], ch.nabc[0],
                                                                            ch.base[1], ch.nabc[1], ch.base[2], ch.nabc[2],
                                                                            io.ybar, bf16 ? 0 : 1, 0));
-                    const int nd = mixed ? n_distinct_ijk(d.o) : 0;
-                    const int np = mixed ? d.o * (d.o - 1) / 2 : 0;   // i = j > k, then as many i > j = k
-                    auto f2t = [&](int rep0, int nrep, int sub0, int nsub_l) -> int {
-                        if (nrep <= 0 || nsub_l <= 0) return TRIPLES_OK;
-                        F.rep0 = rep0;
-                        F.sub0 = sub0;
-                        F.nsub_l = nsub_l;
-                        TB_KLAUNCH(P_F2, (k_f2t<StageT, kSB, false><<<(unsigned)(nrep * nsub_l), F2Smem<kSB>::NT,
-                                                                      f2_smem_bytes<StageT, kSB>(), st>>>(
-                                             F, nullptr, nullptr, 0)));
-                        return TRIPLES_OK;
-                    };
-                    // k_f2p over the representatives [rep0, rep0 + nrep) and the
-                    // leading n_simple_sub sub-range triples
-                    auto f2p = [&](int rep0, int nrep, int deg) -> int {
-                        if (nrep <= 0 || n_simple_sub <= 0) return TRIPLES_OK;
-                        F.rep0 = rep0;
-                        F.sub0 = 0;
-                        F.nsub_l = n_simple_sub;
-                        F2P<float> Ff;
-                        std::memcpy(&Ff, &F, sizeof(F));   // StageT = float in the mixed modes
-                        const int nitems = nrep * n_simple_sub;
-                        const unsigned nb = (unsigned)(nitems < num_sms() ? nitems : num_sms());
-#define TB_F2P(HV, DV) TB_KLAUNCH(P_F2, (k_f2p<HV, DV><<<nb, F2pSmem::NT, F2pSmem::BYTES, st>>>(Ff, nitems)))
-                        if (deg == 1) {
-                            if (bf16) TB_F2P(2, 1);
-                            else TB_F2P(1, 1);
-                        } else if (deg == 2) {
-                            if (bf16) TB_F2P(2, 2);
-                            else TB_F2P(1, 2);
-                        } else {
-                            if (bf16) TB_F2P(2, 0);
-                            else TB_F2P(1, 0);
-                        }
-#undef TB_F2P
-                        return TRIPLES_OK;
-                    };
-                    int frc;
-                    if ((frc = f2p(0, nd, 0)) != TRIPLES_OK) return frc;
-                    if ((frc = f2p(nd, np, 1)) != TRIPLES_OK) return frc;
-                    if ((frc = f2p(nd + np, np, 2)) != TRIPLES_OK) return frc;
-                    if ((frc = f2t(0, nd + 2 * np, n_simple_sub, F.nsub - n_simple_sub)) != TRIPLES_OK) return frc;
-                    if ((frc = f2t(nd + 2 * np, P.n_ijk - nd - 2 * np, 0, F.nsub)) != TRIPLES_OK) return frc;
-                    TB_KLAUNCH(P_F2, k_f2_energy_sum<<<1, 256, 0, st>>>(e_part, P.n_ijk * F.nsub, &ctrl->e_acc));
+                    const int nitems = P.n_ijk * F.nsub;
+                    const int nb = nitems < 2 * num_sms() ? nitems : 2 * num_sms();
+                    if (bf16)
+                        TB_KLAUNCH(P_F2, (k_f2m<2, false><<<nb, kF2mThreads, F2mSmem::BYTES, st>>>(F, nullptr, nullptr, 0, nitems)));
+                    else
+                        TB_KLAUNCH(P_F2, (k_f2m<1, false><<<nb, kF2mThreads, F2mSmem::BYTES, st>>>(F, nullptr, nullptr, 0, nitems)));
+                    TB_KLAUNCH(P_F2, k_f2_energy_sum<<<1, 256, 0, st>>>(e_part, nitems, &ctrl->e_acc, &ctrl->ticket));
+                } else {
+                    F2P F;
+                    f2_params(P, ch, ws, io, F);
+                    TB_KLAUNCH(P_F2, (k_f2t<<<(unsigned)(P.n_ijk * F.nsub), kF2Threads, f2_smem_bytes(), st>>>(F)));
+                    TB_KLAUNCH(P_F2, k_f2_energy_sum<<<1, 256, 0, st>>>(e_part, P.n_ijk * F.nsub, &ctrl->e_acc, nullptr));
                 }
                 if (!P.want_grad) continue;
                 // W-term gradients
@@ -1672,7 +1697,7 @@ struct BatchStep {
     size_t aux;                       // ChunkAux per problem of the step
     int naux;
     size_t f2_jobs, f2_start;
-    int f2_ctas;
+    int f2_items;
     size_t b1_jobs[4], b1_start[4];   // per adjoint kind
     int b1_tiles[4];
 };
@@ -1770,7 +1795,7 @@ static int batch_build(Batch &B, int prec, int nprob, const triples_problem *pro
         }
         S.naux = n;
         S.aux = take(sizeof(ChunkAux) * n);
-        S.f2_jobs = take(sizeof(F2P<float>) * n);
+        S.f2_jobs = take(sizeof(F2M) * n);
         S.f2_start = take(sizeof(int) * (n + 1));
         for (int k = 0; k < 4; k++) {
             S.b1_jobs[k] = take(sizeof(TcB1Params) * n);
@@ -1807,9 +1832,9 @@ static int batch_build(Batch &B, int prec, int nprob, const triples_problem *pro
             const Plan &P = B.plans[p];
             const ChunkDesc &ch = chunks[p][c];
             char *wsp = B.ws + B.ws_off[p];
-            F2P<float> F;
+            F2M F;
             std::memset(&F, 0, sizeof(F));
-            f2_params<float>(P, ch, wsp, B.ios[p], F);   // one segment: every representative, every sub-range triple
+            f2m_params(P, ch, wsp, B.ios[p], true, F);
             std::memcpy(img + S.f2_jobs + sizeof(F) * j, &F, sizeof(F));
             f2s[j + 1] = f2s[j] + P.n_ijk * F.nsub;
             ChunkAux A;
@@ -1833,7 +1858,7 @@ static int batch_build(Batch &B, int prec, int nprob, const triples_problem *pro
                 b1s[k][j + 1] = b1s[k][j] + Bp.cum[ch.nperm];
             }
         }
-        S.f2_ctas = f2s[n];
+        S.f2_items = f2s[n];
         for (int k = 0; k < 4; k++) S.b1_tiles[k] = b1s[k][n];
     }
     if (image) image->resize(t);
@@ -1850,7 +1875,7 @@ static int run_batch(const Batch &B, cudaStream_t st) {
         return TRIPLES_OK;
     }
     int rc;
-    if ((rc = setup_epilogue<float>()) != TRIPLES_OK) return rc;
+    if ((rc = setup_epilogue(true)) != TRIPLES_OK) return rc;
     if ((rc = setup_tensor_cores()) != TRIPLES_OK) return rc;
     for (int p = 0; p < B.nprob; p++)
         if ((rc = prep_launches<float>(B.plans[p], st, B.ios[p])) != TRIPLES_OK) return rc;
@@ -1860,7 +1885,7 @@ static int run_batch(const Batch &B, cudaStream_t st) {
     const F1Maps M0{};
     const TcF1Params T0{};
     const TcB1Params B0{};
-    const F2P<float> F0{};
+    const F2M F0{};
     auto cap = [&](int n) { return n < nsm ? n : nsm; };
     for (const BatchStep &S : B.steps) {
         const F1Job *f1j[2] = {(const F1Job *)(tab + S.f1_jobs[0]), (const F1Job *)(tab + S.f1_jobs[1])};
@@ -1873,8 +1898,13 @@ static int run_batch(const Batch &B, cudaStream_t st) {
                                  M0, T0, f1j[1], f1s[1], S.f1_n[1])));
         const ChunkAux *aux = (const ChunkAux *)(tab + S.aux);
         TB_KLAUNCH(P_PREP, k_chunk_scale_batch<<<S.naux, 32, 0, st>>>(aux, scaled));
-        TB_KLAUNCH(P_F2, (k_f2t<float, 8, true><<<S.f2_ctas, F2Smem<8>::NT, f2_smem_bytes<float, 8>(), st>>>(
-                             F0, (const F2P<float> *)(tab + S.f2_jobs), (const int *)(tab + S.f2_start), S.naux)));
+        const F2M *f2j = (const F2M *)(tab + S.f2_jobs);
+        const int *f2s = (const int *)(tab + S.f2_start);
+        const int f2n = S.f2_items < 2 * nsm ? S.f2_items : 2 * nsm;
+        if (scaled)
+            TB_KLAUNCH(P_F2, (k_f2m<1, true><<<f2n, kF2mThreads, F2mSmem::BYTES, st>>>(F0, f2j, f2s, S.naux, S.f2_items)));
+        else
+            TB_KLAUNCH(P_F2, (k_f2m<2, true><<<f2n, kF2mThreads, F2mSmem::BYTES, st>>>(F0, f2j, f2s, S.naux, S.f2_items)));
         TB_KLAUNCH(P_F2, k_energy_sum_batch<<<S.naux, 256, 0, st>>>(aux));
         const TcB1Params *bj[4];
         const int *bs[4];
@@ -1946,6 +1976,8 @@ static int triples_call(void *stream, int precision, int nocc, int nvir, int ovv
     tb::Plan P;
     int rc = tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, P, 0, opt);
     if (rc != TRIPLES_OK) return rc;
+    // a workspace too small for the V-term tables alone: run without them
+    if (workspace_bytes < P.total) tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, P, 0, opt, false);
     if (!io.workspace || workspace_bytes < P.total) return TRIPLES_ERR_WORKSPACE;
     if (!io.mo_energy || !io.t1 || !io.t2 || !io.ovoo || !io.ovov || !io.ovvv || !io.fvo || !io.e_out)
         return TRIPLES_ERR_INVALID_ARGUMENT;
@@ -2085,9 +2117,9 @@ struct DfLayout {
     size_t off_ovvv, off_gvvv, total;
 };
 
-static int df_layout(int precision, int nocc, int nvir, int naux, int want_grad, DfLayout &L) {
+static int df_layout(int precision, int nocc, int nvir, int naux, int want_grad, DfLayout &L, bool vtables = true) {
     if (naux < 1) return TRIPLES_ERR_INVALID_ARGUMENT;
-    int rc = tb::make_plan(precision, nocc, nvir, 1, want_grad, L.P);
+    int rc = tb::make_plan(precision, nocc, nvir, 1, want_grad, L.P, 0, nullptr, vtables);
     if (rc != TRIPLES_OK) return rc;
     const size_t nov = (size_t)nocc * nvir, npair = (size_t)nvir * (nvir + 1) / 2;
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -2112,6 +2144,7 @@ static int triples_df_call(void *stream, int precision, int nocc, int nvir, int 
     DfLayout L;
     int rc = df_layout(precision, nocc, nvir, naux, want_grad, L);
     if (rc != TRIPLES_OK) return rc;
+    if (workspace_bytes < L.total) df_layout(precision, nocc, nvir, naux, want_grad, L, false);
     if (!io.workspace || workspace_bytes < L.total) return TRIPLES_ERR_WORKSPACE;
     if (!Lov || !Lvv || !io.mo_energy || !io.t1 || !io.t2 || !io.ovoo || !io.ovov || !io.fvo || !io.e_out)
         return TRIPLES_ERR_INVALID_ARGUMENT;
@@ -2205,9 +2238,10 @@ int triples_energy_vjp_static(void *stream, int precision, int nocc, int nvir, i
                               const double *fvo, double ybar, double *e_out, double *mo_energy_bar,
                               double *t1_bar, double *t2_bar, double *ovoo_bar, double *ovov_bar,
                               double *ovvv_bar, double *fvo_bar) {
-    const size_t need = triples_workspace_size(precision, nocc, nvir, ovvv_packed, 1);
-    if (need == 0) return TRIPLES_ERR_INVALID_ARGUMENT;
-    if (need > kStaticScratchBytes) return TRIPLES_ERR_WORKSPACE;   // problem too large for the fixed scratch
+    tb::Plan P;
+    if (tb::make_plan(precision, nocc, nvir, ovvv_packed, 1, P, 0, nullptr, false) != TRIPLES_OK)
+        return TRIPLES_ERR_INVALID_ARGUMENT;
+    if (P.total > kStaticScratchBytes) return TRIPLES_ERR_WORKSPACE;   // problem too large for the fixed scratch
     void *scratch = nullptr;
     const int rc = static_scratch_address(&scratch);
     if (rc != TRIPLES_OK) return rc;

@@ -8,7 +8,6 @@
 
 namespace tb {
 
-constexpr int kF2Threads = 256;   // chunk-epilogue block size
 constexpr int kMaxTv = 16;        // largest virtual block
 constexpr int kMaxCols = 1024;    // largest nocc * Tv (one staged (r, z) row)
 constexpr int kCtrlBytes = 256;   // control block at workspace offset 0
@@ -26,6 +25,7 @@ struct Ctrl {
     double wscale;                // per-chunk power-of-two scale of the split Wbar
     unsigned long long absmax[6]; // bit patterns of max |ovvv|, |ovoo|, |t2|, |ovov|, |t1|, |fvo|
     unsigned wmax_bits;           // bit pattern of max |W| of the current chunk (F1)
+    unsigned ticket;              // work items handed out by the mixed epilogue of the current chunk
     double lno_norm[2];           // LNO projector: max abs row sum, max abs column sum
 };
 
@@ -48,6 +48,8 @@ struct Plan {
     size_t off_A1, off_B1, off_A2, off_B2, off_S, off_SW;
     size_t off_A1h, off_B1h, off_A2h, off_B2h;
     size_t off_GA1, off_GB1, off_GA2, off_GB2;
+    bool vtables;    // the workspace holds the epilogue's FP32 V-term tables
+    size_t off_ot, off_tf;
     size_t off_ijk, off_epart;
     size_t off_L[4], off_lpart;
     size_t total;
@@ -64,7 +66,7 @@ struct TriplesIO {
 };
 
 int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, int lno = 0,
-              const triples_options *opt = nullptr);
+              const triples_options *opt = nullptr, bool vtables = true);
 int run_triples(const Plan &P, cudaStream_t st, const TriplesIO &io);
 
 }  // namespace tb
