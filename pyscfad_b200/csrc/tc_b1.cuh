@@ -35,6 +35,7 @@ struct TcB1Params {
     int nperm;
     int kind;
     int nbatch[6], ntile_m[6], ntile_n;
+    int nw, ncol;           // columns of an N tile (multiple of 16, at most BN), of the gradient rows
     int nk_outer[6], nk_inner[6];
     int cum[7];             // prefix of tile counts over orderings
     double *G;
@@ -51,6 +52,10 @@ constexpr int kB1Threads = 320;   // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 // K <= 512 * 64 keep the rounding of the sum well below the fp16 split error
 constexpr int kB1RunSegments = 512;
 
+// N tiles are nw = 16 n columns wide: nvir (kinds 0, 1) or nocc (2, 3) split
+// evenly over the fewest tiles of at most BN and rounded up to 16, so that nvir
+// 180 takes two tiles of 96 where fixed 128-wide tiles padded it to 256.  K
+// blocks issue only the 16-wide steps that hold values.
 template <bool A_MN, int BN>
 struct TcB1Cfg {
     static constexpr int A_BYTES = kTcBM * kTcBK * 2;
@@ -130,6 +135,11 @@ __global__ void __launch_bounds__(kB1Threads, 1)
     const uint32_t tmem_base = *tmem_slot;
     volatile int *abortp = &s_abort;
     const int total = BATCH ? job_start[njobs] : P0.cum[P0.nperm];
+    // columns an MMA of N tile nt covers
+    auto width = [&](const TcB1Params &P, int nt) -> int {
+        const int left = P.ncol - nt * P.nw;
+        return left < P.nw ? (left + 15) / 16 * 16 : P.nw;
+    };
     // tile t of the chunk with parameters P -> ordering, batch, M tile, N tile
     auto decode = [&](const TcB1Params &P, int t, int &tau, int &b, int &mt, int &nt) {
         tau = 0;
@@ -157,46 +167,43 @@ __global__ void __launch_bounds__(kB1Threads, 1)
             int tau, b, mt, nt;
             decode(P, lt, tau, b, mt, nt);
             const PermBlock &pb = P.pb[tau];
-            const int Ty = pb.Ty, Tz = pb.Tz;
-            const int nk = P.nk_outer[tau] * P.nk_inner[tau];
+            const int Ty = pb.Ty, lz = 31 - __clz(pb.Tz);
+            const int nk_inner = P.nk_inner[tau], nk = P.nk_outer[tau] * nk_inner;
             const CUtensorMap *tmA = &P.tmA[tau], *tmB = &P.tmB[tau];
+            const int nbox = (width(P, nt) + 63) / 64, n0 = nt * P.nw;
+            const uint32_t bytes = (uint32_t)(2 * C::A_BYTES + 2 * nbox * 8192);
+            // K = (ko, ki): kinds 0 and 3 run q in ko with batch y, kinds 1 and 2 y in ko with batch q
+            const bool ko_q = P.kind == 0 || P.kind == 3;
+            int ko = 0, ki = 0;
             for (int kb = 0; kb < nk; kb++) {
                 if (!mbar_wait(&empty[stage], phase ^ 1u, abortp)) {
                     ok = false;
                     break;
                 }
                 pending[stage] = false;
-                mbar_expect_tx(&full[stage], C::STAGE_BYTES);
+                mbar_expect_tx(&full[stage], bytes);
                 uint8_t *sA = smem + stage * C::STAGE_BYTES;
                 uint8_t *sB = sA + 2 * C::A_BYTES;
-                const int ko = kb / P.nk_inner[tau], ki = kb % P.nk_inner[tau];
+                const int aq = ko_q ? ko : b, ay = ko_q ? b : ko;
+                const int b3 = ko_q ? ko : pb.Y0 + ko;
+#pragma unroll
                 for (int h = 0; h < 2; h++) {
                     uint8_t *a = sA + h * C::A_BYTES;
                     uint8_t *bb = sB + h * C::B_BYTES;
-                    switch (P.kind) {
-                    case 0:   // batch y, K = (q = ko, rz block = ki)
-                        tma_load_5d(a, tmA, &full[stage], ki * 64, ko, 0, mt * 8, h * Ty + b);
-                        for (int j = 0; j < BN / 64; j++)
-                            tma_load_5d(bb + j * 8192, tmB, &full[stage], nt * BN + j * 64, pb.Z0, ki * 64 / Tz, ko, h);
-                        break;
-                    case 1:   // batch q, K = (y = ko, p group = ki)
+                    if (A_MN) {
+#pragma unroll
                         for (int j = 0; j < 2; j++)
-                            tma_load_5d(a + j * 8192, tmA, &full[stage], mt * 128 + j * 64, b, 0, ki * 4, h * Ty + ko);
-                        for (int j = 0; j < BN / 64; j++)
-                            tma_load_5d(bb + j * 8192, tmB, &full[stage], nt * BN + j * 64, pb.X0, ki * 4, pb.Y0 + ko, h);
-                        break;
-                    case 2:   // batch q, K = (y = ko, rz block = ki)
-                        tma_load_5d(a, tmA, &full[stage], ki * 64, b, 0, mt * 8, h * Ty + ko);
-                        for (int j = 0; j < BN / 64; j++)
-                            tma_load_5d(bb + j * 8192, tmB, &full[stage], nt * BN + j * 64, pb.Z0, ki * 64 / Tz, pb.Y0 + ko, h);
-                        break;
-                    default:  // batch y, K = (q = ko, p group = ki)
-                        for (int j = 0; j < 2; j++)
-                            tma_load_5d(a + j * 8192, tmA, &full[stage], mt * 128 + j * 64, ko, 0, ki * 4, h * Ty + b);
-                        for (int j = 0; j < BN / 64; j++)
-                            tma_load_5d(bb + j * 8192, tmB, &full[stage], nt * BN + j * 64, pb.X0, ki * 4, ko, h);
-                        break;
+                            tma_load_5d(a + j * 8192, tmA, &full[stage], mt * 128 + j * 64, aq, 0, ki * 4, h * Ty + ay);
+                    } else {
+                        tma_load_5d(a, tmA, &full[stage], ki * 64, aq, 0, mt * 8, h * Ty + ay);
                     }
+                    const int b1 = A_MN ? pb.X0 : pb.Z0, b2 = A_MN ? ki * 4 : (ki * 64) >> lz;
+                    tma_load_5d(bb, tmB, &full[stage], n0, b1, b2, b3, h);
+                    if (BN > 64 && nbox > 1) tma_load_5d(bb + 8192, tmB, &full[stage], n0 + 64, b1, b2, b3, h);
+                }
+                if (++ki == nk_inner) {
+                    ki = 0;
+                    ko++;
                 }
                 pending[stage] = true;
                 pend_phase[stage] = phase;
@@ -217,7 +224,6 @@ __global__ void __launch_bounds__(kB1Threads, 1)
         }
     } else if (warp == 1 && lane == 0) {
         // ---------------- MMA issuer: one TMEM buffer per K segment ----------------
-        const uint32_t idesc = make_idesc_f16(kTcBM, BN, Pfirst.bf16 != 0, A_MN, true);
         int stage = 0;
         uint32_t phase = 0;
         int seg = 0;   // running segment counter (same sequence as the epilogue)
@@ -228,7 +234,11 @@ __global__ void __launch_bounds__(kB1Threads, 1)
             const TcB1Params &P = BATCH ? jobs[jb] : P0;
             int tau, b, mt, nt;
             decode(P, lt, tau, b, mt, nt);
+            const uint32_t idesc = make_idesc_f16(kTcBM, width(P, nt), P.bf16 != 0, A_MN, true);
             const int nk = P.nk_outer[tau] * P.nk_inner[tau];
+            // K values of the inner blocks of one outer index: o Tz, or 16 per p
+            const int klen = A_MN ? 16 * P.d.o : P.d.o * P.pb[tau].Tz;
+            int left = klen;   // K values from the current inner block on
             for (int k0 = 0; k0 < nk && ok; k0 += P.kseg, seg++) {
                 const int acc = seg % C::NACC;
                 const uint32_t accph = (seg / C::NACC) & 1;
@@ -249,8 +259,11 @@ __global__ void __launch_bounds__(kB1Threads, 1)
                     const uint32_t a_l = a_h + C::A_BYTES;
                     const uint32_t b_h = a_l + C::A_BYTES;
                     const uint32_t b_l = b_h + C::B_BYTES;
+                    const int nks = left < kTcBK ? (left + 15) >> 4 : kTcBK / 16;
+                    left = left <= kTcBK ? klen : left - kTcBK;
 #pragma unroll
                     for (int ks = 0; ks < kTcBK / 16; ks++) {
+                        if (ks >= nks) break;
                         uint64_t dah, dal;
                         if (A_MN) {
                             dah = make_sdesc_sw128(a_h + 2048 * ks, 8192, 1024);
@@ -284,9 +297,10 @@ __global__ void __launch_bounds__(kB1Threads, 1)
         }
     } else if (warp >= 2) {
         // ---------------- epilogue: G += sign * sum_seg D_seg / (wscale * oscale) ----------------
-        constexpr int HC = BN / 2;            // columns per epilogue warp
+        constexpr int HC = BN / 2;            // most columns of an epilogue warp: groups of 8,
+                                              // 2 c + half for c = 0, 1, ...
         const int quarter = warp & 3;         // TMEM lane quarter this warp may access
-        const int half = (warp - 2) >> 2;     // which half of the columns
+        const int half = (warp - 2) >> 2;     // which of the column groups
         const int row = quarter * 32 + lane;
         const double sc0 = BATCH ? 0.0 : P0.sign / ((*P0.wscale) * (*P0.oscale));   // single chunk: read once
         int seg = 0;
@@ -321,8 +335,8 @@ __global__ void __launch_bounds__(kB1Threads, 1)
                         roff = ((((long long)pb.Y0 + b) * o + r) * v + pb.Z0 + z) * o;
                 }
             }
-            const int ncol = (P.kind <= 1) ? v : o;
-            const int c0 = nt * BN + half * HC;
+            const int nwid = width(P, nt), c0 = nt * P.nw + half * 8;
+            const int lim = min(P.ncol - nt * P.nw, nwid) - half * 8;   // this warp's columns: c0 + [0, lim)
             float acc[HC];
 #pragma unroll
             for (int j = 0; j < HC; j++) acc[j] = 0.f;
@@ -330,10 +344,11 @@ __global__ void __launch_bounds__(kB1Threads, 1)
             // kB1RunSegments FP32-summed segments
             auto flush = [&]() {
                 if (roff >= 0) {
+                    double *g = P.G + roff + c0;
 #pragma unroll
                     for (int j = 0; j < HC; j++) {
-                        const int col = c0 + j;
-                        if (col < ncol) atomicAdd(&P.G[roff + col], sc * (double)acc[j]);
+                        const int col = (j >> 3) * 16 + (j & 7);
+                        if (col < lim) atomicAdd(g + col, sc * (double)acc[j]);
                     }
                 }
 #pragma unroll
@@ -355,7 +370,8 @@ __global__ void __launch_bounds__(kB1Threads, 1)
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < HC / 8; c++) {
-                    const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * HC + c * 8);
+                    // (columns beyond the tile's width hold nothing and are never added to G)
+                    const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((2 * c + half) * 8);
                     uint32_t va[8], vb[8];
                     tmem_ld8(lane_base + (uint32_t)(accA * BN), va);
                     if (two) tmem_ld8(lane_base + (uint32_t)(accB * BN), vb);

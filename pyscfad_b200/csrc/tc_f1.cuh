@@ -8,8 +8,11 @@
 // both halves.  Each K step issues hi*hi + hi*lo + lo*hi into one FP32 TMEM
 // accumulator.
 //
-// Tile: 128 rows = 8 p x 16 x, BN columns = BN/16 r x 16 z, K blocks of 64.
-// Persistent CTAs (one per SM), warp roles: 0 TMA producer, 1 MMA issuer and
+// Tile: 128 rows = 8 p x 16 x, 16 rt columns = rt r x 16 z (rt even, at most
+// BN / 16), K blocks of 64 (the last of each term issues only the 16-wide steps
+// it holds).  rt divides nocc as evenly as the widest tile allows (f1_tile in
+// triples.cu): nocc 20 takes two tiles of 10 r where fixed 8-wide tiles padded
+// it to 24 and 16-wide ones to 32.  Persistent CTAs (one per SM), warp roles: 0 TMA producer, 1 MMA issuer and
 // TMEM owner, 2-5 epilogue (TMEM -> registers -> staging, FP32).
 #pragma once
 #include "common.cuh"
@@ -29,7 +32,6 @@ struct TcCfg {
     static constexpr int BAR_BYTES = 256;
     static constexpr int STORE_BYTES = 8 * 32 * 32 * 4;   // one 32 x 32 FP32 store box per epilogue warp
     static constexpr int SMEM = STAGES * STAGE_BYTES + STORE_BYTES + BAR_BYTES + 1024;
-    static constexpr int RT = BN / 16;
     static constexpr int TMEM_COLS = 2 * BN;
 };
 
@@ -43,8 +45,9 @@ struct TcF1Params {
     ChunkDesc ch;
     int cum[7];        // prefix over orderings of tile counts
     int mt_count;      // p tiles of 8
-    int nt_count;      // r tiles of BN/16
+    int rt, nt_count;  // r values of a tile (even), r tiles
     int nkb1, nkb2;    // K blocks of the ovvv and ooov terms
+    int k1, k2;        // K lengths of the two terms
     float *S;
     const float *out_scale;   // device scalar: 1 / (scale_A * scale_B)
     unsigned *wmax_bits;      // device: running max |W| of this chunk (float bits)
@@ -190,7 +193,7 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                     break;
                 }
                 pending[stage] = false;
-                mbar_expect_tx(&full[stage], C::STAGE_BYTES);
+                mbar_expect_tx(&full[stage], (uint32_t)(2 * C::A_BYTES + P.rt * (2 * 16 * kTcBK * 2)));
                 uint8_t *sA = smem + stage * C::STAGE_BYTES;
                 uint8_t *sAl = sA + C::A_BYTES;
                 uint8_t *sB = sAl + C::A_BYTES;
@@ -199,14 +202,14 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                     const int f0 = kb * kTcBK;
                     tma_load_5d(sA, &M.a1, &full[stage], f0, pb.X0, T.mt * 8, yg, 0);
                     tma_load_5d(sAl, &M.a1, &full[stage], f0, pb.X0, T.mt * 8, yg, 1);
-                    tma_load_5d(sB, &M.b1, &full[stage], f0, pb.Z0, T.nt * C::RT, T.q, 0);
-                    tma_load_5d(sBl, &M.b1, &full[stage], f0, pb.Z0, T.nt * C::RT, T.q, 1);
+                    tma_load_5d(sB, &M.b1, &full[stage], f0, pb.Z0, T.nt * P.rt, T.q, 0);
+                    tma_load_5d(sBl, &M.b1, &full[stage], f0, pb.Z0, T.nt * P.rt, T.q, 1);
                 } else {
                     const int m0 = (kb - P.nkb1) * kTcBK;
                     tma_load_5d(sA, &M.a2, &full[stage], m0, pb.X0, T.mt * 8, T.q, 0);
                     tma_load_5d(sAl, &M.a2, &full[stage], m0, pb.X0, T.mt * 8, T.q, 1);
-                    tma_load_5d(sB, &M.b2, &full[stage], m0, pb.Z0, T.nt * C::RT, yg, 0);
-                    tma_load_5d(sBl, &M.b2, &full[stage], m0, pb.Z0, T.nt * C::RT, yg, 1);
+                    tma_load_5d(sB, &M.b2, &full[stage], m0, pb.Z0, T.nt * P.rt, yg, 0);
+                    tma_load_5d(sBl, &M.b2, &full[stage], m0, pb.Z0, T.nt * P.rt, yg, 1);
                 }
                 pending[stage] = true;
                 pend_phase[stage] = phase;
@@ -228,7 +231,6 @@ __global__ void __launch_bounds__(kF1Threads, 1)
         }
     } else if (warp == 1 && lane == 0) {
         // ---------------- MMA issuer: one TMEM buffer per K segment ----------------
-        const uint32_t idesc = make_idesc_f16(kTcBM, BN, Pfirst.bf16 != 0, false, false);
         int stage = 0;
         uint32_t phase = 0;
         int seg = 0;
@@ -237,6 +239,7 @@ __global__ void __launch_bounds__(kF1Threads, 1)
             int lt;
             const int jb = job_tile(t, lt);
             const TcF1Params &P = BATCH ? jobs[jb].P : P0;
+            const uint32_t idesc = make_idesc_f16(kTcBM, 16 * P.rt, P.bf16 != 0, false, false);
             const int nkb = P.nkb1 + P.nkb2;
             for (int k0 = 0; k0 < nkb && ok; k0 += P.kseg, seg++) {
                 const int acc = seg & 1;
@@ -258,8 +261,11 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                     const uint32_t a_l = a_h + C::A_BYTES;
                     const uint32_t b_h = a_l + C::A_BYTES;
                     const uint32_t b_l = b_h + C::B_BYTES;
+                    // 16-wide steps that hold K values (the rest of the block is zero)
+                    const int left = kb < P.nkb1 ? P.k1 - kb * kTcBK : P.k2 - (kb - P.nkb1) * kTcBK;
 #pragma unroll
                     for (int ks = 0; ks < kTcBK / 16; ks++) {
+                        if (16 * ks >= left) continue;
                         const uint64_t dah = make_sdesc_sw128(a_h + 32 * ks, 16, 1024);
                         const uint64_t dal = make_sdesc_sw128(a_l + 32 * ks, 16, 1024);
                         const uint64_t dbh = make_sdesc_sw128(b_h + 32 * ks, 16, 1024);
@@ -288,7 +294,8 @@ __global__ void __launch_bounds__(kF1Threads, 1)
         }
     } else if (warp >= 2) {
         // ---------------- epilogue: sum the segments (FP32, round to nearest) ----------------
-        constexpr int HC = BN / 2;          // columns handled by one epilogue warp
+        constexpr int HC = BN / 2;          // most columns of one epilogue warp: pieces of 32
+                                            // (2 r x 16 z), 2 c + half for c = 0, 1, ...
         const int quarter = warp & 3;
         const int half = (warp - 2) >> 2;
         const int row = quarter * 32 + lane;
@@ -324,8 +331,9 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < HC / 32; c++) {
+                    if (4 * c + 2 * half >= P.rt) continue;
                     uint32_t vv[32];
-                    tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * HC + c * 32),
+                    tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + (2 * c + half) * 32),
                               vv);
                     tmem_ld_wait();
 #pragma unroll
@@ -357,6 +365,7 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                 const int brow = (lane >> 4) * 512 + ((lane >> 3) & 1) * 128, bx = (lane & 7) * 8;
                 #pragma unroll
                 for (int c = 0; c < HC / 32; c++) {
+                    if (4 * c + 2 * half >= P.rt) continue;
                     if (c > 0) {
                         if (lane == 0) bulk_wait_read0();
                         __syncwarp();
@@ -376,7 +385,7 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    const int r0 = T.nt * C::RT + half * (HC / 16) + c * 2;
+                    const int r0 = T.nt * P.rt + 4 * c + 2 * half;
                     if (lane == 0 && p0 < o && r0 < o) {
                         if (P.blocked) tma_store_5d(&P.tmS[T.tau], box, (T.y & 7) * 64, (T.y >> 3) * 4, r0, T.q, p0);
                         else tma_store_5d(&P.tmS[T.tau], box, r0 * 16, 0, T.y, T.q, p0);
@@ -389,8 +398,8 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                 const StageRow R = f2m_stage_row(pb, o, p, T.q, T.y, x);
 #pragma unroll
                 for (int h = 0; h < HC / 16; h++) {
-                    const int r = T.nt * C::RT + half * (HC / 16) + h;
-                    if (r >= o) continue;
+                    const int rl = 4 * (h >> 1) + 2 * half + (h & 1), r = T.nt * P.rt + rl;
+                    if (rl >= P.rt || r >= o) continue;
                     float *d = P.S + R.base + (long long)r * R.rs;
                     if (R.ez == 8) {
 #pragma unroll
@@ -418,8 +427,8 @@ __global__ void __launch_bounds__(kF1Threads, 1)
             } else if (vrow) {
 #pragma unroll
                 for (int h = 0; h < HC / 16; h++) {
-                    const int r = T.nt * C::RT + half * (HC / 16) + h;
-                    if (r >= o) continue;
+                    const int rl = 4 * (h >> 1) + 2 * half + (h & 1), r = T.nt * P.rt + rl;
+                    if (rl >= P.rt || r >= o) continue;
                     float *d = dst + (long long)r * pb.Tz;
                     if (pb.Tz == 16) {
                         float4 *d4 = reinterpret_cast<float4 *>(d);

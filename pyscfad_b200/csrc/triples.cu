@@ -169,12 +169,13 @@ int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan
     } else {
         P.kseg = 1;
     }
-    // W-contraction N tile: 256 columns (16 r x 16 z) unless padding nocc to
-    // 16 wastes more than a quarter of the r values and 8-wide r tiles waste
-    // less (measured at nocc = 40: 256 is 3% faster despite 48 padded r)
-    if (P.f1_bn == 0) {
-        const int p16 = ((nocc + 15) / 16) * 16, p8 = ((nocc + 7) / 8) * 8;
-        P.f1_bn = (4 * p16 > 5 * nocc && p8 < p16) ? 128 : 256;
+    // W-contraction N tile: up to 256 columns (16 r x 16 z); 128 (a third pipeline
+    // stage) where nocc needs no more than 8 r values
+    if (P.f1_bn == 0) P.f1_bn = nocc <= 8 ? 128 : 256;
+    // r values per tile: nocc over the fewest tiles, evenly, rounded up to even
+    {
+        const int most = P.f1_bn / 16, nt = (nocc + most - 1) / most;
+        P.f1_rt = ((nocc + nt - 1) / nt + 1) / 2 * 2;
     }
     P.lno = lno ? 1 : 0;
     P.prec = precision;
@@ -1192,15 +1193,14 @@ struct OperandMaps {
     CUtensorMap tmA1m, tmA2m, tmB1z[5], tmB2z[5];   // adjoint contractions, MN-major boxes
 };
 
-// The W contraction's N tile is BN = 16 * RT columns (RT occupied r values x
-// 16 z), P.f1_bn.
+// The W contraction's N tile is 16 * P.f1_rt columns (occupied r values x 16 z).
 static int build_operand_maps(const Plan &P, char *ws, OperandMaps &M) {
     const uint64_t o = P.d.o, v = P.d.v;
     const bool bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16;
     const uint64_t dA1[5] = {(uint64_t)P.Kp8, v, o, v, 2};
     const uint32_t bA[5] = {64, 16, 8, 1, 1};
     const uint64_t dB1[5] = {(uint64_t)P.Kp8, v, o, o, 2};
-    const uint32_t bB[5] = {64, 16, (uint32_t)(P.f1_bn / 16), 1, 1};
+    const uint32_t bB[5] = {64, 16, (uint32_t)P.f1_rt, 1, 1};
     const uint64_t dA2[5] = {(uint64_t)P.Op8, v, o, o, 2};
     const uint64_t dB2[5] = {(uint64_t)P.Op8, v, o, v, 2};
     int rc;
@@ -1234,12 +1234,14 @@ static int f1_params(const Plan &P, const ChunkDesc &ch, char *ws, TcF1Params &T
     T.d = d;
     T.ch = ch;
     T.mt_count = (d.o + 7) / 8;
-    const int rt = P.f1_bn / 16;
-    T.nt_count = (d.o + rt - 1) / rt;
+    T.rt = P.f1_rt;
+    T.nt_count = (d.o + T.rt - 1) / T.rt;
     T.cum[0] = 0;
     for (int t = 0; t < ch.nperm; t++) T.cum[t + 1] = T.cum[t] + ch.pb[t].Ty * d.o * T.mt_count * T.nt_count;
     T.nkb1 = (P.Kp8 + kTcBK - 1) / kTcBK;
     T.nkb2 = (P.Op8 + kTcBK - 1) / kTcBK;
+    T.k1 = P.Kp8;
+    T.k2 = P.Op8;
     T.S = S;
     T.out_scale = &ctrl->out_scale;
     T.wmax_bits = &ctrl->wmax_bits;
@@ -1384,7 +1386,13 @@ static int b1_params(const Plan &P, const ChunkDesc &ch, char *ws, const Operand
     B.bf16 = bf16 ? 1 : 0;
     B.kseg = P.kseg;
     B.kind = kind;
-    B.ntile_n = kind <= 1 ? (d.v + 127) / 128 : (d.o + 63) / 64;
+    {
+        const int most = kind <= 1 ? 128 : 64;
+        B.ncol = kind <= 1 ? d.v : d.o;
+        B.ntile_n = (B.ncol + most - 1) / most;
+        B.nw = ((B.ncol + B.ntile_n - 1) / B.ntile_n + 15) / 16 * 16;
+        B.ntile_n = (B.ncol + B.nw - 1) / B.nw;
+    }
     B.G = (double *)(ws + (kind == 0 ? P.off_GA1 : kind == 1 ? P.off_GB1 : kind == 2 ? P.off_GA2 : P.off_GB2));
     B.oscale = &ctrl->scale[(kind == 0 || kind == 2) ? 1 : 0];
     B.sign = kind == 2 ? -1.0 : 1.0;

@@ -68,3 +68,19 @@ def test_epilogue_without_prepared_tables(o, v, tv, precision):
     for k in G.KEYS:
         assert _relerr(g1[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-12, k
     assert run(full - tables - 1)[0] != 0
+
+
+# W-contraction tiles of 2 to 16 r values (nocc 1-17, with and without a second
+# tile), adjoint tiles of 16 to 128 columns (nvir 7-130), K tails of every length
+@pytest.mark.parametrize("o,v", [(1, 17), (2, 130), (3, 65), (8, 18), (9, 33), (13, 7), (17, 20), (33, 5)])
+@pytest.mark.parametrize("tile_n", [0, 128, 256])
+def test_mixed_contraction_tiles(o, v, tile_n):
+    inp = make_inputs(o, v, 40, seed=o, fvo_sigma=1e-3)
+    ins = [getattr(inp, k) for k in G.KEYS]
+    e0, g0 = triples.energy_vjp(*ins, precision="fp64", device="cuda")
+    e, g = triples.energy_vjp(*ins, precision="mixed", device="cuda", tile_n=tile_n)
+    scale = 1e-14 if o == 1 else 0.0   # one occupied orbital has no triples: both are rounding noise
+    assert abs(float(e) - float(e0)) <= 1e-6 * abs(float(e0)) + scale
+    if o > 1:
+        for k in G.KEYS:
+            assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-5, k
