@@ -91,6 +91,13 @@ size_t triples_workspace_size(int precision, int nocc, int nvir, int ovvv_packed
 size_t triples_workspace_size_ex(int precision, int nocc, int nvir, int ovvv_packed,
                                  int want_grad, const triples_options *opt);
 
+/* Further bytes with which the same call is faster: small problems then run
+ * several chunks in one launch per kernel (0 where it makes no difference, at
+ * most about 2 GiB).  A workspace of triples_workspace_size_ex() bytes, or of
+ * triples_df_workspace_size() for the DF calls, is always enough. */
+size_t triples_workspace_extra(int precision, int nocc, int nvir, int ovvv_packed, int want_grad,
+                               const triples_options *opt);
+
 /* E(T) into *e_out (device FP64 scalar).
  * Replaces the forward of pyscfad/cc/ccsd_t.py:37-42 (pyscf's ccsd_t.kernel). */
 int triples_energy(void *stream, int precision, int nocc, int nvir, int ovvv_packed,

@@ -75,6 +75,8 @@ def load():
     lib.triples_energy_vjp_ex.restype = _c_int
     lib.triples_energy_vjp_ex.argtypes = ([_vp, _c_int, _c_int, _c_int, _c_int] + [_vp] * 7 +
                                           [_c_double, _c_int, _opt, _vp, _c_size, _vp] + [_vp] * 7)
+    lib.triples_workspace_extra.restype = _c_size
+    lib.triples_workspace_extra.argtypes = [_c_int] * 5 + [_opt]
     lib.triples_lno_workspace_size_ex.restype = _c_size
     lib.triples_lno_workspace_size_ex.argtypes = [_c_int] * 5 + [_opt]
     lib.triples_lno_energy_vjp_ex.restype = _c_int

@@ -165,4 +165,52 @@ __host__ __device__ inline long long f2m_stage_offset(const PermBlock &pb, int o
     return R.base + (long long)r * R.rs + R.at(z);
 }
 
+// The jobs of one launch: chunks of one problem by value (Group), or chunks of
+// many problems in device memory (Table).  Work units (tiles, items) are
+// numbered job after job: job j has [start[j], start[j + 1]).  Group<T, 1> is
+// the single-chunk kernel, its parameters compile-time constant addresses.
+constexpr int kMaxGroup = 8;
+
+template <typename T, int N>
+struct Group {
+    static constexpr bool kOne = N == 1;
+    int n;
+    int start[N + 1];
+    T job[N];
+};
+
+template <typename T>
+struct Table {
+    static constexpr bool kOne = false;
+    int n;
+    const int *start;
+    const T *job;
+};
+
+// Job of unit t, for a caller whose t only grows: a binary search once, then
+// the index moves forward.
+struct JobCursor {
+    int j = -1;
+    template <typename JOBS>
+    __device__ __forceinline__ int at(const JOBS &J, int t, int &local) {
+        if constexpr (JOBS::kOne) {
+            local = t;
+            return 0;
+        } else {
+            if (j < 0) {
+                int lo = 0, hi = J.n - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (J.start[mid] <= t) lo = mid;
+                    else hi = mid - 1;
+                }
+                j = lo;
+            }
+            while (j + 1 < J.n && J.start[j + 1] <= t) j++;
+            local = t - J.start[j];
+            return j;
+        }
+    }
+};
+
 }  // namespace tb

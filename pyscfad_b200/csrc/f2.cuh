@@ -220,14 +220,19 @@ __device__ __forceinline__ T group_reduce_scatter(T (&v)[NV], int lane) {
     return r;
 }
 
-__global__ void __launch_bounds__(kF2Threads, 4) k_f2t(const __grid_constant__ F2P P) {
+// One CTA per item of the jobs (chunks) of a launch.
+template <typename JOBS>
+__global__ void __launch_bounds__(kF2Threads, 4) k_f2t(const __grid_constant__ JOBS J) {
     using StageT = double;
     using C = F2Smem;
     constexpr int SB = C::SB, NT = kF2Threads;
     constexpr int REG = C::REG, NV = C::NV, NVP = C::NVP;
     constexpr int SX = C::SX, SY = C::SY;
     constexpr int NW = NT / 32, IPT = C::ITEMS / NT;
-    const int blk = (int)blockIdx.x;
+    JobCursor jcur;
+    int blk;
+    const int jb = jcur.at(J, (int)blockIdx.x, blk);
+    const F2P &P = J.job[JOBS::kOne ? 0 : jb];
     extern __shared__ __align__(16) uint8_t f2_smem[];
     StageT *sW = reinterpret_cast<StageT *>(f2_smem);
     StageT *sG = sW;                      // item results [12][REG] (padded) once W is consumed
@@ -628,12 +633,6 @@ __device__ __forceinline__ void energy_sum_body(const double *__restrict__ e_par
         __syncthreads();
     }
     if (threadIdx.x == 0) *e_acc += s[0];
-}
-
-// ticket (if any): the epilogue's item counter, back to zero for the next launch
-__global__ void k_f2_energy_sum(const double *__restrict__ e_part, int n, double *e_acc, unsigned *ticket) {
-    energy_sum_body(e_part, n, e_acc);
-    if (threadIdx.x == 0 && ticket) *ticket = 0u;
 }
 
 }  // namespace tb

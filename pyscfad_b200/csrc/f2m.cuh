@@ -191,13 +191,11 @@ __device__ __forceinline__ void f2m_bar(int id) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kF2mThreads) : "memory");
 }
 
-// BATCH = false: the items of one chunk (parameters P0).  BATCH = true: those
-// of njobs chunks numbered job after job (job_start[j] = first item of job j),
-// parameters in device memory.
-template <int H, bool BATCH>
-__global__ void __launch_bounds__(kF2mThreads, 2)
-    k_f2m(const __grid_constant__ F2M P0, const F2M *__restrict__ jobs, const int *__restrict__ job_start, int njobs,
-          int nitems) {
+// The items of the jobs (chunks) of a launch.
+template <int H, typename JOBS>
+__global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ JOBS J) {
+    constexpr bool ONE = JOBS::kOne;
+    const int nitems = J.start[J.n];
     using C = F2mSmem;
     extern __shared__ uint8_t f2m_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)f2m_raw + 127) & ~(uintptr_t)127);
@@ -214,7 +212,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2)
     __shared__ int s_abort, s_next[2];             // next item of the CTA, by parity of the current one
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned *ticket = (BATCH ? jobs[0] : P0).ticket;
+    unsigned *ticket = J.job[0].ticket;
     if (tid == 0) {
         s_abort = 0;
         s_next[0] = (int)(gridDim.x + atomicAdd(ticket, 1u));
@@ -241,19 +239,13 @@ __global__ void __launch_bounds__(kF2mThreads, 2)
     struct Item {
         int w, job, sub, rep, i0, i1, i2;
     };
-    int jcur = -1;
+    JobCursor jcur;
     auto item_at = [&](int w) -> Item {
         Item I;
+        int lw;
         I.w = w;
-        I.job = 0;
-        int lw = w;
-        if constexpr (BATCH) {
-            if (jcur < 0) jcur = job_of(job_start, njobs, w);
-            while (jcur + 1 < njobs && job_start[jcur + 1] <= w) jcur++;
-            lw = w - job_start[jcur];
-            I.job = jcur;
-        }
-        const F2M &P = BATCH ? jobs[I.job] : P0;
+        I.job = jcur.at(J, w, lw);
+        const F2M &P = J.job[ONE ? 0 : I.job];
         I.rep = lw / P.nsub;
         I.sub = lw - I.rep * P.nsub;
         I.i0 = P.ijk[3 * I.rep];
@@ -266,13 +258,13 @@ __global__ void __launch_bounds__(kF2mThreads, 2)
     auto wait = [&](uint64_t *bar, uint32_t parity) {
         if (!mbar_wait(bar, parity, abortp)) {
             *abortp = 1;
-            atomicOr((BATCH ? jobs[0] : P0).err, 64);
+            atomicOr(J.job[0].err, 64);
         }
     };
     // ---- the loads, each issued by one warp ----
     // V-term tables and energies of an item into table buffer b (its previous item is done)
     auto issue_tables = [&](const Item &I, int b) {
-        const F2M &P = BATCH ? jobs[I.job] : P0;
+        const F2M &P = J.job[ONE ? 0 : I.job];
         const F2mSub &R = P.sub[I.sub];
         const int o = P.o, v = P.v;
         if (lane < 27) {
@@ -336,7 +328,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2)
     };
     // W stage n of the CTA: the regions of (item, rho); every warp has read the stage's previous content
     auto issue_stage = [&](const Item &I, int rho, int n) {
-        const F2M &P = BATCH ? jobs[I.job] : P0;
+        const F2M &P = J.job[ONE ? 0 : I.job];
         const F2mSub &R = P.sub[I.sub];
         const int st = n & (kF2mStages - 1);
         int pr[3];
@@ -393,7 +385,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2)
     }
 #pragma unroll 1
     for (int k = 0;; k++) {
-        const F2M &P = BATCH ? jobs[cur.job] : P0;
+        const F2M &P = J.job[ONE ? 0 : cur.job];
         const int o = P.o, v = P.v;
         const int sub = cur.sub, rep = cur.rep, i0 = cur.i0, i1 = cur.i1, i2 = cur.i2;
         const float wscf = P.want_grad ? (float)*P.wscale : 1.0f;

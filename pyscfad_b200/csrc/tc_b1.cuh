@@ -68,33 +68,13 @@ struct TcB1Cfg {
     static_assert(NACC * BN <= 512, "TMEM holds 512 columns");
 };
 
-// BATCH = false: one chunk (parameters P0).  BATCH = true: the tiles of njobs
-// chunks (of different problems, one kind) numbered job after job
-// (job_start[j] = first tile of job j, job_start[njobs] = total), parameters
-// in device memory.
-template <bool A_MN, int BN, bool BATCH>
-__global__ void __launch_bounds__(kB1Threads, 1)
-    k_b1_tc(const __grid_constant__ TcB1Params P0, const TcB1Params *__restrict__ jobs,
-            const int *__restrict__ job_start, int njobs) {
+// The tiles of the jobs (chunks, one kind) of a launch.
+template <bool A_MN, int BN, typename JOBS>
+__global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__ JOBS J) {
     using C = TcB1Cfg<A_MN, BN>;
-    // job of global tile t (BATCH) and the tile's index within it (each role
-    // walks its tiles in increasing order: after the first binary search the
-    // job index only moves forward); parameters are bound with
-    // BATCH ? jobs[j] : P0, the __grid_constant__ parameter in the
-    // single-chunk kernel
-    int jcur = -1;
-    auto job_tile = [&](int t, int &lt) -> int {
-        if constexpr (BATCH) {
-            if (jcur < 0) jcur = job_of(job_start, njobs, t);
-            while (jcur + 1 < njobs && job_start[jcur + 1] <= t) jcur++;
-            lt = t - job_start[jcur];
-            return jcur;
-        } else {
-            lt = t;
-            return 0;
-        }
-    };
-    const TcB1Params &Pfirst = BATCH ? jobs[0] : P0;
+    constexpr bool ONE = JOBS::kOne;
+    JobCursor jcur;
+    const TcB1Params &Pfirst = J.job[0];
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = (uint64_t *)(smem + C::STAGES * C::STAGE_BYTES);
@@ -119,10 +99,10 @@ __global__ void __launch_bounds__(kB1Threads, 1)
         mbar_init(drain, 1);
         fence_mbar_init();
     }
-    if (!BATCH && warp == 0 && lane == 0) {
-        for (int t = 0; t < P0.nperm; t++) {
-            tma_prefetch_desc(&P0.tmA[t]);
-            tma_prefetch_desc(&P0.tmB[t]);
+    if (ONE && warp == 0 && lane == 0) {
+        for (int t = 0; t < Pfirst.nperm; t++) {
+            tma_prefetch_desc(&Pfirst.tmA[t]);
+            tma_prefetch_desc(&Pfirst.tmB[t]);
         }
     }
     if (warp == 1) {
@@ -134,7 +114,7 @@ __global__ void __launch_bounds__(kB1Threads, 1)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     volatile int *abortp = &s_abort;
-    const int total = BATCH ? job_start[njobs] : P0.cum[P0.nperm];
+    const int total = J.start[J.n];
     // columns an MMA of N tile nt covers
     auto width = [&](const TcB1Params &P, int nt) -> int {
         const int left = P.ncol - nt * P.nw;
@@ -162,8 +142,8 @@ __global__ void __launch_bounds__(kB1Threads, 1)
         bool ok = true;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
             int lt;
-            const int jb = job_tile(t, lt);
-            const TcB1Params &P = BATCH ? jobs[jb] : P0;
+            const int jb = jcur.at(J, t, lt);
+            const TcB1Params &P = J.job[ONE ? 0 : jb];
             int tau, b, mt, nt;
             decode(P, lt, tau, b, mt, nt);
             const PermBlock &pb = P.pb[tau];
@@ -230,8 +210,8 @@ __global__ void __launch_bounds__(kB1Threads, 1)
         bool ok = true;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
             int lt;
-            const int jb = job_tile(t, lt);
-            const TcB1Params &P = BATCH ? jobs[jb] : P0;
+            const int jb = jcur.at(J, t, lt);
+            const TcB1Params &P = J.job[ONE ? 0 : jb];
             int tau, b, mt, nt;
             decode(P, lt, tau, b, mt, nt);
             const uint32_t idesc = make_idesc_f16(kTcBM, width(P, nt), P.bf16 != 0, A_MN, true);
@@ -302,20 +282,20 @@ __global__ void __launch_bounds__(kB1Threads, 1)
         const int quarter = warp & 3;         // TMEM lane quarter this warp may access
         const int half = (warp - 2) >> 2;     // which of the column groups
         const int row = quarter * 32 + lane;
-        const double sc0 = BATCH ? 0.0 : P0.sign / ((*P0.wscale) * (*P0.oscale));   // single chunk: read once
+        const double sc0 = ONE ? Pfirst.sign / ((*Pfirst.wscale) * (*Pfirst.oscale)) : 0.0;   // single chunk: read once
         int seg = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
             int lt;
-            const int jb = job_tile(t, lt);
-            const TcB1Params &P = BATCH ? jobs[jb] : P0;
+            const int jb = jcur.at(J, t, lt);
+            const TcB1Params &P = J.job[ONE ? 0 : jb];
             const int o = P.d.o, v = P.d.v, Kp = P.d.Kp;
             int tau, b, mt, nt;
             decode(P, lt, tau, b, mt, nt);
             const PermBlock &pb = P.pb[tau];
             const int Tz = pb.Tz;
             const int nk = P.nk_outer[tau] * P.nk_inner[tau];
-            const double sc = BATCH ? P.sign / ((*P.wscale) * (*P.oscale)) : sc0;
+            const double sc = ONE ? sc0 : P.sign / ((*P.wscale) * (*P.oscale));
             long long roff = -1;
             if (P.kind == 0 || P.kind == 2) {
                 const int p = mt * 8 + row / 16, x = row % 16;

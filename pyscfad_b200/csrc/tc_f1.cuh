@@ -83,51 +83,21 @@ struct F1Maps {
     CUtensorMap a1, b1, a2, b2;
 };
 
-// One problem's chunk in a batched launch: its maps and parameters, in device
-// memory (written before the launch, 64-byte aligned).
+// One chunk: its operand maps and parameters (64-byte aligned maps).
 struct alignas(64) F1Job {
     F1Maps m;
     TcF1Params P;
 };
 
-// Index j of the job that holds global work index t: start[j] <= t < start[j+1].
-__device__ __forceinline__ int job_of(const int *__restrict__ start, int njobs, int t) {
-    int lo = 0, hi = njobs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (start[mid] <= t) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// BATCH = false: one chunk (maps M0, parameters P0).  BATCH = true: the tiles
-// of njobs chunks (of different problems) numbered job after job
-// (job_start[j] = first tile of job j, job_start[njobs] = total); every tile
-// reads its job's maps and parameters.
-template <int BN, bool BATCH>
-__global__ void __launch_bounds__(kF1Threads, 1)
-    k_f1_tc(const __grid_constant__ F1Maps M0, const __grid_constant__ TcF1Params P0,
-            const F1Job *__restrict__ jobs, const int *__restrict__ job_start, int njobs) {
+// The tiles of the jobs of a launch.
+template <int BN, typename JOBS>
+__global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__ JOBS J) {
     using C = TcCfg<BN>;
-    // job of global tile t (BATCH) and the tile's index within it
-    // (each role walks its tiles in increasing order: after the first binary
-    // search the job index only moves forward)
-    int jcur = -1;
-    auto job_tile = [&](int t, int &lt) -> int {
-        if constexpr (BATCH) {
-            if (jcur < 0) jcur = job_of(job_start, njobs, t);
-            while (jcur + 1 < njobs && job_start[jcur + 1] <= t) jcur++;
-            lt = t - job_start[jcur];
-            return jcur;
-        } else {
-            lt = t;
-            return 0;
-        }
-    };
-    // the parameters themselves are bound with BATCH ? jobs[j].X : X0, which
-    // folds to the __grid_constant__ parameter in the single-chunk kernel
-    const TcF1Params &Pfirst = BATCH ? jobs[0].P : P0;
+    constexpr bool ONE = JOBS::kOne;
+    JobCursor jcur;
+    // parameters are bound with J.job[ONE ? 0 : j], which folds to the
+    // __grid_constant__ parameter in the single-chunk kernel
+    const TcF1Params &Pfirst = J.job[0].P;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     float *sstore = (float *)(smem + C::STAGES * C::STAGE_BYTES);   // 1024-byte aligned boxes
@@ -153,11 +123,11 @@ __global__ void __launch_bounds__(kF1Threads, 1)
         mbar_init(drain, 1);
         fence_mbar_init();
     }
-    if (!BATCH && warp == 0 && lane == 0) {
-        tma_prefetch_desc(&M0.a1);
-        tma_prefetch_desc(&M0.b1);
-        tma_prefetch_desc(&M0.a2);
-        tma_prefetch_desc(&M0.b2);
+    if (ONE && warp == 0 && lane == 0) {
+        tma_prefetch_desc(&J.job[0].m.a1);
+        tma_prefetch_desc(&J.job[0].m.b1);
+        tma_prefetch_desc(&J.job[0].m.a2);
+        tma_prefetch_desc(&J.job[0].m.b2);
     }
     if (warp == 1) {
         tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -168,7 +138,7 @@ __global__ void __launch_bounds__(kF1Threads, 1)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     volatile int *abortp = &s_abort;
-    const int total = BATCH ? job_start[njobs] : P0.cum[P0.ch.nperm];
+    const int total = J.start[J.n];
 
     if (warp == 0 && lane == 0) {
         // ---------------- TMA producer ----------------
@@ -180,9 +150,9 @@ __global__ void __launch_bounds__(kF1Threads, 1)
         bool ok = true;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
             int lt;
-            const int jb = job_tile(t, lt);
-            const TcF1Params &P = BATCH ? jobs[jb].P : P0;
-            const F1Maps &M = BATCH ? jobs[jb].m : M0;
+            const int jb = jcur.at(J, t, lt);
+            const TcF1Params &P = J.job[ONE ? 0 : jb].P;
+            const F1Maps &M = J.job[ONE ? 0 : jb].m;
             const F1Tile T = f1_decode(P, lt);
             const PermBlock &pb = P.ch.pb[T.tau];
             const int yg = pb.Y0 + T.y;
@@ -237,8 +207,8 @@ __global__ void __launch_bounds__(kF1Threads, 1)
         bool ok = true;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
             int lt;
-            const int jb = job_tile(t, lt);
-            const TcF1Params &P = BATCH ? jobs[jb].P : P0;
+            const int jb = jcur.at(J, t, lt);
+            const TcF1Params &P = J.job[ONE ? 0 : jb].P;
             const uint32_t idesc = make_idesc_f16(kTcBM, 16 * P.rt, P.bf16 != 0, false, false);
             const int nkb = P.nkb1 + P.nkb2;
             for (int k0 = 0; k0 < nkb && ok; k0 += P.kseg, seg++) {
@@ -301,16 +271,16 @@ __global__ void __launch_bounds__(kF1Threads, 1)
         const int row = quarter * 32 + lane;
         float wmax = 0.f;
         unsigned *wmax_dst = Pfirst.wmax_bits;   // running max |W| goes to the tile's problem
-        const float sc0 = BATCH ? 0.f : *P0.out_scale;   // single chunk: read once
+        const float sc0 = ONE ? *Pfirst.out_scale : 0.f;   // single chunk: read once
         int seg = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
             int lt;
-            const int jb = job_tile(t, lt);
-            const TcF1Params &P = BATCH ? jobs[jb].P : P0;
+            const int jb = jcur.at(J, t, lt);
+            const TcF1Params &P = J.job[ONE ? 0 : jb].P;
             const int o = P.d.o;
             const int nkb = P.nkb1 + P.nkb2;
-            if (BATCH && P.wmax_bits != wmax_dst) {
+            if (!ONE && P.wmax_bits != wmax_dst) {
                 for (int off = 16; off > 0; off >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, off));
                 if (lane == 0 && wmax > 0.f) atomicMax(wmax_dst, __float_as_uint(wmax));
                 wmax = 0.f;
@@ -344,7 +314,7 @@ __global__ void __launch_bounds__(kF1Threads, 1)
                 if (lane == 0) mbar_arrive(&tempty[acc]);
             }
             if (!ok) break;
-            const float sc = BATCH ? *P.out_scale : sc0;
+            const float sc = ONE ? sc0 : *P.out_scale;
             const F1Tile T = f1_decode(P, lt);
             const PermBlock &pb = P.ch.pb[T.tau];
             const int p = T.mt * 8 + row / 16;

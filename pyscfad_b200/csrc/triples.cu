@@ -4,6 +4,7 @@
 // Reference path replaced: pyscfad/cc/ccsd_t.py:28-192 (forward through
 // pyscf's ccsd_t.kernel, backward through ccsd_t_energy_vjp,
 // pyscfadlib/pyscfadlib/vjp/cc/ccsd_t_vjp.c:332-497).
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -151,8 +152,8 @@ static long long chunk_stage_elems(const ChunkDesc &ch, const Dims &d) {
     return s;
 }
 
-int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, int lno,
-              const triples_options *opt, bool vtables) {
+static int plan_once(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, int lno,
+                     const triples_options *opt, bool vtables, int most_group) {
     if (nocc < 1 || nvir < 1 || nocc > kMaxCols || nvir > 32767) return TRIPLES_ERR_INVALID_ARGUMENT;
     if (precision < TRIPLES_PRECISION_FP64 || precision > TRIPLES_PRECISION_MIXED_BF16)
         return TRIPLES_ERR_INVALID_ARGUMENT;
@@ -213,6 +214,8 @@ int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan
             }
     P.stage_elems = (size_t)maxst;
     P.wbar_elems = (size_t)maxwb;
+    P.stage_slot = (P.stage_elems + 63) / 64 * 64;   // slots start 256-byte aligned
+    P.wbar_slot = (P.wbar_elems + 63) / 64 * 64;
     P.max_items = maxitems;
     P.f2_gy = kMaxSub;
     const bool mixed = precision != TRIPLES_PRECISION_FP64;
@@ -239,9 +242,19 @@ int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan
         P.off_A2h = take(2 * o * o * v * P.Op8 * 2);
         P.off_B2h = take(2 * v * o * v * P.Op8 * 2);
     }
-    P.off_S = take(P.stage_elems * P.stage_bytes);
+    // Chunk slots: the chunks of a group run in one launch per kernel, as many
+    // as kGroupBytes hold.
+    P.group = 1;
+    if (!lno && most_group > 1) {
+        const size_t chunk = P.stage_slot * P.stage_bytes + (want_grad ? P.wbar_slot * (mixed ? 4 : 8) : 0);
+        long long nchunk = 0;
+        for (int A = P.a0; A < P.nb && (P.a1 <= 0 || A < P.a1); A++) nchunk += (long long)(A + 1) * (A + 2) / 2;
+        const long long fit = (long long)(kGroupBytes / chunk);
+        P.group = (int)std::max(1LL, std::min(std::min(fit, nchunk), (long long)most_group));
+    }
+    P.off_S = take(((P.group - 1) * P.stage_slot + P.stage_elems) * P.stage_bytes);
     if (want_grad) {
-        P.off_SW = take(P.wbar_elems * (mixed ? 4 : 8));
+        P.off_SW = take(((P.group - 1) * P.wbar_slot + P.wbar_elems) * (mixed ? 4 : 8));
         P.off_GA1 = take(v * o * v * Kp * el);
         P.off_GB1 = take(o * o * v * Kp * el);
         P.off_GA2 = take(o * o * v * o * el);
@@ -255,7 +268,7 @@ int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan
         P.off_tf = take(o * nb8 * 8 * sizeof(float2));
     }
     P.off_ijk = take((size_t)P.n_ijk * 3 * sizeof(int));
-    P.off_epart = take((size_t)P.n_ijk * P.f2_gy * el);
+    P.off_epart = take((size_t)P.group * P.n_ijk * P.f2_gy * el);
     if (P.lno) {
         // whole-chunk FP64 arrays: WW / P^T(Wtbar) / vbar (0), Pt(Q) (1), Q / Dbar (2),
         // Zbar (3); the energy alone needs only 0 and 2
@@ -272,6 +285,32 @@ int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan
     }
     P.total = off;
     return TRIPLES_OK;
+}
+
+// vtables: with the V-term tables, which only make a call faster (a problem
+// that fits the fixed scratch without them goes without them when it would not
+// fit it with them); most_group: chunk slots at most.
+int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, int lno,
+              const triples_options *opt, bool vtables, int most_group) {
+    const int rc = plan_once(precision, nocc, nvir, packed, want_grad, P, lno, opt, vtables, most_group);
+    if (rc != TRIPLES_OK || !P.vtables || P.total <= TRIPLES_STATIC_SCRATCH_BYTES) return rc;
+    Plan B;
+    plan_once(precision, nocc, nvir, packed, want_grad, B, lno, opt, false, 1);
+    if (B.total > TRIPLES_STATIC_SCRATCH_BYTES) return rc;
+    return plan_once(precision, nocc, nvir, packed, want_grad, P, lno, opt, false, most_group);
+}
+
+// The plan with the most chunk slots that fits workspace_bytes; failing one,
+// the plan without V-term tables.
+int make_plan_for(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, const triples_options *opt,
+                  size_t workspace_bytes) {
+    for (int g = kMaxGroup; g >= 1; g--) {
+        const int rc = plan_once(precision, nocc, nvir, packed, want_grad, P, 0, opt, true, g);
+        if (rc != TRIPLES_OK) return rc;
+        if (P.total <= workspace_bytes) return TRIPLES_OK;
+        g = std::min(g, P.group);   // fewer slots than asked for: go on from there
+    }
+    return plan_once(precision, nocc, nvir, packed, want_grad, P, 0, opt, false, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -413,69 +452,70 @@ __global__ void k_make_scales(Ctrl *ctrl, int scaled) {
     ctrl->out_scale = (float)(1.0 / (sA * sB));
 }
 
+// What the small per-chunk kernels need: the virtual ranges for the Wbar scale,
+// the energy partials of the epilogue.
+struct ChunkAux {
+    Ctrl *ctrl;
+    ChunkSlot *slot;
+    const double *mo_e;
+    const double *e_part;
+    double ybar;
+    int o, a0, na, b0, nb, c0, nc, n_part;
+    int scaled, lno;
+};
+
 // Per-chunk power-of-two scale for the split Wbar, from a bound that needs no
 // pass over Wbar:  |Wbar| <= 2|ybar| (144 max|w| + 36 max|v|) / min|D| over the
 // chunk (|Z| <= 12 max|X|, |X| <= 6 max|w| + 3 max|v|, |R WW| <= 72 max|w|,
-// orbit weight <= 2).  Resets the running max |w| for the next chunk.
-__device__ __forceinline__ void chunk_scale_body(Ctrl *ctrl, const double *__restrict__ mo_e, int o, int a0,
-                                                 int na, int b0, int nb, int c0, int nc, double ybar, int scaled,
-                                                 int lno) {
+// orbit weight <= 2).  Resets the running max |w| for the slot's next chunk.
+// One 32-thread block per chunk.
+template <typename JOBS>
+__global__ void k_chunk_scale(const __grid_constant__ JOBS J) {
+    const ChunkAux &A = J.job[JOBS::kOne ? 0 : blockIdx.x];
+    const Ctrl *ctrl = A.ctrl;
+    const int o = A.o;
     __shared__ double s_min[3], s_maxo;
     const double inf = 1e300;
     if (threadIdx.x < 4) {
         double m = (threadIdx.x < 3) ? inf : -inf;
-        const int st = threadIdx.x == 0 ? a0 : (threadIdx.x == 1 ? b0 : c0);
-        const int n = threadIdx.x == 0 ? na : (threadIdx.x == 1 ? nb : nc);
+        const int st = threadIdx.x == 0 ? A.a0 : (threadIdx.x == 1 ? A.b0 : A.c0);
+        const int n = threadIdx.x == 0 ? A.na : (threadIdx.x == 1 ? A.nb : A.nc);
         if (threadIdx.x < 3) {
-            for (int t = 0; t < n; t++) m = fmin(m, mo_e[o + st + t]);
+            for (int t = 0; t < n; t++) m = fmin(m, A.mo_e[o + st + t]);
             s_min[threadIdx.x] = m;
         } else {
-            for (int t = 0; t < o; t++) m = fmax(m, mo_e[t]);
+            for (int t = 0; t < o; t++) m = fmax(m, A.mo_e[t]);
             s_maxo = m;
         }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         const double dmin = s_min[0] + s_min[1] + s_min[2] - 3.0 * s_maxo;
-        const double mw = (double)__uint_as_float(ctrl->wmax_bits);
+        const double mw = (double)__uint_as_float(A.slot->wmax_bits);
         const double mv = __longlong_as_double((long long)ctrl->absmax[3]) * __longlong_as_double((long long)ctrl->absmax[4]) +
                           __longlong_as_double((long long)ctrl->absmax[2]) * __longlong_as_double((long long)ctrl->absmax[5]);
         // |wbar| <= 6 |WWbar|; with the LNO projector (row / column abs sums nr, nc)
         // WWbar = P^T(ybar Q / 3) + r3^T(ybar P(WW) / (3 D)), |Q| <= 12 (6 mw + 3 mv) / dmin;
         // nr = nc = 1 is the canonical bound
-        const double nr = lno ? ctrl->lno_norm[0] : 1.0, ncl = lno ? ctrl->lno_norm[1] : 1.0;
-        double bound = 2.0 * fabs(ybar) * (72.0 * (nr + ncl) * mw + 36.0 * nr * mv) / (dmin > 1e-300 ? dmin : 1e-300);
-        ctrl->wscale = scaled ? pow2_scale(bound) : 1.0;
-        ctrl->wmax_bits = 0u;
+        const double nr = A.lno ? ctrl->lno_norm[0] : 1.0, ncl = A.lno ? ctrl->lno_norm[1] : 1.0;
+        double bound = 2.0 * fabs(A.ybar) * (72.0 * (nr + ncl) * mw + 36.0 * nr * mv) / (dmin > 1e-300 ? dmin : 1e-300);
+        A.slot->wscale = A.scaled ? pow2_scale(bound) : 1.0;
+        A.slot->wmax_bits = 0u;
     }
 }
 
-__global__ void k_chunk_scale(Ctrl *ctrl, const double *__restrict__ mo_e, int o, int a0, int na, int b0,
-                              int nb, int c0, int nc, double ybar, int scaled, int lno) {
-    chunk_scale_body(ctrl, mo_e, o, a0, na, b0, nb, c0, nc, ybar, scaled, lno);
-}
-
-// Per problem of a batched chunk step: the chunk's virtual ranges for the
-// Wbar scale, and the energy partials of its epilogue.
-struct ChunkAux {
-    Ctrl *ctrl;
-    const double *mo_e;
-    const double *e_part;
-    double ybar;
-    int o, a0, na, b0, nb, c0, nc, n_part;
-};
-
-// one 32-thread block per problem
-__global__ void k_chunk_scale_batch(const ChunkAux *__restrict__ aux, int scaled) {
-    const ChunkAux &A = aux[blockIdx.x];
-    chunk_scale_body(A.ctrl, A.mo_e, A.o, A.a0, A.na, A.b0, A.nb, A.c0, A.nc, A.ybar, scaled, 0);
-}
-
-// one 256-thread block per problem: the chunk's energy partials, fixed order
-__global__ void k_energy_sum_batch(const ChunkAux *__restrict__ aux) {
-    const ChunkAux &A = aux[blockIdx.x];
-    energy_sum_body(A.e_part, A.n_part, &A.ctrl->e_acc);
-    if (threadIdx.x == 0) A.ctrl->ticket = 0u;   // for the next step's epilogue
+// The chunks' energy partials, each in a fixed order; the epilogue's item
+// counter goes back to zero for its next launch.  Chunks of one problem (a
+// Group) are added by one block, chunk after chunk; those of a Table belong to
+// different problems, one block each.
+template <typename JOBS>
+__global__ void k_energy_sum(const __grid_constant__ JOBS J, int per_block) {
+    for (int c = blockIdx.x * per_block; c < (int)(blockIdx.x + 1) * per_block; c++) {
+        const ChunkAux &A = J.job[JOBS::kOne ? 0 : c];
+        energy_sum_body(A.e_part, A.n_part, &A.ctrl->e_acc);
+        if (threadIdx.x == 0) A.slot->ticket = 0u;
+        __syncthreads();
+    }
 }
 
 template <typename H>
@@ -613,12 +653,15 @@ __global__ void k_prep_B2h(const double *__restrict__ t2, Dims d, int Op8, const
 // ---------------------------------------------------------------------------
 struct GemmLaunch {
     Dims d;
-    ChunkDesc ch;
-    int cum[7];      // prefix sums over orderings of the GEMM problems (blockIdx.z)
-    int nmt, nslice; // M tiles and K slices of blockIdx.x
+    int n;                       // chunks
+    ChunkDesc ch[kMaxGroup];
+    double *S[kMaxGroup];        // staging (F1)
+    double *SW[kMaxGroup];       // Wbar (adjoint kinds)
+    int zstart[kMaxGroup + 1];   // GEMM problems (blockIdx.z) chunk after chunk,
+    int cum[kMaxGroup][7];       // and within a chunk ordering after ordering
+    int nmt, nslice;             // M tiles and K slices of blockIdx.x
     const double *A1, *B1, *A2, *B2;
-    double *S;       // staging, or Wbar
-    double *G;       // gradient target
+    double *G;                   // gradient target
 };
 
 // The five contractions of a chunk.  F1: S_tau[p][q][y][x][r][z] = W for all
@@ -633,19 +676,17 @@ enum GemmKind { GK_F1 = 0, GK_B1A, GK_B1B, GK_B1C, GK_B1D };
 __host__ __device__ constexpr bool gemm_kfa(int kind) { return kind == GK_F1 || kind == GK_B1A || kind == GK_B1C; }
 __host__ __device__ constexpr bool gemm_kfb(int kind) { return kind == GK_F1; }
 
-__device__ __forceinline__ int find_tau(const GemmLaunch &L, int b) {
-    int t = 0;
-    while (t + 1 < L.ch.nperm && b >= L.cum[t + 1]) t++;
-    return t;
-}
-
 template <int KIND, int BM, int BN>
 __global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant__ GemmLaunch L) {
     extern __shared__ __align__(16) double gemm_smem[];
-    const int t = find_tau(L, blockIdx.z);
-    const PermBlock &pb = L.ch.pb[t];
+    int c = 0, t = 0;
+    while (c + 1 < L.n && (int)blockIdx.z >= L.zstart[c + 1]) c++;
+    const int b = (int)blockIdx.z - L.zstart[c];
+    while (t + 1 < L.ch[c].nperm && b >= L.cum[c][t + 1]) t++;
+    const PermBlock &pb = L.ch[c].pb[t];
     const Dims &d = L.d;
-    const int o = d.o, v = d.v, Kp = d.Kp, rem = blockIdx.z - L.cum[t];
+    const int o = d.o, v = d.v, Kp = d.Kp, rem = b - L.cum[c][t];
+    const double *SW = L.SW[c];
     const long long oTz = (long long)o * pb.Tz;
     // Wbar strides
     const long long s_q = pb.rzp, s_x = (long long)o * pb.rzp, s_p = (long long)pb.Tx * s_x, s_y = (long long)o * s_p;
@@ -667,7 +708,7 @@ __global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant_
         g.B = GOp{L.B1 + q * ovK + (long long)pb.Z0 * Kp, map2(pb.Tz, Kp, vK), map1(1)};
         g.A2 = GOp{L.A2 + q * ovo + (long long)pb.X0 * o, map2(pb.Tx, o, vo), map1(1)};
         g.B2 = GOp{L.B2 + yg * ovo + (long long)pb.Z0 * o, map2(pb.Tz, o, vo), map1(1)};
-        g.C = L.S + pb.soff + ((long long)q * pb.Ty + y) * pb.Tx * oTz;
+        g.C = L.S[c] + pb.soff + ((long long)q * pb.Ty + y) * pb.Tx * oTz;
         g.cm = map2(pb.Tx, oTz, (long long)o * pb.Ty * pb.Tx * oTz);
         g.alpha2 = -1.0;
         g.atomic = 0;
@@ -675,7 +716,7 @@ __global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant_
         g.M = o * pb.Tx;
         g.N = v;
         g.K = o * o * pb.Tz;
-        g.A = GOp{L.S + pb.swoff + rem * s_y, map2(pb.Tx, s_x, s_p), map2((int)oTz, 1, s_q)};
+        g.A = GOp{SW + pb.swoff + rem * s_y, map2(pb.Tx, s_x, s_p), map2((int)oTz, 1, s_q)};
         g.B = GOp{L.B1 + (long long)pb.Z0 * Kp, map1(1), map3(pb.Tz, o, Kp, vK, ovK)};
         g.C = L.G + ((long long)pb.Y0 + rem) * ovK + (long long)pb.X0 * Kp;
         g.cm = map2(pb.Tx, Kp, vK);
@@ -683,7 +724,7 @@ __global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant_
         g.M = o * pb.Tz;
         g.N = v;
         g.K = pb.Ty * o * pb.Tx;
-        g.A = GOp{L.S + pb.swoff + rem * s_q, map1(1), map3(pb.Tx, o, s_x, s_p, s_y)};
+        g.A = GOp{SW + pb.swoff + rem * s_q, map1(1), map3(pb.Tx, o, s_x, s_p, s_y)};
         g.B = GOp{L.A1 + (long long)pb.Y0 * ovK + (long long)pb.X0 * Kp, map1(1), map3(pb.Tx, o, Kp, vK, ovK)};
         g.C = L.G + rem * ovK + (long long)pb.Z0 * Kp;
         g.cm = map2(pb.Tz, Kp, vK);
@@ -691,7 +732,7 @@ __global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant_
         g.M = o * pb.Tx;
         g.N = o;
         g.K = pb.Ty * o * pb.Tz;
-        g.A = GOp{L.S + pb.swoff + rem * s_q, map2(pb.Tx, s_x, s_p), map2((int)oTz, 1, s_y)};
+        g.A = GOp{SW + pb.swoff + rem * s_q, map2(pb.Tx, s_x, s_p), map2((int)oTz, 1, s_y)};
         g.B = GOp{L.B2 + (long long)pb.Y0 * ovo + (long long)pb.Z0 * o, map1(1), map3(pb.Tz, o, o, vo, ovo)};
         g.C = L.G + rem * ovo + (long long)pb.X0 * o;
         g.cm = map2(pb.Tx, o, vo);
@@ -700,7 +741,7 @@ __global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant_
         g.M = o * pb.Tz;
         g.N = o;
         g.K = o * o * pb.Tx;
-        g.A = GOp{L.S + pb.swoff + rem * s_y, map1(1), map3(pb.Tx, o, s_x, s_p, s_q)};
+        g.A = GOp{SW + pb.swoff + rem * s_y, map1(1), map3(pb.Tx, o, s_x, s_p, s_q)};
         g.B = GOp{L.A2 + (long long)pb.X0 * o, map1(1), map3(pb.Tx, o, o, vo, ovo)};
         g.C = L.G + ((long long)pb.Y0 + rem) * ovo + (long long)pb.Z0 * o;
         g.cm = map2(pb.Tz, o, vo);
@@ -918,45 +959,48 @@ static int gemm_dispatch(const GemmTile &t, F &&f) {
     return f(integral_constant<int, 128>{}, integral_constant<int, 16>{});
 }
 
+// Shared memory above the default 48 KB needs an opt-in per kernel and device
+// (the attribute call is idempotent and cheap next to a launch).
 template <typename K>
-static int gemm_smem_optin(K kernel, size_t bytes) {
-    // above the default 48 KB a kernel has to opt in, once per device; the
-    // attribute call is idempotent and cheap next to a launch
+static int smem_optin(K kernel, size_t bytes) {
     TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return TRIPLES_OK;
 }
 
-// Largest M, N and K over the orderings; nb: GEMM problems in L.cum.
+// One contraction of the launch's chunks; tiles from the largest M, N and K.
 template <int KIND>
 static int chunk_gemm(cudaStream_t st, int cat, GemmLaunch &L) {
     const long long o = L.d.o, v = L.d.v;
     long long M = 0, N = 0, K = 0;
-    for (int t = 0; t < L.ch.nperm; t++) {
-        const PermBlock &pb = L.ch.pb[t];
-        const long long m = o * (KIND == GK_F1 || KIND == GK_B1A || KIND == GK_B1C ? pb.Tx : pb.Tz);
-        const long long n = KIND == GK_F1 ? o * pb.Tz : (KIND == GK_B1A || KIND == GK_B1B ? v : o);
-        const long long k = KIND == GK_F1 ? v
-                            : KIND == GK_B1A ? o * o * pb.Tz
-                            : KIND == GK_B1B ? o * pb.Ty * pb.Tx
-                            : KIND == GK_B1C ? o * pb.Ty * pb.Tz
-                                             : o * o * pb.Tx;
-        M = m > M ? m : M;
-        N = n > N ? n : N;
-        K = k > K ? k : K;
+    L.zstart[0] = 0;
+    for (int c = 0; c < L.n; c++) {
+        L.cum[c][0] = 0;
+        for (int t = 0; t < L.ch[c].nperm; t++) {
+            const PermBlock &pb = L.ch[c].pb[t];
+            const long long m = o * (KIND == GK_F1 || KIND == GK_B1A || KIND == GK_B1C ? pb.Tx : pb.Tz);
+            const long long n = KIND == GK_F1 ? o * pb.Tz : (KIND == GK_B1A || KIND == GK_B1B ? v : o);
+            const long long k = KIND == GK_F1 ? v
+                                : KIND == GK_B1A ? o * o * pb.Tz
+                                : KIND == GK_B1B ? o * pb.Ty * pb.Tx
+                                : KIND == GK_B1C ? o * pb.Ty * pb.Tz
+                                                 : o * o * pb.Tx;
+            M = std::max(M, m);
+            N = std::max(N, n);
+            K = std::max(K, k);
+            L.cum[c][t + 1] = L.cum[c][t] + (KIND == GK_F1 ? pb.Ty * L.d.o
+                                             : KIND == GK_B1A || KIND == GK_B1D ? pb.Ty : L.d.o);
+        }
+        L.zstart[c + 1] = L.zstart[c] + L.cum[c][L.ch[c].nperm];
     }
-    L.cum[0] = 0;
-    for (int t = 0; t < L.ch.nperm; t++)
-        L.cum[t + 1] = L.cum[t] + (KIND == GK_F1 ? L.ch.pb[t].Ty * L.d.o
-                                   : KIND == GK_B1A || KIND == GK_B1D ? L.ch.pb[t].Ty : L.d.o);
-    const GemmTile tile = gemm_tile(M, N, K, L.cum[L.ch.nperm], KIND != GK_F1);
+    const GemmTile tile = gemm_tile(M, N, K, L.zstart[L.n], KIND != GK_F1);
     return gemm_dispatch(tile, [&](auto bm, auto bn) -> int {
         constexpr int BM = decltype(bm)::value, BN = decltype(bn)::value;
         using C = GemmCfg<BM, BN, gemm_kfa(KIND), gemm_kfb(KIND)>;
-        const int rc = gemm_smem_optin(k_chunk_fp64<KIND, BM, BN>, C::SMEM);
+        const int rc = smem_optin(k_chunk_fp64<KIND, BM, BN>, C::SMEM);
         if (rc != TRIPLES_OK) return rc;
         L.nmt = (int)((M + BM - 1) / BM);
         L.nslice = tile.nslice;
-        const dim3 grid((unsigned)(L.nmt * L.nslice), (unsigned)((N + BN - 1) / BN), (unsigned)L.cum[L.ch.nperm]);
+        const dim3 grid((unsigned)(L.nmt * L.nslice), (unsigned)((N + BN - 1) / BN), (unsigned)L.zstart[L.n]);
         TB_KLAUNCH(cat, (k_chunk_fp64<KIND, BM, BN><<<grid, kGThreads, C::SMEM, st>>>(L)));
         return TRIPLES_OK;
     });
@@ -993,7 +1037,7 @@ static int gemm_plain(cudaStream_t st, int M, int N, int K, const double *A, lon
     using Cfg = GemmCfg<BM, BN, KFA, KFB>;
     const dim3 grid((unsigned)((M + BM - 1) / BM), (unsigned)((N + BN - 1) / BN));
     if (grid.y > 65535) return TRIPLES_ERR_UNSUPPORTED;
-    const int rc = gemm_smem_optin(k_gemm_plain<BM, BN, KFA, KFB>, Cfg::SMEM);
+    const int rc = smem_optin(k_gemm_plain<BM, BN, KFA, KFB>, Cfg::SMEM);
     if (rc != TRIPLES_OK) return rc;
     TB_KLAUNCH(P_PREP, (k_gemm_plain<BM, BN, KFA, KFB><<<grid, kGThreads, Cfg::SMEM, st>>>(g)));
     return TRIPLES_OK;
@@ -1017,6 +1061,24 @@ static int once_per_device(int kind, F &&setup) {
     const int rc = setup();
     if (rc == TRIPLES_OK) g_init_done[dev][kind] = true;
     return rc;
+}
+
+static ChunkAux chunk_aux(const Plan &P, const ChunkDesc &ch, int slot, const TriplesIO &io, int n_part) {
+    char *ws = (char *)io.workspace;
+    ChunkAux A;
+    A.ctrl = (Ctrl *)(ws + P.off_ctrl);
+    A.slot = &A.ctrl->slot[slot];
+    A.mo_e = io.mo_energy;
+    A.e_part = (const double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
+    A.ybar = io.ybar;
+    A.o = P.d.o;
+    A.a0 = ch.base[0]; A.na = ch.nabc[0];
+    A.b0 = ch.base[1]; A.nb = ch.nabc[1];
+    A.c0 = ch.base[2]; A.nc = ch.nabc[2];
+    A.n_part = n_part;
+    A.scaled = P.prec == TRIPLES_PRECISION_MIXED ? 1 : 0;
+    A.lno = P.lno;
+    return A;
 }
 
 // LNO chunk epilogue (FP64): energy of the projected amplitudes and, with
@@ -1083,7 +1145,7 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     A.B3 = (double *)(ws + P.off_L[3]);
     A.mat = io.mat; A.mo_e = io.mo_energy; A.t1 = io.t1; A.t2 = io.t2; A.ovov = io.ovov; A.fvo = io.fvo;
     A.SW = SW;
-    A.wscale = &ctrl->wscale;
+    A.wscale = &ctrl->slot[0].wscale;
     A.mat_bar = io.mat_bar; A.mo_bar = io.mo_energy_bar; A.t1_bar = io.t1_bar; A.t2_bar = io.t2_bar;
     A.ovov_bar = io.ovov_bar; A.fvo_bar = io.fvo_bar;
     A.ybar = io.ybar;
@@ -1106,12 +1168,20 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     const dim3 gproj(clampw((maxcols / d.o + kLnoTile - 1) / kLnoTile), (unsigned)ch.nperm);
     TB_KLAUNCH(P_LNO, k_lno_tile_fwd<StageT><<<gtile, kLnoThreads, lno_tile_smem(), st>>>(A));
     TB_KLAUNCH(P_LNO_PROJ, k_lno_proj<<<gproj, kLnoThreads, lno_proj_smem(d.o), st>>>(A));
-    TB_KLAUNCH(P_PREP, k_f2_energy_sum<<<1, 256, 0, st>>>(A.part, (int)(gproj.x * gproj.y), &ctrl->e_acc, nullptr));
+    {
+        Group<ChunkAux, 1> G;
+        G.n = 1;
+        G.job[0] = chunk_aux(P, ch, 0, io, (int)(gproj.x * gproj.y));
+        G.job[0].e_part = A.part;
+        TB_KLAUNCH(P_PREP, (k_energy_sum<<<1, 256, 0, st>>>(G, 1)));
+    }
     if (!P.want_grad) return TRIPLES_OK;
-    if (split != 0)   // fp16: power-of-two scale of the split Wbar; bf16: scale 1 (both read by the contractions)
-        TB_KLAUNCH(P_PREP, k_chunk_scale<<<1, 32, 0, st>>>(ctrl, io.mo_energy, d.o, ch.base[0], ch.nabc[0], ch.base[1],
-                                                           ch.nabc[1], ch.base[2], ch.nabc[2], io.ybar,
-                                                           split == 1 ? 1 : 0, 1));
+    if (split != 0) {   // fp16: power-of-two scale of the split Wbar; bf16: scale 1 (both read by the contractions)
+        Group<ChunkAux, 1> G;
+        G.n = 1;
+        G.job[0] = chunk_aux(P, ch, 0, io, 0);
+        TB_KLAUNCH(P_PREP, (k_chunk_scale<<<1, 32, 0, st>>>(G)));
+    }
     if (split == 0)
         TB_KLAUNCH(P_LNO_ADJ, k_lno_tile_adj<0><<<gtile, kLnoThreads, lno_tile_smem(), st>>>(A));
     else if (split == 1)
@@ -1141,19 +1211,29 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
 // one-time device set-up and the mixed-precision kernel parameters of a call
 // and of one chunk, shared by the single-problem and the batched drivers
 // ---------------------------------------------------------------------------
+// f(JOBS{}) for each way a launch gets its jobs
+template <typename T, typename F>
+static void for_job_kinds(F &&f) {
+    f(Group<T, 1>{});
+    f(Group<T, kMaxGroup>{});
+    f(Table<T>{});
+}
+
 // once per device and precision: shared-memory opt-ins and the constant tables
 // of the FP64 epilogue's region patterns
 static int setup_epilogue(bool mixed) {
     return once_per_device(mixed ? INIT_F2_F32 : INIT_F2_F64, [&]() -> int {
         if (mixed) {
-            const int bytes = (int)F2mSmem::BYTES;
-            TB_CUDA(cudaFuncSetAttribute(k_f2m<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-            TB_CUDA(cudaFuncSetAttribute(k_f2m<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-            TB_CUDA(cudaFuncSetAttribute(k_f2m<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-            TB_CUDA(cudaFuncSetAttribute(k_f2m<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-            return TRIPLES_OK;
+            int rc = TRIPLES_OK;
+            for_job_kinds<F2M>([&](auto jobs) {
+                using J = decltype(jobs);
+                for (auto k : {k_f2m<1, J>, k_f2m<2, J>})
+                    if (rc == TRIPLES_OK) rc = smem_optin(k, F2mSmem::BYTES);
+            });
+            return rc;
         }
-        TB_CUDA(cudaFuncSetAttribute(k_f2t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f2_smem_bytes()));
+        for (const void *k : {(const void *)k_f2t<Group<F2P, 1>>, (const void *)k_f2t<Group<F2P, kMaxGroup>>})
+            TB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f2_smem_bytes()));
         F2Pattern pats[kF2Patterns];
         f2_build_patterns(pats);
         TB_CUDA(cudaMemcpyToSymbol(c_f2pat, pats, sizeof(pats)));
@@ -1163,27 +1243,23 @@ static int setup_epilogue(bool mixed) {
 
 static int setup_tensor_cores() {
     return once_per_device(INIT_TC, [&]() -> int {
-        TB_CUDA(cudaFuncSetAttribute(k_f1_tc<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_f1_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<128>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_f1_tc<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_f1_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<128>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_b1_tc<false, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcB1Cfg<false, 128>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_b1_tc<false, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcB1Cfg<false, 128>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_b1_tc<true, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcB1Cfg<true, 128>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_b1_tc<true, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcB1Cfg<true, 128>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_b1_tc<false, 64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcB1Cfg<false, 64>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_b1_tc<false, 64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcB1Cfg<false, 64>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_b1_tc<true, 64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcB1Cfg<true, 64>::SMEM));
-        TB_CUDA(cudaFuncSetAttribute(k_b1_tc<true, 64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcB1Cfg<true, 64>::SMEM));
-        return TRIPLES_OK;
+        int rc = TRIPLES_OK;
+        auto opt = [&](auto kernel, size_t bytes) {
+            if (rc == TRIPLES_OK) rc = smem_optin(kernel, bytes);
+        };
+        for_job_kinds<F1Job>([&](auto jobs) {
+            using J = decltype(jobs);
+            opt(k_f1_tc<128, J>, TcCfg<128>::SMEM);
+            opt(k_f1_tc<256, J>, TcCfg<256>::SMEM);
+        });
+        for_job_kinds<TcB1Params>([&](auto jobs) {
+            using J = decltype(jobs);
+            opt(k_b1_tc<false, 128, J>, TcB1Cfg<false, 128>::SMEM);
+            opt(k_b1_tc<true, 128, J>, TcB1Cfg<true, 128>::SMEM);
+            opt(k_b1_tc<false, 64, J>, TcB1Cfg<false, 64>::SMEM);
+            opt(k_b1_tc<true, 64, J>, TcB1Cfg<true, 64>::SMEM);
+        });
+        return rc;
     });
 }
 
@@ -1227,10 +1303,10 @@ static int build_operand_maps(const Plan &P, char *ws, OperandMaps &M) {
 }
 
 // W-contraction parameters of one chunk (tiles ordering by ordering).
-static int f1_params(const Plan &P, const ChunkDesc &ch, char *ws, TcF1Params &T) {
+static int f1_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, TcF1Params &T) {
     const Dims &d = P.d;
     Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
-    float *S = (float *)(ws + P.off_S);
+    float *S = (float *)(ws + P.off_S) + (size_t)slot * P.stage_slot;
     T.d = d;
     T.ch = ch;
     T.mt_count = (d.o + 7) / 8;
@@ -1244,7 +1320,7 @@ static int f1_params(const Plan &P, const ChunkDesc &ch, char *ws, TcF1Params &T
     T.k2 = P.Op8;
     T.S = S;
     T.out_scale = &ctrl->out_scale;
-    T.wmax_bits = &ctrl->wmax_bits;
+    T.wmax_bits = &ctrl->slot[slot].wmax_bits;
     T.err = &ctrl->err;
     T.bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16 ? 1 : 0;
     T.kseg = P.kseg;
@@ -1283,7 +1359,7 @@ static void for_sub_ranges(const ChunkDesc &ch, int sb, F &&f) {
 }
 
 // FP64 epilogue parameters of one chunk.
-static void f2_params(const Plan &P, const ChunkDesc &ch, char *ws, const TriplesIO &io, F2P &F) {
+static void f2_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, const TriplesIO &io, F2P &F) {
     F.d = P.d;
     F.ch = ch;
     F.nsub = 0;
@@ -1296,18 +1372,18 @@ static void f2_params(const Plan &P, const ChunkDesc &ch, char *ws, const Triple
     });
     F.ijk = (int *)(ws + P.off_ijk);
     F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
-    F.S = (const double *)(ws + P.off_S);
-    F.SW = P.want_grad ? (double *)(ws + P.off_SW) : nullptr;
+    F.S = (const double *)(ws + P.off_S) + (size_t)slot * P.stage_slot;
+    F.SW = P.want_grad ? (double *)(ws + P.off_SW) + (size_t)slot * P.wbar_slot : nullptr;
     F.ybar = io.ybar;
     F.want_grad = P.want_grad;
-    F.e_part = (double *)(ws + P.off_epart);
+    F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
     F.n_ijk = P.n_ijk;
     F.mo_bar = io.mo_energy_bar;
     F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
 }
 
 // Mixed-precision epilogue parameters of one chunk.
-static void f2m_params(const Plan &P, const ChunkDesc &ch, char *ws, const TriplesIO &io, bool whole, F2M &F) {
+static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, const TriplesIO &io, bool whole, F2M &F) {
     Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
     const int o = P.d.o;
     F.o = o;
@@ -1356,32 +1432,32 @@ static void f2m_params(const Plan &P, const ChunkDesc &ch, char *ws, const Tripl
     F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
     F.ot = P.vtables ? (const float2 *)(ws + P.off_ot) : nullptr;
     F.tf = P.vtables ? (const float2 *)(ws + P.off_tf) : nullptr;
-    F.S = (const float *)(ws + P.off_S);
-    F.SW = P.want_grad ? (uint16_t *)(ws + P.off_SW) : nullptr;
-    F.wscale = &ctrl->wscale;
+    F.S = (const float *)(ws + P.off_S) + (size_t)slot * P.stage_slot;
+    F.SW = P.want_grad ? (uint16_t *)(ws + P.off_SW) + (size_t)slot * 2 * P.wbar_slot : nullptr;
+    F.wscale = &ctrl->slot[slot].wscale;
     F.ybar = io.ybar;
     F.want_grad = P.want_grad;
-    F.e_part = (double *)(ws + P.off_epart);
+    F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
     F.mo_bar = io.mo_energy_bar;
     F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
     F.err = &ctrl->err;
-    F.ticket = &ctrl->ticket;
+    F.ticket = &ctrl->slot[slot].ticket;
 }
 
 // Adjoint-contraction parameters of one chunk and kind (0: ovvv_bar, 1: t2_bar
 // ovvv term, 2: ovoo_bar, 3: t2_bar ooov term), tiles ordering by ordering.
-static int b1_params(const Plan &P, const ChunkDesc &ch, char *ws, const OperandMaps &M, int kind, TcB1Params &B) {
+static int b1_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, const OperandMaps &M, int kind, TcB1Params &B) {
     const Dims &d = P.d;
     const uint64_t o = d.o;
     const bool bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16;
     Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
-    char *SW = ws + P.off_SW;
+    char *SW = ws + P.off_SW + (size_t)slot * P.wbar_slot * 4;
     const uint32_t bK[5] = {64, 1, 16, 8, 1};   // Wbar K-major (kinds 0, 2)
     const uint32_t bM[5] = {64, 1, 16, 4, 1};   // Wbar MN-major (kinds 1, 3)
     B.d = d;
     B.nperm = ch.nperm;
     for (int t = 0; t < ch.nperm; t++) B.pb[t] = ch.pb[t];
-    B.wscale = &ctrl->wscale;
+    B.wscale = &ctrl->slot[slot].wscale;
     B.err = &ctrl->err;
     B.bf16 = bf16 ? 1 : 0;
     B.kseg = P.kseg;
@@ -1517,7 +1593,7 @@ static int prep_launches(const Plan &P, cudaStream_t st, const TriplesIO &io) {
                 io.ovov, io.t2, io.t1, io.fvo, d.o, d.v, nb8, (float2 *)(ws + P.off_ot), (float2 *)(ws + P.off_tf)));
         }
         TB_LAUNCH_CHECK();
-        if (P.want_grad) TB_CUDA(cudaMemsetAsync(SW, 0, P.wbar_elems * 4, st));
+        if (P.want_grad) TB_CUDA(cudaMemsetAsync(SW, 0, ((P.group - 1) * P.wbar_slot + P.wbar_elems) * 4, st));
     }
     return TRIPLES_OK;
 
@@ -1547,6 +1623,136 @@ static int fold_launches(const Plan &P, cudaStream_t st, const TriplesIO &io) {
     return TRIPLES_OK;
 }
 
+// The work units of a group: start[] from per-job counts.
+template <typename G, typename F>
+static int group_starts(G &g, int n, F &&count) {
+    g.n = n;
+    g.start[0] = 0;
+    for (int j = 0; j < n; j++) g.start[j + 1] = g.start[j] + count(g.job[j]);
+    return g.start[n];
+}
+
+template <typename JOBS>
+static void launch_f1(const Plan &P, cudaStream_t st, int tiles, const JOBS &J) {
+    const int grid = std::min(tiles, num_sms());
+    if (P.f1_bn == 128) k_f1_tc<128, JOBS><<<grid, kF1Threads, TcCfg<128>::SMEM, st>>>(J);
+    else k_f1_tc<256, JOBS><<<grid, kF1Threads, TcCfg<256>::SMEM, st>>>(J);
+}
+
+template <typename JOBS>
+static void launch_f2m(bool bf16, cudaStream_t st, int items, const JOBS &J) {
+    const int grid = std::min(items, 2 * num_sms());
+    if (bf16) k_f2m<2, JOBS><<<grid, kF2mThreads, F2mSmem::BYTES, st>>>(J);
+    else k_f2m<1, JOBS><<<grid, kF2mThreads, F2mSmem::BYTES, st>>>(J);
+}
+
+constexpr int kB1Cat[4] = {P_B1A, P_B1B, P_B1C, P_B1D};
+
+template <typename JOBS>
+static void launch_b1(int kind, cudaStream_t st, int tiles, const JOBS &J) {
+    const int grid = std::min(tiles, num_sms());
+    switch (kind) {
+    case 0: k_b1_tc<false, 128, JOBS><<<grid, kB1Threads, TcB1Cfg<false, 128>::SMEM, st>>>(J); break;
+    case 1: k_b1_tc<true, 128, JOBS><<<grid, kB1Threads, TcB1Cfg<true, 128>::SMEM, st>>>(J); break;
+    case 2: k_b1_tc<false, 64, JOBS><<<grid, kB1Threads, TcB1Cfg<false, 64>::SMEM, st>>>(J); break;
+    default: k_b1_tc<true, 64, JOBS><<<grid, kB1Threads, TcB1Cfg<true, 64>::SMEM, st>>>(J); break;
+    }
+}
+
+// n chunks of one call in the mixed modes: W contraction, epilogue (energy and
+// adjoint of the raw amplitudes), adjoint contractions.
+template <int NG>
+static int mixed_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t st, const TriplesIO &io,
+                        const OperandMaps &M) {
+    const bool bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16;
+    char *ws = (char *)io.workspace;
+    {
+        Group<F1Job, NG> G;
+        for (int c = 0; c < n; c++) {
+            G.job[c].m = F1Maps{M.tmA1, M.tmB1, M.tmA2, M.tmB2};
+            const int rc = f1_params(P, ch[c], c, ws, G.job[c].P);
+            if (rc != TRIPLES_OK) return rc;
+        }
+        const int tiles = group_starts(G, n, [](const F1Job &j) { return j.P.cum[j.P.ch.nperm]; });
+        TB_KLAUNCH(P_F1, launch_f1(P, st, tiles, G));
+    }
+    if (P.lno) {
+        // projected energy: whole-chunk epilogue instead of the orbit tiles (one chunk at a time)
+        const int rc = lno_chunk<float>(P, ch[0], st, io, ws, (Ctrl *)(ws + P.off_ctrl), (const float *)(ws + P.off_S),
+                                        P.want_grad ? (void *)(ws + P.off_SW) : nullptr, (int *)(ws + P.off_ijk),
+                                        bf16 ? 2 : 1);
+        if (rc != TRIPLES_OK) return rc;
+    } else {
+        Group<F2M, NG> G;
+        Group<ChunkAux, NG> X;
+        for (int c = 0; c < n; c++) {
+            f2m_params(P, ch[c], c, ws, io, false, G.job[c]);
+            X.job[c] = chunk_aux(P, ch[c], c, io, P.n_ijk * G.job[c].nsub);
+        }
+        X.n = n;
+        if (P.want_grad) TB_KLAUNCH(P_PREP, (k_chunk_scale<<<n, 32, 0, st>>>(X)));
+        const int items = group_starts(G, n, [&](const F2M &j) { return P.n_ijk * j.nsub; });
+        TB_KLAUNCH(P_F2, launch_f2m(bf16, st, items, G));
+        TB_KLAUNCH(P_F2, (k_energy_sum<<<1, 256, 0, st>>>(X, n)));
+    }
+    if (!P.want_grad) return TRIPLES_OK;
+    for (int kind = 0; kind < 4; kind++) {
+        Group<TcB1Params, NG> G;
+        for (int c = 0; c < n; c++) {
+            const int rc = b1_params(P, ch[c], c, ws, M, kind, G.job[c]);
+            if (rc != TRIPLES_OK) return rc;
+        }
+        const int tiles = group_starts(G, n, [](const TcB1Params &j) { return j.cum[j.nperm]; });
+        TB_KLAUNCH(kB1Cat[kind], launch_b1(kind, st, tiles, G));
+    }
+    return TRIPLES_OK;
+}
+
+// The same in FP64.
+template <int NG>
+static int fp64_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t st, const TriplesIO &io) {
+    char *ws = (char *)io.workspace;
+    GemmLaunch L;
+    L.d = P.d;
+    L.n = n;
+    L.A1 = (const double *)(ws + P.off_A1);
+    L.B1 = (const double *)(ws + P.off_B1);
+    L.A2 = (const double *)(ws + P.off_A2);
+    L.B2 = (const double *)(ws + P.off_B2);
+    L.G = nullptr;
+    for (int c = 0; c < n; c++) {
+        L.ch[c] = ch[c];
+        L.S[c] = (double *)(ws + P.off_S) + c * P.stage_slot;
+        L.SW[c] = P.want_grad ? (double *)(ws + P.off_SW) + c * P.wbar_slot : nullptr;
+    }
+    int rc;
+    if ((rc = chunk_gemm<GK_F1>(st, P_F1, L)) != TRIPLES_OK) return rc;
+    if (P.lno) {
+        rc = lno_chunk<double>(P, ch[0], st, io, ws, (Ctrl *)(ws + P.off_ctrl), L.S[0], L.SW[0], (int *)(ws + P.off_ijk), 0);
+        if (rc != TRIPLES_OK) return rc;
+    } else {
+        Group<F2P, NG> G;
+        Group<ChunkAux, NG> X;
+        for (int c = 0; c < n; c++) {
+            f2_params(P, ch[c], c, ws, io, G.job[c]);
+            X.job[c] = chunk_aux(P, ch[c], c, io, P.n_ijk * G.job[c].nsub);
+        }
+        X.n = n;
+        const int items = group_starts(G, n, [&](const F2P &j) { return P.n_ijk * j.nsub; });
+        TB_KLAUNCH(P_F2, (k_f2t<<<(unsigned)items, kF2Threads, f2_smem_bytes(), st>>>(G)));
+        TB_KLAUNCH(P_F2, (k_energy_sum<<<1, 256, 0, st>>>(X, n)));
+    }
+    if (!P.want_grad) return TRIPLES_OK;
+    L.G = (double *)(ws + P.off_GA1);
+    if ((rc = chunk_gemm<GK_B1A>(st, P_B1A, L)) != TRIPLES_OK) return rc;
+    L.G = (double *)(ws + P.off_GB2);
+    if ((rc = chunk_gemm<GK_B1D>(st, P_B1D, L)) != TRIPLES_OK) return rc;
+    L.G = (double *)(ws + P.off_GB1);
+    if ((rc = chunk_gemm<GK_B1B>(st, P_B1B, L)) != TRIPLES_OK) return rc;
+    L.G = (double *)(ws + P.off_GA2);
+    return chunk_gemm<GK_B1C>(st, P_B1C, L);
+}
+
 template <typename StageT>
 static int run_impl(const Plan &P, cudaStream_t st, const TriplesIO &io) {
     const bool mixed = P.prec != TRIPLES_PRECISION_FP64;
@@ -1554,134 +1760,31 @@ static int run_impl(const Plan &P, cudaStream_t st, const TriplesIO &io) {
     if (prc != TRIPLES_OK) return prc;
     if ((prc = prep_launches<StageT>(P, st, io)) != TRIPLES_OK) return prc;
     const Dims d = P.d;
-    const bool bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16;
     char *ws = (char *)io.workspace;
-    Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
-    double *A1 = (double *)(ws + P.off_A1);
-    double *B1 = (double *)(ws + P.off_B1);
-    double *A2 = (double *)(ws + P.off_A2);
-    double *B2 = (double *)(ws + P.off_B2);
-    StageT *S = (StageT *)(ws + P.off_S);
-    void *SW = P.want_grad ? (void *)(ws + P.off_SW) : nullptr;
-    double *GA1 = P.want_grad ? (double *)(ws + P.off_GA1) : nullptr;
-    double *GB1 = P.want_grad ? (double *)(ws + P.off_GB1) : nullptr;
-    double *GA2 = P.want_grad ? (double *)(ws + P.off_GA2) : nullptr;
-    double *GB2 = P.want_grad ? (double *)(ws + P.off_GB2) : nullptr;
-    int *ijk = (int *)(ws + P.off_ijk);
-    double *e_part = (double *)(ws + P.off_epart);
-    const int f1_bn = P.f1_bn;
     OperandMaps M;
     if (mixed) {
         if ((prc = build_operand_maps(P, ws, M)) != TRIPLES_OK) return prc;
         if ((prc = setup_tensor_cores()) != TRIPLES_OK) return prc;
     }
 
-    for (int A = 0; A < P.nb; A++) {
-        if (A < P.a0 || (P.a1 > 0 && A >= P.a1)) continue;
+    std::vector<ChunkDesc> chunks;
+    for (int A = P.a0; A < P.nb && (P.a1 <= 0 || A < P.a1); A++)
         for (int B = 0; B <= A; B++)
             for (int C = 0; C <= B; C++) {
-                ChunkDesc ch;
-                make_chunk(d, A, B, C, ch);
-                // F1: raw amplitudes
-                if (mixed) {
-                    TcF1Params T;
-                    const int frc = f1_params(P, ch, ws, T);
-                    if (frc != TRIPLES_OK) return frc;
-                    const int tiles = T.cum[ch.nperm];
-                    const int grid = tiles < num_sms() ? tiles : num_sms();
-                    const F1Maps Mf1{M.tmA1, M.tmB1, M.tmA2, M.tmB2};
-                    if (f1_bn == 128)
-                        TB_KLAUNCH(P_F1, (k_f1_tc<128, false><<<grid, kF1Threads, TcCfg<128>::SMEM, st>>>(
-                                             Mf1, T, nullptr, nullptr, 0)));
-                    else
-                        TB_KLAUNCH(P_F1, (k_f1_tc<256, false><<<grid, kF1Threads, TcCfg<256>::SMEM, st>>>(
-                                             Mf1, T, nullptr, nullptr, 0)));
-                } else {
-                    GemmLaunch L;
-                    L.d = d;
-                    L.ch = ch;
-                    L.A1 = A1; L.B1 = B1; L.A2 = A2; L.B2 = B2;
-                    L.S = (double *)S;
-                    L.G = nullptr;
-                    if ((prc = chunk_gemm<GK_F1>(st, P_F1, L)) != TRIPLES_OK) return prc;
-                }
-                if (P.lno) {
-                    // projected energy: whole-chunk epilogue instead of the orbit tiles
-                    const int rc = lno_chunk<StageT>(P, ch, st, io, ws, ctrl, S, SW, ijk, mixed ? (bf16 ? 2 : 1) : 0);
-                    if (rc != TRIPLES_OK) return rc;
-                } else if (mixed) {
-                    // F2: energy (+ adjoint of the raw amplitudes), every item of the chunk in one launch
-                    F2M F;
-                    f2m_params(P, ch, ws, io, false, F);
-                    if (P.want_grad)
-                        TB_KLAUNCH(P_PREP, k_chunk_scale<<<1, 32, 0, st>>>(ctrl, io.mo_energy, d.o, ch.base[0], ch.nabc[0],
-                                                                           ch.base[1], ch.nabc[1], ch.base[2], ch.nabc[2],
-                                                                           io.ybar, bf16 ? 0 : 1, 0));
-                    const int nitems = P.n_ijk * F.nsub;
-                    const int nb = nitems < 2 * num_sms() ? nitems : 2 * num_sms();
-                    if (bf16)
-                        TB_KLAUNCH(P_F2, (k_f2m<2, false><<<nb, kF2mThreads, F2mSmem::BYTES, st>>>(F, nullptr, nullptr, 0, nitems)));
-                    else
-                        TB_KLAUNCH(P_F2, (k_f2m<1, false><<<nb, kF2mThreads, F2mSmem::BYTES, st>>>(F, nullptr, nullptr, 0, nitems)));
-                    TB_KLAUNCH(P_F2, k_f2_energy_sum<<<1, 256, 0, st>>>(e_part, nitems, &ctrl->e_acc, &ctrl->ticket));
-                } else {
-                    F2P F;
-                    f2_params(P, ch, ws, io, F);
-                    TB_KLAUNCH(P_F2, (k_f2t<<<(unsigned)(P.n_ijk * F.nsub), kF2Threads, f2_smem_bytes(), st>>>(F)));
-                    TB_KLAUNCH(P_F2, k_f2_energy_sum<<<1, 256, 0, st>>>(e_part, P.n_ijk * F.nsub, &ctrl->e_acc, nullptr));
-                }
-                if (!P.want_grad) continue;
-                // W-term gradients
-                if (mixed) {
-                    // one launch per kind over all orderings of the chunk
-                    TcB1Params B;
-                    auto launch_b1 = [&](int kind) -> int {
-                        const int brc = b1_params(P, ch, ws, M, kind, B);
-                        if (brc != TRIPLES_OK) return brc;
-                        const int tiles = B.cum[ch.nperm];
-                        const int grid = tiles < num_sms() ? tiles : num_sms();
-                        switch (kind) {
-                        case 0:
-                            TB_KLAUNCH(P_B1A, (k_b1_tc<false, 128, false><<<grid, kB1Threads, TcB1Cfg<false, 128>::SMEM, st>>>(
-                                                  B, nullptr, nullptr, 0)));
-                            break;
-                        case 1:
-                            TB_KLAUNCH(P_B1B, (k_b1_tc<true, 128, false><<<grid, kB1Threads, TcB1Cfg<true, 128>::SMEM, st>>>(
-                                                  B, nullptr, nullptr, 0)));
-                            break;
-                        case 2:
-                            TB_KLAUNCH(P_B1C, (k_b1_tc<false, 64, false><<<grid, kB1Threads, TcB1Cfg<false, 64>::SMEM, st>>>(
-                                                  B, nullptr, nullptr, 0)));
-                            break;
-                        default:
-                            TB_KLAUNCH(P_B1D, (k_b1_tc<true, 64, false><<<grid, kB1Threads, TcB1Cfg<true, 64>::SMEM, st>>>(
-                                                  B, nullptr, nullptr, 0)));
-                            break;
-                        }
-                        return TRIPLES_OK;
-                    };
-                    for (int kind = 0; kind < 4; kind++) {
-                        const int brc = launch_b1(kind);
-                        if (brc != TRIPLES_OK) return brc;
-                    }
-                } else {
-                    GemmLaunch L;
-                    L.d = d;
-                    L.ch = ch;
-                    L.A1 = A1; L.B1 = B1; L.A2 = A2; L.B2 = B2;
-                    L.S = (double *)SW;
-                    L.G = GA1;
-                    if ((prc = chunk_gemm<GK_B1A>(st, P_B1A, L)) != TRIPLES_OK) return prc;
-                    L.G = GB2;
-                    if ((prc = chunk_gemm<GK_B1D>(st, P_B1D, L)) != TRIPLES_OK) return prc;
-                    L.G = GB1;
-                    if ((prc = chunk_gemm<GK_B1B>(st, P_B1B, L)) != TRIPLES_OK) return prc;
-                    L.G = GA2;
-                    if ((prc = chunk_gemm<GK_B1C>(st, P_B1C, L)) != TRIPLES_OK) return prc;
-                }
+                chunks.emplace_back();
+                make_chunk(d, A, B, C, chunks.back());
             }
+    // the chunks of a group (P.group at most) run in one launch per kernel
+    for (size_t c0 = 0; c0 < chunks.size(); c0 += P.group) {
+        const int n = (int)std::min((size_t)P.group, chunks.size() - c0);
+        const ChunkDesc *ch = &chunks[c0];
+        if (mixed) {
+            prc = n == 1 ? mixed_chunks<1>(P, ch, n, st, io, M) : mixed_chunks<kMaxGroup>(P, ch, n, st, io, M);
+        } else {
+            prc = n == 1 ? fp64_chunks<1>(P, ch, n, st, io) : fp64_chunks<kMaxGroup>(P, ch, n, st, io);
+        }
+        if (prc != TRIPLES_OK) return prc;
     }
-
     return fold_launches(P, st, io);
 }
 
@@ -1821,7 +1924,7 @@ static int batch_build(Batch &B, int prec, int nprob, const triples_problem *pro
                 std::memset(&job, 0, sizeof(job));
                 const OperandMaps &M = maps[p];
                 job.m = F1Maps{M.tmA1, M.tmB1, M.tmA2, M.tmB2};
-                const int rc = f1_params(B.plans[p], chunks[p][c], B.ws + B.ws_off[p], job.P);
+                const int rc = f1_params(B.plans[p], chunks[p][c], 0, B.ws + B.ws_off[p], job.P);
                 if (rc != TRIPLES_OK) return rc;
                 std::memcpy(img + S.f1_jobs[g] + sizeof(F1Job) * j, &job, sizeof(job));
                 start[j + 1] = start[j] + job.P.cum[job.P.ch.nperm];
@@ -1842,25 +1945,15 @@ static int batch_build(Batch &B, int prec, int nprob, const triples_problem *pro
             char *wsp = B.ws + B.ws_off[p];
             F2M F;
             std::memset(&F, 0, sizeof(F));
-            f2m_params(P, ch, wsp, B.ios[p], true, F);
+            f2m_params(P, ch, 0, wsp, B.ios[p], true, F);
             std::memcpy(img + S.f2_jobs + sizeof(F) * j, &F, sizeof(F));
             f2s[j + 1] = f2s[j] + P.n_ijk * F.nsub;
-            ChunkAux A;
-            std::memset(&A, 0, sizeof(A));
-            A.ctrl = (Ctrl *)(wsp + P.off_ctrl);
-            A.mo_e = B.ios[p].mo_energy;
-            A.e_part = (const double *)(wsp + P.off_epart);
-            A.ybar = ybar;
-            A.o = P.d.o;
-            A.a0 = ch.base[0]; A.na = ch.nabc[0];
-            A.b0 = ch.base[1]; A.nb = ch.nabc[1];
-            A.c0 = ch.base[2]; A.nc = ch.nabc[2];
-            A.n_part = P.n_ijk * F.nsub;
+            const ChunkAux A = chunk_aux(P, ch, 0, B.ios[p], P.n_ijk * F.nsub);
             std::memcpy(img + S.aux + sizeof(A) * j, &A, sizeof(A));
             for (int k = 0; k < 4; k++) {
                 TcB1Params Bp;
                 std::memset(&Bp, 0, sizeof(Bp));
-                const int rc = b1_params(P, ch, wsp, maps[p], k, Bp);
+                const int rc = b1_params(P, ch, 0, wsp, maps[p], k, Bp);
                 if (rc != TRIPLES_OK) return rc;
                 std::memcpy(img + S.b1_jobs[k] + sizeof(Bp) * j, &Bp, sizeof(Bp));
                 b1s[k][j + 1] = b1s[k][j] + Bp.cum[ch.nperm];
@@ -1888,46 +1981,24 @@ static int run_batch(const Batch &B, cudaStream_t st) {
     for (int p = 0; p < B.nprob; p++)
         if ((rc = prep_launches<float>(B.plans[p], st, B.ios[p])) != TRIPLES_OK) return rc;
     const char *tab = B.ws + B.tables_off;
-    const int nsm = num_sms();
-    const int scaled = B.prec == TRIPLES_PRECISION_MIXED_BF16 ? 0 : 1;
-    const F1Maps M0{};
-    const TcF1Params T0{};
-    const TcB1Params B0{};
-    const F2M F0{};
-    auto cap = [&](int n) { return n < nsm ? n : nsm; };
+    const bool bf16 = B.prec == TRIPLES_PRECISION_MIXED_BF16;
     for (const BatchStep &S : B.steps) {
-        const F1Job *f1j[2] = {(const F1Job *)(tab + S.f1_jobs[0]), (const F1Job *)(tab + S.f1_jobs[1])};
-        const int *f1s[2] = {(const int *)(tab + S.f1_start[0]), (const int *)(tab + S.f1_start[1])};
-        if (S.f1_n[0] > 0)
-            TB_KLAUNCH(P_F1, (k_f1_tc<256, true><<<cap(S.f1_tiles[0]), kF1Threads, TcCfg<256>::SMEM, st>>>(
-                                 M0, T0, f1j[0], f1s[0], S.f1_n[0])));
-        if (S.f1_n[1] > 0)
-            TB_KLAUNCH(P_F1, (k_f1_tc<128, true><<<cap(S.f1_tiles[1]), kF1Threads, TcCfg<128>::SMEM, st>>>(
-                                 M0, T0, f1j[1], f1s[1], S.f1_n[1])));
-        const ChunkAux *aux = (const ChunkAux *)(tab + S.aux);
-        TB_KLAUNCH(P_PREP, k_chunk_scale_batch<<<S.naux, 32, 0, st>>>(aux, scaled));
-        const F2M *f2j = (const F2M *)(tab + S.f2_jobs);
-        const int *f2s = (const int *)(tab + S.f2_start);
-        const int f2n = S.f2_items < 2 * nsm ? S.f2_items : 2 * nsm;
-        if (scaled)
-            TB_KLAUNCH(P_F2, (k_f2m<1, true><<<f2n, kF2mThreads, F2mSmem::BYTES, st>>>(F0, f2j, f2s, S.naux, S.f2_items)));
-        else
-            TB_KLAUNCH(P_F2, (k_f2m<2, true><<<f2n, kF2mThreads, F2mSmem::BYTES, st>>>(F0, f2j, f2s, S.naux, S.f2_items)));
-        TB_KLAUNCH(P_F2, k_energy_sum_batch<<<S.naux, 256, 0, st>>>(aux));
-        const TcB1Params *bj[4];
-        const int *bs[4];
-        for (int k = 0; k < 4; k++) {
-            bj[k] = (const TcB1Params *)(tab + S.b1_jobs[k]);
-            bs[k] = (const int *)(tab + S.b1_start[k]);
+        for (int g = 0; g < 2; g++) {
+            if (S.f1_n[g] == 0) continue;
+            const Table<F1Job> J{S.f1_n[g], (const int *)(tab + S.f1_start[g]), (const F1Job *)(tab + S.f1_jobs[g])};
+            Plan W;   // only the tile width matters to the launch
+            W.f1_bn = g == 0 ? 256 : 128;
+            TB_KLAUNCH(P_F1, launch_f1(W, st, S.f1_tiles[g], J));
         }
-        TB_KLAUNCH(P_B1A, (k_b1_tc<false, 128, true><<<cap(S.b1_tiles[0]), kB1Threads, TcB1Cfg<false, 128>::SMEM, st>>>(
-                              B0, bj[0], bs[0], S.naux)));
-        TB_KLAUNCH(P_B1B, (k_b1_tc<true, 128, true><<<cap(S.b1_tiles[1]), kB1Threads, TcB1Cfg<true, 128>::SMEM, st>>>(
-                              B0, bj[1], bs[1], S.naux)));
-        TB_KLAUNCH(P_B1C, (k_b1_tc<false, 64, true><<<cap(S.b1_tiles[2]), kB1Threads, TcB1Cfg<false, 64>::SMEM, st>>>(
-                              B0, bj[2], bs[2], S.naux)));
-        TB_KLAUNCH(P_B1D, (k_b1_tc<true, 64, true><<<cap(S.b1_tiles[3]), kB1Threads, TcB1Cfg<true, 64>::SMEM, st>>>(
-                              B0, bj[3], bs[3], S.naux)));
+        const Table<ChunkAux> X{S.naux, nullptr, (const ChunkAux *)(tab + S.aux)};
+        TB_KLAUNCH(P_PREP, (k_chunk_scale<<<S.naux, 32, 0, st>>>(X)));
+        const Table<F2M> F{S.naux, (const int *)(tab + S.f2_start), (const F2M *)(tab + S.f2_jobs)};
+        TB_KLAUNCH(P_F2, launch_f2m(bf16, st, S.f2_items, F));
+        TB_KLAUNCH(P_F2, (k_energy_sum<<<S.naux, 256, 0, st>>>(X, 1)));
+        for (int k = 0; k < 4; k++) {
+            const Table<TcB1Params> J{S.naux, (const int *)(tab + S.b1_start[k]), (const TcB1Params *)(tab + S.b1_jobs[k])};
+            TB_KLAUNCH(kB1Cat[k], launch_b1(k, st, S.b1_tiles[k], J));
+        }
     }
     for (int p = 0; p < B.nprob; p++)
         if ((rc = fold_launches(B.plans[p], st, B.ios[p])) != TRIPLES_OK) return rc;
@@ -1979,13 +2050,19 @@ size_t triples_workspace_size_ex(int precision, int nocc, int nvir, int ovvv_pac
     return P.total;
 }
 
+size_t triples_workspace_extra(int precision, int nocc, int nvir, int ovvv_packed, int want_grad,
+                               const triples_options *opt) {
+    tb::Plan P, Q;
+    if (tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, P, 0, opt) != TRIPLES_OK) return 0;
+    if (tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, Q, 0, opt, true, tb::kMaxGroup) != TRIPLES_OK) return 0;
+    return Q.total > P.total ? Q.total - P.total : 0;
+}
+
 static int triples_call(void *stream, int precision, int nocc, int nvir, int ovvv_packed, int want_grad,
                         const triples_options *opt, const tb::TriplesIO &io, size_t workspace_bytes) {
     tb::Plan P;
-    int rc = tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, P, 0, opt);
+    int rc = tb::make_plan_for(precision, nocc, nvir, ovvv_packed, want_grad, P, opt, workspace_bytes);
     if (rc != TRIPLES_OK) return rc;
-    // a workspace too small for the V-term tables alone: run without them
-    if (workspace_bytes < P.total) tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, P, 0, opt, false);
     if (!io.workspace || workspace_bytes < P.total) return TRIPLES_ERR_WORKSPACE;
     if (!io.mo_energy || !io.t1 || !io.t2 || !io.ovoo || !io.ovov || !io.ovvv || !io.fvo || !io.e_out)
         return TRIPLES_ERR_INVALID_ARGUMENT;
@@ -2125,24 +2202,28 @@ struct DfLayout {
     size_t off_ovvv, off_gvvv, total;
 };
 
-static int df_layout(int precision, int nocc, int nvir, int naux, int want_grad, DfLayout &L, bool vtables = true) {
+// workspace_bytes: what the caller has (SIZE_MAX: the size to ask for)
+static int df_layout(int precision, int nocc, int nvir, int naux, int want_grad, DfLayout &L, size_t workspace_bytes) {
     if (naux < 1) return TRIPLES_ERR_INVALID_ARGUMENT;
-    int rc = tb::make_plan(precision, nocc, nvir, 1, want_grad, L.P, 0, nullptr, vtables);
-    if (rc != TRIPLES_OK) return rc;
     const size_t nov = (size_t)nocc * nvir, npair = (size_t)nvir * (nvir + 1) / 2;
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    size_t off = al(L.P.total);
-    L.off_ovvv = off;
-    off = al(off + nov * npair * sizeof(double));
-    L.off_gvvv = off;
-    if (want_grad) off = al(off + nov * npair * sizeof(double));
-    L.total = off;
+    const size_t own = al(nov * npair * sizeof(double)) * (want_grad ? 2 : 1);
+    int rc;
+    if (workspace_bytes == SIZE_MAX)
+        rc = tb::make_plan(precision, nocc, nvir, 1, want_grad, L.P);
+    else
+        rc = tb::make_plan_for(precision, nocc, nvir, 1, want_grad, L.P, nullptr,
+                               workspace_bytes > own ? workspace_bytes - own : 0);
+    if (rc != TRIPLES_OK) return rc;
+    L.off_ovvv = al(L.P.total);
+    L.off_gvvv = L.off_ovvv + al(nov * npair * sizeof(double));
+    L.total = L.off_ovvv + own;
     return TRIPLES_OK;
 }
 
 size_t triples_df_workspace_size(int precision, int nocc, int nvir, int naux, int want_grad) {
     DfLayout L;
-    if (df_layout(precision, nocc, nvir, naux, want_grad, L) != TRIPLES_OK) return 0;
+    if (df_layout(precision, nocc, nvir, naux, want_grad, L, SIZE_MAX) != TRIPLES_OK) return 0;
     return L.total;
 }
 
@@ -2150,9 +2231,8 @@ static int triples_df_call(void *stream, int precision, int nocc, int nvir, int 
                            const double *Lov, const double *Lvv, tb::TriplesIO io, size_t workspace_bytes,
                            double *Lov_bar, double *Lvv_bar) {
     DfLayout L;
-    int rc = df_layout(precision, nocc, nvir, naux, want_grad, L);
+    int rc = df_layout(precision, nocc, nvir, naux, want_grad, L, workspace_bytes);
     if (rc != TRIPLES_OK) return rc;
-    if (workspace_bytes < L.total) df_layout(precision, nocc, nvir, naux, want_grad, L, false);
     if (!io.workspace || workspace_bytes < L.total) return TRIPLES_ERR_WORKSPACE;
     if (!Lov || !Lvv || !io.mo_energy || !io.t1 || !io.t2 || !io.ovoo || !io.ovov || !io.fvo || !io.e_out)
         return TRIPLES_ERR_INVALID_ARGUMENT;
@@ -2246,10 +2326,9 @@ int triples_energy_vjp_static(void *stream, int precision, int nocc, int nvir, i
                               const double *fvo, double ybar, double *e_out, double *mo_energy_bar,
                               double *t1_bar, double *t2_bar, double *ovoo_bar, double *ovov_bar,
                               double *ovvv_bar, double *fvo_bar) {
-    tb::Plan P;
-    if (tb::make_plan(precision, nocc, nvir, ovvv_packed, 1, P, 0, nullptr, false) != TRIPLES_OK)
-        return TRIPLES_ERR_INVALID_ARGUMENT;
-    if (P.total > kStaticScratchBytes) return TRIPLES_ERR_WORKSPACE;   // problem too large for the fixed scratch
+    const size_t need = triples_workspace_size(precision, nocc, nvir, ovvv_packed, 1);
+    if (need == 0) return TRIPLES_ERR_INVALID_ARGUMENT;
+    if (need > kStaticScratchBytes) return TRIPLES_ERR_WORKSPACE;   // problem too large for the fixed scratch
     void *scratch = nullptr;
     const int rc = static_scratch_address(&scratch);
     if (rc != TRIPLES_OK) return rc;

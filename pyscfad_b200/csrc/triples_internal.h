@@ -11,9 +11,23 @@ namespace tb {
 constexpr int kMaxTv = 16;        // largest virtual block
 constexpr int kMaxCols = 1024;    // largest nocc * Tv (one staged (r, z) row)
 constexpr int kCtrlBytes = 256;   // control block at workspace offset 0
+// Chunk slots of a call: most bytes of staging and Wbar.  A chunk of nocc 5 has
+// a few tens of tiles per kernel, one of nocc 13 fills the chip once or twice
+// with a nearly empty last wave; from nocc 20 (1.6 GB a chunk) on a chunk is
+// enough alone.  One chunk at a time / within 1 GB / within 2 GB, E + VJP: nocc
+// 5 nvir 19 mixed 1.26 / 0.45 / 0.45 ms, FP64 kernels 0.95 / 0.45 / 0.45 ms, nocc
+// 13 nvir 83 bf16 41.4 / 35.2 / 33.0 ms, nocc 12 nvir 100 FP64 112 / 112 / 104 ms.
+constexpr size_t kGroupBytes = (size_t)2 << 30;
 constexpr int kLnoGrid = 1184;    // LNO streaming kernels: most blocks per ordering (energy partials)
 constexpr int kLnoArrays = 4;     // LNO whole-chunk FP64 work arrays (with the adjoint)
 constexpr double kLnoBudgetBytes = 96e9;   // their largest total before the block size is halved
+
+// State of one chunk slot
+struct ChunkSlot {
+    double wscale;                // power-of-two scale of the split Wbar
+    unsigned wmax_bits;           // bit pattern of max |W| (F1)
+    unsigned ticket;              // work items handed out by the mixed epilogue (first slot of a launch)
+};
 
 // Control block (workspace offset 0)
 struct Ctrl {
@@ -22,11 +36,9 @@ struct Ctrl {
     double scale[2];              // operand scales (A: ovvv/ovoo, B: t2), powers of two
     float out_scale;              // 1 / (scale[0] * scale[1])
     float pad_;
-    double wscale;                // per-chunk power-of-two scale of the split Wbar
     unsigned long long absmax[6]; // bit patterns of max |ovvv|, |ovoo|, |t2|, |ovov|, |t1|, |fvo|
-    unsigned wmax_bits;           // bit pattern of max |W| of the current chunk (F1)
-    unsigned ticket;              // work items handed out by the mixed epilogue of the current chunk
     double lno_norm[2];           // LNO projector: max abs row sum, max abs column sum
+    ChunkSlot slot[kMaxGroup];
 };
 
 static_assert(sizeof(Ctrl) <= kCtrlBytes, "control block too large");
@@ -45,10 +57,12 @@ struct Plan {
     int f2_gy;       // epilogue grid.y upper bound
     int Kp8, Op8;    // 16-byte padded contraction lengths of the 16-bit operands
     size_t stage_elems, stage_bytes, wbar_elems;
+    size_t stage_slot, wbar_slot;   // elements from one chunk slot to the next
     size_t off_ctrl;
     size_t off_A1, off_B1, off_A2, off_B2, off_S, off_SW;
     size_t off_A1h, off_B1h, off_A2h, off_B2h;
     size_t off_GA1, off_GB1, off_GA2, off_GB2;
+    int group;       // chunk slots: chunks whose kernels run in one launch each
     bool vtables;    // the workspace holds the epilogue's FP32 V-term tables
     size_t off_ot, off_tf;
     size_t off_ijk, off_epart;
@@ -67,7 +81,9 @@ struct TriplesIO {
 };
 
 int make_plan(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, int lno = 0,
-              const triples_options *opt = nullptr, bool vtables = true);
+              const triples_options *opt = nullptr, bool vtables = true, int most_group = 1);
+int make_plan_for(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, const triples_options *opt,
+                  size_t workspace_bytes);
 int run_triples(const Plan &P, cudaStream_t st, const TriplesIO &io);
 
 }  // namespace tb

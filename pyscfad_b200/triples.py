@@ -19,18 +19,42 @@ KEYS = ("mo_energy", "t1", "t2", "ovoo", "ovov", "ovvv", "fvo")
 _workspaces: dict = {}
 
 
-def _workspace(nbytes: int, device: torch.device, stream) -> torch.Tensor:
+# Streams on which the extra bytes once did not fit: their calls do without.
+_no_extra: set = set()
+
+
+def _workspace(nbytes: int, device: torch.device, stream, extra: int = 0) -> torch.Tensor:
+    """At least nbytes of scratch, and `extra` more (triples_workspace_extra) while the device has room."""
     key = (device.type, device.index, int(stream.cuda_stream))
+    if key in _no_extra:
+        extra = 0
     buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
+    if buf is None or buf.numel() < nbytes + extra:
         _workspaces.pop(key, None)
-        buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+        del buf
+        try:
+            buf = torch.empty(max(nbytes + extra, 256), dtype=torch.uint8, device=device)
+        except torch.cuda.OutOfMemoryError:
+            if extra == 0:
+                raise
+            _no_extra.add(key)
+            buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
         _workspaces[key] = buf
     return buf
 
 
+def holds_workspace(nbytes: int) -> bool:
+    """Whether the current stream's cached scratch already has nbytes (asking the
+    device for its free memory costs a millisecond)."""
+    dev = torch.cuda.current_device()
+    stream = int(torch.cuda.current_stream(dev).cuda_stream)
+    return any(buf.numel() >= nbytes for key, buf in _workspaces.items()
+               if key[0] == "cuda" and key[1] in (dev, None) and key[2] == stream)
+
+
 def release_workspace():
     _workspaces.clear()
+    _no_extra.clear()
 
 
 def _as_dev(x, device) -> torch.Tensor:
@@ -105,7 +129,8 @@ def _run(mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, d
     if nbytes == 0:
         raise _lib.TriplesError(1, "triples_workspace_size_ex")
     st = stream if stream is not None else torch.cuda.current_stream(device)
-    ws = _workspace(nbytes, device, st)
+    ws = _workspace(nbytes, device, st,
+                    lib.triples_workspace_extra(prec, o, v, int(packed), int(want_grad), ctypes.byref(opt)))
     e = torch.zeros((), dtype=torch.float64, device=device)
     grads = {k: torch.empty_like(a) for k, a in zip(KEYS, args)} if want_grad else {}
     gptr = [grads[k].data_ptr() for k in KEYS] if want_grad else [None] * len(KEYS)
@@ -221,7 +246,7 @@ def energy_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, precision="fp64", de
     if nbytes == 0:
         raise _lib.TriplesError(1, "triples_df_workspace_size")
     st = stream if stream is not None else torch.cuda.current_stream(device)
-    ws = _workspace(nbytes, device, st)
+    ws = _workspace(nbytes, device, st, lib.triples_workspace_extra(prec, o, v, 1, 0, None))
     e = torch.zeros((), dtype=torch.float64, device=device)
     rc = lib.triples_energy_df(st.cuda_stream, prec, o, v, naux, *[a.data_ptr() for a in args], ws.data_ptr(),
                                ws.numel(), e.data_ptr())
@@ -244,7 +269,7 @@ def energy_vjp_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar=1.0, precis
     if nbytes == 0:
         raise _lib.TriplesError(1, "triples_df_workspace_size")
     st = stream if stream is not None else torch.cuda.current_stream(device)
-    ws = _workspace(nbytes, device, st)
+    ws = _workspace(nbytes, device, st, lib.triples_workspace_extra(prec, o, v, 1, 1, None))
     e = torch.zeros((), dtype=torch.float64, device=device)
     grads = {k: torch.empty_like(a) for k, a in zip(DF_KEYS, args)}
     rc = lib.triples_energy_vjp_df(st.cuda_stream, prec, o, v, naux, *[a.data_ptr() for a in args], float(ybar),

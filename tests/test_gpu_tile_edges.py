@@ -31,12 +31,12 @@ def test_fp64_contraction_tiles(o, v):
         assert _relerr(g[k].cpu().numpy(), g_ref[k]) < 1e-10, k
 
 
-# V-term tables: prepared in the workspace, or gathered when the caller's scratch
-# ends before them; short sub-ranges (nvir 27: blocks 16, 8, 2, 1) start inside
-# an 8-wide table block
+# What only makes a call faster: more than one chunk slot (an extra scratch), and
+# the V-term tables (a scratch without room for them: the entries are gathered).
+# Short sub-ranges (nvir 27: blocks 16, 8, 2, 1) start inside an 8-wide table block
 @pytest.mark.parametrize("o,v,tv", [(3, 27, 16), (2, 40, 8), (5, 9, 2)])
-@pytest.mark.parametrize("precision", ["mixed", "mixed_bf16"])
-def test_epilogue_without_prepared_tables(o, v, tv, precision):
+@pytest.mark.parametrize("precision", ["mixed", "mixed_bf16", "fp64"])
+def test_scratch_sizes_give_the_same(o, v, tv, precision):
     import ctypes
 
     from pyscfad_b200 import _lib
@@ -45,8 +45,6 @@ def test_epilogue_without_prepared_tables(o, v, tv, precision):
     ins = [torch.as_tensor(np.ascontiguousarray(getattr(inp, k)), device="cuda") for k in G.KEYS]
     lib, opt, prec = _lib.load(), _lib.options(tv), _lib.PRECISION[precision]
     full = lib.triples_workspace_size_ex(prec, o, v, 0, 1, ctypes.byref(opt))
-    nb8 = (v + 7) // 8
-    tables = sum((n + 255) // 256 * 256 for n in (o * o * nb8 * nb8 * 512, o * nb8 * 64))
 
     def run(nbytes):
         ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
@@ -61,13 +59,21 @@ def test_epilogue_without_prepared_tables(o, v, tv, precision):
 
     rc, e0, g0 = run(full)
     assert rc == 0
-    rc, e1, g1 = run(full - tables)
-    assert rc == 0
+    extra = lib.triples_workspace_extra(prec, o, v, 0, 1, ctypes.byref(opt))
+    assert extra > 0
+    sizes = [full + extra, full + extra // 2]
+    if precision != "fp64":
+        sizes.append(full - 256)
+    else:
+        assert run(full - 256)[0] != 0
     # the same FP32 values either way; only FP64 sums may be ordered differently
-    assert abs(e1 - e0) <= 1e-13 * abs(e0)
-    for k in G.KEYS:
-        assert _relerr(g1[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-12, k
-    assert run(full - tables - 1)[0] != 0
+    for nbytes in sizes:
+        rc, e1, g1 = run(nbytes)
+        assert rc == 0
+        assert abs(e1 - e0) <= 1e-13 * abs(e0)
+        for k in G.KEYS:
+            assert _relerr(g1[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-12, k
+    assert run(4096)[0] != 0
 
 
 # W-contraction tiles of 2 to 16 r values (nocc 1-17, with and without a second
