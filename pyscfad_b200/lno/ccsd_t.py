@@ -58,7 +58,7 @@ def _check_memory(nocc, nvir, packed, want_grad, precision="fp64"):
     (pyscfad/lno/ccsd_t.py:101-103 and 185-192): RuntimeError when the device
     cannot hold the workspace."""
     need = triples.lno_workspace_size(nocc, nvir, packed, want_grad, precision)
-    if torch.cuda.is_available():
+    if torch.cuda.is_available() and not triples.holds_workspace(need):
         free, _ = torch.cuda.mem_get_info()
         if need > free:
             raise RuntimeError(f"{need / 1e6:.0f} MB more memory is needed "
