@@ -397,13 +397,14 @@ def run_accuracy(args, o, v, naux):
 # ---------------------------------------------------------------------------
 LNO_METRIC = "LNO (T) E+VJP TFLOP/s (projected first occupied index), B200 vs reference CPU kernels"
 # algorithmic bytes per raw amplitude position of each LNO epilogue pass
-# (sz = staging element size: 8 FP64, 4 mixed): tile forward reads w, writes
-# WW and Q; the projection reads WW, Q and writes Zbar, Dbar, P^T(Wtbar);
-# tile adjoint reads Zbar, P^T(Wtbar), writes vbar and the Wbar operand
-# (FP64, or two 16-bit halves); V gradients read vbar, Dbar.
+# (sz = staging element size: 8 FP64, 4 mixed): the forward pass reads w and
+# writes WW and Q, the projections (one per occupied slot) read them and update
+# PW and PQ, the adjoint pass reads Zbar, PQ and Q and writes the Wbar operand
+# (FP64, or two 16-bit halves).
 def lno_pass_bytes(sz):
-    return {"lno_tile_fwd": sz + 16, "lno_projection": 40, "lno_tile_adj": 16 + 8 + (8 if sz == 8 else 4),
-            "lno_vgrad": 16}
+    # the FP64 box arrays hold one value per six raw amplitudes: two written by the forward pass, two read and
+    # two updated by each of the three projections, three read by the adjoint pass
+    return {"lno_tile_fwd": sz + 16 / 6, "lno_projection": 128 / 6, "lno_tile_adj": 24 / 6 + (8 if sz == 8 else 4)}
 
 
 def run_lno(args, o, v, naux):

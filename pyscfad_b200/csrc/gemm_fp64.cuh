@@ -54,7 +54,7 @@ struct GemmCfg {
     static constexpr int LDA = KFA ? kGBK + 4 : BM + 4, LDB = KFB ? kGBK + 4 : BN + 4;
     static constexpr int ELA = KFA ? BM * LDA : kGBK * LDA, ELB = KFB ? BN * LDB : kGBK * LDB;
     static constexpr int RING = kGStages + 1;
-    static constexpr size_t TAB = 2 * (BM + BN) + RING * 2 * kGBK;   // row and k offsets
+    static constexpr size_t TAB = 3 * (BM + BN) + RING * 2 * kGBK;   // row, output and k offsets
     static constexpr size_t SMEM = sizeof(double) * (size_t)(kGStages * (ELA + ELB)) + sizeof(long long) * TAB;
 };
 
@@ -98,6 +98,7 @@ __device__ __forceinline__ void gemm_fp64_tile(const GemmArgs &g, int m0, int n0
     double *sA = smem, *sB = smem + kGStages * C::ELA;
     long long *rowA = reinterpret_cast<long long *>(smem + kGStages * (C::ELA + C::ELB));
     long long *rowB = rowA + BM, *rowA2 = rowB + BN, *rowB2 = rowA2 + BM, *koff = rowB2 + BN;
+    long long *outM = koff + C::RING * 2 * kGBK, *outN = outM + BM;
     for (int t = tid; t < BM; t += kGThreads) {
         const bool ok = m0 + t < g.M;
         rowA[t] = ok ? apply(g.A.mn, m0 + t) : -1;
@@ -149,6 +150,9 @@ __device__ __forceinline__ void gemm_fp64_tile(const GemmArgs &g, int m0, int n0
     __syncthreads();
 #pragma unroll
     for (int s = 0; s < kGStages - 1; s++) issue(ktb + s);
+    // output offsets, while the first tiles arrive (read after the K loop's barriers)
+    for (int t = tid; t < BM; t += kGThreads) outM[t] = apply(g.cm, m0 + t);
+    for (int t = tid; t < BN; t += kGThreads) outN[t] = apply(g.cn, n0 + t);
     for (int kt = ktb; kt < kte; kt++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kGStages - 2) : "memory");
         __syncthreads();   // tile kt is complete, the buffer of tile kt - 1 is free
@@ -183,19 +187,18 @@ __device__ __forceinline__ void gemm_fp64_tile(const GemmArgs &g, int m0, int n0
 
 #pragma unroll
     for (int i = 0; i < C::TM; i++) {
-        const int m = m0 + wm0 + 8 * i + fg;
-        if (m >= g.M) continue;
-        const long long cmo = apply(g.cm, m);
+        const int ml = wm0 + 8 * i + fg;
+        if (m0 + ml >= g.M) continue;
+        double *row = g.C + outM[ml];
 #pragma unroll
         for (int j = 0; j < C::TN; j++)
 #pragma unroll
             for (int c = 0; c < 2; c++) {
-                const int n = n0 + wn0 + 8 * j + 2 * ft + c;
-                if (n >= g.N) continue;
-                const long long off = cmo + apply(g.cn, n);
+                const int nl = wn0 + 8 * j + 2 * ft + c;
+                if (n0 + nl >= g.N) continue;
                 const double val = g.alpha * acc[i][j][c];
-                if (g.atomic) atomicAdd(&g.C[off], val);
-                else g.C[off] = val;
+                if (g.atomic) atomicAdd(row + outN[nl], val);
+                else row[outN[nl]] = val;
             }
     }
 }

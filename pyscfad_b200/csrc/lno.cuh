@@ -4,118 +4,610 @@
 // the energy of lnoccsdt_contract (pyscfadlib/pyscfadlib/vjp/cc/lno_ccsd_t.c:6-29
 // with the job weights of lno_ccsd_t.c:73-94 and the 2/3 of
 // pyscfad/lno/ccsd_t.py:111; mat = identity gives the canonical E(T)), and
-// its adjoint (lnoccsdt_energy_vjp, lno_ccsd_t_vjp.c:74-122 and 400-566):
-//   Qbar = (ybar/3) Wt,   Wtbar = (ybar/3) Q,
-//   mat_bar[l,i] = sum WW[l..] Wtbar[i..],
-//   Zbar = Qbar / D,   Dbar = -Qbar Q / D,   Xbar = r3^T(Zbar),
-//   WWbar = P^T(Wtbar) + Xbar,   VVbar = Xbar / 2,
-//   wbar = sum_sigma WWbar(sigma pos),  vbar = sum_sigma VVbar(sigma pos).
+// its adjoint (lnoccsdt_energy_vjp, lno_ccsd_t_vjp.c:74-122 and 400-566).
 //
-// The projector couples all values of the first occupied index, which the
-// canonical epilogue's orbit tiles keep apart, so one chunk takes four passes
-// over FP64 work arrays in the staging layout (position = (tau; p, q, y, x,
-// r, z), p outermost, "column" = everything after p):
-//   1. tile forward  (orbit tiles in shared memory): WW -> B0, Q -> B2
-//   2. projection    (streaming over columns, all p of a column in a tile):
-//                    energy; with the adjoint also mat_bar, Dbar -> B2 (over Q),
-//                    Zbar -> B3 and P^T(Wtbar) -> B1
-//   3. tile adjoint  (orbit tiles): Xbar, WWbar, VVbar, their orbit sums;
-//                    wbar -> Wbar staging of the adjoint contractions, vbar -> B0
-//   4. V gradients   (streaming over (r, z) rows of vbar and Dbar): the V-term
-//                    gradients and the Dbar reduction into mo_energy_bar
-// An orbit tile is one occupied representative i >= j >= k with all its
-// permutations, times one triple of virtual sub-blocks with all its
-// orderings: closed under the simultaneous permutations of the orbit sums and
-// the virtual-only permutations of r3, so passes 1 and 3 gather only within
-// shared memory.
+// WW and Q are symmetric under simultaneous permutations of the occupied and
+// virtual indices, so one box of virtuals (a in A, b in B, c in C) with all
+// occupied triples (i, j, k) holds everything of a chunk; what the projector
+// breaks is restored by projecting each of the three occupied slots:
+//   E    = g sum_box PW Q,  PW = sum over slots of the projected WW,
+//   PQ   = sum over slots of the transposed projector on Q,
+//   Zbar = f PW / D,  Dbar = -(g ybar / f) Zbar Q,  WWbar = f PQ + r3(Zbar),
+//   VVbar = r3(Zbar) / 2,
+//   mat_bar[l,i] = g ybar sum over slots of sum WW[..l..] Q[..i..]
+// with f = 2 ybar / 3 and g = (distinct orderings of the blocks A, B, C) / 9.  Every
+// raw amplitude of an ordering of the blocks is one box position permuted, and
+// its adjoint is that position's WWbar (VVbar); with equal blocks the box holds
+// each value once per permutation, hence g.
+//
+// Three kernels over FP64 arrays [i][j][k][e] of the box (e: 512 slots per
+// triple of 8-wide sub-ranges, in the thread order of the orbit kernels; slots
+// beyond a short sub-range hold zeros):
+//   k_lno_fwd   an occupied representative and a sub-range triple per CTA: six
+//               orderings of two elements per thread, WW and Q of the six
+//               occupied orders out as whole lines
+//   k_lno_proj  one occupied slot, streaming over columns: three products on the
+//               FP64 tensor cores; the slots add up over three launches, the last
+//               one forms Zbar
+//   k_lno_adj   as k_lno_fwd: r3, Wbar and V-term gradients (FP64 sums) written
+//               back over the leading regions, orbital-energy gradients
+// Bytes per raw amplitude: 4 or 8 + 16/6, 128/6, 24/6 + 4 or 8: a third of what
+// the four passes over arrays of all orderings took (104 and 120), which were
+// bound by shared-memory gathers and memory latency.  Measured, nocc 14 nvir 96
+// mixed, forward / projection / adjoint (+ V gradients): 42.9 / 44.0 / 49.4 + 29.4 ms
+// to 11.6 / 20.6 / 18.0; nocc 9 nvir 45 FP64: 4.7 / 2.2 / 4.5 + 2.7 to 1.2 / 2.6 / 1.4 ms.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "f2m.cuh"
+#include "gemm_fp64.cuh"
 
 namespace tb {
 
 constexpr int kLnoMaxO = 64;    // largest nocc of the LNO path (projection tiles)
-constexpr int kLnoMaxTv = 16;   // largest virtual block
 constexpr int kLnoThreads = 256;
-constexpr int kLnoTile = 32;    // columns per projection tile
-constexpr int kLnoSB = 4;       // virtual sub-block edge of an orbit tile
-constexpr int kLnoRegion = kLnoSB * kLnoSB * kLnoSB;
-// slab layout in shared memory: slot s at s + 3 (s / 16) (fewer bank conflicts
-// on the permuted gathers), 73 doubles per slab
-constexpr int kLnoSlab = kLnoRegion + 3 * (kLnoRegion / 16 - 1) + 1;
-__host__ __device__ constexpr int lno_pad(int slot) { return slot + 3 * (slot >> 4); }
-constexpr int kLnoMaxSub = 64;  // sub-block triples per chunk: (16/4)^3
-constexpr int kLnoWaves = 4;    // waves of the streaming passes
-
-struct LnoSub {
-    int st[3];
-    int len[3];
-};
 
 struct LnoArgs {
-    Dims d;
-    ChunkDesc ch;
-    signed char tau_of[27];                // ordering of (slot x, slot y, slot z); slots 0..2 = A, B, C
-    int nsub;
-    LnoSub sub[kLnoMaxSub];
-    const int *ijk;                        // occupied representatives i >= j >= k
-    const void *S;                         // raw w of the chunk (staging, FP64 or FP32)
-    double *B0, *B1, *B2, *B3;             // chunk-shaped work arrays (staging layout)
+    int o, v;
+    int nsub;                   // sub-range triples of the box (all of them)
+    F2mSub sub[kF2mMaxSub];     // pat: equal blocks; regions as in the canonical epilogue
+    int n_ijk;
+    const int *ijk;             // occupied representatives i >= j >= k
+    const void *S;              // raw w of the chunk (blocked staging, FP64 or FP32)
+    double *WW, *Q, *PW, *PQ;   // box arrays; PW becomes Zbar
     const double *mat, *mo_e, *t1, *t2, *ovov, *fvo;
-    void *SW;                              // Wbar staging per ordering: FP64 [y][p][x][q][rzp], or
-                                           // 16-bit hi/lo planes [h][y][p][x][q][rzp] at 2 swoff
-    const double *wscale;                  // power-of-two scale of the fp16 split
+    void *SW;                   // Wbar staging per ordering: FP64 [y][p][x][q][rzp], or
+                                // 16-bit hi/lo planes [h][y][p][x][q][rzp] at 2 swoff
+    const double *wscale;       // power-of-two scale of the fp16 split
     double *mat_bar, *mo_bar, *t1_bar, *t2_bar, *ovov_bar, *fvo_bar;
-    double ybar;
+    double ybar, f, g;
     int want_grad;
-    double *part;                          // energy partials, gridDim.x * nperm
-    int n_ijk;                             // occupied representatives
+    double *part;               // energy partials, one per block and slot
 };
 
-// r3 on the virtual indices (pyscfad/cc/ccsd_t_slow.py:84-87):
-// Z(j) = sum_s c_s X(i) with i[s[k]] = j[k], s = (0,1,2), (1,2,0), (2,0,1),
-// (2,1,0), (0,2,1), (1,0,2) (the orderings of lno_build_tables).
-__constant__ double c_r3_coef[6] = {4.0, 1.0, 1.0, -2.0, -2.0, -2.0};
-
-__device__ __forceinline__ int lno_slot(const ChunkDesc &ch, int g) {
-    return (g >= ch.base[0] && g < ch.base[0] + ch.nabc[0]) ? 0
-           : (g >= ch.base[1] && g < ch.base[1] + ch.nabc[1]) ? 1
-                                                               : 2;
+// ---------------------------------------------------------------------------
+// orbit kernels: two elements (a, b, c), (a + 4, b, c) per thread, as in f2m.cuh
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void lno_element(int t, int &a, int &b, int &c) {
+    a = ((t >> 4) & 1) | (((t >> 7) & 1) << 1);
+    b = ((t >> 2) & 3) | (((t >> 6) & 1) << 2);
+    c = (t & 3) | (((t >> 5) & 1) << 2);
 }
 
-__device__ __forceinline__ double lno_warp_sum(double s) {
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    return s;
+// 64-entry table block of 16-byte entries: eight lanes of a gather hit eight banks
+__device__ __forceinline__ int lno_tab(int x, int y) { return y * 8 + (x ^ ((y & 1) << 2) ^ (y & 2)); }
+
+// FP64 V-term tables of an item: {ovov[p,x,q,y], t2[q,p,y,x]} per (rho, pi), {t1[r,z], fvo[z,r]}
+__device__ __forceinline__ void lno_load_tables(const LnoArgs &A, const F2mSub &R, int i0, int i1, int i2,
+                                                double2 *tab, double2 *tf) {
+    const int o = A.o, v = A.v;
+    double *ts = reinterpret_cast<double *>(tab);
+#pragma unroll 3
+    for (int e = threadIdx.x; e < 36 * 64; e += kLnoThreads) {
+        const int blk = e >> 6, hi = (e >> 3) & 7, lo = e & 7;
+        int pr[3], pp[3];
+        perm_of(blk / 6, pr);
+        perm_of(blk % 6, pp);
+        const int p = sel3(i0, i1, i2, pr[0]), q = sel3(i0, i1, i2, pr[1]);
+        const int lx = sel3(R.len[0], R.len[1], R.len[2], pp[0]), ly = sel3(R.len[0], R.len[1], R.len[2], pp[1]);
+        const int sx = sel3(R.st[0], R.st[1], R.st[2], pp[0]), sy = sel3(R.st[0], R.st[1], R.st[2], pp[1]);
+        // the fast index of each factor in turn runs over the lanes
+        ts[2 * (blk * 64 + lno_tab(hi, lo))] =
+            hi < lx && lo < ly ? __ldg(&A.ovov[(((long long)p * v + sx + hi) * o + q) * v + sy + lo]) : 0.0;
+        ts[2 * (blk * 64 + lno_tab(lo, hi)) + 1] =
+            lo < lx && hi < ly ? __ldg(&A.t2[(((long long)q * o + p) * v + sy + hi) * v + sx + lo]) : 0.0;
+    }
+    for (int e = threadIdx.x; e < 72; e += kLnoThreads) {
+        const int r = sel3(i0, i1, i2, e / 24), s = (e >> 3) % 3, zl = e & 7;
+        const int z = sel3(R.st[0], R.st[1], R.st[2], s) + zl;
+        const bool in = zl < sel3(R.len[0], R.len[1], R.len[2], s);
+        tf[e] = in ? make_double2(__ldg(&A.t1[(long long)r * v + z]), __ldg(&A.fvo[(long long)z * o + r]))
+                   : make_double2(0.0, 0.0);
+    }
+}
+
+// box index of ordering s at slot e: the occupied index paired with virtual slot c is ijk[t] with s[t] = c
+template <int S>
+__device__ __forceinline__ long long lno_box(int o, long long ne, int i0, int i1, int i2) {
+    int ps[3] = {0, 0, 0}, inv[3] = {0, 0, 0};
+    perm_of(S, ps);
+    inv[ps[0]] = 0;
+    inv[ps[1]] = 1;
+    inv[ps[2]] = 2;
+    const int ids[3] = {i0, i1, i2};
+    return (((long long)ids[inv[0]] * o + ids[inv[1]]) * o + ids[inv[2]]) * ne;
+}
+
+template <typename F>
+__device__ __forceinline__ void lno_for_s(F &&f) {
+    f(std::integral_constant<int, 0>{});
+    f(std::integral_constant<int, 1>{});
+    f(std::integral_constant<int, 2>{});
+    f(std::integral_constant<int, 3>{});
+    f(std::integral_constant<int, 4>{});
+    f(std::integral_constant<int, 5>{});
+}
+
+__device__ __forceinline__ void lno_r3(const double (&x)[6], double (&z)[6]) {
+#pragma unroll
+    for (int s = 0; s < 6; s++)
+        z[s] = 4.0 * x[s] + x[perm_compose(s, 4)] + x[perm_compose(s, 3)] -
+               2.0 * (x[perm_compose(s, 5)] + x[perm_compose(s, 1)] + x[perm_compose(s, 2)]);
+}
+
+inline size_t lno_fwd_smem() { return (36 * 64 + 72) * sizeof(double2); }
+
+template <typename StageT>
+__global__ void __launch_bounds__(kLnoThreads, 2) k_lno_fwd(const __grid_constant__ LnoArgs A) {
+    extern __shared__ __align__(16) uint8_t lno_raw[];
+    double2 *tab = reinterpret_cast<double2 *>(lno_raw), *tf = tab + 36 * 64;
+    const int o = A.o;
+    // sub-range triple fastest: the CTAs of one representative run together
+    const int rep = blockIdx.x / A.nsub, sub = blockIdx.x - rep * A.nsub;
+    const F2mSub &R = A.sub[sub];
+    const int i0 = A.ijk[3 * rep], i1 = A.ijk[3 * rep + 1], i2 = A.ijk[3 * rep + 2];
+    int ca, cb, cc;
+    lno_element(threadIdx.x, ca, cb, cc);
+    const bool ok0 = ca < R.len[0] && cb < R.len[1] && cc < R.len[2];
+    const bool ok1 = ok0 && ca + 4 < R.len[0];
+    lno_load_tables(A, R, i0, i1, i2, tab, tf);
+    const StageT *S = reinterpret_cast<const StageT *>(A.S);
+    const int loc[3] = {ca, cb, cc};
+    int w0[6], w1[6], t0[6];   // this thread's positions in the regions (elements a, a + 4) and tables
+#pragma unroll
+    for (int pi = 0; pi < 6; pi++) {
+        int pp[3] = {0, 0, 0};
+        perm_of(pi, pp);
+        const int x = loc[pp[0]], y = loc[pp[1]], z = loc[pp[2]];
+        const int ex = R.len[pp[0]], ez = R.len[pp[2]];
+        const bool swz = sizeof(StageT) == 4 && ex == 8 && ez == 8;
+        const int dx = pp[0] == 0 ? 4 : 0, dy = pp[1] == 0 ? 4 : 0, dz = pp[2] == 0 ? 4 : 0;
+        const int s0 = (x * ez + z) ^ (swz ? f2m_row_swizzle(y) : 0);
+        const int s1 = ((x + dx) * ez + z + dz) ^ (swz ? f2m_row_swizzle(y + dy) : 0);
+        w0[pi] = ok0 ? y * ex * ez + s0 : 0;
+        w1[pi] = ok1 ? (y + dy) * ex * ez + s1 : w0[pi];
+        t0[pi] = lno_tab(x, y);
+    }
+    double WW[2][6], VV[2][6];
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+#pragma unroll
+        for (int s = 0; s < 6; s++) WW[e][s] = VV[e][s] = 0.0;
+    __syncthreads();
+#pragma unroll
+    for (int rho = 0; rho < 6; rho++) {
+        int pr[3] = {0, 0, 0};
+        perm_of(rho, pr);
+        const int ids[3] = {i0, i1, i2};
+        const long long idx = ((long long)ids[pr[0]] * o + ids[pr[1]]) * o + ids[pr[2]];
+        const double2 *tr = tf + pr[2] * 24;
+        const double2 tz[3] = {tr[ca], tr[8 + cb], tr[16 + cc]}, tz4 = tr[(ca + 4) & 7];
+#pragma unroll
+        for (int pi = 0; pi < 6; pi++) {
+            const int s = f2m_sof(pi, rho);
+            int pp[3] = {0, 0, 0};
+            perm_of(pi, pp);
+            const StageT *base = S + R.pi[pi].s0 + idx * R.pi[pi].rs;
+            WW[0][s] += (double)__ldg(base + w0[pi]);
+            WW[1][s] += (double)__ldg(base + w1[pi]);
+            const double2 *tp = tab + (rho * 6 + pi) * 64;
+            // a + 4 in slot x or y of the table block
+            const double2 ot0 = tp[t0[pi]];
+            const double2 ot1 = pp[0] == 0 ? tp[t0[pi] ^ 4] : (pp[1] == 0 ? tp[t0[pi] ^ 32] : ot0);
+            const double2 z0 = tz[pp[2]], z1 = pp[2] == 0 ? tz4 : tz[pp[2]];
+            VV[0][s] += ot0.x * z0.x + ot0.y * z0.y;
+            VV[1][s] += ot1.x * z1.x + ot1.y * z1.y;
+        }
+    }
+    const double *ev = A.mo_e + o;
+    const double e_occ = A.mo_e[i0] + A.mo_e[i1] + A.mo_e[i2];
+    const double e_bc = ok0 ? ev[R.st[1] + cb] + ev[R.st[2] + cc] : 0.0;
+    const long long ne = (long long)A.nsub * 512;
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const bool ok = e == 0 ? ok0 : ok1;
+        double X[6], Z[6];
+#pragma unroll
+        for (int s = 0; s < 6; s++) X[s] = WW[e][s] + 0.5 * VV[e][s];
+        lno_r3(X, Z);
+        const double rD = ok ? 1.0 / (e_occ - ev[R.st[0] + ca + 4 * e] - e_bc) : 0.0;
+        const int slot = sub * 512 + e * 256 + threadIdx.x;
+        lno_for_s([&](auto sc) {
+            constexpr int s = decltype(sc)::value;
+            const long long at = lno_box<s>(o, ne, i0, i1, i2) + slot;
+            A.WW[at] = ok ? WW[e][s] : 0.0;
+            A.Q[at] = ok ? Z[s] * rD : 0.0;
+        });
+    }
 }
 
 // ---------------------------------------------------------------------------
-// orbit tiles
+// projection of one occupied slot (0, 1, 2), streaming over columns
 // ---------------------------------------------------------------------------
-// Candidate region c = 6 pi + rho: occupied triple (ijk[pi0], ijk[pi1], ijk[pi2])
-// and virtual sub-ranges (U[rho0], U[rho1], U[rho2]).  Candidates with the same
-// triple and ranges hold the same positions; the first of them is "primary"
-// and owns a 4x4x4 slab of the shared arrays.  A position is (slab, slot),
-// slot = (4 l0 + l1) 4 + l2 for local virtual indices l.  The gather tables
-// give, per candidate and permutation, the candidate holding the permuted
-// position, and per slot and permutation the permuted slot.
-constexpr int kLnoIt = (36 * kLnoRegion + kLnoThreads - 1) / kLnoThreads;   // positions per thread
+// Rows: all o values of the slot, a row stride apart; columns: the other two
+// occupied indices and e, COLS at a time (consecutive e).  Per tile
+//   PW[i] = sum_l mat[l,i] WW[l],  energy += PW Q,  PQ[l] = sum_i mat[l,i] Q[i],
+//   Gram += WW Q^T
+// on the FP64 tensor cores (per 8x8 output tile a thread holds D[g][2t],
+// D[g][2t+1], A[g][t] and B[t][g] of each k-step, g = lane / 4, t = lane % 4).
+// FIRST: PW and PQ are stored, else added to; slot 0 runs last and forms Zbar
+// and f PQ.  Streams WW, Q and the running sums: HBM; wide tiles at small o and the
+// running sums loaded before the tile's copies are waited for keep enough bytes
+// in flight.  The Gram tiles belong to warps; every CTA adds its o x o sums to
+// mat_bar once, so the grid is what is resident (those atomics all meet on o^2
+// addresses: with the columns of four Gram tiles split over eight warps the
+// kernel took twice as long).
+template <int COLS>
+struct LnoProj {
+    static constexpr int LD = COLS + 4;   // conflict-free fragment loads
+    static constexpr int MAXO = 2048 / COLS;                      // 16, 32, 64
+    static constexpr int NG = (MAXO / 8) * (MAXO / 8);            // Gram tiles
+    static constexpr int GW = NG < kLnoThreads / 32 ? 1 : NG / (kLnoThreads / 32);   // Gram tiles per warp
+    static constexpr int TW = (MAXO / 8) * (COLS / 8) / (kLnoThreads / 32);   // output tiles per warp
+    static size_t smem(int o) {
+        const int rows = (o + 7) / 8 * 8;
+        return (size_t)(4 * rows * LD + o * o + kLnoMaxO + 2 * COLS) * sizeof(double);
+    }
+};
 
-// Gather tables, the same for every tile (built on the host, lno_build_tables):
-// per candidate and permutation the candidate holding the permuted position,
-// per permutation and slot the permuted slot; sigma runs over the six
-// simultaneous permutations, s over the six terms of r3 (0: forward
-// i[m] = j[sinv[m]], 1: adjoint j[k] = i[s[k]]).
+template <int COLS>
+__global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_constant__ LnoArgs A, int slot, int first) {
+    using C = LnoProj<COLS>;
+    constexpr int LD = C::LD, CT = COLS / 8;
+    extern __shared__ __align__(16) uint8_t lno_raw[];
+    const int o = A.o, o4 = (o + 3) & ~3, o8 = (o + 7) / 8, rows = 8 * o8;
+    double *sw_b = reinterpret_cast<double *>(lno_raw), *sq_b = sw_b + 2 * rows * LD, *sM = sq_b + 2 * rows * LD;
+    double *s_eo = sM + o * o, *s_ecol_b = s_eo + kLnoMaxO;
+    __shared__ double red[kLnoThreads / 32];
+    const long long ne = (long long)A.nsub * 512;
+    const long long rstride = slot == 0 ? o * o * ne : (slot == 1 ? o * ne : ne);
+    const int per = (int)(ne / COLS), ntile = o * o * per;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int fg = lane >> 2, ft = lane & 3;
+    const bool grad = A.want_grad != 0, last = slot == 0;
+    const double gy = A.g * A.ybar;
+    for (int k = threadIdx.x; k < o * o; k += blockDim.x) sM[k] = A.mat[k];
+    for (int k = threadIdx.x; k < o; k += blockDim.x) s_eo[k] = A.mo_e[k];
+    const int ngram = o8 * o8;
+    double acc[C::GW][2];
+#pragma unroll
+    for (int k = 0; k < C::GW; k++) acc[k][0] = acc[k][1] = 0.0;
+    double en = 0.0;
+    // first element of tile t (row 0)
+    auto tile_base = [&](int t) -> long long {
+        const int oth = t / per;
+        const long long e0 = (long long)(t - oth * per) * COLS;
+        return slot == 1 ? (long long)(oth / o) * o * o * ne + (oth % o) * ne + e0
+                         : (slot == 0 ? oth * ne : oth * o * ne) + e0;
+    };
+    auto issue = [&](int t, int b) {
+        const long long base = tile_base(t);
+        double *sw = sw_b + b * rows * LD, *sq = sq_b + b * rows * LD;
+        for (int e = threadIdx.x; e < rows * (COLS / 2); e += blockDim.x) {
+            const int l = e / (COLS / 2), j = e % (COLS / 2) * 2;
+            const long long at = base + (l < o ? l * rstride + j : 0);
+            const int bytes = l < o ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sw + l * LD + j)), "l"(A.WW + at), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sq + l * LD + j)), "l"(A.Q + at), "r"(bytes) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (grad && last && threadIdx.x < COLS) {
+            // energies of the column: the other two occupied indices, a, b and c
+            const int oth = t / per, e = (t - oth * per) * COLS + threadIdx.x;
+            const F2mSub &R = A.sub[e >> 9];
+            int a, b2, c;
+            lno_element(e & 255, a, b2, c);
+            a += 4 * ((e >> 8) & 1);
+            double ec = -1.0;   // a slot beyond a short range: any non-zero value
+            if (a < R.len[0] && b2 < R.len[1] && c < R.len[2]) {
+                const double *ev = A.mo_e + o;
+                ec = A.mo_e[oth / o] + A.mo_e[oth % o] - ev[R.st[0] + a] - ev[R.st[1] + b2] - ev[R.st[2] + c];
+            } else {
+                ec = -1e30;
+            }
+            s_ecol_b[b * COLS + threadIdx.x] = ec;
+        }
+    };
+    int buf = 0;
+    if ((int)blockIdx.x < ntile) issue(blockIdx.x, 0);
+    for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
+        if (t + (int)gridDim.x < ntile) issue(t + gridDim.x, buf ^ 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");   // keeps the wait count uniform
+        const long long base = tile_base(t);
+        double2 pw[C::TW], pq[C::TW];   // running sums of this thread's output positions
+#pragma unroll
+        for (int k = 0; k < C::TW; k++) {
+            const int tile = warp + k * (kLnoThreads / 32), i = tile / CT * 8 + fg;
+            pw[k] = pq[k] = double2{0.0, 0.0};
+            if (grad && !first && i < o) {
+                const long long at = base + i * rstride + tile % CT * 8 + 2 * ft;
+                pw[k] = *reinterpret_cast<const double2 *>(A.PW + at);
+                pq[k] = *reinterpret_cast<const double2 *>(A.PQ + at);
+            }
+        }
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const double *sw = sw_b + buf * rows * LD, *sq = sq_b + buf * rows * LD;
+        const double *s_ecol = s_ecol_b + buf * COLS;
+#pragma unroll
+        for (int k = 0; k < C::TW; k++) {
+            const int tile = warp + k * (kLnoThreads / 32);
+            if (tile >= o8 * CT) break;
+            const int nt = tile % CT, i = tile / CT * 8 + fg, cl = nt * 8 + 2 * ft;
+            const long long at = base + i * rstride + cl;
+            double u0 = 0.0, u1 = 0.0, p0 = 0.0, p1 = 0.0;
+            for (int k0 = 0; k0 < o4; k0 += 4) {
+                const int l = k0 + ft;
+                const bool in = i < o && l < o;
+                dmma_884(u0, u1, in ? sM[l * o + i] : 0.0, sw[l * LD + nt * 8 + fg]);
+                if (grad) dmma_884(p0, p1, in ? sM[i * o + l] : 0.0, sq[l * LD + nt * 8 + fg]);
+            }
+            if (i < o) {
+                en += u0 * sq[i * LD + cl] + u1 * sq[i * LD + cl + 1];
+                if (grad) {
+                    double2 w = pw[k], r = pq[k];
+                    w.x += u0;
+                    w.y += u1;
+                    r.x += p0;
+                    r.y += p1;
+                    if (last) {
+                        w.x = A.f * w.x / (s_eo[i] + s_ecol[cl]);
+                        w.y = A.f * w.y / (s_eo[i] + s_ecol[cl + 1]);
+                        r.x *= A.f;
+                        r.y *= A.f;
+                    }
+                    *reinterpret_cast<double2 *>(A.PW + at) = w;
+                    *reinterpret_cast<double2 *>(A.PQ + at) = r;
+                }
+            }
+        }
+        if (grad) {
+            // Gram[l, i] += sum_c WW[l, c] Q[i, c]
+#pragma unroll
+            for (int k = 0; k < C::GW; k++) {
+                const int gt = warp + k * (kLnoThreads / 32);
+                if (gt < ngram) {
+                    const int mt = gt / o8, nt = gt % o8;
+#pragma unroll 8
+                    for (int k0 = 0; k0 < COLS; k0 += 4)
+                        dmma_884(acc[k][0], acc[k][1], sw[(mt * 8 + fg) * LD + k0 + ft], sq[(nt * 8 + fg) * LD + k0 + ft]);
+                }
+            }
+        }
+        __syncthreads();   // buffer buf is refilled two tiles from now
+        buf ^= 1;
+    }
+    for (int off = 16; off > 0; off >>= 1) en += __shfl_xor_sync(0xffffffffu, en, off);
+    if (lane == 0) red[warp] = en;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < kLnoThreads / 32; w++) s += red[w];
+        A.part[slot * gridDim.x + blockIdx.x] = A.g * s;
+    }
+    if (!grad) return;
+#pragma unroll
+    for (int k = 0; k < C::GW; k++) {
+        const int gt = warp + k * (kLnoThreads / 32);
+        if (gt < ngram) {
+            const int l = (gt / o8) * 8 + fg;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int i = (gt % o8) * 8 + 2 * ft + h;
+                const double gv = h ? acc[k][1] : acc[k][0];
+                if (l < o && i < o && gv != 0.0) atomicAdd(&A.mat_bar[l * o + i], gy * gv);
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// adjoint of the raw amplitudes, V-term and orbital-energy gradients
+// ---------------------------------------------------------------------------
+// SPLIT 0: FP64 Wbar; 1: fp16 hi/lo of wbar * wscale (exact power of two); 2: bf16
+// hi/lo, unscaled -- the operand formats of the adjoint contractions.
+template <int SPLIT>
+struct LnoAdj {
+    using W = typename std::conditional<SPLIT == 0, double, uint32_t>::type;   // FP64, or hi and lo halves
+    static constexpr size_t TABLES = (36 * 64 + 72) * sizeof(double2);
+    static constexpr size_t SMEM = TABLES + 6 * 512 * (sizeof(double) + sizeof(W));
+};
+
+template <int SPLIT>
+__global__ void __launch_bounds__(kLnoThreads, 2) k_lno_adj(const __grid_constant__ LnoArgs A) {
+    using WT = typename LnoAdj<SPLIT>::W;
+    extern __shared__ __align__(16) uint8_t lno_raw[];
+    double2 *tab = reinterpret_cast<double2 *>(lno_raw), *tf = tab + 36 * 64;
+    double *sV = reinterpret_cast<double *>(lno_raw + LnoAdj<SPLIT>::TABLES);
+    WT *sW = reinterpret_cast<WT *>(sV + 6 * 512);
+    __shared__ int s_res[3][8];
+    __shared__ double s_part[8][12];
+    const int o = A.o, v = A.v;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rep = blockIdx.x / A.nsub, sub = blockIdx.x - rep * A.nsub;
+    const F2mSub &R = A.sub[sub];
+    const int i0 = A.ijk[3 * rep], i1 = A.ijk[3 * rep + 1], i2 = A.ijk[3 * rep + 2];
+    const int opat = (i0 == i2) ? 3 : (i0 == i1 ? 1 : (i1 == i2 ? 2 : 0));
+    const int vpat = R.pat;
+    const int l0 = R.len[0], l1 = R.len[1], l2 = R.len[2];
+    if (tid < 24) s_res[tid >> 3][tid & 7] = f2m_res(tid >> 3, tid & 7);
+    int ca, cb, cc;
+    lno_element(tid, ca, cb, cc);
+    const int gidx = f2m_res(0, ca) ^ f2m_res(1, cb) ^ f2m_res(2, cc);
+    const long long ne = (long long)A.nsub * 512;
+    const float wsc = SPLIT == 1 ? (float)*A.wscale : 1.0f;
+    // Dbar = -(g ybar / f) Zbar Q, each occupied order once
+    const double dfac = -(A.g * A.ybar / A.f) / (opat == 0 ? 1.0 : (opat == 3 ? 6.0 : 2.0));
+    double dd[2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const int slot = sub * 512 + e * 256 + tid;
+        double Z[6], P[6], X[6];
+        double ds = 0.0;
+        lno_for_s([&](auto sc) {
+            constexpr int s = decltype(sc)::value;
+            const long long at = lno_box<s>(o, ne, i0, i1, i2) + slot;
+            Z[s] = __ldg(&A.PW[at]);
+            P[s] = __ldg(&A.PQ[at]);
+            ds += Z[s] * __ldg(&A.Q[at]);
+        });
+        dd[e] = A.f != 0.0 ? dfac * ds : 0.0;
+        lno_r3(Z, X);
+        const int g = e == 0 ? gidx : gidx ^ 4;
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            const double wb = P[s] + X[s];
+            sV[s * 512 + g] = 0.5 * X[s];
+            if constexpr (SPLIT == 0) sW[s * 512 + g] = wb;
+            else sW[s * 512 + g] = f2m_split<SPLIT>((float)wb, wsc);
+        }
+    }
+    lno_load_tables(A, R, i0, i1, i2, tab, tf);
+    {
+        // -dE/d e of the element's virtuals: per-warp sums over the other two slots
+        double dc = dd[0] + dd[1], db = dc;
+        dc += __shfl_xor_sync(0xffffffffu, dc, 4);
+        dc += __shfl_xor_sync(0xffffffffu, dc, 8);
+        dc += __shfl_xor_sync(0xffffffffu, dc, 16);
+        db += __shfl_xor_sync(0xffffffffu, db, 1);
+        db += __shfl_xor_sync(0xffffffffu, db, 2);
+        db += __shfl_xor_sync(0xffffffffu, db, 16);
+        const bool up = lane & 1;
+        double da = (up ? dd[1] : dd[0]) + __shfl_xor_sync(0xffffffffu, up ? dd[0] : dd[1], 1);
+        da += __shfl_xor_sync(0xffffffffu, da, 2);
+        da += __shfl_xor_sync(0xffffffffu, da, 4);
+        da += __shfl_xor_sync(0xffffffffu, da, 8);
+        if (lane < 4) s_part[warp][lane] = dc;
+        if ((lane & 19) == 0) s_part[warp][4 + (lane >> 2)] = db;
+        if ((lane & 14) == 0) s_part[warp][8 + (lane >> 4) + 2 * (lane & 1)] = da;
+    }
+    __syncthreads();
+    if (warp == 0 && lane < 24) {
+        // warps with bit 0, 1, 2 = bit 2 of c, bit 2 of b, bit 1 of a (lanes: c, b, a)
+        double acc = 0.0;
+        const int l = lane & 7;
+        for (int u = 0; u < 4; u++)
+            acc += lane < 8 ? s_part[(l >> 2) + 2 * u][l & 3]
+                   : lane < 16 ? s_part[2 * (l >> 2) + (u & 1) + 4 * (u >> 1)][4 + (l & 3)]
+                               : s_part[4 * ((l >> 1) & 1) + u][8 + (l & 1) + 2 * (l >> 2)];
+        double tot = acc;
+        tot += __shfl_xor_sync(0x00ffffffu, tot, 1);
+        tot += __shfl_xor_sync(0x00ffffffu, tot, 2);
+        tot += __shfl_xor_sync(0x00ffffffu, tot, 4);
+        const int slot = 2 - (lane >> 3);
+        if (l < sel3(l0, l1, l2, slot)) atomicAdd(&A.mo_bar[o + sel3(R.st[0], R.st[1], R.st[2], slot) + l], -acc);
+        if (lane < 3) atomicAdd(&A.mo_bar[sel3(i0, i1, i2, lane)], tot);
+    }
+    // ---- write-back: a region per warp, runs (yy, xx) of lane and u ----
+    const int nro = f2m_nlead(opat), ntask = f2m_nlead(vpat) * nro;
+    const int xx = lane & 7, y4 = lane >> 3;
+#pragma unroll 1
+    for (int task = 7 - warp; task < ntask; task += 8) {
+        const int pi = f2m_lead(vpat, task / nro), rho = f2m_lead(opat, task % nro);
+        int pp[3], pr[3];
+        perm_of(pi, pp);
+        perm_of(rho, pr);
+        const int p = sel3(i0, i1, i2, pr[0]), q = sel3(i0, i1, i2, pr[1]), r = sel3(i0, i1, i2, pr[2]);
+        const int lx = sel3(l0, l1, l2, pp[0]), ly = sel3(l0, l1, l2, pp[1]), lz = sel3(l0, l1, l2, pp[2]);
+        const int inv0 = pr[0] == 0 ? 0 : (pr[1] == 0 ? 1 : 2), inv1 = pr[0] == 1 ? 0 : (pr[1] == 1 ? 1 : 2);
+        const int s = perm_index(sel3(pp[0], pp[1], pp[2], inv0), sel3(pp[0], pp[1], pp[2], inv1));
+        const F2mPi &D = R.pi[pi];
+        const long long wl = D.w0 + (long long)p * D.wp + (long long)q * D.rzp + (long long)r * D.tz + (long long)xx * D.wx;
+        const double2 *trow = tf + (pr[2] * 3 + pp[2]) * 8;
+        const double2 *tp = tab + (rho * 6 + pi) * 64;
+        const int x = sel3(R.st[0], R.st[1], R.st[2], pp[0]) + xx;
+        const int y0 = sel3(R.st[0], R.st[1], R.st[2], pp[1]);
+        const int gx = s * 512, gxx = s_res[pp[0]][xx];
+        double col[16];
+#pragma unroll
+        for (int c = 0; c < 16; c++) col[c] = 0.0;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int yy = y4 + 4 * u;
+            const int g0 = gxx ^ s_res[pp[1]][yy];
+            const bool in = xx < lx && yy < ly;
+            int gz[8];
+#pragma unroll
+            for (int z = 0; z < 8; z++) gz[z] = gx + (g0 ^ s_res[pp[2]][z]);
+            if (in) {
+                if constexpr (SPLIT == 0) {
+                    double *dst = reinterpret_cast<double *>(A.SW) + wl + (long long)yy * D.wy;
+                    if (lz == 8) {
+#pragma unroll
+                        for (int z = 0; z < 8; z += 2)
+                            *reinterpret_cast<double2 *>(dst + z) = make_double2(sW[gz[z]], sW[gz[z + 1]]);
+                    } else {
+#pragma unroll
+                        for (int z = 0; z < 4; z++)
+                            if (z < lz) dst[z] = sW[gz[z]];
+                    }
+                } else {
+                    uint16_t *dst = reinterpret_cast<uint16_t *>(A.SW) + wl + (long long)yy * D.wy;
+                    uint32_t pk[8];
+#pragma unroll
+                    for (int z = 0; z < 8; z++) pk[z] = (uint32_t)sW[gz[z]];
+                    if (lz == 8) {
+                        uint4 hi, lo;
+                        hi.x = __byte_perm(pk[0], pk[1], 0x5410); lo.x = __byte_perm(pk[0], pk[1], 0x7632);
+                        hi.y = __byte_perm(pk[2], pk[3], 0x5410); lo.y = __byte_perm(pk[2], pk[3], 0x7632);
+                        hi.z = __byte_perm(pk[4], pk[5], 0x5410); lo.z = __byte_perm(pk[4], pk[5], 0x7632);
+                        hi.w = __byte_perm(pk[6], pk[7], 0x5410); lo.w = __byte_perm(pk[6], pk[7], 0x7632);
+                        *reinterpret_cast<uint4 *>(dst) = hi;
+                        *reinterpret_cast<uint4 *>(dst + D.half) = lo;
+                    } else {
+#pragma unroll
+                        for (int z = 0; z < 4; z++)
+                            if (z < lz) {
+                                dst[z] = (uint16_t)pk[z];
+                                dst[D.half + z] = (uint16_t)(pk[z] >> 16);
+                            }
+                    }
+                }
+            }
+            // v = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r] (results and tables are zero beyond a short range)
+            const double2 ot = tp[lno_tab(xx, yy)];
+            double r1 = 0.0, r2 = 0.0;
+#pragma unroll
+            for (int z = 0; z < 8; z++) {
+                const double vb = sV[gz[z]];
+                const double2 tr = trow[z];
+                r1 += vb * tr.x;
+                r2 += vb * tr.y;
+                col[z] += vb * ot.x;
+                col[8 + z] += vb * ot.y;
+            }
+            if (in) {
+                atomicAdd(&A.ovov_bar[(((long long)p * v + x) * o + q) * v + y0 + yy], r1);
+                atomicAdd(&A.t2_bar[(((long long)q * o + p) * v + y0 + yy) * v + x], r2);
+            }
+        }
+        // column sums t1_bar[r, z] (values 0-7), fvo_bar[z, r] (8-15) over the region's runs
+        const double cv = group_reduce_scatter<16, 32>(col, lane);
+        if (lane < 16 && (lane & 7) < lz) {
+            const int z = sel3(R.st[0], R.st[1], R.st[2], pp[2]) + (lane & 7);
+            if (lane < 8) atomicAdd(&A.t1_bar[(long long)r * v + z], cv);
+            else atomicAdd(&A.fvo_bar[(long long)z * o + r], cv);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// orbit bookkeeping as host tables (introspection only): candidate region
+// c = 6 pi + rho holds occupied triple (ijk[pi0], ijk[pi1], ijk[pi2]) over the
+// 4-wide virtual sub-ranges (U[rho0], U[rho1], U[rho2])
+// ---------------------------------------------------------------------------
+constexpr int kLnoSB = 4;
+constexpr int kLnoRegion = kLnoSB * kLnoSB * kLnoSB;
+__host__ __device__ constexpr int lno_pad(int slot) { return slot + 3 * (slot >> 4); }
+
 struct alignas(16) LnoTables {
     unsigned char symsl[6][kLnoRegion];      // 16-byte multiples first: copied as uint4
     unsigned char r3sl[2][6][kLnoRegion];
     unsigned char symc[36][6];
     unsigned char r3c[2][36][6];
 };
-// global (not constant) memory: threads read different entries at once
-__device__ LnoTables c_lno_tab;
-
 inline void lno_build_tables(LnoTables &t) {
     static const int r3p[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}, {0, 2, 1}, {1, 0, 2}};
     for (int cc = 0; cc < 36; cc++)
@@ -143,16 +635,11 @@ inline void lno_build_tables(LnoTables &t) {
         }
 }
 
-// Duplicate candidates depend only on which occupied indices coincide
-// (i == j, j == k) and which virtual sub-ranges coincide (U0 == U1, U1 == U2):
-// 16 patterns, each listing its slabs' candidates and every candidate's slab.
 struct LnoPattern {
     unsigned char nslab;
     unsigned char cand[36];
     unsigned char prim[36];
 };
-__device__ LnoPattern c_lno_pat[16];
-
 inline void lno_build_patterns(LnoPattern pats[16]) {
     for (int pid = 0; pid < 16; pid++) {
         const int eo01 = (pid >> 3) & 1, eo12 = (pid >> 2) & 1, ev01 = (pid >> 1) & 1, ev12 = pid & 1;
@@ -192,586 +679,5 @@ inline void lno_build_patterns(LnoPattern pats[16]) {
         P.nslab = (unsigned char)n;
     }
 }
-
-// A block handles one virtual sub-block triple and kLnoReps consecutive
-// occupied representatives.  What depends only on the virtual side (per
-// candidate ordering: staging bases and strides, validity, energies) is set
-// up once per block; per representative only the occupied offsets of the
-// slabs are recomputed (ALU and shared memory only).
-constexpr int kLnoReps = 16;
-
-struct LnoTile {
-    // per candidate (virtual side)
-    long long soff_v[36], swoff_v[36], swbase_c[36], plane_c[36];
-    int strP[36], strQ[36], swP[36], rzp[36], tz[36];
-    long long bov_v[36];
-    int bt2_v[36], bt1_v[36], bfv_v[36];
-    int roff[36][kLnoSB * kLnoSB];  // staging offset of local (l0, l1, 0)
-    int swro[36][kLnoSB * kLnoSB];  // Wbar staging offset of local (l0, l1, 0)
-    unsigned long long vmask_c[36]; // slots inside the ranges
-    unsigned char cpr[36][3];       // which sub-range fills each virtual slot
-    double ev_r[3][kLnoSB];         // virtual orbital energies of the three sub-ranges
-    double s_eo[kLnoMaxO];
-    unsigned char symc[36][6], r3c[2][36][6];
-    LnoPattern pat[16];
-    int ijk[kLnoReps][3];
-    // per slab (current representative)
-    long long soff[36], swoff[36], b_ov[36], b_t2[36];
-    int b_t1[36], b_fv[36], cand[36];
-    double eocc[36];
-    short symg[36][6], r3g[2][36][6];
-    int nslab, nrep;
-};
-
-// once per block: the virtual side of all 36 candidates
-__device__ void lno_tile_setup_block(const LnoArgs &A, LnoTile &T) {
-    const int o = A.d.o, v = A.d.v;
-    const LnoSub &U = A.sub[blockIdx.x];
-    const int r0 = blockIdx.y * kLnoReps;
-    if (threadIdx.x == 0) T.nrep = min(kLnoReps, A.n_ijk - r0);
-    for (int e = threadIdx.x; e < kLnoReps * 3; e += blockDim.x)
-        T.ijk[e / 3][e % 3] = r0 + e / 3 < A.n_ijk ? A.ijk[3 * r0 + e] : 0;
-    for (int e = threadIdx.x; e < o; e += blockDim.x) T.s_eo[e] = A.mo_e[e];
-    for (int e = threadIdx.x; e < 36; e += blockDim.x) T.cand[e] = 0;
-    for (int e = threadIdx.x; e < 3 * kLnoSB; e += blockDim.x) {
-        const int k = e / kLnoSB, l = e % kLnoSB;
-        T.ev_r[k][l] = l < U.len[k] ? A.mo_e[o + U.st[k] + l] : 0.0;
-    }
-    for (int e = threadIdx.x; e < 36 * 6; e += blockDim.x) {
-        T.symc[e / 6][e % 6] = c_lno_tab.symc[e / 6][e % 6];
-        T.r3c[0][e / 6][e % 6] = c_lno_tab.r3c[0][e / 6][e % 6];
-        T.r3c[1][e / 6][e % 6] = c_lno_tab.r3c[1][e / 6][e % 6];
-    }
-    for (int e = threadIdx.x; e < (int)sizeof(T.pat); e += blockDim.x)
-        reinterpret_cast<unsigned char *>(T.pat)[e] = reinterpret_cast<const unsigned char *>(c_lno_pat)[e];
-    const int cc = threadIdx.x;
-    if (cc < 36) {
-        int pr[3], vst[3], vl[3];
-        perm_of(cc % 6, pr);
-        for (int k = 0; k < 3; k++) {
-            vst[k] = U.st[pr[k]];
-            vl[k] = U.len[pr[k]];
-            T.cpr[cc][k] = (unsigned char)pr[k];
-        }
-        const int x0 = vst[0], y0 = vst[1], z0 = vst[2];
-        const int t = A.tau_of[(lno_slot(A.ch, x0) * 3 + lno_slot(A.ch, y0)) * 3 + lno_slot(A.ch, z0)];
-        const PermBlock &pb = A.ch.pb[t];
-        const int oTz = o * pb.Tz;
-        const int sx = oTz, sy = pb.Tx * oTz;
-        T.strQ[cc] = pb.Ty * sy;
-        T.strP[cc] = o * pb.Ty * sy;
-        T.tz[cc] = pb.Tz;
-        T.soff_v[cc] = pb.soff + (long long)(y0 - pb.Y0) * sy + (long long)(x0 - pb.X0) * sx + (z0 - pb.Z0);
-        const int wx = o * pb.rzp, wy = o * pb.Tx * wx;
-        T.swP[cc] = pb.Tx * wx;
-        T.rzp[cc] = pb.rzp;
-        T.swoff_v[cc] = pb.swoff + (long long)(y0 - pb.Y0) * wy + (long long)(x0 - pb.X0) * wx + (z0 - pb.Z0);
-        T.plane_c[cc] = (long long)pb.Ty * wy;
-        T.swbase_c[cc] = pb.swoff;
-        T.bov_v[cc] = (long long)x0 * o * v + y0;
-        T.bt2_v[cc] = y0 * v + x0;
-        T.bt1_v[cc] = z0;
-        T.bfv_v[cc] = z0 * o;
-        for (int l01 = 0; l01 < kLnoSB * kLnoSB; l01++) {
-            const int l0 = l01 / kLnoSB, l1 = l01 % kLnoSB;
-            T.roff[cc][l01] = l1 * sy + l0 * sx;
-            T.swro[cc][l01] = l1 * wy + l0 * wx;
-        }
-        unsigned long long m = 0ull;
-        for (int sl = 0; sl < kLnoRegion; sl++) {
-            const int l0 = sl / (kLnoSB * kLnoSB), l1 = (sl / kLnoSB) % kLnoSB, l2 = sl % kLnoSB;
-            if (l0 < vl[0] && l1 < vl[1] && l2 < vl[2]) m |= 1ull << sl;
-        }
-        T.vmask_c[cc] = m;
-    }
-    __syncthreads();
-}
-
-// per representative n: the occupied side of its slabs
-__device__ void lno_tile_setup_rep(const LnoArgs &A, LnoTile &T, int n) {
-    const int o = A.d.o, v = A.d.v;
-    const LnoSub &U = A.sub[blockIdx.x];
-    const int ijk[3] = {T.ijk[n][0], T.ijk[n][1], T.ijk[n][2]};
-    const int pid = ((ijk[0] == ijk[1]) << 3) | ((ijk[1] == ijk[2]) << 2) | ((U.st[0] == U.st[1]) << 1) |
-                    (U.st[1] == U.st[2]);
-    const LnoPattern &P = T.pat[pid];
-    const int c = threadIdx.x;
-    if (c == 0) T.nslab = P.nslab;
-    if (c < P.nslab) {
-        const int cc = P.cand[c];
-        int pp[3];
-        perm_of(cc / 6, pp);
-        const int p = ijk[pp[0]], q = ijk[pp[1]], r = ijk[pp[2]];
-        T.cand[c] = cc;
-        T.soff[c] = T.soff_v[cc] + (long long)p * T.strP[cc] + (long long)q * T.strQ[cc] + r * T.tz[cc];
-        T.swoff[c] = T.swoff_v[cc] + (long long)p * T.swP[cc] + (long long)q * T.rzp[cc] + r * T.tz[cc];
-        T.b_ov[c] = ((long long)p * v * o + q) * v + T.bov_v[cc];
-        T.b_t2[c] = ((long long)q * o + p) * v * v + T.bt2_v[cc];
-        T.b_t1[c] = r * v + T.bt1_v[cc];
-        T.b_fv[c] = T.bfv_v[cc] + r;
-        T.eocc[c] = T.s_eo[p] + T.s_eo[q] + T.s_eo[r];
-        for (int s = 0; s < 6; s++) {
-            T.symg[c][s] = (short)(P.prim[T.symc[cc][s]] * kLnoSlab);
-            T.r3g[0][c][s] = (short)(P.prim[T.r3c[0][cc][s]] * kLnoSlab);
-            T.r3g[1][c][s] = (short)(P.prim[T.r3c[1][cc][s]] * kLnoSlab);
-        }
-    }
-    __syncthreads();
-}
-
-// Per-thread constants: a thread's slot in its slabs is the same at every
-// iteration (kLnoThreads is a multiple of the slab size), so its local
-// indices and the permuted slots of its gathers are loaded once.
-struct LnoLane {
-    int sl, l0, l1, l2, l01, psl;
-    unsigned sym[2], r3[2][2];   // 8-bit permuted padded slots, four per word (six used)
-
-    __device__ __forceinline__ void init() {
-        sl = threadIdx.x % kLnoRegion;
-        l0 = sl / (kLnoSB * kLnoSB);
-        l1 = (sl / kLnoSB) % kLnoSB;
-        l2 = sl % kLnoSB;
-        l01 = l0 * kLnoSB + l1;
-        psl = lno_pad(sl);
-        sym[0] = sym[1] = r3[0][0] = r3[0][1] = r3[1][0] = r3[1][1] = 0u;
-        for (int s = 0; s < 6; s++) {
-            sym[s >> 2] |= (unsigned)c_lno_tab.symsl[s][sl] << (8 * (s & 3));
-            r3[0][s >> 2] |= (unsigned)c_lno_tab.r3sl[0][s][sl] << (8 * (s & 3));
-            r3[1][s >> 2] |= (unsigned)c_lno_tab.r3sl[1][s][sl] << (8 * (s & 3));
-        }
-    }
-    __device__ __forceinline__ int symsl(int s) const { return (sym[s >> 2] >> (8 * (s & 3))) & 0xff; }
-    __device__ __forceinline__ int r3sl(int a, int s) const { return (r3[a][s >> 2] >> (8 * (s & 3))) & 0xff; }
-};
-
-// it-th position of this thread: slab g (candidate cg), shared index si, staging offset goff
-#define LNO_POS(T, L, it)                                                                                           \
-    const int g = (int)(threadIdx.x / kLnoRegion) + (it) * (kLnoThreads / kLnoRegion);                            \
-    const bool inr = g < (T).nslab;                                                                               \
-    const int cg = inr ? (T).cand[g] : 0;                                                                         \
-    const int si = g * kLnoSlab + (L).psl;                                                                        \
-    const bool valid = inr && (((T).vmask_c[cg] >> (L).sl) & 1ull);                                                \
-    const long long goff = (T).soff[g] + (T).roff[cg][(L).l01] + (L).l2
-
-// pass 1: WW -> B0, Q = r3(WW + VV/2) / D -> B2
-template <typename StageT>
-__global__ void __launch_bounds__(kLnoThreads) k_lno_tile_fwd(LnoArgs A) {
-    const StageT *S = reinterpret_cast<const StageT *>(A.S);
-    __shared__ LnoTile T;
-    extern __shared__ double lno_sm[];
-    double *sW = lno_sm, *sV = lno_sm + 36 * kLnoSlab;
-    LnoLane L;
-    L.init();
-    lno_tile_setup_block(A, T);
-    const int o = A.d.o, v = A.d.v;
-    const int ovl = L.l0 * o * v + L.l1, t2l = L.l1 * v + L.l0, fvl = L.l2 * o;
-    for (int n = 0; n < T.nrep; n++) {
-    lno_tile_setup_rep(A, T, n);
-#pragma unroll
-    for (int it = 0; it < kLnoIt; it++) {
-        LNO_POS(T, L, it);
-        if (!inr) break;
-        double w = 0.0, vv = 0.0;
-        if (valid) {
-            // v = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r]
-            w = (double)S[goff];
-            vv = A.ovov[T.b_ov[g] + ovl] * A.t1[T.b_t1[g] + L.l2] + A.t2[T.b_t2[g] + t2l] * A.fvo[T.b_fv[g] + fvl];
-        }
-        sW[si] = w;
-        sV[si] = vv;
-    }
-    __syncthreads();
-    double xr[kLnoIt];
-#pragma unroll
-    for (int it = 0; it < kLnoIt; it++) {
-        LNO_POS(T, L, it);
-        (void)si;
-        xr[it] = 0.0;
-        if (!valid) continue;
-        double ww = 0.0, vv = 0.0;
-#pragma unroll
-        for (int s = 0; s < 6; s++) {
-            const int k = T.symg[g][s] + L.symsl(s);
-            ww += sW[k];
-            vv += sV[k];
-        }
-        A.B0[goff] = ww;
-        xr[it] = ww + 0.5 * vv;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < kLnoIt; it++) {
-        LNO_POS(T, L, it);
-        (void)valid;
-        (void)goff;
-        if (inr) sW[si] = xr[it];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < kLnoIt; it++) {
-        LNO_POS(T, L, it);
-        (void)si;
-        if (!valid) continue;
-        double z = 0.0;
-#pragma unroll
-        for (int s = 0; s < 6; s++) z += c_r3_coef[s] * sW[T.r3g[0][g][s] + L.r3sl(0, s)];
-        const double D = T.eocc[g] - T.ev_r[T.cpr[cg][0]][L.l0] - T.ev_r[T.cpr[cg][1]][L.l1] -
-                         T.ev_r[T.cpr[cg][2]][L.l2];
-        A.B2[goff] = z / D;
-    }
-    __syncthreads();   // slab data and shared arrays are reused by the next representative
-    }
-}
-
-// pass 3: Xbar = r3^T(Zbar (B3)), WWbar = P^T(Wtbar) (B1) + Xbar, VVbar = Xbar/2;
-// wbar = orbit sum of WWbar -> Wbar staging, vbar = orbit sum of VVbar -> B0.
-// SPLIT 0: FP64 staging; 1: fp16 hi/lo of wbar * wscale (exact power of two);
-// 2: bf16 hi/lo, unscaled -- the operand formats of the adjoint contractions.
-template <int SPLIT>
-__global__ void __launch_bounds__(kLnoThreads) k_lno_tile_adj(LnoArgs A) {
-    __shared__ LnoTile T;
-    extern __shared__ double lno_sm[];
-    double *sZ = lno_sm, *sW = lno_sm + 36 * kLnoSlab;
-    LnoLane L;
-    L.init();
-    lno_tile_setup_block(A, T);
-    const float wsc = SPLIT == 1 ? (float)*A.wscale : 1.0f;
-    for (int n = 0; n < T.nrep; n++) {
-    lno_tile_setup_rep(A, T, n);
-#pragma unroll
-    for (int it = 0; it < kLnoIt; it++) {
-        LNO_POS(T, L, it);
-        if (!inr) break;
-        sZ[si] = valid ? A.B3[goff] : 0.0;
-        sW[si] = valid ? A.B1[goff] : 0.0;
-    }
-    __syncthreads();
-    double xr[kLnoIt];
-#pragma unroll
-    for (int it = 0; it < kLnoIt; it++) {
-        LNO_POS(T, L, it);
-        (void)goff;
-        xr[it] = 0.0;
-        if (!valid) continue;
-        double xb = 0.0;
-#pragma unroll
-        for (int s = 0; s < 6; s++) xb += c_r3_coef[s] * sZ[T.r3g[1][g][s] + L.r3sl(1, s)];
-        xr[it] = xb;
-        sW[si] += xb;   // only this thread reads sW[si] in this phase
-    }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < kLnoIt; it++) {
-        LNO_POS(T, L, it);
-        (void)valid;
-        (void)goff;
-        if (inr) sZ[si] = 0.5 * xr[it];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < kLnoIt; it++) {
-        LNO_POS(T, L, it);
-        (void)si;
-        if (!valid) continue;
-        double wb = 0.0, vb = 0.0;
-#pragma unroll
-        for (int s = 0; s < 6; s++) {
-            const int k = T.symg[g][s] + L.symsl(s);
-            wb += sW[k];
-            vb += sZ[k];
-        }
-        const long long wl = T.swoff[g] + T.swro[cg][L.l01] + L.l2;
-        if (SPLIT == 0) {
-            reinterpret_cast<double *>(A.SW)[wl] = wb;
-        } else if (SPLIT == 1) {
-            const float xs = (float)wb * wsc;
-            const __half h = __float2half_rn(xs);
-            __half *dst = reinterpret_cast<__half *>(A.SW) + T.swbase_c[cg] + wl;   // 2 swoff + local offset
-            dst[0] = h;
-            dst[T.plane_c[cg]] = __float2half_rn(xs - __half2float(h));
-        } else {
-            const float xs = (float)wb;
-            const __nv_bfloat16 h = __float2bfloat16_rn(xs);
-            __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(A.SW) + T.swbase_c[cg] + wl;
-            dst[0] = h;
-            dst[T.plane_c[cg]] = __float2bfloat16_rn(xs - __bfloat162float(h));
-        }
-        A.B0[goff] = vb;
-    }
-    __syncthreads();   // slab data and shared arrays are reused by the next representative
-    }
-}
-
-#undef LNO_POS
-
-// ---------------------------------------------------------------------------
-// pass 2: projection along the first occupied index, streaming over columns
-// ---------------------------------------------------------------------------
-// Column c of ordering pb = (((q Ty + y) Tx + x) o + r) Tz + z (< 2^31); position p c.
-// Per 32-column tile with all o rows of WW (B0) and Q (B2) in shared memory:
-//   Wt[i,c] = sum_l mat[l,i] WW[l,c],  energy += Wt Q;
-//   with the adjoint: Zbar = f Wt / D -> B3, Dbar = -f Wt Q / D -> B2 (over Q),
-//   P^T(Wtbar)[l,c] = f sum_i mat[l,i] Q[i,c] -> B1, Gram WW Q^T -> mat_bar
-//   (f = ybar / 3).
-// The three products run on the FP64 tensor cores (mma.sync m8n8k4, FP64 in
-// and out): per 8x8 output tile a thread holds D[g][2t], D[g][2t+1]
-// (g = lane / 4, t = lane % 4), A[g][t] and B[t][g] of each k-step.
-constexpr int kLnoLd = 36;   // row stride of the shared tiles (conflict-free fragment loads)
-
-inline size_t lno_proj_smem(int o) {
-    return (size_t)(4 * kLnoMaxO * kLnoLd + o * o + kLnoMaxO + 2 * kLnoTile) * sizeof(double);
-}
-
-// 8-byte global -> shared copy that bypasses registers; ok = false writes zero
-__device__ __forceinline__ void lno_cp_async8(double *dst, const double *src, bool ok) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void lno_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void lno_cp_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-
-__device__ __forceinline__ void lno_dmma(double &d0, double &d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
-__global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(LnoArgs A) {
-    extern __shared__ double lno_sm[];
-    // two buffers of the WW / Q tiles: the next tile streams in while this one is used
-    double *sw_b = lno_sm, *sq_b = sw_b + 2 * kLnoMaxO * kLnoLd, *sM = sq_b + 2 * kLnoMaxO * kLnoLd;
-    const int o = A.d.o;
-    double *s_eo = sM + o * o, *s_ecol_b = s_eo + kLnoMaxO;
-    __shared__ double red[kLnoThreads / 32];
-    const int o4 = (o + 3) & ~3, o8 = (o + 7) / 8, rows = 8 * o8;
-    const PermBlock &pb = A.ch.pb[blockIdx.y];
-    const int stride_p = o * o * pb.Tx * pb.Ty * pb.Tz;
-    const int ntile = (stride_p + kLnoTile - 1) / kLnoTile;
-    const double f = A.ybar / 3.0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int fg = lane >> 2, ft = lane & 3;   // fragment row group / thread in group
-    const bool grad = A.want_grad != 0;
-    for (int k = threadIdx.x; k < o * o; k += blockDim.x) sM[k] = A.mat[k];
-    for (int k = threadIdx.x; k < o; k += blockDim.x) s_eo[k] = A.mo_e[k];
-    constexpr int kG = (kLnoMaxO / 8) * (kLnoMaxO / 8) / (kLnoThreads / 32);   // Gram tiles per warp
-    const int ngram = o8 * o8;
-    double acc[kG][2];
-#pragma unroll
-    for (int k = 0; k < kG; k++) acc[k][0] = acc[k][1] = 0.0;
-    double en = 0.0;
-    const double *W = A.B0 + pb.soff, *Qg = A.B2 + pb.soff;
-    // issue the copies of tile tb into buffer b (and its column energies)
-    auto issue = [&](int tb, int b) {
-        const int c0 = tb * kLnoTile;
-        double *sw = sw_b + b * kLnoMaxO * kLnoLd, *sq = sq_b + b * kLnoMaxO * kLnoLd;
-        for (int e = threadIdx.x; e < rows * kLnoTile; e += blockDim.x) {
-            const int l = e / kLnoTile, j = e % kLnoTile;
-            const bool ok = l < o && c0 + j < stride_p;
-            const long long at = ok ? (long long)l * stride_p + c0 + j : 0;
-            lno_cp_async8(sw + l * kLnoLd + j, W + at, ok);
-            lno_cp_async8(sq + l * kLnoLd + j, Qg + at, ok);
-        }
-        lno_cp_commit();
-        if (grad && threadIdx.x < kLnoTile) {
-            int cc = c0 + threadIdx.x;
-            double ec = 0.0;
-            if (cc < stride_p) {
-                const int zl = cc % pb.Tz;
-                cc /= pb.Tz;
-                const int r = cc % o;
-                cc /= o;
-                const int xl = cc % pb.Tx;
-                cc /= pb.Tx;
-                const int yl = cc % pb.Ty;
-                const int q = cc / pb.Ty;
-                ec = A.mo_e[q] + A.mo_e[r] - A.mo_e[o + pb.X0 + xl] - A.mo_e[o + pb.Y0 + yl] -
-                     A.mo_e[o + pb.Z0 + zl];
-            }
-            s_ecol_b[b * kLnoTile + threadIdx.x] = ec;
-        }
-    };
-    int buf = 0;
-    if ((int)blockIdx.x < ntile) issue(blockIdx.x, 0);
-    for (int tb = blockIdx.x; tb < ntile; tb += gridDim.x) {
-        const int c0 = tb * kLnoTile;
-        if (tb + (int)gridDim.x < ntile)
-            issue(tb + gridDim.x, buf ^ 1);
-        else
-            lno_cp_commit();   // empty group: keeps the wait count uniform
-        lno_cp_wait1();        // this thread's copies of tile tb have landed
-        __syncthreads();       // ... and everyone's
-        const double *sw = sw_b + buf * kLnoMaxO * kLnoLd, *sq = sq_b + buf * kLnoMaxO * kLnoLd;
-        const double *s_ecol = s_ecol_b + buf * kLnoTile;
-        // Wt and P^T(Q) tiles (rows i / l in 8-blocks, columns in 8-blocks) and their epilogue
-        for (int tile = warp; tile < o8 * (kLnoTile / 8); tile += kLnoThreads / 32) {
-            const int mt = tile / (kLnoTile / 8), nt = tile % (kLnoTile / 8);
-            const int i = mt * 8 + fg;
-            double w0 = 0.0, w1 = 0.0, p0 = 0.0, p1 = 0.0;
-            for (int k0 = 0; k0 < o4; k0 += 4) {
-                const int l = k0 + ft;
-                const bool in = i < o && l < o;
-                lno_dmma(w0, w1, in ? sM[l * o + i] : 0.0, sw[l * kLnoLd + nt * 8 + fg]);
-                if (grad) lno_dmma(p0, p1, in ? sM[i * o + l] : 0.0, sq[l * kLnoLd + nt * 8 + fg]);
-            }
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int cl = nt * 8 + 2 * ft + h;
-                const double wt = h ? w1 : w0;
-                const double qv = sq[i * kLnoLd + cl];
-                en += wt * qv;
-                const int c = c0 + cl;
-                if (grad && i < o && c < stride_p) {
-                    const double D = s_eo[i] + s_ecol[cl];
-                    const double qb = f * wt;
-                    const long long at = pb.soff + (long long)i * stride_p + c;
-                    A.B3[at] = qb / D;
-                    A.B2[at] = -qb * qv / D;
-                    A.B1[at] = f * (h ? p1 : p0);
-                }
-            }
-        }
-        if (grad) {
-            // Gram[l, i] += sum_c WW[l, c] Q[i, c]: warp-owned 8x8 tiles, k over the 32 columns
-#pragma unroll
-            for (int k = 0; k < kG; k++) {
-                const int gt = warp + k * (kLnoThreads / 32);
-                if (gt < ngram) {
-                    const int mt = gt / o8, nt = gt % o8;
-#pragma unroll
-                    for (int k0 = 0; k0 < kLnoTile; k0 += 4)
-                        lno_dmma(acc[k][0], acc[k][1], sw[(mt * 8 + fg) * kLnoLd + k0 + ft],
-                                 sq[(nt * 8 + fg) * kLnoLd + k0 + ft]);
-                }
-            }
-        }
-        __syncthreads();   // buffer buf is refilled two tiles from now
-        buf ^= 1;
-    }
-    en = lno_warp_sum(en);
-    if (lane == 0) red[warp] = en;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < kLnoThreads / 32; w++) s += red[w];
-        A.part[blockIdx.y * gridDim.x + blockIdx.x] = s / 3.0;
-    }
-    if (!grad) return;
-#pragma unroll
-    for (int k = 0; k < kG; k++) {
-        const int gt = warp + k * (kLnoThreads / 32);
-        if (gt < ngram) {
-            const int l = (gt / o8) * 8 + fg;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int i = (gt % o8) * 8 + 2 * ft + h;
-                const double gv = h ? acc[k][1] : acc[k][0];
-                if (l < o && i < o && gv != 0.0) atomicAdd(&A.mat_bar[l * o + i], f * gv);
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// pass 4: V-term and denominator gradients from vbar (B0) and Dbar (B2), one
-// warp per (p, q, y, x) row of o Tz contiguous (r, z) values:
-//   ovov_bar[p,x,q,y] += sum_rz vbar t1[r,z],   t2_bar[q,p,y,x] += sum_rz vbar fvo[z,r],
-//   t1_bar[r,z] += sum vbar ovov[p,x,q,y],      fvo_bar[z,r] += sum vbar t2[q,p,y,x],
-//   mo_bar[p], [q], [r] += sum Dbar;  mo_bar[o+x], [o+y], [o+z] -= sum Dbar.
-// Lane k of every warp owns elements k, k+32, ... of the row (M per lane) and
-// keeps their sums in registers across rows.
-// ---------------------------------------------------------------------------
-template <int M>
-__global__ void __launch_bounds__(kLnoThreads) k_lno_vgrad(LnoArgs A) {
-    __shared__ double s_t1[kLnoMaxO * kLnoMaxTv], s_fv[kLnoMaxO * kLnoMaxTv], s_rz[kLnoMaxO * kLnoMaxTv];
-    __shared__ double s_occ[kLnoThreads / 32][kLnoMaxO], s_vir[kLnoThreads / 32][2][kLnoMaxTv];
-    const int o = A.d.o, v = A.d.v;
-    const PermBlock &pb = A.ch.pb[blockIdx.y];
-    const int oTz = o * pb.Tz;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = threadIdx.x; k < oTz; k += blockDim.x) s_t1[k] = s_fv[k] = s_rz[k] = 0.0;
-    for (int k = lane; k < kLnoMaxO; k += 32) s_occ[warp][k] = 0.0;
-    for (int k = lane; k < 2 * kLnoMaxTv; k += 32) s_vir[warp][k / kLnoMaxTv][k % kLnoMaxTv] = 0.0;
-    __syncthreads();
-    double a1[M], af[M], ar[M];
-#pragma unroll
-    for (int m = 0; m < M; m++) a1[m] = af[m] = ar[m] = 0.0;
-    const int npr = o * o * pb.Ty * pb.Tx;
-    const int nwarp = gridDim.x * (blockDim.x >> 5);
-    for (int pr = blockIdx.x * (blockDim.x >> 5) + warp; pr < npr; pr += nwarp) {
-        const int xl = pr % pb.Tx, yl = (pr / pb.Tx) % pb.Ty;
-        const int q = (pr / (pb.Tx * pb.Ty)) % o, p = pr / (pb.Tx * pb.Ty * o);
-        const int x = pb.X0 + xl, y = pb.Y0 + yl;
-        const long long iov = (((long long)p * v + x) * o + q) * v + y;
-        const long long it2 = (((long long)q * o + p) * v + y) * v + x;
-        const double ovv = A.ovov[iov], t2v = A.t2[it2];
-        const double *rv = A.B0 + pb.soff + (long long)pr * oTz;
-        const double *rd = A.B2 + pb.soff + (long long)pr * oTz;
-        double s_ov = 0.0, s_t2 = 0.0, s_d = 0.0;
-#pragma unroll
-        for (int m = 0; m < M; m++) {
-            const int k = lane + 32 * m;
-            if (k < oTz) {
-                const int r = k / pb.Tz, z = pb.Z0 + k % pb.Tz;
-                const double vb = rv[k], db = rd[k];
-                s_ov += vb * __ldg(&A.t1[r * v + z]);
-                s_t2 += vb * __ldg(&A.fvo[z * o + r]);
-                s_d += db;
-                a1[m] += vb * ovv;
-                af[m] += vb * t2v;
-                ar[m] += db;
-            }
-        }
-        s_ov = lno_warp_sum(s_ov);
-        s_t2 = lno_warp_sum(s_t2);
-        s_d = lno_warp_sum(s_d);
-        if (lane == 0) {
-            if (s_ov != 0.0) atomicAdd(&A.ovov_bar[iov], s_ov);
-            if (s_t2 != 0.0) atomicAdd(&A.t2_bar[it2], s_t2);
-            s_occ[warp][p] += s_d;
-            s_occ[warp][q] += s_d;
-            s_vir[warp][0][xl] -= s_d;
-            s_vir[warp][1][yl] -= s_d;
-        }
-    }
-    // combine the warps' register sums (one warp at a time: no atomics)
-    for (int w = 0; w < kLnoThreads / 32; w++) {
-        if (warp == w) {
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                const int k = lane + 32 * m;
-                if (k < oTz) {
-                    s_t1[k] += a1[m];
-                    s_fv[k] += af[m];
-                    s_rz[k] += ar[m];
-                }
-            }
-        }
-        __syncthreads();
-    }
-    for (int k = threadIdx.x; k < oTz; k += blockDim.x) {
-        const int r = k / pb.Tz, z = pb.Z0 + k % pb.Tz;
-        if (s_t1[k] != 0.0) atomicAdd(&A.t1_bar[(long long)r * v + z], s_t1[k]);
-        if (s_fv[k] != 0.0) atomicAdd(&A.fvo_bar[(long long)z * o + r], s_fv[k]);
-        if (s_rz[k] != 0.0) {
-            atomicAdd(&A.mo_bar[r], s_rz[k]);
-            atomicAdd(&A.mo_bar[o + z], -s_rz[k]);
-        }
-    }
-    for (int k = threadIdx.x; k < o; k += blockDim.x) {
-        double t = 0.0;
-        for (int w = 0; w < kLnoThreads / 32; w++) t += s_occ[w][k];
-        if (t != 0.0) atomicAdd(&A.mo_bar[k], t);
-    }
-    for (int k = threadIdx.x; k < 2 * kLnoMaxTv; k += blockDim.x) {
-        const int role = k / kLnoMaxTv, kk = k % kLnoMaxTv;
-        const int len = role == 0 ? pb.Tx : pb.Ty;
-        if (kk >= len) continue;
-        double t = 0.0;
-        for (int w = 0; w < kLnoThreads / 32; w++) t += s_vir[w][role][kk];
-        if (t != 0.0) atomicAdd(&A.mo_bar[o + (role == 0 ? pb.X0 : pb.Y0) + kk], t);
-    }
-}
-
-inline size_t lno_tile_smem() { return 2 * 36 * kLnoSlab * sizeof(double); }
 
 }  // namespace tb

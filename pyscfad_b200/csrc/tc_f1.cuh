@@ -36,10 +36,9 @@ struct TcCfg {
 };
 
 struct TcF1Params {
-    CUtensorMap tmS[6];       // per ordering with full 16 x 16 (x, z) blocks, one 32 x 32 piece of
-                              // an epilogue warp per store: S_tau as [p][q][y][x][r*16+z], box
-                              // {32, 16, 1, 1, 2}, 128B swizzle; or (blocked) as [p][q][r][block]
-                              // [y*64 + slot], box {64, 4, 2, 1, 2}: the four (x, z) blocks of a y
+    CUtensorMap tmS[6];       // per ordering with full 16 x 16 (x, z) blocks: S_tau as [p][q][r][block]
+                              // [y*64 + slot], box {64, 4, 2, 1, 2} (the four (x, z) blocks of a y):
+                              // one 32 x 32 piece of an epilogue warp per store
     int tmS_ok[6];            // 1 where tmS is valid (else plain stores)
     Dims d;
     ChunkDesc ch;
@@ -54,7 +53,6 @@ struct TcF1Params {
     int *err;
     int bf16;
     int kseg;                 // K blocks per TMEM accumulation segment
-    int blocked;              // staging in the epilogue's 8 x 8 x 8 blocks (f2m_stage_offset)
 };
 
 constexpr int kF1Threads = 320;   // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
@@ -320,17 +318,13 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
             const int p = T.mt * 8 + row / 16;
             const int x = row % 16;
             const bool vrow = (p < o) && (x < pb.Tx);
-            float *dst = P.S + pb.soff +
-                         ((((long long)(p * o + T.q) * pb.Ty + T.y) * pb.Tx + x) * o) * pb.Tz;
             if (P.tmS_ok[T.tau]) {
-                // Full blocks: each 32 x 32 piece (lane = row = 16 p-local x 16 x) goes to
-                // this warp's 128B-swizzled shared box and leaves as one TMA store, so the
-                // rows reach HBM as whole 128-byte lines instead of 32 scattered 16-byte
-                // pieces per warp store.
+                // Full blocks: each 32 x 32 piece (lane = row = 2 p x 16 x) goes to this warp's
+                // shared box and leaves as one TMA store of 256-byte rows instead of 32
+                // scattered 16-byte pieces per warp store.
                 float *box = sstore + (warp - 2) * 32 * 32;
                 const int p0 = T.mt * 8 + quarter * 2;
-                // this lane's float4 slot ch of its row: 128B-swizzled row of 32, or
-                // [p][r][x block, z block][x][z] with the row exchange of f2m_row_swizzle
+                // the box as [p][r][x block, z block][x][z] with the row exchange of f2m_row_swizzle
                 const int bsw = f2m_row_swizzle(T.y);
                 const int brow = (lane >> 4) * 512 + ((lane >> 3) & 1) * 128, bx = (lane & 7) * 8;
                 #pragma unroll
@@ -349,22 +343,20 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
                         w.w = accf[c * 32 + ch * 4 + 3] * sc;
                         if (vrow)
                             wmax = fmaxf(wmax, fmaxf(fmaxf(fabsf(w.x), fabsf(w.y)), fmaxf(fabsf(w.z), fabsf(w.w))));
-                        const int at = P.blocked ? brow + (ch >> 2) * 256 + ((ch >> 1) & 1) * 64 + ((bx + (ch & 1) * 4) ^ bsw)
-                                                 : lane * 32 + 4 * (ch ^ (lane & 7));
+                        const int at = brow + (ch >> 2) * 256 + ((ch >> 1) & 1) * 64 + ((bx + (ch & 1) * 4) ^ bsw);
                         *reinterpret_cast<float4 *>(box + at) = w;
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
                     const int r0 = T.nt * P.rt + 4 * c + 2 * half;
                     if (lane == 0 && p0 < o && r0 < o) {
-                        if (P.blocked) tma_store_5d(&P.tmS[T.tau], box, (T.y & 7) * 64, (T.y >> 3) * 4, r0, T.q, p0);
-                        else tma_store_5d(&P.tmS[T.tau], box, r0 * 16, 0, T.y, T.q, p0);
+                        tma_store_5d(&P.tmS[T.tau], box, (T.y & 7) * 64, (T.y >> 3) * 4, r0, T.q, p0);
                         bulk_commit();
                     }
                 }
                 if (lane == 0) bulk_wait_read0();
                 __syncwarp();
-            } else if (vrow && P.blocked) {
+            } else if (vrow) {
                 const StageRow R = f2m_stage_row(pb, o, p, T.q, T.y, x);
 #pragma unroll
                 for (int h = 0; h < HC / 16; h++) {
@@ -390,35 +382,6 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
                                 const float w1 = accf[h * 16 + z] * sc;
                                 wmax = fmaxf(wmax, fabsf(w1));
                                 d[R.slot + z] = w1;
-                            }
-                        }
-                    }
-                }
-            } else if (vrow) {
-#pragma unroll
-                for (int h = 0; h < HC / 16; h++) {
-                    const int rl = 4 * (h >> 1) + 2 * half + (h & 1), r = T.nt * P.rt + rl;
-                    if (rl >= P.rt || r >= o) continue;
-                    float *d = dst + (long long)r * pb.Tz;
-                    if (pb.Tz == 16) {
-                        float4 *d4 = reinterpret_cast<float4 *>(d);
-#pragma unroll
-                        for (int z4 = 0; z4 < 4; z4++) {
-                            float4 w;
-                            w.x = accf[h * 16 + z4 * 4 + 0] * sc;
-                            w.y = accf[h * 16 + z4 * 4 + 1] * sc;
-                            w.z = accf[h * 16 + z4 * 4 + 2] * sc;
-                            w.w = accf[h * 16 + z4 * 4 + 3] * sc;
-                            wmax = fmaxf(wmax, fmaxf(fmaxf(fabsf(w.x), fabsf(w.y)), fmaxf(fabsf(w.z), fabsf(w.w))));
-                            d4[z4] = w;
-                        }
-                    } else {
-#pragma unroll
-                        for (int z = 0; z < 16; z++) {
-                            if (z < pb.Tz) {
-                                const float w1 = accf[h * 16 + z] * sc;
-                                wmax = fmaxf(wmax, fabsf(w1));
-                                d[z] = w1;
                             }
                         }
                     }

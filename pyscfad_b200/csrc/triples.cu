@@ -188,8 +188,8 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
     d.n = nocc + nvir;
     d.Tv = choose_tv(nocc, opt ? opt->block_size : 0);
     if (lno) {
-        // the projected epilogue keeps whole-chunk FP64 work arrays (6 o^3 Tv^3
-        // values each at most): halve the block until they fit the budget
+        // halve the block until four FP64 arrays of a chunk's raw amplitudes fit the
+        // budget (the box arrays take a sixth; the rule fixes the decomposition)
         const double o3 = (double)nocc * nocc * nocc;
         while (d.Tv > 4 && kLnoArrays * 6.0 * o3 * d.Tv * d.Tv * d.Tv * sizeof(double) > kLnoBudgetBytes) d.Tv >>= 1;
     }
@@ -199,7 +199,7 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
     P.nb = num_blocks(d);
     P.n_ijk = nocc * (nocc + 1) * (nocc + 2) / 6;
     long long maxst = 0, maxwb = 0;
-    int maxitems = 0;
+    int maxitems = 0, maxsub = 1;
     for (int A = 0; A < P.nb; A++)
         for (int B = 0; B <= A; B++)
             for (int C = 0; C <= B; C++) {
@@ -211,6 +211,7 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
                 if (w > maxwb) maxwb = w;
                 int it = ch.nabc[0] * ch.nabc[1] * ch.nabc[2];
                 if (it > maxitems) maxitems = it;
+                maxsub = std::max(maxsub, ((ch.nabc[0] + 7) / 8) * ((ch.nabc[1] + 7) / 8) * ((ch.nabc[2] + 7) / 8));
             }
     P.stage_elems = (size_t)maxst;
     P.wbar_elems = (size_t)maxwb;
@@ -270,13 +271,13 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
     P.off_ijk = take((size_t)P.n_ijk * 3 * sizeof(int));
     P.off_epart = take((size_t)P.group * P.n_ijk * P.f2_gy * el);
     if (P.lno) {
-        // whole-chunk FP64 arrays: WW / P^T(Wtbar) / vbar (0), Pt(Q) (1), Q / Dbar (2),
-        // Zbar (3); the energy alone needs only 0 and 2
-        P.off_L[0] = take(P.stage_elems * el);
-        P.off_L[2] = take(P.stage_elems * el);
+        // FP64 box arrays: WW (0), PQ (1), Q (2), PW / Zbar (3); the energy alone needs only 0 and 2
+        const size_t box = o * o * o * 512 * (size_t)maxsub;
+        P.off_L[0] = take(box * el);
+        P.off_L[2] = take(box * el);
         if (want_grad) {
-            P.off_L[1] = take(P.stage_elems * el);
-            P.off_L[3] = take(P.stage_elems * el);
+            P.off_L[1] = take(box * el);
+            P.off_L[3] = take(box * el);
         } else {
             P.off_L[1] = P.off_L[0];
             P.off_L[3] = P.off_L[2];
@@ -660,6 +661,7 @@ struct GemmLaunch {
     int zstart[kMaxGroup + 1];   // GEMM problems (blockIdx.z) chunk after chunk,
     int cum[kMaxGroup][7];       // and within a chunk ordering after ordering
     int nmt, nslice;             // M tiles and K slices of blockIdx.x
+    int blocked;                 // staging in 8 x 8 x 8 blocks (StageRow, no exchange): the LNO kernels
     const double *A1, *B1, *A2, *B2;
     double *G;                   // gradient target
 };
@@ -708,8 +710,16 @@ __global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant_
         g.B = GOp{L.B1 + q * ovK + (long long)pb.Z0 * Kp, map2(pb.Tz, Kp, vK), map1(1)};
         g.A2 = GOp{L.A2 + q * ovo + (long long)pb.X0 * o, map2(pb.Tx, o, vo), map1(1)};
         g.B2 = GOp{L.B2 + yg * ovo + (long long)pb.Z0 * o, map2(pb.Tz, o, vo), map1(1)};
-        g.C = L.S[c] + pb.soff + ((long long)q * pb.Ty + y) * pb.Tx * oTz;
-        g.cm = map2(pb.Tx, oTz, (long long)o * pb.Ty * pb.Tx * oTz);
+        if (L.blocked) {
+            const int ex = min(8, pb.Tx), ey = min(8, pb.Ty), ez = min(8, pb.Tz), nx = pb.Tx / ex, nz = pb.Tz / ez;
+            const long long es = ex * ey * ez, rs = (long long)pb.Tx * pb.Ty * pb.Tz;
+            g.C = L.S[c] + pb.soff + (long long)q * o * rs + (y / ey) * nx * nz * es + (y % ey) * (ex * ez);
+            g.cm = map3(ex, nx, ez, nz * es, (long long)o * o * rs);
+            g.cn = map3(ez, nz, 1, es, rs);
+        } else {
+            g.C = L.S[c] + pb.soff + ((long long)q * pb.Ty + y) * pb.Tx * oTz;
+            g.cm = map2(pb.Tx, oTz, (long long)o * pb.Ty * pb.Tx * oTz);
+        }
         g.alpha2 = -1.0;
         g.atomic = 0;
     } else if (KIND == GK_B1A) {
@@ -876,24 +886,20 @@ static int make_tmap5(CUtensorMap *tm, void *base, bool bf16, const uint64_t dim
     return r == CUDA_SUCCESS ? TRIPLES_OK : TRIPLES_ERR_CUDA;
 }
 
-// 5-D map over S_tau (FP32), used by the W-contraction epilogue to store 32 x 32
-// pieces of full (x, z) blocks: [p][q][y][x][rz] (rz innermost, o*16 values,
-// 128B swizzle), or blocked, [p][q][r][y block, x block, z block][y][64].
-static int make_tmap_stage(CUtensorMap *tm, float *base, int o, int Tx, int Ty, bool blocked) {
+// 5-D map over S_tau (FP32) as [p][q][r][y block, x block, z block][y][64], used
+// by the W-contraction epilogue to store 32 x 32 pieces of full (x, z) blocks.
+static int make_tmap_stage(CUtensorMap *tm, float *base, int o, int Ty) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return TRIPLES_ERR_UNSUPPORTED;
     const int ey = Ty < 8 ? Ty : 8;
-    const cuuint64_t gdim_rows[5] = {(cuuint64_t)o * 16, (cuuint64_t)Tx, (cuuint64_t)Ty, (cuuint64_t)o, (cuuint64_t)o};
-    const cuuint64_t gdim_blk[5] = {(cuuint64_t)ey * 64, (cuuint64_t)(Ty / ey) * 4, (cuuint64_t)o, (cuuint64_t)o,
-                                    (cuuint64_t)o};
-    const cuuint64_t *gdim = blocked ? gdim_blk : gdim_rows;
+    const cuuint64_t gdim[5] = {(cuuint64_t)ey * 64, (cuuint64_t)(Ty / ey) * 4, (cuuint64_t)o, (cuuint64_t)o, (cuuint64_t)o};
     cuuint64_t gstr[4];
     gstr[0] = gdim[0] * sizeof(float);
     for (int i = 1; i < 4; i++) gstr[i] = gstr[i - 1] * gdim[i];
-    const cuuint32_t box_rows[5] = {32, 16, 1, 1, 2}, box_blk[5] = {64, 4, 2, 1, 2}, es[5] = {1, 1, 1, 1, 1};
-    CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, gdim, gstr, blocked ? box_blk : box_rows, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, blocked ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
-                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint32_t box[5] = {64, 4, 2, 1, 2}, es[5] = {1, 1, 1, 1, 1};
+    CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, gdim, gstr, box, es,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? TRIPLES_OK : TRIPLES_ERR_CUDA;
 }
 
@@ -1047,7 +1053,7 @@ static int gemm_plain(cudaStream_t st, int M, int N, int K, const double *A, lon
 // constant tables), under a lock so that host threads making their first
 // call at the same time do it once.  Assumes the device's primary context
 // lives as long as the process (a cudaDeviceReset would need it again).
-enum InitKind { INIT_F2_F32 = 0, INIT_F2_F64, INIT_TC, INIT_LNO, INIT_NKINDS };
+enum InitKind { INIT_F2_F32 = 0, INIT_F2_F64, INIT_TC, INIT_LNO, INIT_LNO64, INIT_NKINDS };
 static std::mutex g_init_mu;
 static bool g_init_done[kMaxDev][INIT_NKINDS];
 
@@ -1079,132 +1085,6 @@ static ChunkAux chunk_aux(const Plan &P, const ChunkDesc &ch, int slot, const Tr
     A.scaled = P.prec == TRIPLES_PRECISION_MIXED ? 1 : 0;
     A.lno = P.lno;
     return A;
-}
-
-// LNO chunk epilogue (FP64): energy of the projected amplitudes and, with
-// want_grad, mat_bar, the D and V-term gradients and the FP64 Wbar staging
-// that the adjoint contractions read next (four passes, see lno.cuh).
-template <typename StageT>
-static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const TriplesIO &io, char *ws,
-                     Ctrl *ctrl, const StageT *S, void *SW, const int *ijk, int split) {
-    {
-        const int rc = once_per_device(INIT_LNO, [&]() -> int {
-            const int ts = (int)lno_tile_smem();
-            TB_CUDA(cudaFuncSetAttribute(k_lno_tile_fwd<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, ts));
-            TB_CUDA(cudaFuncSetAttribute(k_lno_tile_fwd<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, ts));
-            TB_CUDA(cudaFuncSetAttribute(k_lno_tile_adj<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, ts));
-            TB_CUDA(cudaFuncSetAttribute(k_lno_tile_adj<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ts));
-            TB_CUDA(cudaFuncSetAttribute(k_lno_tile_adj<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ts));
-            LnoTables tabs;
-            lno_build_tables(tabs);
-            TB_CUDA(cudaMemcpyToSymbol(c_lno_tab, &tabs, sizeof(tabs)));
-            LnoPattern pats[16];
-            lno_build_patterns(pats);
-            TB_CUDA(cudaMemcpyToSymbol(c_lno_pat, pats, sizeof(pats)));
-            const int ps = (int)lno_proj_smem(kLnoMaxO);
-            TB_CUDA(cudaFuncSetAttribute(k_lno_proj, cudaFuncAttributeMaxDynamicSharedMemorySize, ps));
-            return TRIPLES_OK;
-        });
-        if (rc != TRIPLES_OK) return rc;
-    }
-    const Dims &d = P.d;
-    LnoArgs A;
-    A.d = d;
-    A.ch = ch;
-    for (int k = 0; k < 27; k++) A.tau_of[k] = 0;
-    for (int sx = 0; sx < 3; sx++)
-        for (int sy = 0; sy < 3; sy++)
-            for (int sz = 0; sz < 3; sz++)
-                for (int t = 0; t < ch.nperm; t++)
-                    if (ch.pb[t].bx == ch.blk[sx] && ch.pb[t].by == ch.blk[sy] && ch.pb[t].bz == ch.blk[sz])
-                        A.tau_of[(sx * 3 + sy) * 3 + sz] = (signed char)t;
-    // virtual sub-block triples, one per orbit of orderings
-    A.nsub = 0;
-    int nsb[3];
-    for (int t = 0; t < 3; t++) nsb[t] = (ch.nabc[t] + kLnoSB - 1) / kLnoSB;
-    for (int sa = 0; sa < nsb[0]; sa++)
-        for (int sb = 0; sb < nsb[1]; sb++) {
-            if (ch.blk[0] == ch.blk[1] && sb > sa) continue;
-            for (int sc = 0; sc < nsb[2]; sc++) {
-                if (ch.blk[1] == ch.blk[2] && sc > sb) continue;
-                if (A.nsub >= kLnoMaxSub) return TRIPLES_ERR_UNSUPPORTED;
-                LnoSub &u = A.sub[A.nsub++];
-                const int si[3] = {sa, sb, sc};
-                for (int t = 0; t < 3; t++) {
-                    u.st[t] = ch.base[t] + si[t] * kLnoSB;
-                    const int len = ch.nabc[t] - si[t] * kLnoSB;
-                    u.len[t] = len < kLnoSB ? len : kLnoSB;
-                }
-            }
-        }
-    A.ijk = ijk;
-    A.S = S;
-    A.B0 = (double *)(ws + P.off_L[0]);
-    A.B1 = (double *)(ws + P.off_L[1]);
-    A.B2 = (double *)(ws + P.off_L[2]);
-    A.B3 = (double *)(ws + P.off_L[3]);
-    A.mat = io.mat; A.mo_e = io.mo_energy; A.t1 = io.t1; A.t2 = io.t2; A.ovov = io.ovov; A.fvo = io.fvo;
-    A.SW = SW;
-    A.wscale = &ctrl->slot[0].wscale;
-    A.mat_bar = io.mat_bar; A.mo_bar = io.mo_energy_bar; A.t1_bar = io.t1_bar; A.t2_bar = io.t2_bar;
-    A.ovov_bar = io.ovov_bar; A.fvo_bar = io.fvo_bar;
-    A.ybar = io.ybar;
-    A.want_grad = P.want_grad;
-    A.part = (double *)(ws + P.off_lpart);
-    long long maxcols = 0, maxrows = 0;
-    for (int t = 0; t < ch.nperm; t++) {
-        const long long rows = (long long)d.o * d.o * ch.pb[t].Tx * ch.pb[t].Ty;
-        if (rows * d.o * ch.pb[t].Tz > maxcols) maxcols = rows * d.o * ch.pb[t].Tz;
-        if (rows > maxrows) maxrows = rows;
-    }
-    auto clampg = [](long long n) { return (unsigned)(n < kLnoGrid ? (n > 0 ? n : 1) : kLnoGrid); };
-    A.n_ijk = P.n_ijk;
-    const dim3 gtile((unsigned)A.nsub, (unsigned)((P.n_ijk + kLnoReps - 1) / kLnoReps));
-    // streaming passes: a few full waves of two blocks per SM over the chunk's
-    // orderings (their per-block reductions end in global atomics on a few
-    // hundred entries, so the grid stays small)
-    const long long wave = (long long)kLnoWaves * 2 * num_sms() / ch.nperm;
-    auto clampw = [&](long long n) { return clampg(n < wave ? n : wave); };
-    const dim3 gproj(clampw((maxcols / d.o + kLnoTile - 1) / kLnoTile), (unsigned)ch.nperm);
-    TB_KLAUNCH(P_LNO, k_lno_tile_fwd<StageT><<<gtile, kLnoThreads, lno_tile_smem(), st>>>(A));
-    TB_KLAUNCH(P_LNO_PROJ, k_lno_proj<<<gproj, kLnoThreads, lno_proj_smem(d.o), st>>>(A));
-    {
-        Group<ChunkAux, 1> G;
-        G.n = 1;
-        G.job[0] = chunk_aux(P, ch, 0, io, (int)(gproj.x * gproj.y));
-        G.job[0].e_part = A.part;
-        TB_KLAUNCH(P_PREP, (k_energy_sum<<<1, 256, 0, st>>>(G, 1)));
-    }
-    if (!P.want_grad) return TRIPLES_OK;
-    if (split != 0) {   // fp16: power-of-two scale of the split Wbar; bf16: scale 1 (both read by the contractions)
-        Group<ChunkAux, 1> G;
-        G.n = 1;
-        G.job[0] = chunk_aux(P, ch, 0, io, 0);
-        TB_KLAUNCH(P_PREP, (k_chunk_scale<<<1, 32, 0, st>>>(G)));
-    }
-    if (split == 0)
-        TB_KLAUNCH(P_LNO_ADJ, k_lno_tile_adj<0><<<gtile, kLnoThreads, lno_tile_smem(), st>>>(A));
-    else if (split == 1)
-        TB_KLAUNCH(P_LNO_ADJ, k_lno_tile_adj<1><<<gtile, kLnoThreads, lno_tile_smem(), st>>>(A));
-    else
-        TB_KLAUNCH(P_LNO_ADJ, k_lno_tile_adj<2><<<gtile, kLnoThreads, lno_tile_smem(), st>>>(A));
-    const dim3 gv(clampw((maxrows + kLnoThreads / 32 - 1) / (kLnoThreads / 32)), (unsigned)ch.nperm);
-    int maxTz = 0;
-    for (int t = 0; t < ch.nperm; t++) maxTz = ch.pb[t].Tz > maxTz ? ch.pb[t].Tz : maxTz;
-    const int per_lane = (d.o * maxTz + 31) / 32;
-    if (per_lane <= 2)
-        TB_KLAUNCH(P_LNO_VG, k_lno_vgrad<2><<<gv, kLnoThreads, 0, st>>>(A));
-    else if (per_lane <= 4)
-        TB_KLAUNCH(P_LNO_VG, k_lno_vgrad<4><<<gv, kLnoThreads, 0, st>>>(A));
-    else if (per_lane <= 8)
-        TB_KLAUNCH(P_LNO_VG, k_lno_vgrad<8><<<gv, kLnoThreads, 0, st>>>(A));
-    else if (per_lane <= 12)
-        TB_KLAUNCH(P_LNO_VG, k_lno_vgrad<12><<<gv, kLnoThreads, 0, st>>>(A));
-    else if (per_lane <= 16)
-        TB_KLAUNCH(P_LNO_VG, k_lno_vgrad<16><<<gv, kLnoThreads, 0, st>>>(A));
-    else
-        TB_KLAUNCH(P_LNO_VG, k_lno_vgrad<32><<<gv, kLnoThreads, 0, st>>>(A));
-    return TRIPLES_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1324,12 +1204,11 @@ static int f1_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, TcF
     T.err = &ctrl->err;
     T.bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16 ? 1 : 0;
     T.kseg = P.kseg;
-    T.blocked = P.lno ? 0 : 1;
     for (int t = 0; t < 6; t++) T.tmS_ok[t] = 0;
     for (int t = 0; t < ch.nperm; t++) {
         const PermBlock &pb = ch.pb[t];
         if (pb.Tx == 16 && pb.Tz == 16 && d.o >= 2) {
-            const int trc = make_tmap_stage(&T.tmS[t], S + pb.soff, d.o, pb.Tx, pb.Ty, T.blocked != 0);
+            const int trc = make_tmap_stage(&T.tmS[t], S + pb.soff, d.o, pb.Ty);
             if (trc != TRIPLES_OK) return trc;
             T.tmS_ok[t] = 1;
         }
@@ -1382,6 +1261,43 @@ static void f2_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, co
     F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
 }
 
+// Where the regions of a sub-range triple lie in the (blocked) staging and in
+// Wbar (wmul: 2 for the 16-bit hi and lo planes, 1 for FP64).
+static void sub_regions(const ChunkDesc &ch, int o, const int *st, const int *len, int wmul, int elem, F2mSub &u) {
+    u.full = 1;
+    for (int t = 0; t < 3; t++) {
+        u.st[t] = st[t];
+        u.len[t] = len[t];
+        if (len[t] != 8) u.full = 0;
+    }
+    u.bulk = u.bulk_bytes = 0;
+    for (int pi = 0; pi < 6; pi++) {
+        int pp[3];
+        perm_of(pi, pp);
+        int t = 0;
+        while (t + 1 < ch.nperm && !(ch.pb[t].bx == ch.blk[pp[0]] && ch.pb[t].by == ch.blk[pp[1]] &&
+                                     ch.pb[t].bz == ch.blk[pp[2]]))
+            t++;
+        const PermBlock &pb = ch.pb[t];
+        const int xs = st[pp[0]] - pb.X0, ys = st[pp[1]] - pb.Y0, zs = st[pp[2]] - pb.Z0;
+        F2mPi &D = u.pi[pi];
+        D.s0 = f2m_stage_offset(pb, o, 0, 0, 0, ys, xs, zs);   // (y, x, z) at a block's origin: no exchange
+        D.rs = pb.Tx * pb.Ty * pb.Tz;
+        D.wx = o * pb.rzp;
+        D.wp = pb.Tx * D.wx;
+        D.wy = o * D.wp;
+        D.rzp = pb.rzp;
+        D.tz = pb.Tz;
+        D.w0 = wmul * pb.swoff + (long long)ys * D.wy + (long long)xs * D.wx + zs;
+        D.half = (long long)pb.Ty * D.wy;
+        D.bytes = elem * len[0] * len[1] * len[2];
+        if (D.bytes % 16 == 0) {
+            u.bulk |= 1 << pi;
+            u.bulk_bytes += D.bytes;
+        }
+    }
+}
+
 // Mixed-precision epilogue parameters of one chunk.
 static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, const TriplesIO &io, bool whole, F2M &F) {
     Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
@@ -1394,39 +1310,8 @@ static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, c
     F.whole = whole ? 1 : 0;
     for_sub_ranges(ch, 8, [&](const int *st, const int *len) {
         F2mSub &u = F.sub[F.nsub++];
-        u.full = 1;
-        for (int t = 0; t < 3; t++) {
-            u.st[t] = st[t];
-            u.len[t] = len[t];
-            if (len[t] != 8) u.full = 0;
-        }
+        sub_regions(ch, o, st, len, 2, 4, u);
         u.pat = st[0] == st[2] ? 3 : (st[0] == st[1] ? 1 : (st[1] == st[2] ? 2 : 0));
-        u.bulk = u.bulk_bytes = 0;
-        for (int pi = 0; pi < 6; pi++) {
-            int pp[3];
-            perm_of(pi, pp);
-            int t = 0;
-            while (t + 1 < ch.nperm && !(ch.pb[t].bx == ch.blk[pp[0]] && ch.pb[t].by == ch.blk[pp[1]] &&
-                                         ch.pb[t].bz == ch.blk[pp[2]]))
-                t++;
-            const PermBlock &pb = ch.pb[t];
-            const int xs = st[pp[0]] - pb.X0, ys = st[pp[1]] - pb.Y0, zs = st[pp[2]] - pb.Z0;
-            F2mPi &D = u.pi[pi];
-            D.s0 = f2m_stage_offset(pb, o, 0, 0, 0, ys, xs, zs);   // (y, x, z) at a block's origin: no exchange
-            D.rs = pb.Tx * pb.Ty * pb.Tz;
-            D.wx = o * pb.rzp;
-            D.wp = pb.Tx * D.wx;
-            D.wy = o * D.wp;
-            D.rzp = pb.rzp;
-            D.tz = pb.Tz;
-            D.w0 = 2 * pb.swoff + (long long)ys * D.wy + (long long)xs * D.wx + zs;
-            D.half = (long long)pb.Ty * D.wy;
-            D.bytes = 4 * len[0] * len[1] * len[2];
-            if (D.bytes % 16 == 0) {
-                u.bulk |= 1 << pi;
-                u.bulk_bytes += D.bytes;
-            }
-        }
     });
     F.ijk = (int *)(ws + P.off_ijk);
     F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
@@ -1442,6 +1327,95 @@ static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, c
     F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
     F.err = &ctrl->err;
     F.ticket = &ctrl->slot[slot].ticket;
+}
+
+// LNO chunk epilogue: energy of the projected amplitudes and, with want_grad,
+// mat_bar, the orbital-energy and V-term gradients and the Wbar staging that
+// the adjoint contractions read next (lno.cuh).
+template <int COLS>
+static int lno_projections(const LnoArgs &A, cudaStream_t st, unsigned &grid) {
+    const long long tiles = (long long)A.o * A.o * A.nsub * (512 / COLS);
+    grid = (unsigned)std::min(tiles, (long long)2 * num_sms());
+    const size_t smem = LnoProj<COLS>::smem(A.o);
+    const int rc = smem_optin(k_lno_proj<COLS>, smem);
+    if (rc != TRIPLES_OK) return rc;
+    for (int slot = 2; slot >= 0; slot--)
+        TB_KLAUNCH(P_LNO_PROJ, (k_lno_proj<COLS><<<grid, kLnoThreads, smem, st>>>(A, slot, slot == 2 ? 1 : 0)));
+    return TRIPLES_OK;
+}
+
+template <typename StageT>
+static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const TriplesIO &io, char *ws) {
+    const bool mixed = sizeof(StageT) == 4, bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16;
+    {
+        const int rc = once_per_device(mixed ? INIT_LNO : INIT_LNO64, [&]() -> int {
+            int rc = smem_optin(k_lno_fwd<StageT>, lno_fwd_smem());
+            if (rc != TRIPLES_OK) return rc;
+            if (!mixed) return smem_optin(k_lno_adj<0>, LnoAdj<0>::SMEM);
+            if ((rc = smem_optin(k_lno_adj<1>, LnoAdj<1>::SMEM)) != TRIPLES_OK) return rc;
+            return smem_optin(k_lno_adj<2>, LnoAdj<2>::SMEM);
+        });
+        if (rc != TRIPLES_OK) return rc;
+    }
+    const int o = P.d.o;
+    Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
+    LnoArgs A;
+    A.o = o;
+    A.v = P.d.v;
+    A.nsub = 0;
+    int n[3];
+    for (int t = 0; t < 3; t++) n[t] = (ch.nabc[t] + 7) / 8;
+    for (int c = 0; c < n[0] * n[1] * n[2]; c++) {
+        const int idx[3] = {c / (n[1] * n[2]), c / n[2] % n[1], c % n[2]};
+        int sst[3], len[3];
+        for (int t = 0; t < 3; t++) {
+            sst[t] = ch.base[t] + 8 * idx[t];
+            len[t] = std::min(8, ch.nabc[t] - 8 * idx[t]);
+        }
+        F2mSub &u = A.sub[A.nsub++];
+        sub_regions(ch, o, sst, len, mixed ? 2 : 1, (int)sizeof(StageT), u);
+        u.pat = ch.blk[0] == ch.blk[2] ? 3 : (ch.blk[0] == ch.blk[1] ? 1 : (ch.blk[1] == ch.blk[2] ? 2 : 0));
+    }
+    A.n_ijk = P.n_ijk;
+    A.ijk = (int *)(ws + P.off_ijk);
+    A.S = ws + P.off_S;
+    A.WW = (double *)(ws + P.off_L[0]);
+    A.PQ = (double *)(ws + P.off_L[1]);
+    A.Q = (double *)(ws + P.off_L[2]);
+    A.PW = (double *)(ws + P.off_L[3]);
+    A.mat = io.mat; A.mo_e = io.mo_energy; A.t1 = io.t1; A.t2 = io.t2; A.ovov = io.ovov; A.fvo = io.fvo;
+    A.SW = P.want_grad ? (void *)(ws + P.off_SW) : nullptr;
+    A.wscale = &ctrl->slot[0].wscale;
+    A.mat_bar = io.mat_bar; A.mo_bar = io.mo_energy_bar; A.t1_bar = io.t1_bar; A.t2_bar = io.t2_bar;
+    A.ovov_bar = io.ovov_bar; A.fvo_bar = io.fvo_bar;
+    A.ybar = io.ybar;
+    A.f = 2.0 * io.ybar / 3.0;
+    A.g = ch.nperm / 9.0;
+    A.want_grad = P.want_grad;
+    A.part = (double *)(ws + P.off_lpart);
+    const unsigned items = (unsigned)(P.n_ijk * A.nsub);
+    TB_KLAUNCH(P_LNO, (k_lno_fwd<StageT><<<items, kLnoThreads, lno_fwd_smem(), st>>>(A)));
+    // columns per tile: 128 while two buffers of all rows leave room for two CTAs per SM
+    unsigned parts = 0;
+    const int prc = o <= 16   ? lno_projections<128>(A, st, parts)
+                    : o <= 32 ? lno_projections<64>(A, st, parts)
+                              : lno_projections<32>(A, st, parts);
+    if (prc != TRIPLES_OK) return prc;
+    Group<ChunkAux, 1> G;
+    G.n = 1;
+    G.job[0] = chunk_aux(P, ch, 0, io, 3 * (int)parts);
+    G.job[0].e_part = A.part;
+    TB_KLAUNCH(P_PREP, (k_energy_sum<<<1, 256, 0, st>>>(G, 1)));
+    if (!P.want_grad) return TRIPLES_OK;
+    if (!mixed) {
+        TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<0><<<items, kLnoThreads, LnoAdj<0>::SMEM, st>>>(A)));
+        return TRIPLES_OK;
+    }
+    // fp16: power-of-two scale of the split Wbar; bf16: scale 1 (both read by the contractions)
+    TB_KLAUNCH(P_PREP, (k_chunk_scale<<<1, 32, 0, st>>>(G)));
+    if (bf16) TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<2><<<items, kLnoThreads, LnoAdj<2>::SMEM, st>>>(A)));
+    else TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<1><<<items, kLnoThreads, LnoAdj<1>::SMEM, st>>>(A)));
+    return TRIPLES_OK;
 }
 
 // Adjoint-contraction parameters of one chunk and kind (0: ovvv_bar, 1: t2_bar
@@ -1678,9 +1652,7 @@ static int mixed_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t 
     }
     if (P.lno) {
         // projected energy: whole-chunk epilogue instead of the orbit tiles (one chunk at a time)
-        const int rc = lno_chunk<float>(P, ch[0], st, io, ws, (Ctrl *)(ws + P.off_ctrl), (const float *)(ws + P.off_S),
-                                        P.want_grad ? (void *)(ws + P.off_SW) : nullptr, (int *)(ws + P.off_ijk),
-                                        bf16 ? 2 : 1);
+        const int rc = lno_chunk<float>(P, ch[0], st, io, ws);
         if (rc != TRIPLES_OK) return rc;
     } else {
         Group<F2M, NG> G;
@@ -1715,6 +1687,7 @@ static int fp64_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t s
     GemmLaunch L;
     L.d = P.d;
     L.n = n;
+    L.blocked = P.lno;
     L.A1 = (const double *)(ws + P.off_A1);
     L.B1 = (const double *)(ws + P.off_B1);
     L.A2 = (const double *)(ws + P.off_A2);
@@ -1728,7 +1701,7 @@ static int fp64_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t s
     int rc;
     if ((rc = chunk_gemm<GK_F1>(st, P_F1, L)) != TRIPLES_OK) return rc;
     if (P.lno) {
-        rc = lno_chunk<double>(P, ch[0], st, io, ws, (Ctrl *)(ws + P.off_ctrl), L.S[0], L.SW[0], (int *)(ws + P.off_ijk), 0);
+        rc = lno_chunk<double>(P, ch[0], st, io, ws);
         if (rc != TRIPLES_OK) return rc;
     } else {
         Group<F2P, NG> G;
