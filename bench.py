@@ -396,14 +396,22 @@ def run_accuracy(args, o, v, naux):
 # LNO fragment (T): projector on the first occupied index
 # ---------------------------------------------------------------------------
 LNO_METRIC = "LNO (T) E+VJP TFLOP/s (projected first occupied index), B200 vs reference CPU kernels"
-# algorithmic bytes per raw amplitude position of each LNO epilogue pass
-# (sz = staging element size: 8 FP64, 4 mixed): the forward pass reads w and
-# writes WW and Q, the projections (one per occupied slot) read them and update
-# PW and PQ, the adjoint pass reads Zbar, PQ and Q and writes the Wbar operand
-# (FP64, or two 16-bit halves).
+# algorithmic bytes per raw amplitude position of the LNO epilogue (sz = staging
+# element size: 8 FP64, 4 mixed) as four passes over work arrays of every
+# ordering of a chunk: the forward pass reads w and writes WW and Q; the
+# projection reads them and writes Zbar, Dbar and P^T(Wtbar); the adjoint pass
+# reads the last two and writes vbar and the Wbar operand (FP64, or two 16-bit
+# halves); the V gradients read vbar and Dbar.
 def lno_pass_bytes(sz):
-    # the FP64 box arrays hold one value per six raw amplitudes: two written by the forward pass, two read and
-    # two updated by each of the three projections, three read by the adjoint pass
+    return {"lno_tile_fwd": sz + 16, "lno_projection": 40, "lno_tile_adj": 16 + 8 + (8 if sz == 8 else 4),
+            "lno_vgrad": 16}
+
+
+# ... and as the library does it, over one box of virtual indices (one value per
+# six raw amplitudes): WW and Q written by the forward pass; read, and PW and PQ
+# updated, by the projection of each of the three occupied slots; Zbar, PQ and
+# Q read by the adjoint pass, which writes the Wbar operand.
+def lno_box_bytes(sz):
     return {"lno_tile_fwd": sz + 16 / 6, "lno_projection": 128 / 6, "lno_tile_adj": 24 / 6 + (8 if sz == 8 else 4)}
 
 
@@ -488,7 +496,7 @@ def run_lno(args, o, v, naux):
         pass
     hpeak, hnote = (float(peaks["hbm_gbs"]), "of measured (copy)") if "hbm_gbs" in peaks else (6650.0, "of fallback")
     positions = float(o) ** 3 * float(v) ** 3
-    pbytes = lno_pass_bytes(8 if args.precision == "fp64" else 4)
+    pbytes = lno_box_bytes(8 if args.precision == "fp64" else 4)
     total_ms = sum(m for m, _ in prof.values()) or 1.0
     classes = {}
     for k, b in pbytes.items():
