@@ -1,203 +1,45 @@
-// FP64 chunk epilogue: energy and adjoint of the raw triples amplitudes (the
-// mixed-precision modes use f2m.cuh).
-//
-// One CTA owns one occupied representative i >= j >= k and one triple of
-// virtual sub-ranges (a-sub >= b-sub >= c-sub, SB wide).  Every raw
-// amplitude w^{pqr}_{xyz} with {p,q,r} = {i,j,k} and {x,y,z} one value from
-// each sub-range belongs to exactly one such CTA, and the CTA holds all of
-// them: 36 regions = (distinct orderings of the sub-ranges) x (distinct
-// orderings of ijk), each SB^3 values, staged in shared memory with
-// coalesced loads.
-//
-// Per orbit item (a >= b >= c), with d = sigma_s(abc) the six orderings,
-//   WW(d) = sum_tau w(tau(ijk), tau(d)),  VV(d) likewise from v,
-//   Z(d)  = 4X(d) + X(d2,d0,d1) + X(d1,d2,d0) - 2[X(d2,d1,d0) + X(d0,d2,d1) + X(d1,d0,d2)],
-//   X = WW + VV/2,
-//   E    += (n_ijk n_abc / 18) sum_s WW Z / D,   D = e_i+e_j+e_k-e_a-e_b-e_c
-// (the a>=b>=c restricted sum of pyscfad/cc/ccsd_t_slow.py:46-124 rewritten
-// over occupied-triplet orbits), and the adjoint
-//   Wbar(d) = c (Z + R WW)/D, Vbar(d) = c (R WW)/(2D), dE/dD = -c sum WW Z / D^2
-// (ccsd_t_vjp.c:64-117) scattered back to every raw position of the orbit.
-// Wbar goes to its own buffer in the layout the gradient contractions read:
-// [h][y][p][x][q][r][z].  Vbar never leaves the CTA: since
-//   v^{pqr}_{xyz} = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r]
-// and the CTA already holds those factors in its V-term tables, its
-// contributions to ovov_bar / t2_bar (row sums over the z run of a thread)
-// and to t1_bar / fvo_bar (column sums, reduced across the warp) are added
-// to the global gradients directly (FP64 reductions).
-//
-// Item results (Wbar, Vbar per ordering s) are written once per item into
-// shared memory over the dead W tile; the write-back maps every raw position
-// to its item(s) through the (sub-range ordering, occupied ordering) pairs of
-// its region, which in degenerate cases (repeated indices) are several.
+// FP64 orbit kernels: the chunk epilogue of the FP64 mode (k_f2t) and what the
+// LNO kernels (lno.cuh) share with it.  The work items, the region layout and
+// the treatment of repeated indices are those of f2m.cuh; here everything is
+// FP64, one CTA of 256 threads takes one item, and the raw amplitudes are
+// gathered straight from the contiguous regions of the staging buffer (every
+// sector of a region is read by the CTA, the permuted gathers meet it in L1):
+// V-term tables and element results fill the shared memory of two CTAs per SM.
+// What bounds it: latency of the gathers and tables at 16 warps per SM, then the
+// FP64 column sums.  Measured at nocc 12 nvir 100, E + VJP: 33.8 to 18.5 ms (4-wide sub-ranges,
+// 64 threads per CTA and staged regions before).
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
+#include "f2m.cuh"
 
 namespace tb {
 
-struct F2Sub {
-    int st[3];
-    int len[3];
-};
-constexpr int kMaxSub = 64;    // sub-range triples of a chunk: (16 / 4)^3
-constexpr int kF2SB = 4;       // sub-range width
-constexpr int kF2Threads = kF2SB * kF2SB * kF2SB;
+constexpr int kF2Threads = 256;
 
 struct F2P {
-    Dims d;
-    ChunkDesc ch;
-    int nsub;
-    F2Sub sub[kMaxSub];
+    int o, v;
+    int nsub, n_ijk;
     const int *ijk;
     const double *mo_e, *t1, *t2, *ovov, *fvo;
-    const double *S;    // W per ordering tau: [p][q][y][x][r][z] at ch.pb[tau].soff
+    const double *S;    // W per ordering tau, blocked staging (no row exchange)
     double *SW;         // Wbar out, per tau at ch.pb[tau].swoff: [y][p][x][q][r][z]
     double ybar;
     int want_grad;
-    double *e_part;     // energy partial of each CTA, at sub * n_ijk + rep
-    int n_ijk;          // occupied representatives (stride of e_part)
+    double *e_part;     // energy partial of each item, at sub * n_ijk + rep
     double *mo_bar, *t1_bar, *fvo_bar, *ovov_bar, *t2_bar;
+    F2mSub sub[kF2mMaxSub];
 };
 
-// Shared-memory region layout: element (y,x,z) at y*SY + x*SX + z.  The padded
-// strides keep the permuted gathers of a warp within 2-way bank conflicts.
+// Shared memory: V-term tables, element results V (FP64) and W (FP64, or the
+// 16-bit halves of the LNO mixed modes).
+template <int SPLIT>
 struct F2Smem {
-    static constexpr int SB = kF2SB;
-    static constexpr int SX = SB;
-    static constexpr int SY = SB * SB + 1;
-    static constexpr int REG = SY * SB;
-    static constexpr int NV = 3 * SB;
-    static constexpr int NVP = NV + 1;
-    static constexpr int TAB = 6 * NV * NVP;
-    static constexpr int ITEMS = SB * SB * SB;
-    static_assert(ITEMS == kF2Threads, "one orbit item per thread");
+    using W = typename std::conditional<SPLIT == 0, double, uint32_t>::type;
+    static constexpr size_t TABLES = (36 * 64 + 72) * sizeof(double2);
+    static constexpr size_t BYTES = TABLES + 6 * 512 * (sizeof(double) + sizeof(W));
 };
-
-__host__ __device__ constexpr size_t f2_smem_bytes() {
-    return sizeof(double) * (36 * F2Smem::REG + 2 * F2Smem::TAB + 2 * 3 * F2Smem::NV);
-}
-
-__host__ __device__ constexpr inline int pair_index(int sp, int sq) { return 2 * sp + (sq > sp ? sq - 1 : sq); }
-
-// A z run of N contiguous values moved with the widest aligned vector access:
-// one warp instruction then fills whole 32-byte sectors instead of touching
-// 32 sectors with a 2- or 4-byte write each.  Partial or unaligned runs
-// (remainder blocks) fall back to scalar accesses.
-template <typename T, int N>
-union RunBuf {
-    static constexpr int BYTES = N * (int)sizeof(T);
-    static constexpr int VB = BYTES >= 16 ? 16 : (BYTES >= 8 ? 8 : 4);
-    T e[N];
-    uint4 u4[BYTES / 16 > 0 ? BYTES / 16 : 1];
-    uint2 u2[BYTES / 8 > 0 ? BYTES / 8 : 1];
-};
-
-template <typename T, int N>
-__device__ __forceinline__ void st_run(T *dst, const RunBuf<T, N> &b, int n) {
-    using B = RunBuf<T, N>;
-    const uintptr_t a = reinterpret_cast<uintptr_t>(dst);
-    if (n == N && B::VB == 16 && (a & 15) == 0) {
-#pragma unroll
-        for (int c = 0; c < B::BYTES / 16; c++) reinterpret_cast<uint4 *>(dst)[c] = b.u4[c];
-    } else if (n == N && B::VB == 8 && (a & 7) == 0) {
-#pragma unroll
-        for (int c = 0; c < B::BYTES / 8; c++) reinterpret_cast<uint2 *>(dst)[c] = b.u2[c];
-    } else {
-#pragma unroll
-        for (int z = 0; z < N; z++)
-            if (z < n) dst[z] = b.e[z];
-    }
-}
-
-template <typename T, int N>
-__device__ __forceinline__ void ld_run(RunBuf<T, N> &b, const T *src, int n) {
-    using B = RunBuf<T, N>;
-    const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-    if (n == N && B::VB == 16 && (a & 15) == 0) {
-#pragma unroll
-        for (int c = 0; c < B::BYTES / 16; c++) b.u4[c] = reinterpret_cast<const uint4 *>(src)[c];
-    } else {
-#pragma unroll
-        for (int z = 0; z < N; z++) b.e[z] = (z < n) ? src[z] : (T)0;
-    }
-}
-
-// Region bookkeeping of a CTA depends only on which of i, j, k coincide and
-// which sub-ranges coincide (4 x 4 patterns), so it is tabulated once on the
-// host and read from constant memory.  For a pattern:
-//   reg[pi*6 + rho]   region of (sub-range ordering pi, occupied ordering rho)
-//   rep[g]            representative pi*6 + rho of region g (first in order)
-//   combo[g][0..ncombo[g])  all pi*6 + rho of region g, ascending
-//   sof[pi*6 + rho]   the ordering s with perm_compose(s, rho) = pi
-struct F2Pattern {
-    unsigned char nrole, npi;
-    unsigned char reg[36];
-    unsigned char rep[36];
-    unsigned char ncombo[36];
-    unsigned char combo[36][36];
-    unsigned char sof[36];
-};
-constexpr int kF2Patterns = 16;
-__constant__ F2Pattern c_f2pat[kF2Patterns];
-
-// pattern index: 4 * (i==j==k ? 3 : i==j ? 1 : j==k ? 2 : 0) + (sub-ranges likewise)
-__host__ __device__ inline int f2_pattern_index(int i, int j, int k, int a, int b, int c) {
-    const int pij = (i == k) ? 3 : (i == j ? 1 : (j == k ? 2 : 0));
-    const int pab = (a == c) ? 3 : (a == b ? 1 : (b == c ? 2 : 0));
-    return 4 * pij + pab;
-}
-
-inline void f2_build_patterns(F2Pattern out[kF2Patterns]) {
-    const int vals[4][3] = {{2, 1, 0}, {1, 1, 0}, {1, 0, 0}, {0, 0, 0}};
-    for (int pij = 0; pij < 4; pij++)
-        for (int pab = 0; pab < 4; pab++) {
-            F2Pattern &T = out[4 * pij + pab];
-            const int *ijk = vals[pij], *st = vals[pab];
-            auto same = [&](const int *val, int ra, int rb) {
-                int qa[3], qb[3];
-                perm_of(ra, qa);
-                perm_of(rb, qb);
-                return val[qa[0]] == val[qb[0]] && val[qa[1]] == val[qb[1]] && val[qa[2]] == val[qb[2]];
-            };
-            // dense index of an ordering among the distinct orderings (first occurrence order)
-            auto dense = [&](const int *val, int r, int &count) {
-                int first_at = r;
-                for (int r2 = 5; r2 >= 0; r2--)
-                    if (same(val, r2, r)) first_at = r2;
-                int id = 0;
-                count = 0;
-                for (int r2 = 0; r2 < 6; r2++) {
-                    bool first = true;
-                    for (int r3 = 0; r3 < r2; r3++)
-                        if (same(val, r2, r3)) first = false;
-                    if (first) {
-                        count++;
-                        if (r2 < first_at) id++;
-                    }
-                }
-                return id;
-            };
-            int nrole = 0, npi = 0;
-            for (int t = 0; t < 36; t++) {
-                const int pi = t / 6, rho = t % 6;
-                const int rid = dense(ijk, rho, nrole), pid = dense(st, pi, npi);
-                T.reg[t] = (unsigned char)(pid * nrole + rid);
-                for (int s2 = 0; s2 < 6; s2++)
-                    if (perm_compose(s2, rho) == pi) T.sof[t] = (unsigned char)s2;
-            }
-            T.nrole = (unsigned char)nrole;
-            T.npi = (unsigned char)npi;
-            for (int g = 0; g < 36; g++) {
-                T.ncombo[g] = 0;
-                T.rep[g] = 0;
-            }
-            for (int t = 0; t < 36; t++) {
-                const int g = T.reg[t];
-                if (T.ncombo[g] == 0) T.rep[g] = (unsigned char)t;
-                T.combo[g][T.ncombo[g]++] = (unsigned char)t;
-            }
-        }
-}
 
 // Sum NV (power of two) per-lane values over aligned groups of G lanes
 // (NV <= G <= 32, G a power of two); afterwards lane l holds the group total
@@ -220,408 +62,345 @@ __device__ __forceinline__ T group_reduce_scatter(T (&v)[NV], int lane) {
     return r;
 }
 
-// One CTA per item of the jobs (chunks) of a launch.
-template <typename JOBS>
-__global__ void __launch_bounds__(kF2Threads, 4) k_f2t(const __grid_constant__ JOBS J) {
-    using StageT = double;
-    using C = F2Smem;
-    constexpr int SB = C::SB, NT = kF2Threads;
-    constexpr int REG = C::REG, NV = C::NV, NVP = C::NVP;
-    constexpr int SX = C::SX, SY = C::SY;
-    constexpr int NW = NT / 32, IPT = C::ITEMS / NT;
-    JobCursor jcur;
-    int blk;
-    const int jb = jcur.at(J, (int)blockIdx.x, blk);
-    const F2P &P = J.job[JOBS::kOne ? 0 : jb];
-    extern __shared__ __align__(16) uint8_t f2_smem[];
-    StageT *sW = reinterpret_cast<StageT *>(f2_smem);
-    StageT *sG = sW;                      // item results [12][REG] (padded) once W is consumed
-    StageT *tOV = sW + 36 * REG;
-    StageT *tT2 = tOV + C::TAB;
-    StageT *tT1 = tT2 + C::TAB;
-    StageT *tFV = tT1 + 3 * NV;
-    __shared__ double s_ev[NV];
-    __shared__ double s_red[2][NW];
-    __shared__ int s_rd[36][9];               // per region: pi, rho, tau, lx, ly, lz, p, q, r
-    __shared__ long long s_gb[36], s_wb[36];  // staging / Wbar base offsets of each region
-    __shared__ int s_gs[36][2], s_ws[36][2];  // (y, x) strides in staging / Wbar
+// element (a, b, c) of thread t; its second one is (a + 4, b, c).  A warp spans 2 x 4 x 4 of them
+__device__ __forceinline__ void f2_element(int t, int &a, int &b, int &c) {
+    a = ((t >> 4) & 1) | (((t >> 7) & 1) << 1);
+    b = ((t >> 2) & 3) | (((t >> 6) & 1) << 2);
+    c = (t & 3) | (((t >> 5) & 1) << 2);
+}
 
-    const Dims &d = P.d;
-    const int o = d.o, v = d.v;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // linear grid, sub-range triple fastest: the blocks of one representative run together
-    const int sub = blk % P.nsub, rep = blk / P.nsub;
-    const F2Sub &R = P.sub[sub];
-    const int ijk[3] = {P.ijk[3 * rep], P.ijk[3 * rep + 1], P.ijk[3 * rep + 2]};
+// 64-entry table block of 16-byte entries: eight lanes of a gather hit eight banks
+__device__ __forceinline__ int f2_tab(int x, int y) { return y * 8 + (x ^ ((y & 1) << 2) ^ (y & 2)); }
 
-    // canonical sub-range slot of each role (identical ranges share a slot)
-    int cs[3];
-    cs[0] = 0;
-    cs[1] = (R.st[1] == R.st[0]) ? 0 : 1;
-    cs[2] = (R.st[2] == R.st[1]) ? cs[1] : ((R.st[2] == R.st[0]) ? 0 : 2);
-    const F2Pattern &pat = c_f2pat[f2_pattern_index(ijk[0], ijk[1], ijk[2], R.st[0], R.st[1], R.st[2])];
-    const int nreg = pat.nrole * pat.npi;
-    for (int e = tid; e < NV; e += NT) s_ev[e] = 0.0;
+// FP64 V-term tables of an item: {ovov[p,x,q,y], t2[q,p,y,x]} per (rho, pi), {t1[r,z], fvo[z,r]}
+template <typename ARGS>
+__device__ __forceinline__ void f2_load_tables(const ARGS &A, const F2mSub &R, int i0, int i1, int i2, double2 *tab,
+                                               double2 *tf) {
+    const int o = A.o, v = A.v;
+    double *ts = reinterpret_cast<double *>(tab);
+#pragma unroll 3
+    for (int e = threadIdx.x; e < 36 * 64; e += kF2Threads) {
+        const int blk = e >> 6, hi = (e >> 3) & 7, lo = e & 7;
+        int pr[3], pp[3];
+        perm_of(blk / 6, pr);
+        perm_of(blk % 6, pp);
+        const int p = sel3(i0, i1, i2, pr[0]), q = sel3(i0, i1, i2, pr[1]);
+        const int lx = sel3(R.len[0], R.len[1], R.len[2], pp[0]), ly = sel3(R.len[0], R.len[1], R.len[2], pp[1]);
+        const int sx = sel3(R.st[0], R.st[1], R.st[2], pp[0]), sy = sel3(R.st[0], R.st[1], R.st[2], pp[1]);
+        // the fast index of each factor in turn runs over the lanes
+        ts[2 * (blk * 64 + f2_tab(hi, lo))] =
+            hi < lx && lo < ly ? __ldg(&A.ovov[(((long long)p * v + sx + hi) * o + q) * v + sy + lo]) : 0.0;
+        ts[2 * (blk * 64 + f2_tab(lo, hi)) + 1] =
+            lo < lx && hi < ly ? __ldg(&A.t2[(((long long)q * o + p) * v + sy + hi) * v + sx + lo]) : 0.0;
+    }
+    for (int e = threadIdx.x; e < 72; e += kF2Threads) {
+        const int r = sel3(i0, i1, i2, e / 24), s = (e >> 3) % 3, zl = e & 7;
+        const int z = sel3(R.st[0], R.st[1], R.st[2], s) + zl;
+        const bool in = zl < sel3(R.len[0], R.len[1], R.len[2], s);
+        tf[e] = in ? make_double2(__ldg(&A.t1[(long long)r * v + z]), __ldg(&A.fvo[(long long)z * o + r]))
+                   : make_double2(0.0, 0.0);
+    }
+}
 
-    // region descriptors; find the staging ordering tau of a sub-range ordering
-    auto block_of = [&](int start) {
-        for (int t = 0; t < 3; t++)
-            if (start >= P.ch.base[t] && start < P.ch.base[t] + P.ch.nabc[t]) return P.ch.blk[t];
-        return -1;
-    };
-    auto tau_of = [&](int pi) {
-        int pp[3];
+__device__ __forceinline__ void f2_r3(const double (&x)[6], double (&z)[6]) {
+#pragma unroll
+    for (int s = 0; s < 6; s++)
+        z[s] = 4.0 * x[s] + x[perm_compose(s, 4)] + x[perm_compose(s, 3)] -
+               2.0 * (x[perm_compose(s, 5)] + x[perm_compose(s, 1)] + x[perm_compose(s, 2)]);
+}
+
+// WW and VV of the thread's two elements, six orderings each: orbit sums over
+// the regions of the item (StageT staging: FP32 rows are exchanged, FP64 rows not)
+template <typename StageT>
+__device__ __forceinline__ void f2_amplitudes(const StageT *__restrict__ S, const F2mSub &R, int o, int i0, int i1, int i2,
+                                              int ca, int cb, int cc, bool ok0, bool ok1, const double2 *tab,
+                                              const double2 *tf, double (&WW)[2][6], double (&VV)[2][6]) {
+    const int loc[3] = {ca, cb, cc};
+    int w0[6], w1[6], t0[6];   // this thread's positions in the regions (elements a, a + 4) and tables
+#pragma unroll
+    for (int pi = 0; pi < 6; pi++) {
+        int pp[3] = {0, 0, 0};
         perm_of(pi, pp);
-        const int bx = block_of(R.st[pp[0]]), by = block_of(R.st[pp[1]]), bz = block_of(R.st[pp[2]]);
-        int t = 0;
-        for (; t < P.ch.nperm - 1; t++)
-            if (P.ch.pb[t].bx == bx && P.ch.pb[t].by == by && P.ch.pb[t].bz == bz) break;
-        return t;
-    };
-    if (tid < nreg) {
-        const int pi = pat.rep[tid] / 6, rho = pat.rep[tid] % 6;
-        int pp[3], pr[3];
-        perm_of(pi, pp);
+        const int x = loc[pp[0]], y = loc[pp[1]], z = loc[pp[2]];
+        const int ex = R.len[pp[0]], ez = R.len[pp[2]];
+        const bool swz = sizeof(StageT) == 4 && ex == 8 && ez == 8;
+        const int dx = pp[0] == 0 ? 4 : 0, dy = pp[1] == 0 ? 4 : 0, dz = pp[2] == 0 ? 4 : 0;
+        const int s0 = (x * ez + z) ^ (swz ? f2m_row_swizzle(y) : 0);
+        const int s1 = ((x + dx) * ez + z + dz) ^ (swz ? f2m_row_swizzle(y + dy) : 0);
+        w0[pi] = ok0 ? y * ex * ez + s0 : 0;
+        w1[pi] = ok1 ? (y + dy) * ex * ez + s1 : w0[pi];
+        t0[pi] = f2_tab(x, y);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+#pragma unroll
+        for (int s = 0; s < 6; s++) WW[e][s] = VV[e][s] = 0.0;
+    __syncthreads();   // the tables are complete
+#pragma unroll
+    for (int rho = 0; rho < 6; rho++) {
+        int pr[3] = {0, 0, 0};
         perm_of(rho, pr);
-        const int tau = tau_of(pi);
-        const int p = pr[0] == 0 ? ijk[0] : (pr[0] == 1 ? ijk[1] : ijk[2]);
-        const int q = pr[1] == 0 ? ijk[0] : (pr[1] == 1 ? ijk[1] : ijk[2]);
-        const int r = pr[2] == 0 ? ijk[0] : (pr[2] == 1 ? ijk[1] : ijk[2]);
-        int *rd = s_rd[tid];
-        rd[0] = pi;
-        rd[1] = rho;
-        rd[2] = tau;
-        rd[3] = R.len[pp[0]];
-        rd[4] = R.len[pp[1]];
-        rd[5] = R.len[pp[2]];
-        rd[6] = p;
-        rd[7] = q;
-        rd[8] = r;
-        const PermBlock &pb = P.ch.pb[tau];
-        const int xs = R.st[pp[0]] - pb.X0, ys = R.st[pp[1]] - pb.Y0, zs = R.st[pp[2]] - pb.Z0;
-        // staging S_tau[p][q][y][x][r][z]
-        const long long gy = (long long)pb.Tx * o * pb.Tz, gx = (long long)o * pb.Tz;
-        s_gb[tid] = pb.soff + (long long)(p * o + q) * pb.Ty * gy + ys * gy + xs * gx + (long long)r * pb.Tz + zs;
-        s_gs[tid][0] = (int)gy;
-        s_gs[tid][1] = (int)gx;
-        // Wbar_tau[y][p][x][q][rzp]
-        const long long wx = (long long)o * pb.rzp, wy = (long long)o * pb.Tx * wx;
-        s_wb[tid] = (long long)ys * wy + (long long)p * pb.Tx * wx + xs * wx + (long long)q * pb.rzp + (long long)r * pb.Tz + zs;
-        s_ws[tid][0] = (int)wy;
-        s_ws[tid][1] = (int)wx;
-    }
-    __syncthreads();
-
-    // ---- load the distinct regions, one (y, x) run of z values per thread step;
-    //      LB runs are fetched before any is stored, so their latencies overlap ----
-    // distinct sub-ranges: the tables need only the blocks of two different ranges
-    const bool distinct_rng = (cs[1] == 1 && cs[2] == 2);
-    {
-        constexpr int LB = 3;
-        const int nrun = nreg * SB * SB;
-        for (int e0 = tid; e0 < nrun; e0 += LB * NT) {
-            RunBuf<StageT, SB> b[LB];
-            StageT *dst[LB];
-            int lzs[LB];
+        const int ids[3] = {i0, i1, i2};
+        const long long idx = ((long long)ids[pr[0]] * o + ids[pr[1]]) * o + ids[pr[2]];
+        const double2 *tr = tf + pr[2] * 24;
+        const double2 tz[3] = {tr[ca], tr[8 + cb], tr[16 + cc]}, tz4 = tr[(ca + 4) & 7];
 #pragma unroll
-            for (int u = 0; u < LB; u++) {
-                const int e = e0 + u * NT;
-                dst[u] = nullptr;
-                lzs[u] = 0;
-                if (e < nrun) {
-                    const int reg = e / (SB * SB), yy = (e / SB) % SB, xx = e % SB;
-                    const int *rd = s_rd[reg];
-                    if (xx < rd[3] && yy < rd[4]) {
-                        lzs[u] = rd[5];
-                        ld_run(b[u], P.S + s_gb[reg] + (long long)yy * s_gs[reg][0] + (long long)xx * s_gs[reg][1],
-                               lzs[u]);
-                        dst[u] = sW + reg * REG + yy * SY + xx * SX;
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < LB; u++)
-                if (dst[u] != nullptr) {
-#pragma unroll
-                    for (int zz = 0; zz < SB; zz++)
-                        if (zz < lzs[u]) dst[u][zz] = b[u].e[zz];
-                }
-        }
-    }
-    // ---- tables for the V terms (TB entries fetched per batch) ----
-    {
-        constexpr int TB = 4;
-        for (int e0 = tid; e0 < 6 * NV * NV; e0 += TB * NT) {
-            double ov[TB], tt[TB];
-            int te[TB];
-#pragma unroll
-            for (int u = 0; u < TB; u++) {
-                const int e = e0 + u * NT;
-                ov[u] = tt[u] = 0.0;
-                te[u] = -1;
-                if (e < 6 * NV * NV) {
-                    const int pair = e / (NV * NV), xl = (e / NV) % NV, yl = e % NV;
-                    te[u] = (pair * NV + xl) * NVP + yl;
-                    const int sp = pair / 2, rem = pair % 2;
-                    const int sq = (rem < sp) ? rem : rem + 1;   // inverse of pair_index
-                    const int sx = xl / SB, sy = yl / SB;
-                    if (xl % SB < R.len[sx] && yl % SB < R.len[sy] && !(distinct_rng && sx == sy)) {
-                        const int x = R.st[sx] + xl % SB, y = R.st[sy] + yl % SB;
-                        const int p = (sp == 0) ? ijk[0] : (sp == 1 ? ijk[1] : ijk[2]);
-                        const int q = (sq == 0) ? ijk[0] : (sq == 1 ? ijk[1] : ijk[2]);
-                        ov[u] = P.ovov[(((long long)p * v + x) * o + q) * v + y];
-                        tt[u] = P.t2[(((long long)q * o + p) * v + y) * v + x];
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < TB; u++)
-                if (te[u] >= 0) {
-                    tOV[te[u]] = (StageT)ov[u];
-                    tT2[te[u]] = (StageT)tt[u];
-                }
-        }
-    }
-    for (int e = tid; e < 3 * NV; e += NT) {
-        const int sr = e / NV, zl = e % NV, sz = zl / SB;
-        StageT a1 = 0, f1 = 0;
-        if (zl % SB < R.len[sz]) {
-            const int z = R.st[sz] + zl % SB, r = (sr == 0) ? ijk[0] : (sr == 1 ? ijk[1] : ijk[2]);
-            a1 = (StageT)P.t1[(long long)r * v + z];
-            f1 = (StageT)P.fvo[(long long)z * o + r];
-        }
-        tT1[e] = a1;
-        tFV[e] = f1;
-    }
-    __syncthreads();
-
-    // ---- orbit items (IPT per thread) ----
-    const int i = ijk[0], j = ijk[1], k = ijk[2];
-    const int n_ijk = (i == k) ? 1 : ((i == j || j == k) ? 3 : 6);
-    const double e_ijk = P.mo_e[i] + P.mo_e[j] + P.mo_e[k];
-    double e_loc = 0.0, dd_loc = 0.0;
-    StageT gres[IPT][12];
-    bool gvalid[IPT];
-#pragma unroll
-    for (int it = 0; it < IPT; it++) {
-        const int item = tid + it * NT;
-        const int loc[3] = {item / (SB * SB), (item / SB) % SB, item % SB};
-        bool valid = loc[0] < R.len[0] && loc[1] < R.len[1] && loc[2] < R.len[2];
-        const int abc[3] = {R.st[0] + loc[0], R.st[1] + loc[1], R.st[2] + loc[2]};
-        if (valid && cs[1] == 0 && abc[0] < abc[1]) valid = false;
-        if (valid && cs[2] == cs[1] && abc[1] < abc[2]) valid = false;
-        gvalid[it] = valid;
-        double ddi = 0.0;
-        if (valid) {
-            const int vl[3] = {cs[0] * SB + loc[0], cs[1] * SB + loc[1], cs[2] * SB + loc[2]};
-            double WW[6], X[6];
-#pragma unroll
-            for (int s = 0; s < 6; s++) {
-                double sw = 0.0;
-                StageT sv = 0;   // V term: products of staged (StageT) factors
-#pragma unroll
-                for (int tau = 0; tau < 6; tau++) {
-                    const int pi = perm_compose(s, tau);
-                    int pp[3], pt[3];
-                    perm_of(pi, pp);
-                    perm_of(tau, pt);
-                    sw += (double)sW[pat.reg[pi * 6 + tau] * REG + loc[pp[1]] * SY + loc[pp[0]] * SX + loc[pp[2]]];
-                    const int pair = pair_index(pt[0], pt[1]);
-                    const int xl = vl[pp[0]], yl = vl[pp[1]], zl = vl[pp[2]];
-                    sv += tOV[(pair * NV + xl) * NVP + yl] * tT1[pt[2] * NV + zl] +
-                          tT2[(pair * NV + xl) * NVP + yl] * tFV[pt[2] * NV + zl];
-                }
-                WW[s] = sw;
-                X[s] = sw + 0.5 * (double)sv;
-            }
-            double Z[6], RW[6];
-#pragma unroll
-            for (int s = 0; s < 6; s++) {
-                Z[s] = 4.0 * X[s] + X[perm_compose(s, 4)] + X[perm_compose(s, 3)] -
-                       2.0 * (X[perm_compose(s, 5)] + X[perm_compose(s, 1)] + X[perm_compose(s, 2)]);
-                RW[s] = 4.0 * WW[s] + WW[perm_compose(s, 4)] + WW[perm_compose(s, 3)] -
-                        2.0 * (WW[perm_compose(s, 5)] + WW[perm_compose(s, 1)] + WW[perm_compose(s, 2)]);
-            }
-            const int n_abc = (abc[0] == abc[2]) ? 1 : ((abc[0] == abc[1] || abc[1] == abc[2]) ? 3 : 6);
-            const double cfac = (double)(n_ijk * n_abc) / 18.0;
-            const double Dn = e_ijk - P.mo_e[o + abc[0]] - P.mo_e[o + abc[1]] - P.mo_e[o + abc[2]];
-            const double rD = 1.0 / Dn;
-            double esum = 0.0;
-#pragma unroll
-            for (int s = 0; s < 6; s++) esum += WW[s] * Z[s];
-            e_loc += cfac * esum * rD;
-            if (P.want_grad) {
-                const double g0 = P.ybar * cfac * rD;
-                ddi = -P.ybar * cfac * esum * rD * rD;
-#pragma unroll
-                for (int s = 0; s < 6; s++) {
-                    gres[it][s] = (StageT)(g0 * (Z[s] + RW[s]));
-                    gres[it][6 + s] = (StageT)(g0 * 0.5 * RW[s]);
-                }
-                atomicAdd(&s_ev[vl[0]], -ddi);
-                atomicAdd(&s_ev[vl[1]], -ddi);
-                atomicAdd(&s_ev[vl[2]], -ddi);
-            }
-        }
-        dd_loc += ddi;
-    }
-
-    // ---- block reductions: chunk energy partial, occupied-energy gradient ----
-    for (int off = 16; off > 0; off >>= 1) {
-        e_loc += __shfl_down_sync(0xffffffffu, e_loc, off);
-        dd_loc += __shfl_down_sync(0xffffffffu, dd_loc, off);
-    }
-    if (lane == 0) {
-        s_red[0][warp] = e_loc;
-        s_red[1][warp] = dd_loc;
-    }
-    __syncthreads();   // all reads of the W tile are done: it becomes the item-result buffer
-    if (tid == 0) {
-        double es = 0.0, ds = 0.0;
-        for (int w = 0; w < NW; w++) {
-            es += s_red[0][w];
-            ds += s_red[1][w];
-        }
-        P.e_part[(long long)sub * P.n_ijk + rep] = es;
-        if (P.want_grad && ds != 0.0) {
-            atomicAdd(&P.mo_bar[ijk[0]], ds);
-            atomicAdd(&P.mo_bar[ijk[1]], ds);
-            atomicAdd(&P.mo_bar[ijk[2]], ds);
-        }
-    }
-    if (!P.want_grad) return;
-#pragma unroll
-    for (int it = 0; it < IPT; it++)
-        if (gvalid[it]) {
-            const int item = tid + it * NT;
-            // item (l0, l1, l2) at l0*SY + l1*SX + l2 in each of the 12 planes: the
-            // padded strides keep the write-back gathers within 2-way bank conflicts
-            const int gi = (item / (SB * SB)) * SY + ((item / SB) % SB) * SX + item % SB;
-#pragma unroll
-            for (int c = 0; c < 12; c++) sG[c * REG + gi] = gres[it][c];
-        }
-    __syncthreads();
-    for (int e = tid; e < NV; e += NT) {
-        const int sl = e / SB, l = e % SB;
-        if (l < R.len[sl] && s_ev[e] != 0.0) atomicAdd(&P.mo_bar[o + R.st[sl] + l], s_ev[e]);
-    }
-
-    // ---- write back Wbar; V-term gradients from the run's Vbar ----
-    // A group of GL lanes takes whole regions (RPL runs of z values per lane),
-    // so the columns (r, z) of the t1 / fvo sums are fixed per group and the
-    // column partials of all its runs are reduced once per region.
-    constexpr int RPR = SB * SB;                 // runs per region
-    constexpr int GL = RPR < 32 ? RPR : 32;      // lanes per region group
-    constexpr int RPL = RPR / GL;                // runs per lane
-    constexpr int NG = NT / GL;                  // groups per CTA
-    // every region holds one (pi, rho) pair and no ordering constraint applies
-    const bool simple = (n_ijk == 6) && distinct_rng;
-    const int grp = tid / GL, gl = tid % GL;
-    const int nround = (nreg + NG - 1) / NG;
-    for (int rr = 0; rr < nround; rr++) {
-        const int reg_ = grp + rr * NG;
-        const bool inrange = reg_ < nreg;
-        const int reg = inrange ? reg_ : 0;
-        const int *rd = s_rd[reg];
-        const int lx = rd[3], ly = rd[4], lz = rd[5];
-        int pp[3], pt[3];
-        perm_of(rd[0], pp);
-        perm_of(rd[1], pt);
-        auto cslot = [&](int j) { return j == 0 ? cs[0] : (j == 1 ? cs[1] : cs[2]); };
-        auto stride = [&](int j) { return j == 0 ? SY : (j == 1 ? SX : 1); };   // item-result layout
-        const int zl0 = cslot(pp[2]) * SB;
-        const int p = rd[6], q = rd[7], r = rd[8];
-        const int pair = pair_index(pt[0], pt[1]);
-        const StageT *a1 = tT1 + pt[2] * NV + zl0, *f1 = tFV + pt[2] * NV + zl0;
-        const PermBlock &pb = P.ch.pb[rd[2]];
-        // V-term partials in the staging precision (FP32 in the mixed modes: 8-term
-        // row sums and the warp's 64-run column sums), added to the FP64 gradients
-        StageT colv[2 * SB];
-#pragma unroll
-        for (int c = 0; c < 2 * SB; c++) colv[c] = 0;
-#pragma unroll
-        for (int u = 0; u < RPL; u++) {
-            const int run = gl + u * GL;
-            const int yy = run / SB, xx = run % SB;
-            if (!(inrange && xx < lx && yy < ly)) continue;
-            StageT wb[SB], vb[SB];
-            if (simple) {
-                const int s = pat.sof[rd[0] * 6 + rd[1]];
-                const int base = xx * stride(pp[0]) + yy * stride(pp[1]), st2 = stride(pp[2]);
-                const StageT *gw = sG + s * REG + base, *gv = sG + (6 + s) * REG + base;
-#pragma unroll
-                for (int zz = 0; zz < SB; zz++) {
-                    wb[zz] = (zz < lz) ? gw[zz * st2] : (StageT)0;
-                    vb[zz] = (zz < lz) ? gv[zz * st2] : (StageT)0;
-                }
-            } else {
-                double wd[SB], vd[SB];   // several (s, tau) per position: sum in FP64
-#pragma unroll
-                for (int zz = 0; zz < SB; zz++) wd[zz] = vd[zz] = 0.0;
-                const int nc = pat.ncombo[reg];
-                for (int c = 0; c < nc; c++) {
-                    const int pr = pat.combo[reg][c];
-                    const int s = pat.sof[pr];
-                    int q3[3];
-                    perm_of(pr / 6, q3);
-                    // item slot j takes the region coordinate whose ordering slot is j
-                    const int base = xx * stride(q3[0]) + yy * stride(q3[1]), st2 = stride(q3[2]);
-                    const StageT *gw = sG + s * REG, *gv = sG + (6 + s) * REG;
-#pragma unroll
-                    for (int zz = 0; zz < SB; zz++) {
-                        if (zz >= lz) continue;
-                        const int l0 = (q3[0] == 0) ? xx : ((q3[1] == 0) ? yy : zz);
-                        const int l1 = (q3[0] == 1) ? xx : ((q3[1] == 1) ? yy : zz);
-                        const int l2 = (q3[0] == 2) ? xx : ((q3[1] == 2) ? yy : zz);
-                        bool ok = true;
-                        if (cs[1] == 0 && l0 < l1) ok = false;
-                        if (cs[2] == cs[1] && l1 < l2) ok = false;
-                        if (ok) {
-                            const int item = base + zz * st2;
-                            wd[zz] += (double)gw[item];
-                            vd[zz] += (double)gv[item];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int zz = 0; zz < SB; zz++) {
-                    wb[zz] = (StageT)wd[zz];
-                    vb[zz] = (StageT)vd[zz];
-                }
-            }
-            // Wbar out
-            const long long wl = s_wb[reg] + (long long)yy * s_ws[reg][0] + (long long)xx * s_ws[reg][1];
-            RunBuf<StageT, SB> bw;
-#pragma unroll
-            for (int zz = 0; zz < SB; zz++) bw.e[zz] = wb[zz];
-            st_run(P.SW + pb.swoff + wl, bw, lz);
-            // V-term gradients: v = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r]
-            const int x = R.st[pp[0]] + xx, y = R.st[pp[1]] + yy;
-            const int te = (pair * NV + cslot(pp[0]) * SB + xx) * NVP + cslot(pp[1]) * SB + yy;
-            const StageT ovv = tOV[te], t2v = tT2[te];
-            StageT rs1 = 0, rs2 = 0;
-#pragma unroll
-            for (int zz = 0; zz < SB; zz++) {
-                rs1 += vb[zz] * a1[zz];
-                rs2 += vb[zz] * f1[zz];
-                colv[zz] += vb[zz] * ovv;
-                colv[SB + zz] += vb[zz] * t2v;
-            }
-            atomicAdd(&P.ovov_bar[(((long long)p * v + x) * o + q) * v + y], (double)rs1);
-            atomicAdd(&P.t2_bar[(((long long)q * o + p) * v + y) * v + x], (double)rs2);
-        }
-        // column sums over the region's runs: t1_bar[r, z], fvo_bar[z, r]
-        const double cv = (double)group_reduce_scatter<2 * SB, GL>(colv, lane);
-        const int cidx = lane % (2 * SB);
-        if (inrange && gl < 2 * SB && (cidx % SB) < lz && cv != 0.0) {
-            const int z = R.st[pp[2]] + cidx % SB;
-            if (cidx < SB) atomicAdd(&P.t1_bar[(long long)r * v + z], cv);
-            else atomicAdd(&P.fvo_bar[(long long)z * o + r], cv);
+        for (int pi = 0; pi < 6; pi++) {
+            const int s = f2m_sof(pi, rho);
+            int pp[3] = {0, 0, 0};
+            perm_of(pi, pp);
+            const StageT *base = S + R.pi[pi].s0 + idx * R.pi[pi].rs;
+            WW[0][s] += (double)__ldg(base + w0[pi]);
+            WW[1][s] += (double)__ldg(base + w1[pi]);
+            const double2 *tp = tab + (rho * 6 + pi) * 64;
+            // a + 4 in slot x or y of the table block
+            const double2 ot0 = tp[t0[pi]];
+            const double2 ot1 = pp[0] == 0 ? tp[t0[pi] ^ 4] : (pp[1] == 0 ? tp[t0[pi] ^ 32] : ot0);
+            const double2 z0 = tz[pp[2]], z1 = pp[2] == 0 ? tz4 : tz[pp[2]];
+            VV[0][s] += ot0.x * z0.x + ot0.y * z0.y;
+            VV[1][s] += ot1.x * z1.x + ot1.y * z1.y;
         }
     }
 }
 
-// Sum of the per-CTA energy partials of one epilogue launch, in a fixed order.
+// Orbital-energy gradient: dd = dE/dD of the thread's elements.  Per-warp sums
+// over two of the slots each, then dE/de of i, j, k (+ the total) and of the
+// virtuals (- the sums of their slot).
+__device__ __forceinline__ void f2_dd_partials(const double (&dd)[2], double (*s_part)[12]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double dc = dd[0] + dd[1], db = dc;
+    dc += __shfl_xor_sync(0xffffffffu, dc, 4);
+    dc += __shfl_xor_sync(0xffffffffu, dc, 8);
+    dc += __shfl_xor_sync(0xffffffffu, dc, 16);
+    db += __shfl_xor_sync(0xffffffffu, db, 1);
+    db += __shfl_xor_sync(0xffffffffu, db, 2);
+    db += __shfl_xor_sync(0xffffffffu, db, 16);
+    const bool up = lane & 1;
+    double da = (up ? dd[1] : dd[0]) + __shfl_xor_sync(0xffffffffu, up ? dd[0] : dd[1], 1);
+    da += __shfl_xor_sync(0xffffffffu, da, 2);
+    da += __shfl_xor_sync(0xffffffffu, da, 4);
+    da += __shfl_xor_sync(0xffffffffu, da, 8);
+    if (lane < 4) s_part[warp][lane] = dc;
+    if ((lane & 19) == 0) s_part[warp][4 + (lane >> 2)] = db;
+    if ((lane & 14) == 0) s_part[warp][8 + (lane >> 4) + 2 * (lane & 1)] = da;
+}
+
+__device__ __forceinline__ void f2_dd_add(double (*s_part)[12], const F2mSub &R, int o, int i0, int i1, int i2,
+                                          double *mo_bar) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x >= 24) return;
+    // warps with bit 0, 1, 2 = bit 2 of c, bit 2 of b, bit 1 of a (lanes: c, b, a)
+    double acc = 0.0;
+    const int l = lane & 7;
+    for (int u = 0; u < 4; u++)
+        acc += lane < 8 ? s_part[(l >> 2) + 2 * u][l & 3]
+               : lane < 16 ? s_part[2 * (l >> 2) + (u & 1) + 4 * (u >> 1)][4 + (l & 3)]
+                           : s_part[4 * ((l >> 1) & 1) + u][8 + (l & 1) + 2 * (l >> 2)];
+    double tot = acc;
+    tot += __shfl_xor_sync(0x00ffffffu, tot, 1);
+    tot += __shfl_xor_sync(0x00ffffffu, tot, 2);
+    tot += __shfl_xor_sync(0x00ffffffu, tot, 4);
+    const int slot = 2 - (lane >> 3);
+    if (l < sel3(R.len[0], R.len[1], R.len[2], slot))
+        atomicAdd(&mo_bar[o + sel3(R.st[0], R.st[1], R.st[2], slot) + l], -acc);
+    if (lane < 3) atomicAdd(&mo_bar[sel3(i0, i1, i2, lane)], tot);
+}
+
+// Write-back of the element results sW, sV (planes of 512 in f2m_res order): the
+// leading regions, one per warp at a time, runs (yy, xx) of lane and u.  Wbar
+// leaves as whole runs; V-term gradients v = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r]
+// as row sums per run and column sums over the region.  Results and tables are
+// zero beyond a short range.
+template <int SPLIT, typename ARGS>
+__device__ __forceinline__ void f2_writeback(const ARGS &A, const F2mSub &R, int i0, int i1, int i2, int opat, int vpat,
+                                             const double2 *tab, const double2 *tf, const int (*s_res)[8],
+                                             const typename F2Smem<SPLIT>::W *sW, const double *sV) {
+    const int o = A.o, v = A.v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int l0 = R.len[0], l1 = R.len[1], l2 = R.len[2];
+    const int nro = f2m_nlead(opat), ntask = f2m_nlead(vpat) * nro;
+    const int xx = lane & 7, y4 = lane >> 3;
+#pragma unroll 1
+    for (int task = 7 - warp; task < ntask; task += 8) {
+        const int pi = f2m_lead(vpat, task / nro), rho = f2m_lead(opat, task % nro);
+        int pp[3], pr[3];
+        perm_of(pi, pp);
+        perm_of(rho, pr);
+        const int p = sel3(i0, i1, i2, pr[0]), q = sel3(i0, i1, i2, pr[1]), r = sel3(i0, i1, i2, pr[2]);
+        const int lx = sel3(l0, l1, l2, pp[0]), ly = sel3(l0, l1, l2, pp[1]), lz = sel3(l0, l1, l2, pp[2]);
+        const int inv0 = pr[0] == 0 ? 0 : (pr[1] == 0 ? 1 : 2), inv1 = pr[0] == 1 ? 0 : (pr[1] == 1 ? 1 : 2);
+        const int s = perm_index(sel3(pp[0], pp[1], pp[2], inv0), sel3(pp[0], pp[1], pp[2], inv1));
+        const F2mPi &D = R.pi[pi];
+        const long long wl = D.w0 + (long long)p * D.wp + (long long)q * D.rzp + (long long)r * D.tz + (long long)xx * D.wx;
+        const double2 *trow = tf + (pr[2] * 3 + pp[2]) * 8;
+        const double2 *tp = tab + (rho * 6 + pi) * 64;
+        const int x = sel3(R.st[0], R.st[1], R.st[2], pp[0]) + xx;
+        const int y0 = sel3(R.st[0], R.st[1], R.st[2], pp[1]);
+        const int gx = s * 512, gxx = s_res[pp[0]][xx];
+        double col[16];
+#pragma unroll
+        for (int c = 0; c < 16; c++) col[c] = 0.0;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int yy = y4 + 4 * u;
+            const int g0 = gxx ^ s_res[pp[1]][yy];
+            const bool in = xx < lx && yy < ly;
+            int gz[8];
+#pragma unroll
+            for (int z = 0; z < 8; z++) gz[z] = gx + (g0 ^ s_res[pp[2]][z]);
+            if (in) {
+                if constexpr (SPLIT == 0) {
+                    double *dst = reinterpret_cast<double *>(A.SW) + wl + (long long)yy * D.wy;
+                    if (lz == 8) {
+#pragma unroll
+                        for (int z = 0; z < 8; z += 2)
+                            *reinterpret_cast<double2 *>(dst + z) = make_double2(sW[gz[z]], sW[gz[z + 1]]);
+                    } else {
+#pragma unroll
+                        for (int z = 0; z < 4; z++)
+                            if (z < lz) dst[z] = sW[gz[z]];
+                    }
+                } else {
+                    uint16_t *dst = reinterpret_cast<uint16_t *>(A.SW) + wl + (long long)yy * D.wy;
+                    uint32_t pk[8];
+#pragma unroll
+                    for (int z = 0; z < 8; z++) pk[z] = (uint32_t)sW[gz[z]];
+                    if (lz == 8) {
+                        uint4 hi, lo;
+                        hi.x = __byte_perm(pk[0], pk[1], 0x5410); lo.x = __byte_perm(pk[0], pk[1], 0x7632);
+                        hi.y = __byte_perm(pk[2], pk[3], 0x5410); lo.y = __byte_perm(pk[2], pk[3], 0x7632);
+                        hi.z = __byte_perm(pk[4], pk[5], 0x5410); lo.z = __byte_perm(pk[4], pk[5], 0x7632);
+                        hi.w = __byte_perm(pk[6], pk[7], 0x5410); lo.w = __byte_perm(pk[6], pk[7], 0x7632);
+                        *reinterpret_cast<uint4 *>(dst) = hi;
+                        *reinterpret_cast<uint4 *>(dst + D.half) = lo;
+                    } else {
+#pragma unroll
+                        for (int z = 0; z < 4; z++)
+                            if (z < lz) {
+                                dst[z] = (uint16_t)pk[z];
+                                dst[D.half + z] = (uint16_t)(pk[z] >> 16);
+                            }
+                    }
+                }
+            }
+            // v = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r] (results and tables are zero beyond a short range)
+            const double2 ot = tp[f2_tab(xx, yy)];
+            double r1 = 0.0, r2 = 0.0;
+#pragma unroll
+            for (int z = 0; z < 8; z++) {
+                const double vb = sV[gz[z]];
+                const double2 tr = trow[z];
+                r1 += vb * tr.x;
+                r2 += vb * tr.y;
+                col[z] += vb * ot.x;
+                col[8 + z] += vb * ot.y;
+            }
+            if (in) {
+                atomicAdd(&A.ovov_bar[(((long long)p * v + x) * o + q) * v + y0 + yy], r1);
+                atomicAdd(&A.t2_bar[(((long long)q * o + p) * v + y0 + yy) * v + x], r2);
+            }
+        }
+        // column sums t1_bar[r, z] (values 0-7), fvo_bar[z, r] (8-15) over the region's runs
+        const double cv = group_reduce_scatter<16, 32>(col, lane);
+        if (lane < 16 && (lane & 7) < lz) {
+            const int z = sel3(R.st[0], R.st[1], R.st[2], pp[2]) + (lane & 7);
+            if (lane < 8) atomicAdd(&A.t1_bar[(long long)r * v + z], cv);
+            else atomicAdd(&A.fvo_bar[(long long)z * o + r], cv);
+        }
+    }
+}
+
+// One CTA per item of the jobs (chunks) of a launch.
+template <typename JOBS>
+__global__ void __launch_bounds__(kF2Threads, 2) k_f2t(const __grid_constant__ JOBS J) {
+    extern __shared__ __align__(16) uint8_t f2_raw[];
+    double2 *tab = reinterpret_cast<double2 *>(f2_raw), *tf = tab + 36 * 64;
+    double *sV = reinterpret_cast<double *>(f2_raw + F2Smem<0>::TABLES), *sW = sV + 6 * 512;
+    __shared__ int s_res[3][8];
+    __shared__ double s_part[8][12], s_e[8];
+    JobCursor jcur;
+    int blk;
+    const int jb = jcur.at(J, (int)blockIdx.x, blk);
+    const F2P &A = J.job[JOBS::kOne ? 0 : jb];
+    const int o = A.o, tid = threadIdx.x;
+    // sub-range triple fastest: the CTAs of one representative run together
+    const int rep = blk / A.nsub, sub = blk - rep * A.nsub;
+    const F2mSub &R = A.sub[sub];
+    const int i0 = A.ijk[3 * rep], i1 = A.ijk[3 * rep + 1], i2 = A.ijk[3 * rep + 2];
+    const int opat = (i0 == i2) ? 3 : (i0 == i1 ? 1 : (i1 == i2 ? 2 : 0));
+    const int vpat = R.pat;
+    if (tid < 24) s_res[tid >> 3][tid & 7] = f2m_res(tid >> 3, tid & 7);
+    int ca, cb, cc;
+    f2_element(tid, ca, cb, cc);
+    const bool ok0 = ca < R.len[0] && cb < R.len[1] && cc < R.len[2];
+    const bool ok1 = ok0 && ca + 4 < R.len[0];
+    f2_load_tables(A, R, i0, i1, i2, tab, tf);
+    const double *ev = A.mo_e + o;
+    const double e_occ = A.mo_e[i0] + A.mo_e[i1] + A.mo_e[i2];
+    const double e_bc = ok0 ? ev[R.st[1] + cb] + ev[R.st[2] + cc] : 0.0;
+    double WW[2][6], VV[2][6];
+    f2_amplitudes(A.S, R, o, i0, i1, i2, ca, cb, cc, ok0, ok1, tab, tf, WW, VV);
+    // orbit weights: n_ijk n_abc / 18 for three distinct virtuals; the energy
+    // counts each orbit once per ordering of equal sub-ranges
+    const double cocc = opat == 0 ? 2.0 : (opat == 3 ? 6.0 / 18.0 : 1.0);
+    const double cen = vpat == 0 ? cocc : (vpat == 3 ? cocc / 6.0 : cocc * 0.5);
+    const int gidx = f2m_res(0, ca) ^ f2m_res(1, cb) ^ f2m_res(2, cc);
+    double e_loc = 0.0, dd[2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const bool ok = e == 0 ? ok0 : ok1;
+        double X[6], Z[6], RW[6];
+#pragma unroll
+        for (int s = 0; s < 6; s++) X[s] = WW[e][s] + 0.5 * VV[e][s];
+        f2_r3(X, Z);
+        f2_r3(WW[e], RW);
+        const double rD = ok ? 1.0 / (e_occ - ev[R.st[0] + ca + 4 * e] - e_bc) : 0.0;
+        double esum = 0.0;
+#pragma unroll
+        for (int s = 0; s < 6; s++) esum += WW[e][s] * Z[s];
+        e_loc += ok ? cen * esum * rD : 0.0;
+        dd[e] = ok ? -cen * A.ybar * esum * rD * rD : 0.0;
+        if (A.want_grad) {
+            const double g0 = cocc * A.ybar * rD;
+            double wb[6], vb[6];
+#pragma unroll
+            for (int s = 0; s < 6; s++) {
+                wb[s] = ok ? g0 * (Z[s] + RW[s]) : 0.0;
+                vb[s] = ok ? g0 * 0.5 * RW[s] : 0.0;
+            }
+            const int g = e == 0 ? gidx : gidx ^ 4;
+            // equal occupied indices: the orderings that name the same raw amplitudes add up
+            double w3 = 0.0, v3 = 0.0;
+            if (opat == 3) {
+#pragma unroll
+                for (int s = 0; s < 6; s++) {
+                    w3 += wb[s];
+                    v3 += vb[s];
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < 6; s++) {
+                const int s1 = perm_compose(s, 2), s2 = perm_compose(s, 1);
+                sW[s * 512 + g] = opat == 0 ? wb[s] : opat == 1 ? wb[s] + wb[s1] : opat == 2 ? wb[s] + wb[s2] : w3;
+                sV[s * 512 + g] = opat == 0 ? vb[s] : opat == 1 ? vb[s] + vb[s1] : opat == 2 ? vb[s] + vb[s2] : v3;
+            }
+        }
+    }
+    for (int off = 16; off > 0; off >>= 1) e_loc += __shfl_xor_sync(0xffffffffu, e_loc, off);
+    if ((tid & 31) == 0) s_e[tid >> 5] = e_loc;
+    f2_dd_partials(dd, s_part);
+    __syncthreads();
+    if (tid == 32) {
+        double es = 0.0;
+        for (int w = 0; w < kF2Threads / 32; w++) es += s_e[w];
+        A.e_part[(long long)sub * A.n_ijk + rep] = es;
+    }
+    if (!A.want_grad) return;
+    f2_dd_add(s_part, R, o, i0, i1, i2, A.mo_bar);
+    f2_writeback<0>(A, R, i0, i1, i2, opat, vpat, tab, tf, s_res, sW, sV);
+}
+
+// Sum of the energy partials of one epilogue launch, in a fixed order.
 __device__ __forceinline__ void energy_sum_body(const double *__restrict__ e_part, int n, double *e_acc) {
     __shared__ double s[256];
     double acc = 0.0;

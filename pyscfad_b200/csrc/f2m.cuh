@@ -57,7 +57,6 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
-#include "f2.cuh"
 #include "tc_f1.cuh"
 #include "tc_ptx.cuh"
 

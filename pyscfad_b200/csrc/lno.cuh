@@ -41,13 +41,14 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "f2.cuh"
 #include "f2m.cuh"
 #include "gemm_fp64.cuh"
 
 namespace tb {
 
 constexpr int kLnoMaxO = 64;    // largest nocc of the LNO path (projection tiles)
-constexpr int kLnoThreads = 256;
+constexpr int kLnoThreads = kF2Threads;
 
 struct LnoArgs {
     int o, v;
@@ -68,46 +69,8 @@ struct LnoArgs {
 };
 
 // ---------------------------------------------------------------------------
-// orbit kernels: two elements (a, b, c), (a + 4, b, c) per thread, as in f2m.cuh
+// orbit kernels: two elements (a, b, c), (a + 4, b, c) per thread, as in f2.cuh
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void lno_element(int t, int &a, int &b, int &c) {
-    a = ((t >> 4) & 1) | (((t >> 7) & 1) << 1);
-    b = ((t >> 2) & 3) | (((t >> 6) & 1) << 2);
-    c = (t & 3) | (((t >> 5) & 1) << 2);
-}
-
-// 64-entry table block of 16-byte entries: eight lanes of a gather hit eight banks
-__device__ __forceinline__ int lno_tab(int x, int y) { return y * 8 + (x ^ ((y & 1) << 2) ^ (y & 2)); }
-
-// FP64 V-term tables of an item: {ovov[p,x,q,y], t2[q,p,y,x]} per (rho, pi), {t1[r,z], fvo[z,r]}
-__device__ __forceinline__ void lno_load_tables(const LnoArgs &A, const F2mSub &R, int i0, int i1, int i2,
-                                                double2 *tab, double2 *tf) {
-    const int o = A.o, v = A.v;
-    double *ts = reinterpret_cast<double *>(tab);
-#pragma unroll 3
-    for (int e = threadIdx.x; e < 36 * 64; e += kLnoThreads) {
-        const int blk = e >> 6, hi = (e >> 3) & 7, lo = e & 7;
-        int pr[3], pp[3];
-        perm_of(blk / 6, pr);
-        perm_of(blk % 6, pp);
-        const int p = sel3(i0, i1, i2, pr[0]), q = sel3(i0, i1, i2, pr[1]);
-        const int lx = sel3(R.len[0], R.len[1], R.len[2], pp[0]), ly = sel3(R.len[0], R.len[1], R.len[2], pp[1]);
-        const int sx = sel3(R.st[0], R.st[1], R.st[2], pp[0]), sy = sel3(R.st[0], R.st[1], R.st[2], pp[1]);
-        // the fast index of each factor in turn runs over the lanes
-        ts[2 * (blk * 64 + lno_tab(hi, lo))] =
-            hi < lx && lo < ly ? __ldg(&A.ovov[(((long long)p * v + sx + hi) * o + q) * v + sy + lo]) : 0.0;
-        ts[2 * (blk * 64 + lno_tab(lo, hi)) + 1] =
-            lo < lx && hi < ly ? __ldg(&A.t2[(((long long)q * o + p) * v + sy + hi) * v + sx + lo]) : 0.0;
-    }
-    for (int e = threadIdx.x; e < 72; e += kLnoThreads) {
-        const int r = sel3(i0, i1, i2, e / 24), s = (e >> 3) % 3, zl = e & 7;
-        const int z = sel3(R.st[0], R.st[1], R.st[2], s) + zl;
-        const bool in = zl < sel3(R.len[0], R.len[1], R.len[2], s);
-        tf[e] = in ? make_double2(__ldg(&A.t1[(long long)r * v + z]), __ldg(&A.fvo[(long long)z * o + r]))
-                   : make_double2(0.0, 0.0);
-    }
-}
-
 // box index of ordering s at slot e: the occupied index paired with virtual slot c is ijk[t] with s[t] = c
 template <int S>
 __device__ __forceinline__ long long lno_box(int o, long long ne, int i0, int i1, int i2) {
@@ -130,15 +93,6 @@ __device__ __forceinline__ void lno_for_s(F &&f) {
     f(std::integral_constant<int, 5>{});
 }
 
-__device__ __forceinline__ void lno_r3(const double (&x)[6], double (&z)[6]) {
-#pragma unroll
-    for (int s = 0; s < 6; s++)
-        z[s] = 4.0 * x[s] + x[perm_compose(s, 4)] + x[perm_compose(s, 3)] -
-               2.0 * (x[perm_compose(s, 5)] + x[perm_compose(s, 1)] + x[perm_compose(s, 2)]);
-}
-
-inline size_t lno_fwd_smem() { return (36 * 64 + 72) * sizeof(double2); }
-
 template <typename StageT>
 __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_fwd(const __grid_constant__ LnoArgs A) {
     extern __shared__ __align__(16) uint8_t lno_raw[];
@@ -149,58 +103,12 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_fwd(const __grid_constan
     const F2mSub &R = A.sub[sub];
     const int i0 = A.ijk[3 * rep], i1 = A.ijk[3 * rep + 1], i2 = A.ijk[3 * rep + 2];
     int ca, cb, cc;
-    lno_element(threadIdx.x, ca, cb, cc);
+    f2_element(threadIdx.x, ca, cb, cc);
     const bool ok0 = ca < R.len[0] && cb < R.len[1] && cc < R.len[2];
     const bool ok1 = ok0 && ca + 4 < R.len[0];
-    lno_load_tables(A, R, i0, i1, i2, tab, tf);
-    const StageT *S = reinterpret_cast<const StageT *>(A.S);
-    const int loc[3] = {ca, cb, cc};
-    int w0[6], w1[6], t0[6];   // this thread's positions in the regions (elements a, a + 4) and tables
-#pragma unroll
-    for (int pi = 0; pi < 6; pi++) {
-        int pp[3] = {0, 0, 0};
-        perm_of(pi, pp);
-        const int x = loc[pp[0]], y = loc[pp[1]], z = loc[pp[2]];
-        const int ex = R.len[pp[0]], ez = R.len[pp[2]];
-        const bool swz = sizeof(StageT) == 4 && ex == 8 && ez == 8;
-        const int dx = pp[0] == 0 ? 4 : 0, dy = pp[1] == 0 ? 4 : 0, dz = pp[2] == 0 ? 4 : 0;
-        const int s0 = (x * ez + z) ^ (swz ? f2m_row_swizzle(y) : 0);
-        const int s1 = ((x + dx) * ez + z + dz) ^ (swz ? f2m_row_swizzle(y + dy) : 0);
-        w0[pi] = ok0 ? y * ex * ez + s0 : 0;
-        w1[pi] = ok1 ? (y + dy) * ex * ez + s1 : w0[pi];
-        t0[pi] = lno_tab(x, y);
-    }
+    f2_load_tables(A, R, i0, i1, i2, tab, tf);
     double WW[2][6], VV[2][6];
-#pragma unroll
-    for (int e = 0; e < 2; e++)
-#pragma unroll
-        for (int s = 0; s < 6; s++) WW[e][s] = VV[e][s] = 0.0;
-    __syncthreads();
-#pragma unroll
-    for (int rho = 0; rho < 6; rho++) {
-        int pr[3] = {0, 0, 0};
-        perm_of(rho, pr);
-        const int ids[3] = {i0, i1, i2};
-        const long long idx = ((long long)ids[pr[0]] * o + ids[pr[1]]) * o + ids[pr[2]];
-        const double2 *tr = tf + pr[2] * 24;
-        const double2 tz[3] = {tr[ca], tr[8 + cb], tr[16 + cc]}, tz4 = tr[(ca + 4) & 7];
-#pragma unroll
-        for (int pi = 0; pi < 6; pi++) {
-            const int s = f2m_sof(pi, rho);
-            int pp[3] = {0, 0, 0};
-            perm_of(pi, pp);
-            const StageT *base = S + R.pi[pi].s0 + idx * R.pi[pi].rs;
-            WW[0][s] += (double)__ldg(base + w0[pi]);
-            WW[1][s] += (double)__ldg(base + w1[pi]);
-            const double2 *tp = tab + (rho * 6 + pi) * 64;
-            // a + 4 in slot x or y of the table block
-            const double2 ot0 = tp[t0[pi]];
-            const double2 ot1 = pp[0] == 0 ? tp[t0[pi] ^ 4] : (pp[1] == 0 ? tp[t0[pi] ^ 32] : ot0);
-            const double2 z0 = tz[pp[2]], z1 = pp[2] == 0 ? tz4 : tz[pp[2]];
-            VV[0][s] += ot0.x * z0.x + ot0.y * z0.y;
-            VV[1][s] += ot1.x * z1.x + ot1.y * z1.y;
-        }
-    }
+    f2_amplitudes(reinterpret_cast<const StageT *>(A.S), R, o, i0, i1, i2, ca, cb, cc, ok0, ok1, tab, tf, WW, VV);
     const double *ev = A.mo_e + o;
     const double e_occ = A.mo_e[i0] + A.mo_e[i1] + A.mo_e[i2];
     const double e_bc = ok0 ? ev[R.st[1] + cb] + ev[R.st[2] + cc] : 0.0;
@@ -211,7 +119,7 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_fwd(const __grid_constan
         double X[6], Z[6];
 #pragma unroll
         for (int s = 0; s < 6; s++) X[s] = WW[e][s] + 0.5 * VV[e][s];
-        lno_r3(X, Z);
+        f2_r3(X, Z);
         const double rD = ok ? 1.0 / (e_occ - ev[R.st[0] + ca + 4 * e] - e_bc) : 0.0;
         const int slot = sub * 512 + e * 256 + threadIdx.x;
         lno_for_s([&](auto sc) {
@@ -298,7 +206,7 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
             const int oth = t / per, e = (t - oth * per) * COLS + threadIdx.x;
             const F2mSub &R = A.sub[e >> 9];
             int a, b2, c;
-            lno_element(e & 255, a, b2, c);
+            f2_element(e & 255, a, b2, c);
             a += 4 * ((e >> 8) & 1);
             double ec = -1.0;   // a slot beyond a short range: any non-zero value
             if (a < R.len[0] && b2 < R.len[1] && c < R.len[2]) {
@@ -409,32 +317,23 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
 // SPLIT 0: FP64 Wbar; 1: fp16 hi/lo of wbar * wscale (exact power of two); 2: bf16
 // hi/lo, unscaled -- the operand formats of the adjoint contractions.
 template <int SPLIT>
-struct LnoAdj {
-    using W = typename std::conditional<SPLIT == 0, double, uint32_t>::type;   // FP64, or hi and lo halves
-    static constexpr size_t TABLES = (36 * 64 + 72) * sizeof(double2);
-    static constexpr size_t SMEM = TABLES + 6 * 512 * (sizeof(double) + sizeof(W));
-};
-
-template <int SPLIT>
 __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_adj(const __grid_constant__ LnoArgs A) {
-    using WT = typename LnoAdj<SPLIT>::W;
+    using WT = typename F2Smem<SPLIT>::W;
     extern __shared__ __align__(16) uint8_t lno_raw[];
     double2 *tab = reinterpret_cast<double2 *>(lno_raw), *tf = tab + 36 * 64;
-    double *sV = reinterpret_cast<double *>(lno_raw + LnoAdj<SPLIT>::TABLES);
+    double *sV = reinterpret_cast<double *>(lno_raw + F2Smem<SPLIT>::TABLES);
     WT *sW = reinterpret_cast<WT *>(sV + 6 * 512);
     __shared__ int s_res[3][8];
     __shared__ double s_part[8][12];
-    const int o = A.o, v = A.v;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int o = A.o, tid = threadIdx.x;
     const int rep = blockIdx.x / A.nsub, sub = blockIdx.x - rep * A.nsub;
     const F2mSub &R = A.sub[sub];
     const int i0 = A.ijk[3 * rep], i1 = A.ijk[3 * rep + 1], i2 = A.ijk[3 * rep + 2];
     const int opat = (i0 == i2) ? 3 : (i0 == i1 ? 1 : (i1 == i2 ? 2 : 0));
     const int vpat = R.pat;
-    const int l0 = R.len[0], l1 = R.len[1], l2 = R.len[2];
     if (tid < 24) s_res[tid >> 3][tid & 7] = f2m_res(tid >> 3, tid & 7);
     int ca, cb, cc;
-    lno_element(tid, ca, cb, cc);
+    f2_element(tid, ca, cb, cc);
     const int gidx = f2m_res(0, ca) ^ f2m_res(1, cb) ^ f2m_res(2, cc);
     const long long ne = (long long)A.nsub * 512;
     const float wsc = SPLIT == 1 ? (float)*A.wscale : 1.0f;
@@ -454,7 +353,7 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_adj(const __grid_constan
             ds += Z[s] * __ldg(&A.Q[at]);
         });
         dd[e] = A.f != 0.0 ? dfac * ds : 0.0;
-        lno_r3(Z, X);
+        f2_r3(Z, X);
         const int g = e == 0 ? gidx : gidx ^ 4;
 #pragma unroll
         for (int s = 0; s < 6; s++) {
@@ -464,133 +363,11 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_adj(const __grid_constan
             else sW[s * 512 + g] = f2m_split<SPLIT>((float)wb, wsc);
         }
     }
-    lno_load_tables(A, R, i0, i1, i2, tab, tf);
-    {
-        // -dE/d e of the element's virtuals: per-warp sums over the other two slots
-        double dc = dd[0] + dd[1], db = dc;
-        dc += __shfl_xor_sync(0xffffffffu, dc, 4);
-        dc += __shfl_xor_sync(0xffffffffu, dc, 8);
-        dc += __shfl_xor_sync(0xffffffffu, dc, 16);
-        db += __shfl_xor_sync(0xffffffffu, db, 1);
-        db += __shfl_xor_sync(0xffffffffu, db, 2);
-        db += __shfl_xor_sync(0xffffffffu, db, 16);
-        const bool up = lane & 1;
-        double da = (up ? dd[1] : dd[0]) + __shfl_xor_sync(0xffffffffu, up ? dd[0] : dd[1], 1);
-        da += __shfl_xor_sync(0xffffffffu, da, 2);
-        da += __shfl_xor_sync(0xffffffffu, da, 4);
-        da += __shfl_xor_sync(0xffffffffu, da, 8);
-        if (lane < 4) s_part[warp][lane] = dc;
-        if ((lane & 19) == 0) s_part[warp][4 + (lane >> 2)] = db;
-        if ((lane & 14) == 0) s_part[warp][8 + (lane >> 4) + 2 * (lane & 1)] = da;
-    }
+    f2_load_tables(A, R, i0, i1, i2, tab, tf);
+    f2_dd_partials(dd, s_part);
     __syncthreads();
-    if (warp == 0 && lane < 24) {
-        // warps with bit 0, 1, 2 = bit 2 of c, bit 2 of b, bit 1 of a (lanes: c, b, a)
-        double acc = 0.0;
-        const int l = lane & 7;
-        for (int u = 0; u < 4; u++)
-            acc += lane < 8 ? s_part[(l >> 2) + 2 * u][l & 3]
-                   : lane < 16 ? s_part[2 * (l >> 2) + (u & 1) + 4 * (u >> 1)][4 + (l & 3)]
-                               : s_part[4 * ((l >> 1) & 1) + u][8 + (l & 1) + 2 * (l >> 2)];
-        double tot = acc;
-        tot += __shfl_xor_sync(0x00ffffffu, tot, 1);
-        tot += __shfl_xor_sync(0x00ffffffu, tot, 2);
-        tot += __shfl_xor_sync(0x00ffffffu, tot, 4);
-        const int slot = 2 - (lane >> 3);
-        if (l < sel3(l0, l1, l2, slot)) atomicAdd(&A.mo_bar[o + sel3(R.st[0], R.st[1], R.st[2], slot) + l], -acc);
-        if (lane < 3) atomicAdd(&A.mo_bar[sel3(i0, i1, i2, lane)], tot);
-    }
-    // ---- write-back: a region per warp, runs (yy, xx) of lane and u ----
-    const int nro = f2m_nlead(opat), ntask = f2m_nlead(vpat) * nro;
-    const int xx = lane & 7, y4 = lane >> 3;
-#pragma unroll 1
-    for (int task = 7 - warp; task < ntask; task += 8) {
-        const int pi = f2m_lead(vpat, task / nro), rho = f2m_lead(opat, task % nro);
-        int pp[3], pr[3];
-        perm_of(pi, pp);
-        perm_of(rho, pr);
-        const int p = sel3(i0, i1, i2, pr[0]), q = sel3(i0, i1, i2, pr[1]), r = sel3(i0, i1, i2, pr[2]);
-        const int lx = sel3(l0, l1, l2, pp[0]), ly = sel3(l0, l1, l2, pp[1]), lz = sel3(l0, l1, l2, pp[2]);
-        const int inv0 = pr[0] == 0 ? 0 : (pr[1] == 0 ? 1 : 2), inv1 = pr[0] == 1 ? 0 : (pr[1] == 1 ? 1 : 2);
-        const int s = perm_index(sel3(pp[0], pp[1], pp[2], inv0), sel3(pp[0], pp[1], pp[2], inv1));
-        const F2mPi &D = R.pi[pi];
-        const long long wl = D.w0 + (long long)p * D.wp + (long long)q * D.rzp + (long long)r * D.tz + (long long)xx * D.wx;
-        const double2 *trow = tf + (pr[2] * 3 + pp[2]) * 8;
-        const double2 *tp = tab + (rho * 6 + pi) * 64;
-        const int x = sel3(R.st[0], R.st[1], R.st[2], pp[0]) + xx;
-        const int y0 = sel3(R.st[0], R.st[1], R.st[2], pp[1]);
-        const int gx = s * 512, gxx = s_res[pp[0]][xx];
-        double col[16];
-#pragma unroll
-        for (int c = 0; c < 16; c++) col[c] = 0.0;
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int yy = y4 + 4 * u;
-            const int g0 = gxx ^ s_res[pp[1]][yy];
-            const bool in = xx < lx && yy < ly;
-            int gz[8];
-#pragma unroll
-            for (int z = 0; z < 8; z++) gz[z] = gx + (g0 ^ s_res[pp[2]][z]);
-            if (in) {
-                if constexpr (SPLIT == 0) {
-                    double *dst = reinterpret_cast<double *>(A.SW) + wl + (long long)yy * D.wy;
-                    if (lz == 8) {
-#pragma unroll
-                        for (int z = 0; z < 8; z += 2)
-                            *reinterpret_cast<double2 *>(dst + z) = make_double2(sW[gz[z]], sW[gz[z + 1]]);
-                    } else {
-#pragma unroll
-                        for (int z = 0; z < 4; z++)
-                            if (z < lz) dst[z] = sW[gz[z]];
-                    }
-                } else {
-                    uint16_t *dst = reinterpret_cast<uint16_t *>(A.SW) + wl + (long long)yy * D.wy;
-                    uint32_t pk[8];
-#pragma unroll
-                    for (int z = 0; z < 8; z++) pk[z] = (uint32_t)sW[gz[z]];
-                    if (lz == 8) {
-                        uint4 hi, lo;
-                        hi.x = __byte_perm(pk[0], pk[1], 0x5410); lo.x = __byte_perm(pk[0], pk[1], 0x7632);
-                        hi.y = __byte_perm(pk[2], pk[3], 0x5410); lo.y = __byte_perm(pk[2], pk[3], 0x7632);
-                        hi.z = __byte_perm(pk[4], pk[5], 0x5410); lo.z = __byte_perm(pk[4], pk[5], 0x7632);
-                        hi.w = __byte_perm(pk[6], pk[7], 0x5410); lo.w = __byte_perm(pk[6], pk[7], 0x7632);
-                        *reinterpret_cast<uint4 *>(dst) = hi;
-                        *reinterpret_cast<uint4 *>(dst + D.half) = lo;
-                    } else {
-#pragma unroll
-                        for (int z = 0; z < 4; z++)
-                            if (z < lz) {
-                                dst[z] = (uint16_t)pk[z];
-                                dst[D.half + z] = (uint16_t)(pk[z] >> 16);
-                            }
-                    }
-                }
-            }
-            // v = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r] (results and tables are zero beyond a short range)
-            const double2 ot = tp[lno_tab(xx, yy)];
-            double r1 = 0.0, r2 = 0.0;
-#pragma unroll
-            for (int z = 0; z < 8; z++) {
-                const double vb = sV[gz[z]];
-                const double2 tr = trow[z];
-                r1 += vb * tr.x;
-                r2 += vb * tr.y;
-                col[z] += vb * ot.x;
-                col[8 + z] += vb * ot.y;
-            }
-            if (in) {
-                atomicAdd(&A.ovov_bar[(((long long)p * v + x) * o + q) * v + y0 + yy], r1);
-                atomicAdd(&A.t2_bar[(((long long)q * o + p) * v + y0 + yy) * v + x], r2);
-            }
-        }
-        // column sums t1_bar[r, z] (values 0-7), fvo_bar[z, r] (8-15) over the region's runs
-        const double cv = group_reduce_scatter<16, 32>(col, lane);
-        if (lane < 16 && (lane & 7) < lz) {
-            const int z = sel3(R.st[0], R.st[1], R.st[2], pp[2]) + (lane & 7);
-            if (lane < 8) atomicAdd(&A.t1_bar[(long long)r * v + z], cv);
-            else atomicAdd(&A.fvo_bar[(long long)z * o + r], cv);
-        }
-    }
+    f2_dd_add(s_part, R, o, i0, i1, i2, A.mo_bar);
+    f2_writeback<SPLIT>(A, R, i0, i1, i2, opat, vpat, tab, tf, s_res, sW, sV);
 }
 
 // ---------------------------------------------------------------------------

@@ -19,8 +19,8 @@
 
 #include "gemm_fp64.cuh"
 #include "tc_f1.cuh"
-#include "f2.cuh"
 #include "f2m.cuh"
+#include "f2.cuh"
 #include "tc_b1.cuh"
 #include "lno.cuh"
 #include "pyscfad_b200.h"
@@ -661,7 +661,6 @@ struct GemmLaunch {
     int zstart[kMaxGroup + 1];   // GEMM problems (blockIdx.z) chunk after chunk,
     int cum[kMaxGroup][7];       // and within a chunk ordering after ordering
     int nmt, nslice;             // M tiles and K slices of blockIdx.x
-    int blocked;                 // staging in 8 x 8 x 8 blocks (StageRow, no exchange): the LNO kernels
     const double *A1, *B1, *A2, *B2;
     double *G;                   // gradient target
 };
@@ -710,16 +709,12 @@ __global__ void __launch_bounds__(kGThreads) k_chunk_fp64(const __grid_constant_
         g.B = GOp{L.B1 + q * ovK + (long long)pb.Z0 * Kp, map2(pb.Tz, Kp, vK), map1(1)};
         g.A2 = GOp{L.A2 + q * ovo + (long long)pb.X0 * o, map2(pb.Tx, o, vo), map1(1)};
         g.B2 = GOp{L.B2 + yg * ovo + (long long)pb.Z0 * o, map2(pb.Tz, o, vo), map1(1)};
-        if (L.blocked) {
-            const int ex = min(8, pb.Tx), ey = min(8, pb.Ty), ez = min(8, pb.Tz), nx = pb.Tx / ex, nz = pb.Tz / ez;
-            const long long es = ex * ey * ez, rs = (long long)pb.Tx * pb.Ty * pb.Tz;
-            g.C = L.S[c] + pb.soff + (long long)q * o * rs + (y / ey) * nx * nz * es + (y % ey) * (ex * ez);
-            g.cm = map3(ex, nx, ez, nz * es, (long long)o * o * rs);
-            g.cn = map3(ez, nz, 1, es, rs);
-        } else {
-            g.C = L.S[c] + pb.soff + ((long long)q * pb.Ty + y) * pb.Tx * oTz;
-            g.cm = map2(pb.Tx, oTz, (long long)o * pb.Ty * pb.Tx * oTz);
-        }
+        // staging in 8 x 8 x 8 blocks (StageRow, rows not exchanged)
+        const int ex = min(8, pb.Tx), ey = min(8, pb.Ty), ez = min(8, pb.Tz), nx = pb.Tx / ex, nz = pb.Tz / ez;
+        const long long es = ex * ey * ez, rs = (long long)pb.Tx * pb.Ty * pb.Tz;
+        g.C = L.S[c] + pb.soff + (long long)q * o * rs + (y / ey) * nx * nz * es + (y % ey) * (ex * ez);
+        g.cm = map3(ex, nx, ez, nz * es, (long long)o * o * rs);
+        g.cn = map3(ez, nz, 1, es, rs);
         g.alpha2 = -1.0;
         g.atomic = 0;
     } else if (KIND == GK_B1A) {
@@ -1112,12 +1107,9 @@ static int setup_epilogue(bool mixed) {
             });
             return rc;
         }
-        for (const void *k : {(const void *)k_f2t<Group<F2P, 1>>, (const void *)k_f2t<Group<F2P, kMaxGroup>>})
-            TB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f2_smem_bytes()));
-        F2Pattern pats[kF2Patterns];
-        f2_build_patterns(pats);
-        TB_CUDA(cudaMemcpyToSymbol(c_f2pat, pats, sizeof(pats)));
-        return TRIPLES_OK;
+        int rc = smem_optin(k_f2t<Group<F2P, 1>>, F2Smem<0>::BYTES);
+        if (rc == TRIPLES_OK) rc = smem_optin(k_f2t<Group<F2P, kMaxGroup>>, F2Smem<0>::BYTES);
+        return rc;
     });
 }
 
@@ -1216,9 +1208,10 @@ static int f1_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, TcF
     return TRIPLES_OK;
 }
 
-// Sub-range triples of a chunk (edge sb), one per orbit of orderings: f(start, length).
+// Triples of 8-wide sub-ranges of a chunk, one per orbit of orderings: f(start, length).
 template <typename F>
-static void for_sub_ranges(const ChunkDesc &ch, int sb, F &&f) {
+static void for_sub_ranges(const ChunkDesc &ch, F &&f) {
+    constexpr int sb = 8;
     int n[3];
     for (int t = 0; t < 3; t++) n[t] = (ch.nabc[t] + sb - 1) / sb;
     for (int ia = 0; ia < n[0]; ia++)
@@ -1235,30 +1228,6 @@ static void for_sub_ranges(const ChunkDesc &ch, int sb, F &&f) {
                 f(st, len);
             }
         }
-}
-
-// FP64 epilogue parameters of one chunk.
-static void f2_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, const TriplesIO &io, F2P &F) {
-    F.d = P.d;
-    F.ch = ch;
-    F.nsub = 0;
-    for_sub_ranges(ch, kF2SB, [&](const int *st, const int *len) {
-        F2Sub &u = F.sub[F.nsub++];
-        for (int t = 0; t < 3; t++) {
-            u.st[t] = st[t];
-            u.len[t] = len[t];
-        }
-    });
-    F.ijk = (int *)(ws + P.off_ijk);
-    F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
-    F.S = (const double *)(ws + P.off_S) + (size_t)slot * P.stage_slot;
-    F.SW = P.want_grad ? (double *)(ws + P.off_SW) + (size_t)slot * P.wbar_slot : nullptr;
-    F.ybar = io.ybar;
-    F.want_grad = P.want_grad;
-    F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
-    F.n_ijk = P.n_ijk;
-    F.mo_bar = io.mo_energy_bar;
-    F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
 }
 
 // Where the regions of a sub-range triple lie in the (blocked) staging and in
@@ -1298,6 +1267,28 @@ static void sub_regions(const ChunkDesc &ch, int o, const int *st, const int *le
     }
 }
 
+// FP64 epilogue parameters of one chunk.
+static void f2_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, const TriplesIO &io, F2P &F) {
+    F.o = P.d.o;
+    F.v = P.d.v;
+    F.nsub = 0;
+    for_sub_ranges(ch, [&](const int *st, const int *len) {
+        F2mSub &u = F.sub[F.nsub++];
+        sub_regions(ch, F.o, st, len, 1, 8, u);
+        u.pat = st[0] == st[2] ? 3 : (st[0] == st[1] ? 1 : (st[1] == st[2] ? 2 : 0));
+    });
+    F.n_ijk = P.n_ijk;
+    F.ijk = (int *)(ws + P.off_ijk);
+    F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
+    F.S = (const double *)(ws + P.off_S) + (size_t)slot * P.stage_slot;
+    F.SW = P.want_grad ? (double *)(ws + P.off_SW) + (size_t)slot * P.wbar_slot : nullptr;
+    F.ybar = io.ybar;
+    F.want_grad = P.want_grad;
+    F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
+    F.mo_bar = io.mo_energy_bar;
+    F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
+}
+
 // Mixed-precision epilogue parameters of one chunk.
 static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, const TriplesIO &io, bool whole, F2M &F) {
     Ctrl *ctrl = (Ctrl *)(ws + P.off_ctrl);
@@ -1308,7 +1299,7 @@ static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, c
     F.nsub = 0;
     F.n_ijk = P.n_ijk;
     F.whole = whole ? 1 : 0;
-    for_sub_ranges(ch, 8, [&](const int *st, const int *len) {
+    for_sub_ranges(ch, [&](const int *st, const int *len) {
         F2mSub &u = F.sub[F.nsub++];
         sub_regions(ch, o, st, len, 2, 4, u);
         u.pat = st[0] == st[2] ? 3 : (st[0] == st[1] ? 1 : (st[1] == st[2] ? 2 : 0));
@@ -1349,11 +1340,11 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     const bool mixed = sizeof(StageT) == 4, bf16 = P.prec == TRIPLES_PRECISION_MIXED_BF16;
     {
         const int rc = once_per_device(mixed ? INIT_LNO : INIT_LNO64, [&]() -> int {
-            int rc = smem_optin(k_lno_fwd<StageT>, lno_fwd_smem());
+            int rc = smem_optin(k_lno_fwd<StageT>, F2Smem<0>::TABLES);
             if (rc != TRIPLES_OK) return rc;
-            if (!mixed) return smem_optin(k_lno_adj<0>, LnoAdj<0>::SMEM);
-            if ((rc = smem_optin(k_lno_adj<1>, LnoAdj<1>::SMEM)) != TRIPLES_OK) return rc;
-            return smem_optin(k_lno_adj<2>, LnoAdj<2>::SMEM);
+            if (!mixed) return smem_optin(k_lno_adj<0>, F2Smem<0>::BYTES);
+            if ((rc = smem_optin(k_lno_adj<1>, F2Smem<1>::BYTES)) != TRIPLES_OK) return rc;
+            return smem_optin(k_lno_adj<2>, F2Smem<2>::BYTES);
         });
         if (rc != TRIPLES_OK) return rc;
     }
@@ -1394,7 +1385,7 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     A.want_grad = P.want_grad;
     A.part = (double *)(ws + P.off_lpart);
     const unsigned items = (unsigned)(P.n_ijk * A.nsub);
-    TB_KLAUNCH(P_LNO, (k_lno_fwd<StageT><<<items, kLnoThreads, lno_fwd_smem(), st>>>(A)));
+    TB_KLAUNCH(P_LNO, (k_lno_fwd<StageT><<<items, kLnoThreads, F2Smem<0>::TABLES, st>>>(A)));
     // columns per tile: 128 while two buffers of all rows leave room for two CTAs per SM
     unsigned parts = 0;
     const int prc = o <= 16   ? lno_projections<128>(A, st, parts)
@@ -1408,13 +1399,13 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     TB_KLAUNCH(P_PREP, (k_energy_sum<<<1, 256, 0, st>>>(G, 1)));
     if (!P.want_grad) return TRIPLES_OK;
     if (!mixed) {
-        TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<0><<<items, kLnoThreads, LnoAdj<0>::SMEM, st>>>(A)));
+        TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<0><<<items, kLnoThreads, F2Smem<0>::BYTES, st>>>(A)));
         return TRIPLES_OK;
     }
     // fp16: power-of-two scale of the split Wbar; bf16: scale 1 (both read by the contractions)
     TB_KLAUNCH(P_PREP, (k_chunk_scale<<<1, 32, 0, st>>>(G)));
-    if (bf16) TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<2><<<items, kLnoThreads, LnoAdj<2>::SMEM, st>>>(A)));
-    else TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<1><<<items, kLnoThreads, LnoAdj<1>::SMEM, st>>>(A)));
+    if (bf16) TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<2><<<items, kLnoThreads, F2Smem<2>::BYTES, st>>>(A)));
+    else TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<1><<<items, kLnoThreads, F2Smem<1>::BYTES, st>>>(A)));
     return TRIPLES_OK;
 }
 
@@ -1687,7 +1678,6 @@ static int fp64_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t s
     GemmLaunch L;
     L.d = P.d;
     L.n = n;
-    L.blocked = P.lno;
     L.A1 = (const double *)(ws + P.off_A1);
     L.B1 = (const double *)(ws + P.off_B1);
     L.A2 = (const double *)(ws + P.off_A2);
@@ -1712,7 +1702,7 @@ static int fp64_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t s
         }
         X.n = n;
         const int items = group_starts(G, n, [&](const F2P &j) { return P.n_ijk * j.nsub; });
-        TB_KLAUNCH(P_F2, (k_f2t<<<(unsigned)items, kF2Threads, f2_smem_bytes(), st>>>(G)));
+        TB_KLAUNCH(P_F2, (k_f2t<<<(unsigned)items, kF2Threads, F2Smem<0>::BYTES, st>>>(G)));
         TB_KLAUNCH(P_F2, (k_energy_sum<<<1, 256, 0, st>>>(X, n)));
     }
     if (!P.want_grad) return TRIPLES_OK;

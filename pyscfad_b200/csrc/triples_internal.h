@@ -3,12 +3,12 @@
 #include <cstddef>
 
 #include "common.cuh"
-#include "f2.cuh"
 #include "pyscfad_b200.h"
 
 namespace tb {
 
 constexpr int kMaxTv = 16;        // largest virtual block
+constexpr int kMaxSub = 64;       // energy partials per occupied representative
 constexpr int kMaxCols = 1024;    // largest nocc * Tv (one staged (r, z) row)
 constexpr int kCtrlBytes = 256;   // control block at workspace offset 0
 // Chunk slots of a call: most bytes of staging and Wbar.  A chunk of nocc 5 has
