@@ -65,6 +65,14 @@ struct PermBlock {
     long long swoff;       // offset of Wbar_tau (values) in the Wbar buffer
 };
 
+// 16-bit Wbar_tau: blocks of at least 8 x values are stored as 8 x 8 tiles
+// [h][y][q][p][x / 8][rz / 8][x % 8][rz % 8] (rz = r Tz + z), smaller ones as rows
+// [h][y][p][x][q][rz].  A tile is one 128-byte line, the 8 z runs of eight x that
+// one epilogue region holds for a y: as rows they were 16-byte halves of 32-byte
+// sectors whose other half came from another work item.  It is also a core
+// matrix of the adjoint contractions' first operand, K- or MN-major.
+__host__ __device__ inline bool wbar_tiled(const PermBlock &pb) { return pb.Tx >= 8; }
+
 struct ChunkDesc {
     int nperm;
     int blk[3];            // A >= B >= C block indices

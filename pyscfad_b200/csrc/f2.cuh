@@ -231,7 +231,7 @@ __device__ __forceinline__ void f2_writeback(const ARGS &A, const F2mSub &R, int
         const int inv0 = pr[0] == 0 ? 0 : (pr[1] == 0 ? 1 : 2), inv1 = pr[0] == 1 ? 0 : (pr[1] == 1 ? 1 : 2);
         const int s = perm_index(sel3(pp[0], pp[1], pp[2], inv0), sel3(pp[0], pp[1], pp[2], inv1));
         const F2mPi &D = R.pi[pi];
-        const long long wl = D.w0 + (long long)p * D.wp + (long long)q * D.rzp + (long long)r * D.tz + (long long)xx * D.wx;
+        const long long wl = f2m_wbar(D, p, q, r) + (long long)xx * D.wx;
         const double2 *trow = tf + (pr[2] * 3 + pp[2]) * 8;
         const double2 *tp = tab + (rho * 6 + pi) * 64;
         const int x = sel3(R.st[0], R.st[1], R.st[2], pp[0]) + xx;

@@ -25,10 +25,9 @@
 //   regions are written back.
 //
 // Persistent, two CTAs of 8 warps per SM.  Items are handed out in order by a
-// counter: the two 16-byte halves of a Wbar sector (the two 8-wide halves of a
-// z block) come from neighbouring items, and only while these run at the same
-// time do the halves meet in L2.  With a fixed stride the CTAs drift apart and
-// the half sectors reach DRAM one by one.  Bulk copies stream the items in:
+// counter, so that neighbouring items run at the same time: they read the same
+// tables, and where Wbar is stored in rows (x blocks below 8) the two 16-byte
+// halves of a sector come from two of them and meet in L2.  Bulk copies stream the items in:
 // the regions of one rho at a time (6 x 2 KB, a ring of four that runs ahead
 // into the next item; the last warp to read a stage refills it), and the
 // V-term tables of the next item (FP32 pairs
@@ -42,12 +41,14 @@
 // run) and column sums (over the region's runs) added to the FP64 gradients.
 //
 // What bounds it: instruction issue and shared-memory latency at 16 warps per
-// SM, then the half-sector Wbar stores; HBM is at a quarter of its rate.
+// SM; HBM is at a quarter of its rate.
 // Measured against the kernels it replaced (a one-CTA persistent kernel for
 // the all-distinct items and a CTA per item for the rest): nocc 40 nvir 360,
 // virtual block 6: 343 to 266 ms; nocc 40 nvir 72: 285 to 199 ms; nocc 20 nvir
-// 180: 493 to 397 ms; with items in fixed strides instead of by the counter the
-// first took 454 ms.
+// 180: 493 to 397 ms.  Wbar in 8 x 8 tiles, whole 128-byte lines per warp, in
+// place of rows whose half sectors two items wrote: the three to 213, 165 and
+// 325 ms (with rows, items in fixed strides instead of by the counter took 454
+// ms in the first, the halves reaching DRAM one by one).
 //
 // The FP32 sums keep a fixed order: rows run over z; columns over
 // half regions of 32 runs where nothing coincides and every sub-range is
@@ -72,10 +73,17 @@ struct F2mPi {
     long long w0;         // Wbar (hi plane): first position of that region
     long long half;       // lo plane - hi plane
     int rs;               // staging stride of r (q: o rs, p: o o rs)
-    int wx, wy, wp;       // Wbar strides of x, y, p
-    int rzp, tz;          // Wbar strides of q, r
+    int wx, wy, wp, wq;   // Wbar strides of x, y, p, q
+    int tz, zs;           // rz = r tz + zs + z
+    int tiled;            // rz strides by 64 per 8 values (8 x 8 tiles), else by 1
     int bytes;            // of a region
 };
+
+// Wbar offset of (p, q, r), first x, y and z of a region
+__device__ __forceinline__ long long f2m_wbar(const F2mPi &D, int p, int q, int r) {
+    const int rz = r * D.tz + D.zs;
+    return D.w0 + (long long)p * D.wp + (long long)q * D.wq + (D.tiled ? (rz >> 3) * 64 + (rz & 7) : rz);
+}
 
 struct F2mSub {
     int st[3], len[3];
@@ -605,8 +613,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
                 const int4 zb = *reinterpret_cast<const int4 *>(&s_res[pp[2]][4]);
                 const int zo[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
                 const F2mPi &D = R.pi[pi];
-                const long long wl = D.w0 + (long long)p * D.wp + (long long)q * D.rzp + (long long)r * D.tz +
-                                     (long long)xx * D.wx;
+                const long long wl = f2m_wbar(D, p, q, r) + (long long)xx * D.wx;
                 const float2 *trow = tf + (pr[2] * 3 + pp[2]) * 8;
                 float2 trz[8];
                 if (R.full) {

@@ -60,7 +60,7 @@ struct LnoArgs {
     double *WW, *Q, *PW, *PQ;   // box arrays; PW becomes Zbar
     const double *mat, *mo_e, *t1, *t2, *ovov, *fvo;
     void *SW;                   // Wbar staging per ordering: FP64 [y][p][x][q][rzp], or
-                                // 16-bit hi/lo planes [h][y][p][x][q][rzp] at 2 swoff
+                                // 16-bit hi/lo planes (rows or 8 x 8 tiles, wbar_tiled) at 2 swoff
     const double *wscale;       // power-of-two scale of the fp16 split
     double *mat_bar, *mo_bar, *t1_bar, *t2_bar, *ovov_bar, *fvo_bar;
     double ybar, f, g;

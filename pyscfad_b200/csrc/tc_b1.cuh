@@ -1,7 +1,11 @@
 // Tensor-core (tcgen05) form of the adjoint contractions, one launch per
 // ordering tau of a chunk.  Wbar_tau is staged by the epilogue as fp16/bf16
-// hi/lo splits in the layout [h][y][p][x][q][r][z] (scaled by a per-chunk
-// power of two), which serves all four products through 5-D TMA boxes:
+// hi/lo splits (scaled by a per-chunk power of two), as rows
+// [h][y][p][x][q][r][z] or, for x blocks of 8 and 16, as 8 x 8 tiles of (x, rz)
+// (wbar_tiled); either serves all four products through TMA boxes, 128B-swizzled
+// rows or unswizzled core matrices.  The MMA thread forms a step's descriptors
+// by one addition each: field by field, it held up the MN-major kinds (8 % at
+// nocc 40 nvir 72).
 //
 //   kind 0  ovvv:  G_A1[y][p][x][f] += sum_{q,rz} Wbar[y][p][x][q][rz] B1[q][rz][f]
 //                  rows (p,x) K-major, batch y, K = (q, rz)
@@ -62,7 +66,13 @@ struct TcB1Cfg {
     static constexpr int B_BYTES = BN * kTcBK * 2;
     static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
     static constexpr int STAGES = (200 * 1024) / STAGE_BYTES;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 256 + 1024;
+    // A 128 x 8 block of zeros: second K half of an 8-wide x block.
+    static constexpr int ZERO_BYTES = A_MN ? 2048 : 0;
+    // Barriers in the first 1024 bytes.  With the 1 KB that a block has reserved this stays within a
+    // shared memory of 196 KB: a few hundred bytes more take the next size, 228 KB, and leave
+    // 28 KB of L1 instead of 60 (the adjoint contractions of batched jobs then ran 1.25x as long).
+    static constexpr int SMEM = 1024 + STAGES * STAGE_BYTES + ZERO_BYTES;
+    static_assert(SMEM + 1024 <= 196 * 1024, "one shared memory size up");
     static constexpr int NACC = 4;   // TMEM accumulators: the epilogue sums them in pairs
     static constexpr int TMEM_COLS = NACC * BN < 32 ? 32 : NACC * BN;
     static_assert(NACC * BN <= 512, "TMEM holds 512 columns");
@@ -75,15 +85,20 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
     constexpr bool ONE = JOBS::kOne;
     JobCursor jcur;
     const TcB1Params &Pfirst = J.job[0];
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t *full = (uint64_t *)(smem + C::STAGES * C::STAGE_BYTES);
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    if ((smem_u32(smem_raw) & 1023u) != 0) {   // the swizzle's pattern counts from 1024 B boundaries
+        if (threadIdx.x == 0) atomicOr(Pfirst.err, 64);
+        return;
+    }
+    uint8_t *smem = smem_raw + 1024;
+    uint8_t *zero = smem + C::STAGES * C::STAGE_BYTES;
+    uint64_t *full = (uint64_t *)smem_raw;
     uint64_t *empty = full + C::STAGES;
     uint64_t *tfull = empty + C::STAGES;
     uint64_t *tempty = tfull + C::NACC;
     uint64_t *drain = tempty + C::NACC;
     uint32_t *tmem_slot = (uint32_t *)(drain + 1);
-    __shared__ int s_abort;
+    int &s_abort = *(int *)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -108,6 +123,10 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
     if (warp == 1) {
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
+    }
+    if (A_MN) {
+        for (int e = threadIdx.x; e < C::ZERO_BYTES / 4; e += kB1Threads) reinterpret_cast<uint32_t *>(zero)[e] = 0u;
+        fence_proxy_async_smem();
     }
     tc_fence_before();
     __syncthreads();
@@ -151,7 +170,12 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
             const int nk_inner = P.nk_inner[tau], nk = P.nk_outer[tau] * nk_inner;
             const CUtensorMap *tmA = &P.tmA[tau], *tmB = &P.tmB[tau];
             const int nbox = (width(P, nt) + 63) / 64, n0 = nt * P.nw;
-            const uint32_t bytes = (uint32_t)(2 * C::A_BYTES + 2 * nbox * 8192);
+            // A_MN K blocks hold 4 p: half the rows where an x block is one tile wide
+            const bool tiled = wbar_tiled(pb);
+            const int nxb = pb.Tx >> 3, o = P.d.o;
+            const int bx = A_MN ? pb.X0 : pb.Z0, y0 = pb.Y0;
+            const uint32_t abytes = A_MN && tiled && nxb == 1 ? C::A_BYTES / 2 : C::A_BYTES;
+            const uint32_t bytes = 2 * abytes + (uint32_t)(2 * nbox * 8192);
             // K = (ko, ki): kinds 0 and 3 run q in ko with batch y, kinds 1 and 2 y in ko with batch q
             const bool ko_q = P.kind == 0 || P.kind == 3;
             int ko = 0, ki = 0;
@@ -165,21 +189,25 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
                 uint8_t *sA = smem + stage * C::STAGE_BYTES;
                 uint8_t *sB = sA + 2 * C::A_BYTES;
                 const int aq = ko_q ? ko : b, ay = ko_q ? b : ko;
-                const int b3 = ko_q ? ko : pb.Y0 + ko;
+                const int b3 = ko_q ? ko : y0 + ko;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     uint8_t *a = sA + h * C::A_BYTES;
                     uint8_t *bb = sB + h * C::B_BYTES;
-                    if (A_MN) {
+                    if (tiled) {
+                        const int hyq = (h * Ty + ay) * o + aq;
+                        if (A_MN) tma_load_5d(a, tmA, &full[stage], 0, mt * 16, ki * 4 * nxb, hyq, 0);
+                        else tma_load_5d(a, tmA, &full[stage], 0, ki * 8, mt * 16, hyq, 0);
+                    } else if (A_MN) {
 #pragma unroll
                         for (int j = 0; j < 2; j++)
                             tma_load_5d(a + j * 8192, tmA, &full[stage], mt * 128 + j * 64, aq, 0, ki * 4, h * Ty + ay);
                     } else {
                         tma_load_5d(a, tmA, &full[stage], ki * 64, aq, 0, mt * 8, h * Ty + ay);
                     }
-                    const int b1 = A_MN ? pb.X0 : pb.Z0, b2 = A_MN ? ki * 4 : (ki * 64) >> lz;
-                    tma_load_5d(bb, tmB, &full[stage], n0, b1, b2, b3, h);
-                    if (BN > 64 && nbox > 1) tma_load_5d(bb + 8192, tmB, &full[stage], n0 + 64, b1, b2, b3, h);
+                    const int b2 = A_MN ? ki * 4 : (ki * 64) >> lz;
+                    tma_load_5d(bb, tmB, &full[stage], n0, bx, b2, b3, h);
+                    if (BN > 64 && nbox > 1) tma_load_5d(bb + 8192, tmB, &full[stage], n0 + 64, bx, b2, b3, h);
                 }
                 if (++ki == nk_inner) {
                     ki = 0;
@@ -219,6 +247,15 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
             // K values of the inner blocks of one outer index: o Tz, or 16 per p
             const int klen = A_MN ? 16 * P.d.o : P.d.o * P.pb[tau].Tz;
             int left = klen;   // K values from the current inner block on
+            // First operand: 128B-swizzled rows, or core matrices.  An 8-wide x block is the first
+            // half of each 16-wide K step and a block of zeros the second: there the K stride is
+            // the distance to that block, which falls as the address rises.
+            const bool tiled = wbar_tiled(P.pb[tau]), half_k = A_MN && tiled && P.pb[tau].Tx == 8;
+            const uint64_t a_unit = half_k ? 1ull - (1ull << 16) : 1ull;   // descriptor per 16 bytes of address
+            const uint64_t a_base = !tiled  ? make_sdesc_sw128(0, A_MN ? 8192 : 16, 1024)
+                                    : !A_MN ? make_sdesc_none(0, 128, 1024)
+                                            : make_sdesc_none(0, half_k ? smem_u32(zero) : 2048u, 128);
+            const uint64_t a_step = (tiled ? (A_MN ? (half_k ? 128 : 256) : 16) : (A_MN ? 128 : 2)) * a_unit;
             for (int k0 = 0; k0 < nk && ok; k0 += P.kseg, seg++) {
                 const int acc = seg % C::NACC;
                 const uint32_t accph = (seg / C::NACC) & 1;
@@ -235,25 +272,16 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t a_h = smem_u32(smem + stage * C::STAGE_BYTES);
-                    const uint32_t a_l = a_h + C::A_BYTES;
-                    const uint32_t b_h = a_l + C::A_BYTES;
-                    const uint32_t b_l = b_h + C::B_BYTES;
+                    const uint32_t sA = smem_u32(smem + stage * C::STAGE_BYTES), sB = sA + 2 * C::A_BYTES;
+                    const uint64_t a_h = a_base + (sA >> 4) * a_unit, a_l = a_h + (C::A_BYTES >> 4) * a_unit;
+                    const uint64_t b_h = make_sdesc_sw128(sB, 8192, 1024), b_l = b_h + (C::B_BYTES >> 4);
                     const int nks = left < kTcBK ? (left + 15) >> 4 : kTcBK / 16;
                     left = left <= kTcBK ? klen : left - kTcBK;
 #pragma unroll
                     for (int ks = 0; ks < kTcBK / 16; ks++) {
                         if (ks >= nks) break;
-                        uint64_t dah, dal;
-                        if (A_MN) {
-                            dah = make_sdesc_sw128(a_h + 2048 * ks, 8192, 1024);
-                            dal = make_sdesc_sw128(a_l + 2048 * ks, 8192, 1024);
-                        } else {
-                            dah = make_sdesc_sw128(a_h + 32 * ks, 16, 1024);
-                            dal = make_sdesc_sw128(a_l + 32 * ks, 16, 1024);
-                        }
-                        const uint64_t dbh = make_sdesc_sw128(b_h + 2048 * ks, 8192, 1024);
-                        const uint64_t dbl = make_sdesc_sw128(b_l + 2048 * ks, 8192, 1024);
+                        const uint64_t dah = a_h + a_step * ks, dal = a_l + a_step * ks;
+                        const uint64_t dbh = b_h + 128 * ks, dbl = b_l + 128 * ks;
                         umma_f16(d_tmem, dah, dbh, idesc, (kb > k0 || ks > 0) ? 1u : 0u);
                         umma_f16(d_tmem, dah, dbl, idesc, 1u);
                         umma_f16(d_tmem, dal, dbh, idesc, 1u);
@@ -298,7 +326,8 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
             const double sc = ONE ? sc0 : P.sign / ((*P.wscale) * (*P.oscale));
             long long roff = -1;
             if (P.kind == 0 || P.kind == 2) {
-                const int p = mt * 8 + row / 16, x = row % 16;
+                const int xw = pb.Tx == 8 ? 8 : 16;   // rows of a p in the tile
+                const int p = mt * (kTcBM / xw) + row / xw, x = row % xw;
                 if (p < o && x < pb.Tx) {
                     if (P.kind == 0)
                         roff = ((((long long)pb.Y0 + b) * o + p) * v + pb.X0 + x) * Kp;
@@ -369,10 +398,9 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
                     if (two) mbar_arrive(&tempty[accB]);
                 }
                 if (!two) seg -= 1;   // an odd tail used one accumulator
-                if ((s0 + 2) % kB1RunSegments == 0 && s0 + 2 < nseg) flush();
+                if ((s0 + 2) % kB1RunSegments == 0 || s0 + 2 >= nseg) flush();
             }
             if (!ok) break;
-            flush();
         }
     }
     tc_fence_before();

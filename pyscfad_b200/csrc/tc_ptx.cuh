@@ -175,6 +175,19 @@ __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t saddr, uint32_t lb
     return d;
 }
 
+// Shared-memory matrix descriptor without swizzle: 8 x 8 core matrices of 128
+// contiguous bytes (eight 16-byte rows).
+// K-major: a row is 8 K elements; lbo = core matrices adjacent in K, sbo = adjacent in MN.
+// MN-major: a row is 8 MN elements of one K; lbo = adjacent in K, sbo = adjacent in MN.
+__device__ __forceinline__ uint64_t make_sdesc_none(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)1 << 46;   // descriptor version for sm_100
+    return d;
+}
+
 // Instruction descriptor, kind::f16: fp32 accumulate, fp16 (bf16 = false) or
 // bf16 inputs (both operands the same type), K- or MN-major operands.
 __host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N, bool bf16, bool a_mn, bool b_mn) {

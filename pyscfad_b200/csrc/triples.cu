@@ -860,8 +860,9 @@ static EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
-// 5-D map over a [2][d3][d2][d1][d0] 16-bit array (d0 innermost), 128B swizzle.
-static int make_tmap5(CUtensorMap *tm, void *base, bool bf16, const uint64_t dims[5], const uint32_t box[5]) {
+// 5-D map over a dense 16-bit array of dims[0] (innermost) to dims[4], 128B swizzle or none.
+static int make_tmap5(CUtensorMap *tm, void *base, bool bf16, const uint64_t dims[5], const uint32_t box[5],
+                      bool swizzle = true) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return TRIPLES_ERR_UNSUPPORTED;
     cuuint64_t gdim[5], gstr[4];
@@ -876,8 +877,8 @@ static int make_tmap5(CUtensorMap *tm, void *base, bool bf16, const uint64_t dim
     cuuint32_t bx[5], es[5] = {1, 1, 1, 1, 1};
     for (int i = 0; i < 5; i++) bx[i] = box[i];
     CUresult r = enc(tm, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, base, gdim,
-                     gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? TRIPLES_OK : TRIPLES_ERR_CUDA;
 }
 
@@ -1252,12 +1253,23 @@ static void sub_regions(const ChunkDesc &ch, int o, const int *st, const int *le
         F2mPi &D = u.pi[pi];
         D.s0 = f2m_stage_offset(pb, o, 0, 0, 0, ys, xs, zs);   // (y, x, z) at a block's origin: no exchange
         D.rs = pb.Tx * pb.Ty * pb.Tz;
-        D.wx = o * pb.rzp;
-        D.wp = pb.Tx * D.wx;
-        D.wy = o * D.wp;
-        D.rzp = pb.rzp;
         D.tz = pb.Tz;
-        D.w0 = wmul * pb.swoff + (long long)ys * D.wy + (long long)xs * D.wx + zs;
+        D.zs = zs;
+        D.tiled = wmul == 2 && wbar_tiled(pb) ? 1 : 0;
+        if (D.tiled) {
+            const int tile_row = 8 * pb.rzp;   // the tiles of 8 x values
+            D.wx = 8;
+            D.wp = pb.Tx / 8 * tile_row;
+            D.wq = o * D.wp;
+            D.wy = o * D.wq;
+            D.w0 = wmul * pb.swoff + (long long)ys * D.wy + xs / 8 * tile_row;
+        } else {
+            D.wq = pb.rzp;
+            D.wx = o * D.wq;
+            D.wp = pb.Tx * D.wx;
+            D.wy = o * D.wp;
+            D.w0 = wmul * pb.swoff + (long long)ys * D.wy + (long long)xs * D.wx;
+        }
         D.half = (long long)pb.Ty * D.wy;
         D.bytes = elem * len[0] * len[1] * len[2];
         if (D.bytes % 16 == 0) {
@@ -1439,15 +1451,26 @@ static int b1_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, con
     B.sign = kind == 2 ? -1.0 : 1.0;
     for (int t = 0; t < ch.nperm; t++) {
         const PermBlock &pb = ch.pb[t];
-        const uint64_t dW[5] = {(uint64_t)pb.rzp, o, (uint64_t)pb.Tx, o, (uint64_t)(2 * pb.Ty)};
-        const int rc = make_tmap5(&B.tmA[t], SW + 2 * pb.swoff * 2, bf16, dW, (kind == 0 || kind == 2) ? bK : bM);
+        const bool kmajor = kind == 0 || kind == 2;
+        int rc;
+        if (wbar_tiled(pb)) {
+            // [h y q][p, x tile][rz tile][64]; boxes of 128 rows x 64 K values (K = 4 p in the MN-major kinds)
+            const uint64_t nxb = pb.Tx / 8;
+            const uint64_t dT[5] = {64, (uint64_t)pb.rzp / 8, o * nxb, 2 * pb.Ty * o, 1};
+            const uint32_t bTK[5] = {64, 8, 16, 1, 1}, bTM[5] = {64, 16, (uint32_t)(4 * nxb), 1, 1};
+            rc = make_tmap5(&B.tmA[t], SW + 2 * pb.swoff * 2, bf16, dT, kmajor ? bTK : bTM, false);
+        } else {
+            const uint64_t dW[5] = {(uint64_t)pb.rzp, o, (uint64_t)pb.Tx, o, (uint64_t)(2 * pb.Ty)};
+            rc = make_tmap5(&B.tmA[t], SW + 2 * pb.swoff * 2, bf16, dW, kmajor ? bK : bM);
+        }
         if (rc != TRIPLES_OK) return rc;
+        const int mt_px = (d.o * (pb.Tx == 8 ? 8 : 16) + kTcBM - 1) / kTcBM;   // M tiles over (p, x)
         int lz = 0;
         while ((1 << lz) < pb.Tz) lz++;
         switch (kind) {
         case 0:
             B.tmB[t] = M.tmB1z[lz];
-            B.nbatch[t] = pb.Ty; B.ntile_m[t] = (d.o + 7) / 8;
+            B.nbatch[t] = pb.Ty; B.ntile_m[t] = mt_px;
             B.nk_outer[t] = d.o; B.nk_inner[t] = (d.o * pb.Tz + 63) / 64;
             break;
         case 1:
@@ -1457,7 +1480,7 @@ static int b1_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, con
             break;
         case 2:
             B.tmB[t] = M.tmB2z[lz];
-            B.nbatch[t] = d.o; B.ntile_m[t] = (d.o + 7) / 8;
+            B.nbatch[t] = d.o; B.ntile_m[t] = mt_px;
             B.nk_outer[t] = pb.Ty; B.nk_inner[t] = (d.o * pb.Tz + 63) / 64;
             break;
         default:

@@ -90,3 +90,20 @@ def test_mixed_contraction_tiles(o, v, tile_n):
     if o > 1:
         for k in G.KEYS:
             assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-5, k
+
+
+# The adjoint tiles of x blocks of 16 and 8 virtuals (two and one 8 x 8 tiles
+# wide: K blocks of 64 and of half as many stored values) and of the shorter
+# remainder blocks kept in rows, for occupied counts off the 4 per K block and
+# the 8 and 16 per M tile.  The mixed mode's parity bounds.
+@pytest.mark.parametrize("o,v,tv", [(2, 24, 16), (5, 40, 16), (9, 28, 8), (17, 40, 16), (18, 27, 8)])
+@pytest.mark.parametrize("precision", ["mixed", "mixed_bf16"])
+def test_adjoint_tiles(o, v, tv, precision):
+    inp = make_inputs(o, v, 40, seed=v, fvo_sigma=1e-3)
+    ins = [getattr(inp, k) for k in G.KEYS]
+    e0, g0 = triples.energy_vjp(*ins, precision="fp64", device="cuda")
+    e, g = triples.energy_vjp(*ins, precision=precision, device="cuda", block_size=tv)
+    e_tol, g_tol = (1e-6, 1e-5) if precision == "mixed" else (1e-4, 1e-3)
+    assert abs(float(e) - float(e0)) <= e_tol * abs(float(e0))
+    for k in G.KEYS:
+        assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < g_tol, k
