@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
     uint32_t *tmem_slot = (uint32_t *)(drain + 1);
     int &s_abort = *(int *)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t leader = lane == 0 ? 1u : 0u;   // issues for the producer and MMA warps
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int s = 0; s < C::STAGES; s++) {
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
         nt = rem % P.ntile_n;
     };
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------- TMA producer ----------------
         int stage = 0;
         uint32_t phase = 0;
@@ -180,12 +181,12 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
             const bool ko_q = P.kind == 0 || P.kind == 3;
             int ko = 0, ki = 0;
             for (int kb = 0; kb < nk; kb++) {
-                if (!mbar_wait(&empty[stage], phase ^ 1u, abortp)) {
+                if (!mbar_wait_warp(&empty[stage], phase ^ 1u, abortp)) {
                     ok = false;
                     break;
                 }
                 pending[stage] = false;
-                mbar_expect_tx(&full[stage], bytes);
+                mbar_expect_tx(leader, &full[stage], bytes);
                 uint8_t *sA = smem + stage * C::STAGE_BYTES;
                 uint8_t *sB = sA + 2 * C::A_BYTES;
                 const int aq = ko_q ? ko : b, ay = ko_q ? b : ko;
@@ -196,18 +197,18 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
                     uint8_t *bb = sB + h * C::B_BYTES;
                     if (tiled) {
                         const int hyq = (h * Ty + ay) * o + aq;
-                        if (A_MN) tma_load_5d(a, tmA, &full[stage], 0, mt * 16, ki * 4 * nxb, hyq, 0);
-                        else tma_load_5d(a, tmA, &full[stage], 0, ki * 8, mt * 16, hyq, 0);
+                        if (A_MN) tma_load_5d(leader, a, tmA, &full[stage], 0, mt * 16, ki * 4 * nxb, hyq, 0);
+                        else tma_load_5d(leader, a, tmA, &full[stage], 0, ki * 8, mt * 16, hyq, 0);
                     } else if (A_MN) {
 #pragma unroll
                         for (int j = 0; j < 2; j++)
-                            tma_load_5d(a + j * 8192, tmA, &full[stage], mt * 128 + j * 64, aq, 0, ki * 4, h * Ty + ay);
+                            tma_load_5d(leader, a + j * 8192, tmA, &full[stage], mt * 128 + j * 64, aq, 0, ki * 4, h * Ty + ay);
                     } else {
-                        tma_load_5d(a, tmA, &full[stage], ki * 64, aq, 0, mt * 8, h * Ty + ay);
+                        tma_load_5d(leader, a, tmA, &full[stage], ki * 64, aq, 0, mt * 8, h * Ty + ay);
                     }
                     const int b2 = A_MN ? ki * 4 : (ki * 64) >> lz;
-                    tma_load_5d(bb, tmB, &full[stage], n0, bx, b2, b3, h);
-                    if (BN > 64 && nbox > 1) tma_load_5d(bb + 8192, tmB, &full[stage], n0 + 64, bx, b2, b3, h);
+                    tma_load_5d(leader, bb, tmB, &full[stage], n0, bx, b2, b3, h);
+                    if (BN > 64 && nbox > 1) tma_load_5d(leader, bb + 8192, tmB, &full[stage], n0 + 64, bx, b2, b3, h);
                 }
                 if (++ki == nk_inner) {
                     ki = 0;
@@ -223,14 +224,14 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
         }
         if (!ok) {
             *abortp = 1;
-            atomicOr(Pfirst.err, 8);
+            if (leader) atomicOr(Pfirst.err, 8);
             for (int s = 0; s < C::STAGES; s++)
                 if (pending[s]) {
                     for (uint32_t i = 0; i < kSpinLimit && !mbar_try_wait(&full[s], pend_phase[s]); i++) {
                     }
                 }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // ---------------- MMA issuer: one TMEM buffer per K segment ----------------
         int stage = 0;
         uint32_t phase = 0;
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
             for (int k0 = 0; k0 < nk && ok; k0 += P.kseg, seg++) {
                 const int acc = seg % C::NACC;
                 const uint32_t accph = (seg / C::NACC) & 1;
-                if (!mbar_wait(&tempty[acc], accph ^ 1u, abortp)) {
+                if (!mbar_wait_warp(&tempty[acc], accph ^ 1u, abortp)) {
                     ok = false;
                     break;
                 }
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
                 const int k1 = (k0 + P.kseg < nk) ? k0 + P.kseg : nk;
                 for (int kb = k0; kb < k1; kb++) {
-                    if (!mbar_wait(&full[stage], phase, abortp)) {
+                    if (!mbar_wait_warp(&full[stage], phase, abortp)) {
                         ok = false;
                         break;
                     }
@@ -282,25 +283,25 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
                         if (ks >= nks) break;
                         const uint64_t dah = a_h + a_step * ks, dal = a_l + a_step * ks;
                         const uint64_t dbh = b_h + 128 * ks, dbl = b_l + 128 * ks;
-                        umma_f16(d_tmem, dah, dbh, idesc, (kb > k0 || ks > 0) ? 1u : 0u);
-                        umma_f16(d_tmem, dah, dbl, idesc, 1u);
-                        umma_f16(d_tmem, dal, dbh, idesc, 1u);
+                        umma_f16(leader, d_tmem, dah, dbh, idesc, (kb > k0 || ks > 0) ? 1u : 0u);
+                        umma_f16(leader, d_tmem, dah, dbl, idesc, 1u);
+                        umma_f16(leader, d_tmem, dal, dbh, idesc, 1u);
                     }
-                    umma_commit(&empty[stage]);
+                    umma_commit(leader, &empty[stage]);
                     if (++stage == C::STAGES) {
                         stage = 0;
                         phase ^= 1u;
                     }
                 }
                 if (!ok) break;
-                umma_commit(&tfull[acc]);
+                umma_commit(leader, &tfull[acc]);
             }
         }
         if (!ok) {
             *abortp = 1;
-            atomicOr(Pfirst.err, 16);
+            if (leader) atomicOr(Pfirst.err, 16);
         }
-        umma_commit(drain);
+        umma_commit(leader, drain);
         for (uint32_t i = 0; i < kSpinLimit && !mbar_try_wait(drain, 0); i++) {
         }
     } else if (warp >= 2) {

@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
     uint32_t *tmem_slot = (uint32_t *)(drain + 1);
     __shared__ int s_abort;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t leader = lane == 0 ? 1u : 0u;   // issues for the producer and MMA warps
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int s = 0; s < C::STAGES; s++) {
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
     volatile int *abortp = &s_abort;
     const int total = J.start[J.n];
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------- TMA producer ----------------
         int stage = 0;
         uint32_t phase = 0;
@@ -156,28 +157,28 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
             const int yg = pb.Y0 + T.y;
             const int nkb = P.nkb1 + P.nkb2;
             for (int kb = 0; kb < nkb; kb++) {
-                if (!mbar_wait(&empty[stage], phase ^ 1u, abortp)) {
+                if (!mbar_wait_warp(&empty[stage], phase ^ 1u, abortp)) {
                     ok = false;
                     break;
                 }
                 pending[stage] = false;
-                mbar_expect_tx(&full[stage], (uint32_t)(2 * C::A_BYTES + P.rt * (2 * 16 * kTcBK * 2)));
+                mbar_expect_tx(leader, &full[stage], (uint32_t)(2 * C::A_BYTES + P.rt * (2 * 16 * kTcBK * 2)));
                 uint8_t *sA = smem + stage * C::STAGE_BYTES;
                 uint8_t *sAl = sA + C::A_BYTES;
                 uint8_t *sB = sAl + C::A_BYTES;
                 uint8_t *sBl = sB + C::B_BYTES;
                 if (kb < P.nkb1) {
                     const int f0 = kb * kTcBK;
-                    tma_load_5d(sA, &M.a1, &full[stage], f0, pb.X0, T.mt * 8, yg, 0);
-                    tma_load_5d(sAl, &M.a1, &full[stage], f0, pb.X0, T.mt * 8, yg, 1);
-                    tma_load_5d(sB, &M.b1, &full[stage], f0, pb.Z0, T.nt * P.rt, T.q, 0);
-                    tma_load_5d(sBl, &M.b1, &full[stage], f0, pb.Z0, T.nt * P.rt, T.q, 1);
+                    tma_load_5d(leader, sA, &M.a1, &full[stage], f0, pb.X0, T.mt * 8, yg, 0);
+                    tma_load_5d(leader, sAl, &M.a1, &full[stage], f0, pb.X0, T.mt * 8, yg, 1);
+                    tma_load_5d(leader, sB, &M.b1, &full[stage], f0, pb.Z0, T.nt * P.rt, T.q, 0);
+                    tma_load_5d(leader, sBl, &M.b1, &full[stage], f0, pb.Z0, T.nt * P.rt, T.q, 1);
                 } else {
                     const int m0 = (kb - P.nkb1) * kTcBK;
-                    tma_load_5d(sA, &M.a2, &full[stage], m0, pb.X0, T.mt * 8, T.q, 0);
-                    tma_load_5d(sAl, &M.a2, &full[stage], m0, pb.X0, T.mt * 8, T.q, 1);
-                    tma_load_5d(sB, &M.b2, &full[stage], m0, pb.Z0, T.nt * P.rt, yg, 0);
-                    tma_load_5d(sBl, &M.b2, &full[stage], m0, pb.Z0, T.nt * P.rt, yg, 1);
+                    tma_load_5d(leader, sA, &M.a2, &full[stage], m0, pb.X0, T.mt * 8, T.q, 0);
+                    tma_load_5d(leader, sAl, &M.a2, &full[stage], m0, pb.X0, T.mt * 8, T.q, 1);
+                    tma_load_5d(leader, sB, &M.b2, &full[stage], m0, pb.Z0, T.nt * P.rt, yg, 0);
+                    tma_load_5d(leader, sBl, &M.b2, &full[stage], m0, pb.Z0, T.nt * P.rt, yg, 1);
                 }
                 pending[stage] = true;
                 pend_phase[stage] = phase;
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
         }
         if (!ok) {
             *abortp = 1;
-            atomicOr(Pfirst.err, 1);
+            if (leader) atomicOr(Pfirst.err, 1);
             // let copies already in flight land before the CTA can exit
             for (int s = 0; s < C::STAGES; s++)
                 if (pending[s]) {
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
                     }
                 }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // ---------------- MMA issuer: one TMEM buffer per K segment ----------------
         int stage = 0;
         uint32_t phase = 0;
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
             for (int k0 = 0; k0 < nkb && ok; k0 += P.kseg, seg++) {
                 const int acc = seg & 1;
                 const uint32_t accph = (seg >> 1) & 1;
-                if (!mbar_wait(&tempty[acc], accph ^ 1u, abortp)) {
+                if (!mbar_wait_warp(&tempty[acc], accph ^ 1u, abortp)) {
                     ok = false;
                     break;
                 }
@@ -220,44 +221,40 @@ __global__ void __launch_bounds__(kF1Threads, 1) k_f1_tc(const __grid_constant__
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
                 const int k1 = (k0 + P.kseg < nkb) ? k0 + P.kseg : nkb;
                 for (int kb = k0; kb < k1; kb++) {
-                    if (!mbar_wait(&full[stage], phase, abortp)) {
+                    if (!mbar_wait_warp(&full[stage], phase, abortp)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t a_h = smem_u32(smem + stage * C::STAGE_BYTES);
-                    const uint32_t a_l = a_h + C::A_BYTES;
-                    const uint32_t b_h = a_l + C::A_BYTES;
-                    const uint32_t b_l = b_h + C::B_BYTES;
+                    const uint64_t a_h = make_sdesc_sw128(smem_u32(smem + stage * C::STAGE_BYTES), 16, 1024);
+                    const uint64_t a_l = a_h + (C::A_BYTES >> 4), b_h = a_l + (C::A_BYTES >> 4);
+                    const uint64_t b_l = b_h + (C::B_BYTES >> 4);
                     // 16-wide steps that hold K values (the rest of the block is zero)
                     const int left = kb < P.nkb1 ? P.k1 - kb * kTcBK : P.k2 - (kb - P.nkb1) * kTcBK;
 #pragma unroll
                     for (int ks = 0; ks < kTcBK / 16; ks++) {
                         if (16 * ks >= left) continue;
-                        const uint64_t dah = make_sdesc_sw128(a_h + 32 * ks, 16, 1024);
-                        const uint64_t dal = make_sdesc_sw128(a_l + 32 * ks, 16, 1024);
-                        const uint64_t dbh = make_sdesc_sw128(b_h + 32 * ks, 16, 1024);
-                        const uint64_t dbl = make_sdesc_sw128(b_l + 32 * ks, 16, 1024);
-                        umma_f16(d_tmem, dah, dbh, idesc, (kb > k0 || ks > 0) ? 1u : 0u);
-                        umma_f16(d_tmem, dah, dbl, idesc, 1u);
-                        umma_f16(d_tmem, dal, dbh, idesc, 1u);
+                        const uint64_t dah = a_h + 2 * ks, dal = a_l + 2 * ks, dbh = b_h + 2 * ks, dbl = b_l + 2 * ks;
+                        umma_f16(leader, d_tmem, dah, dbh, idesc, (kb > k0 || ks > 0) ? 1u : 0u);
+                        umma_f16(leader, d_tmem, dah, dbl, idesc, 1u);
+                        umma_f16(leader, d_tmem, dal, dbh, idesc, 1u);
                     }
-                    umma_commit(&empty[stage]);
+                    umma_commit(leader, &empty[stage]);
                     if (++stage == C::STAGES) {
                         stage = 0;
                         phase ^= 1u;
                     }
                 }
                 if (!ok) break;
-                umma_commit(&tfull[acc]);
+                umma_commit(leader, &tfull[acc]);
             }
         }
         if (!ok) {
             *abortp = 1;
-            atomicOr(Pfirst.err, 2);
+            if (leader) atomicOr(Pfirst.err, 2);
         }
         // all MMAs of this thread complete before TMEM can be released
-        umma_commit(drain);
+        umma_commit(leader, drain);
         for (uint32_t i = 0; i < kSpinLimit && !mbar_try_wait(drain, 0); i++) {
         }
     } else if (warp >= 2) {
