@@ -40,15 +40,27 @@
 // leaves as 16-byte hi and lo runs, the V-term gradients as row sums (per
 // run) and column sums (over the region's runs) added to the FP64 gradients.
 //
-// What bounds it: instruction issue and shared-memory latency at 16 warps per
-// SM; HBM is at a quarter of its rate.
-// Measured against the kernels it replaced (a one-CTA persistent kernel for
-// the all-distinct items and a CTA per item for the rest): nocc 40 nvir 360,
-// virtual block 6: 343 to 266 ms; nocc 40 nvir 72: 285 to 199 ms; nocc 20 nvir
-// 180: 493 to 397 ms.  Wbar in 8 x 8 tiles, whole 128-byte lines per warp, in
-// place of rows whose half sectors two items wrote: the three to 213, 165 and
-// 325 ms (with rows, items in fixed strides instead of by the counter took 454
-// ms in the first, the halves reaching DRAM one by one).
+// What bounds it: latency at 16 warps per SM (registers and shared memory allow
+// no more); issue slots are 45 % busy, HBM is at a quarter of its rate.  What
+// holds the warps up are barriers, instruction fetch and memory in equal parts,
+// so the code an item runs through is kept short (the instruction cache does
+// not hold it otherwise): rare paths and the copies are out of line, the second
+// element takes a second turn of the same code, regions are described once per
+// item in shared memory.  Everything that prepares later items (next item's
+// tables, the load record of the one after) is done by one warp each during the
+// write-back, whose regions go to the warps as they come free.  The gradients
+// are reached by explicitly global reductions: through generic pointers each
+// one first tests for shared memory.
+// Measured (nocc 40 nvir 360, one virtual block; nocc 40 nvir 72; nocc 20 nvir
+// 180; 48 batched problems, ms):
+//   a one-CTA persistent kernel for the all-distinct items and
+//   a CTA per item for the rest                               343  285  493  119
+//   this kernel, Wbar in rows                                 266  198  396   91
+//   Wbar in 8 x 8 tiles: whole lines per warp, where rows
+//   were 16-byte halves of sectors from two items             213  165  324   89
+//   short code, records, preparation in the write-back              132  265   60
+//   global reductions                                               119  242   56
+// (In rows, items in fixed strides instead of by the counter: 454 ms in the first.)
 //
 // The FP32 sums keep a fixed order: rows run over z; columns over
 // half regions of 32 runs where nothing coincides and every sub-range is
@@ -143,6 +155,15 @@ __device__ __forceinline__ int f2m_nlead(int pat) { return pat == 0 ? 6 : (pat =
 
 __device__ __forceinline__ int sel3(int a, int b, int c, int i) { return i == 0 ? a : (i == 1 ? b : c); }
 
+// A region to write back, formed once per item by one thread each.
+struct __align__(16) F2mTask {
+    uint16_t *w;          // Wbar: hi plane, first position
+    double *ob, *tb;      // ovov_bar, t2_bar: first x and y
+    unsigned code;        // bits 0-2 pi, 3-5 rho, 6-11 slots of pi, 12-14 s with s o rho = pi,
+                          // 15-16 slot of r, 17-28 lx, ly, lz
+    unsigned rz;          // r, first z << 16
+};
+
 struct F2mSmem {
     static constexpr int REGION = 512;                                    // floats
     static constexpr int STAGE = 6 * REGION;
@@ -151,7 +172,9 @@ struct F2mSmem {
     static constexpr size_t OFF_TAB = sizeof(float) * kF2mStages * STAGE;
     static constexpr size_t OFF_TF = OFF_TAB + sizeof(float2) * 2 * TAB;
     static constexpr size_t OFF_RES = OFF_TF + sizeof(float2) * 2 * TF;
-    static constexpr size_t BYTES = OFF_RES + sizeof(uint2) * 6 * 512 + 128;   // +128: base alignment
+    static constexpr size_t OFF_REC = OFF_RES + sizeof(uint2) * 6 * 512;
+    static constexpr size_t BYTES = OFF_REC + sizeof(F2mTask) * 36 + 128;   // +128: base alignment
+    static_assert(2 * (BYTES + 2048 + 1024) <= 228 * 1024, "two blocks per SM, with the static arrays");
     static_assert(OFF_TAB % 16 == 0 && OFF_TF % 16 == 0 && OFF_RES % 16 == 0, "bulk copy destinations");
 };
 
@@ -194,6 +217,57 @@ __device__ __forceinline__ uint32_t f2m_split(float w, float scale) {
     return (uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(l) << 16);
 }
 
+// What the loads of an item's regions need.
+struct F2mSrc {
+    const float *src;     // staging: region of pi, p = q = r = 0
+    int rs;               // staging stride of r
+    int bytes;            // of a region; negative: no bulk copies
+};
+struct F2mItem {
+    int job, sub, rep, i0, i1, i2;
+    float wscale;
+};
+struct F2mLoad {
+    F2mSrc pi[6];
+    int idx[6];           // (p o + q) o + r of each rho
+    int bulk_bytes, pad;
+};
+
+// Out of line: the instruction cache holds the code of an item only if its
+// rare paths are short.
+__device__ __noinline__ void f2m_wait_slow(uint64_t *bar, uint32_t parity, volatile int *abortp, int *err) {
+    if (!mbar_wait(bar, parity, abortp)) {
+        *abortp = 1;
+        atomicOr(err, 64);
+    }
+}
+
+// W stage n of the CTA (one warp): the regions of (item, rho) of a load record;
+// every warp has read the stage's previous content.
+__device__ __noinline__ void f2m_issue(const F2mLoad *L, int rho, int n, float *sW, uint64_t *full) {
+    const int lane = threadIdx.x & 31, st = n & (kF2mStages - 1);
+    fence_proxy_async_smem();
+    if (lane == 0) mbar_expect_tx(&full[st], (uint32_t)L->bulk_bytes);
+    __syncwarp();
+    if (lane < 6) {
+        const F2mSrc D = L->pi[lane];
+        float *dst = sW + st * F2mSmem::STAGE + lane * F2mSmem::REGION;
+        const float *src = D.src + (long long)L->idx[rho] * D.rs;
+        if (D.bytes > 0) {
+            bulk_load(dst, src, (uint32_t)D.bytes, &full[st]);
+        } else {
+#pragma unroll 1
+            for (int e = 0; e < -D.bytes / 4; e++) dst[e] = src[e];   // one or two values
+        }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&full[st]);
+}
+
+__device__ __forceinline__ void f2m_red(double *p, float v) {
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"((double)v) : "memory");
+}
+
 __device__ __forceinline__ void f2m_bar(int id) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kF2mThreads) : "memory");
 }
@@ -210,6 +284,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
     float2 *sTab = reinterpret_cast<float2 *>(smem + C::OFF_TAB);
     float2 *sTF = reinterpret_cast<float2 *>(smem + C::OFF_TF);
     uint2 *sRes = reinterpret_cast<uint2 *>(smem + C::OFF_RES);
+    F2mTask *s_rec = reinterpret_cast<F2mTask *>(smem + C::OFF_REC);
     __shared__ uint64_t full[kF2mStages], tfull[2];
     __shared__ unsigned s_read[kF2mStages];        // warps that have read the stage
     __shared__ unsigned s_task[36];                // per (pi, rho): slots of pi, of rho, and s with s o rho = pi
@@ -217,6 +292,9 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
     __shared__ __align__(16) int s_res[3][8];      // byte offsets of f2m_res
     __shared__ double s_part[8][14];               // per-warp partials: c, b, a sums (4 each), energy
     __shared__ int s_abort, s_next[2];             // next item of the CTA, by parity of the current one
+    __shared__ __align__(16) F2mLoad s_load[2];    // of the current and the next item
+    __shared__ F2mItem s_item[2];
+    __shared__ unsigned s_tasks[2];                // regions handed out for write-back
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned *ticket = J.job[0].ticket;
@@ -243,14 +321,11 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
     __syncthreads();
     volatile int *abortp = &s_abort;
     // Job of global item w and the item in it (w only grows).
-    struct Item {
-        int w, job, sub, rep, i0, i1, i2;
-    };
+    using Item = F2mItem;
     JobCursor jcur;
     auto item_at = [&](int w) -> Item {
         Item I;
         int lw;
-        I.w = w;
         I.job = jcur.at(J, w, lw);
         const F2M &P = J.job[ONE ? 0 : I.job];
         I.rep = lw / P.nsub;
@@ -258,15 +333,13 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
         I.i0 = P.ijk[3 * I.rep];
         I.i1 = P.ijk[3 * I.rep + 1];
         I.i2 = P.ijk[3 * I.rep + 2];
+        I.wscale = P.want_grad ? (float)*P.wscale : 1.0f;
         return I;
     };
     // every wait is bounded; after a timeout the remaining items run through
     // without waiting (no address depends on the data) and the status bit is set
     auto wait = [&](uint64_t *bar, uint32_t parity) {
-        if (!mbar_wait(bar, parity, abortp)) {
-            *abortp = 1;
-            atomicOr(J.job[0].err, 64);
-        }
+        if (!mbar_try_wait(bar, parity)) f2m_wait_slow(bar, parity, abortp, J.job[0].err);
     };
     // ---- the loads, each issued by one warp ----
     // V-term tables and energies of an item into table buffer b (its previous item is done)
@@ -333,32 +406,21 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
         }
         if (lane == 0) mbar_arrive(&tfull[b]);
     };
-    // W stage n of the CTA: the regions of (item, rho); every warp has read the stage's previous content
-    auto issue_stage = [&](const Item &I, int rho, int n) {
+    // the load record of an item (one warp; the readers are ordered behind it by the stage counts)
+    auto load_record = [&](const Item &I, F2mLoad &L) {
         const F2M &P = J.job[ONE ? 0 : I.job];
         const F2mSub &R = P.sub[I.sub];
-        const int st = n & (kF2mStages - 1);
-        int pr[3];
-        perm_of(rho, pr);
-        const long long idx = ((long long)sel3(I.i0, I.i1, I.i2, pr[0]) * P.o + sel3(I.i0, I.i1, I.i2, pr[1])) * P.o +
-                              sel3(I.i0, I.i1, I.i2, pr[2]);
-        fence_proxy_async_smem();
-        float *dst = sW + st * C::STAGE;
-        if (lane == 0) mbar_expect_tx(&full[st], (uint32_t)R.bulk_bytes);
-        __syncwarp();
         if (lane < 6) {
             const F2mPi &D = R.pi[lane];
-            const float *src = P.S + D.s0 + idx * D.rs;
-            if ((R.bulk >> lane) & 1) {
-                bulk_load(dst + lane * C::REGION, src, (uint32_t)D.bytes, &full[st]);
-            } else {
-                for (int e = 0; e < D.bytes / 4; e++) dst[lane * C::REGION + e] = src[e];   // one or two values
-            }
+            L.pi[lane] = F2mSrc{P.S + D.s0, D.rs, (R.bulk >> lane) & 1 ? D.bytes : -D.bytes};
+            int pr[3];
+            perm_of(lane, pr);
+            L.idx[lane] = (sel3(I.i0, I.i1, I.i2, pr[0]) * P.o + sel3(I.i0, I.i1, I.i2, pr[1])) * P.o +
+                          sel3(I.i0, I.i1, I.i2, pr[2]);
         }
+        if (lane == 0) L.bulk_bytes = R.bulk_bytes;
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full[st]);
     };
-
     // elements (a, b, c) and (a + 4, b, c); a warp spans 2 x 4 x 4 of them
     const int ca = ((tid >> 4) & 1) | (((tid >> 7) & 1) << 1);
     const int cb = ((tid >> 2) & 3) | (((tid >> 6) & 1) << 2);
@@ -383,30 +445,31 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
     };
 
     if ((int)blockIdx.x >= nitems) return;
-    Item cur = item_at(blockIdx.x), nxt = cur;
+    Item cur = item_at(blockIdx.x);
+    if (tid == 0) s_item[0] = cur;
     bool full_offsets = false;
     if (warp == 0) {
         issue_tables(cur, 0);
+        load_record(cur, s_load[0]);
 #pragma unroll 1
-        for (int n = 0; n < kF2mStages; n++) issue_stage(cur, n, n);
+        for (int n = 0; n < kF2mStages; n++) f2m_issue(&s_load[0], n, n, sW, full);
     }
+    // item w of the CTA's parity b, formed by one warp ahead of the first use
+    auto announce = [&](int w, int b) {
+        const Item I = item_at(w);
+        if (lane == 0) s_item[b] = I;
+        load_record(I, s_load[b]);
+    };
+    if (warp == 2 && s_next[0] < nitems) announce(s_next[0], 1);
 #pragma unroll 1
     for (int k = 0;; k++) {
         const F2M &P = J.job[ONE ? 0 : cur.job];
-        const int o = P.o, v = P.v;
-        const int sub = cur.sub, rep = cur.rep, i0 = cur.i0, i1 = cur.i1, i2 = cur.i2;
-        const float wscf = P.want_grad ? (float)*P.wscale : 1.0f;
         const int wn = s_next[k & 1];
         const bool more = wn < nitems;
-        if (more) nxt = item_at(wn);
         unsigned tk = 0;
         if (tid == 0 && more) tk = atomicAdd(ticket, 1u);
-        const F2mSub &R = P.sub[sub];
-        const int opat = (i0 == i2) ? 3 : (i0 == i1 ? 1 : (i1 == i2 ? 2 : 0));
-        const int vpat = R.pat;
-        const int l0 = R.len[0], l1 = R.len[1], l2 = R.len[2];
-        const bool plain = !P.whole && R.full && vpat == 0 && opat != 3;
-        const bool ok0 = ca < l0 && cb < l1 && cc < l2, ok1 = ca + 4 < l0 && cb < l1 && cc < l2;
+        const F2mSub &R = P.sub[cur.sub];
+        const bool plain = !P.whole && R.full && R.pat == 0 && cur.i0 != cur.i2;
         if (!R.full || !full_offsets) {
             offsets(R, P.ot != nullptr);
             full_offsets = R.full != 0;
@@ -470,41 +533,69 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
             if (seen == 7u) {
                 __threadfence_block();
                 if (lane == 0) s_read[st] = 0u;
-                if (rho + kF2mStages < 6) issue_stage(cur, rho + kF2mStages, n + kF2mStages);
-                else if (more) issue_stage(nxt, rho + kF2mStages - 6, n + kF2mStages);
+                if (rho + kF2mStages < 6) f2m_issue(&s_load[k & 1], rho + kF2mStages, n + kF2mStages, sW, full);
+                else if (more) f2m_issue(&s_load[(k & 1) ^ 1], rho + kF2mStages - 6, n + kF2mStages, sW, full);
             }
         }
 
+        // what only the second half needs is read here, not held in registers through the first
+        const F2mItem it = s_item[k & 1];
+        const int o = P.o, v = P.v;
+        const int i0 = it.i0, i1 = it.i1, i2 = it.i2;
+        const int opat = (i0 == i2) ? 3 : (i0 == i1 ? 1 : (i1 == i2 ? 2 : 0));
+        const int vpat = R.pat;
+        const int l0 = R.len[0], l1 = R.len[1], l2 = R.len[2];
+        const bool ok0 = ca < l0 && cb < l1 && cc < l2, ok1 = ca + 4 < l0 && cb < l1 && cc < l2;
         // orbit weights: n_ijk n_abc / 18 for three distinct virtuals; the energy
         // counts each orbit once per ordering of equal sub-ranges
         const double cocc = opat == 0 ? 2.0 : (opat == 3 ? 6.0 / 18.0 : 1.0);
         const double cen = vpat == 0 ? cocc : (vpat == 3 ? cocc / 6.0 : cocc * 0.5);
         if (tid == 0) s_next[(k & 1) ^ 1] = more ? (int)(gridDim.x + tk) : nitems;
+        if (tid == 0) s_tasks[k & 1] = 0u;   // (last used two items ago)
         f2m_bar(1);   // every warp is done with the previous item's results, partials and tables
-        if (warp == 1 && more) issue_tables(nxt, tb_ ^ 1);
         const double *en = s_en[tb_];
         const double e_occ = en[24] + en[25] + en[26];
-        double e_loc = 0.0, dd[2];
-#pragma unroll
+        const int nro = f2m_nlead(opat), ntask = P.want_grad ? f2m_nlead(vpat) * nro : 0;
+        if (tid >= 192 && tid - 192 < ntask) {
+            const int pi = f2m_lead(vpat, (tid - 192) / nro), rho = f2m_lead(opat, (tid - 192) % nro);
+            const unsigned code = s_task[pi * 6 + rho];
+            const int p0 = code & 3u, p1 = (code >> 2) & 3u, p2 = (code >> 4) & 3u;
+            const int p = sel3(i0, i1, i2, (code >> 6) & 3u), q = sel3(i0, i1, i2, (code >> 8) & 3u);
+            const int r = sel3(i0, i1, i2, (code >> 10) & 3u);
+            const int x = sel3(R.st[0], R.st[1], R.st[2], p0), y = sel3(R.st[0], R.st[1], R.st[2], p1);
+            F2mTask t;
+            t.w = P.SW + f2m_wbar(R.pi[pi], p, q, r);
+            t.ob = P.ovov_bar + (((long long)p * v + x) * o + q) * v + y;
+            t.tb = P.t2_bar + (((long long)q * o + p) * v + y) * v + x;
+            t.code = (unsigned)(pi | (rho << 3)) | ((code & 63u) << 6) | (((code >> 12) & 7u) << 12) |
+                     (((code >> 10) & 3u) << 15) | ((unsigned)sel3(l0, l1, l2, p0) << 17) |
+                     ((unsigned)sel3(l0, l1, l2, p1) << 21) | ((unsigned)sel3(l0, l1, l2, p2) << 25);
+            t.rz = (unsigned)r | ((unsigned)sel3(R.st[0], R.st[1], R.st[2], p2) << 16);
+            s_rec[tid - 192] = t;
+        }
+        double e_loc = 0.0, dd[2] = {0.0, 0.0};
+        // (a loop of two turns: the element's registers move down, half the code)
+#pragma unroll 1
         for (int e = 0; e < 2; e++) {
             const bool ok = e == 0 ? ok0 : ok1;
             double X[6], Z[6], RW[6];
 #pragma unroll
-            for (int s = 0; s < 6; s++) X[s] = WW[e][s] + 0.5 * (double)VV[e][s];
+            for (int s = 0; s < 6; s++) X[s] = WW[0][s] + 0.5 * (double)VV[0][s];
 #pragma unroll
             for (int s = 0; s < 6; s++) {
                 Z[s] = 4.0 * X[s] + X[perm_compose(s, 4)] + X[perm_compose(s, 3)] -
                        2.0 * (X[perm_compose(s, 5)] + X[perm_compose(s, 1)] + X[perm_compose(s, 2)]);
-                RW[s] = 4.0 * WW[e][s] + WW[e][perm_compose(s, 4)] + WW[e][perm_compose(s, 3)] -
-                        2.0 * (WW[e][perm_compose(s, 5)] + WW[e][perm_compose(s, 1)] + WW[e][perm_compose(s, 2)]);
+                RW[s] = 4.0 * WW[0][s] + WW[0][perm_compose(s, 4)] + WW[0][perm_compose(s, 3)] -
+                        2.0 * (WW[0][perm_compose(s, 5)] + WW[0][perm_compose(s, 1)] + WW[0][perm_compose(s, 2)]);
             }
             const double Dn = e_occ - en[ca + 4 * e] - en[8 + cb] - en[16 + cc];
             const double rD = 1.0 / Dn;
             double esum = 0.0;
 #pragma unroll
-            for (int s = 0; s < 6; s++) esum += WW[e][s] * Z[s];
+            for (int s = 0; s < 6; s++) esum += WW[0][s] * Z[s];
             e_loc += ok ? cen * esum * rD : 0.0;
-            dd[e] = ok ? cen * P.ybar * esum * rD * rD : 0.0;   // dE/d e_abc (minus dE/dD)
+            dd[0] = dd[1];
+            dd[1] = ok ? cen * P.ybar * esum * rD * rD : 0.0;   // dE/d e_abc (minus dE/dD)
             if (P.want_grad) {
                 const double g0 = cocc * P.ybar * rD;
                 float wb[6], vb[6];
@@ -541,7 +632,12 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
                 uint2 *g = sRes + (e == 0 ? gidx : gidx ^ 4);
 #pragma unroll
                 for (int s = 0; s < 6; s++)
-                    g[s * 512] = make_uint2(f2m_split<H>(wb[s], wscf), __float_as_uint(vb[s]));
+                    g[s * 512] = make_uint2(f2m_split<H>(wb[s], it.wscale), __float_as_uint(vb[s]));
+            }
+#pragma unroll
+            for (int s = 0; s < 6; s++) {
+                WW[0][s] = WW[1][s];
+                VV[0][s] = VV[1][s];
             }
         }
         // per-warp partials: dE/d e_c (lanes 0-3), e_b (0, 4, 8, 12), e_a and e_(a+4), energy
@@ -566,6 +662,9 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
             if (lane == 0) s_part[warp][12] = e_loc;
         }
         f2m_bar(2);   // results and partials visible
+        // (these warps take fewer regions below)
+        if (warp == 1 && more) issue_tables(s_item[(k & 1) ^ 1], tb_ ^ 1);
+        if (warp == 2 && s_next[(k & 1) ^ 1] < nitems) announce(s_next[(k & 1) ^ 1], k & 1);
         if (warp == 0) {
             // warps with bit 0, 1, 2 = bit 2 of c, bit 2 of b, bit 1 of a
             double acc = 0.0;
@@ -584,7 +683,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
             tot += __shfl_xor_sync(0xffffffffu, tot, 1);
             tot += __shfl_xor_sync(0xffffffffu, tot, 2);
             tot += __shfl_xor_sync(0xffffffffu, tot, 4);
-            if (lane == 24) P.e_part[(long long)sub * P.n_ijk + rep] = tot;
+            if (lane == 24) P.e_part[(long long)it.sub * P.n_ijk + it.rep] = tot;
             if (P.want_grad) {
                 const int slot = 2 - (lane >> 3), l = lane & 7;
                 if (lane < 24 && l < sel3(l0, l1, l2, slot))
@@ -595,26 +694,26 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
 
         if (P.want_grad) {
             // ---- write-back: a region per warp, runs (yy, xx) of lane and u ----
-            const int nro = f2m_nlead(opat), ntask = f2m_nlead(vpat) * nro;
             const int xx = lane & 7, h3 = (lane >> 3) & 1, h4 = lane >> 4;
             const int ys0 = plain ? 2 * h3 + 4 * h4 : h3 + 2 * h4, ydu = plain ? 1 : 4;
 #pragma unroll 1
-            for (int task = 7 - warp; task < ntask; task += 8) {   // warps 0 and 1 have other work too
-                const int pi = f2m_lead(vpat, task / nro), rho = f2m_lead(opat, task % nro);
-                const unsigned code = s_task[pi * 6 + rho];
-                const int pp[3] = {(int)(code & 3u), (int)((code >> 2) & 3u), (int)((code >> 4) & 3u)};
-                const int pr[3] = {(int)((code >> 6) & 3u), (int)((code >> 8) & 3u), (int)((code >> 10) & 3u)};
-                const int s = (int)(code >> 12);
-                const int p = sel3(i0, i1, i2, pr[0]), q = sel3(i0, i1, i2, pr[1]), r = sel3(i0, i1, i2, pr[2]);
-                const int lx = sel3(l0, l1, l2, pp[0]), ly = sel3(l0, l1, l2, pp[1]), lz = sel3(l0, l1, l2, pp[2]);
+            for (int task = warp, next; task < ntask; task = next) {
+                next = 0;
+                if (lane == 0) next = 8 + (int)atomicAdd(&s_tasks[k & 1], 1u);   // further ones in order of arrival
+                next = __shfl_sync(0xffffffffu, next, 0);
+                const F2mTask T = s_rec[task];
+                const int pi = T.code & 7u, rho = (T.code >> 3) & 7u;
+                const int pp[3] = {(int)((T.code >> 6) & 3u), (int)((T.code >> 8) & 3u), (int)((T.code >> 10) & 3u)};
+                const int s = (T.code >> 12) & 7u, pr2 = (T.code >> 15) & 3u;
+                const int lx = (T.code >> 17) & 15u, ly = (T.code >> 21) & 15u, lz = (T.code >> 25) & 15u;
                 const uint8_t *plane = reinterpret_cast<const uint8_t *>(sRes + s * 512);
                 const int gx = s_res[pp[0]][xx];
                 const int4 za = *reinterpret_cast<const int4 *>(&s_res[pp[2]][0]);
                 const int4 zb = *reinterpret_cast<const int4 *>(&s_res[pp[2]][4]);
                 const int zo[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
                 const F2mPi &D = R.pi[pi];
-                const long long wl = f2m_wbar(D, p, q, r) + (long long)xx * D.wx;
-                const float2 *trow = tf + (pr[2] * 3 + pp[2]) * 8;
+                uint16_t *const wl = T.w + (long long)xx * D.wx;
+                const float2 *trow = tf + (pr2 * 3 + pp[2]) * 8;
                 float2 trz[8];
                 if (R.full) {
 #pragma unroll
@@ -650,7 +749,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
                     hi.z = __byte_perm(pk[4], pk[5], 0x5410); lo.z = __byte_perm(pk[4], pk[5], 0x7632);
                     hi.w = __byte_perm(pk[6], pk[7], 0x5410); lo.w = __byte_perm(pk[6], pk[7], 0x7632);
                     if (xx < lx && yy < ly) {
-                        uint16_t *dst = P.SW + wl + (long long)yy * D.wy;
+                        uint16_t *dst = wl + (long long)yy * D.wy;
                         if (lz == 8) {
                             *reinterpret_cast<uint4 *>(dst) = hi;
                             *reinterpret_cast<uint4 *>(dst + D.half) = lo;
@@ -695,8 +794,6 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
                         }
                     }
                 }
-                const int x = sel3(R.st[0], R.st[1], R.st[2], pp[0]) + xx;
-                const int y0 = sel3(R.st[0], R.st[1], R.st[2], pp[1]);
                 // row sums: lanes of one x take four consecutive y (one sector of ovov_bar)
                 int yr0 = ys0, yr1 = ys0 + ydu;
                 if (plain) {
@@ -711,15 +808,15 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
                     yr0 = 2 * h3 + h4;
                     yr1 = yr0 + 4;
                 }
-                double *ob = P.ovov_bar + (((long long)p * v + x) * o + q) * v + y0;
-                double *tb2 = P.t2_bar + (((long long)q * o + p) * v + y0) * v + x;
+                double *ob = T.ob + (long long)(xx * o) * v;
+                double *tb2 = T.tb + xx;
                 if (xx < lx && yr0 < ly) {
-                    atomicAdd(ob + yr0, (double)rs1[0]);
-                    atomicAdd(tb2 + (long long)yr0 * v, (double)rs2[0]);
+                    f2m_red(ob + yr0, rs1[0]);
+                    f2m_red(tb2 + (long long)yr0 * v, rs2[0]);
                 }
                 if (xx < lx && yr1 < ly) {
-                    atomicAdd(ob + yr1, (double)rs1[1]);
-                    atomicAdd(tb2 + (long long)yr1 * v, (double)rs2[1]);
+                    f2m_red(ob + yr1, rs1[1]);
+                    f2m_red(tb2 + (long long)yr1 * v, rs2[1]);
                 }
                 // column sums t1_bar[r, z] (values 0-7), fvo_bar[z, r] (8-15); every
                 // level adds lane pairs in the order bit 3, 2, 1, 0, 4 of the run
@@ -735,30 +832,28 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
                             col[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
                         }
                 };
+                // plain: bits 4, 2, 1, 8 (a half region per result), else 8, 4, 2, 1, then 16
+                const int sh = plain ? 1 : 0;
+                fold(8, 8 >> sh);
+                fold(4, 4 >> sh);
+                fold(2, 2 >> sh);
+                fold(1, plain ? 8 : 1);
                 if (plain) {
-                    fold(8, 4);
-                    fold(4, 2);
-                    fold(2, 1);
-                    fold(1, 8);
-                    ci = ((lane & 4) << 1) | ((lane & 2) << 1) | ((lane & 1) << 1) | h3;
+                    ci = ((lane & 7) << 1) | h3;
                 } else {
-                    fold(8, 8);
-                    fold(4, 4);
-                    fold(2, 2);
-                    fold(1, 1);
                     col[0] += __shfl_xor_sync(0xffffffffu, col[0], 16);
                     ci = lane & 15;
                     act = lane < 16;
                 }
                 if (act && (ci & 7) < lz) {
-                    const int z = sel3(R.st[0], R.st[1], R.st[2], pp[2]) + (ci & 7);
-                    if (ci < 8) atomicAdd(&P.t1_bar[(long long)r * v + z], (double)col[0]);
-                    else atomicAdd(&P.fvo_bar[(long long)z * o + r], (double)col[0]);
+                    const int r = T.rz & 0xffffu, z = (int)(T.rz >> 16) + (ci & 7);
+                    if (ci < 8) f2m_red(&P.t1_bar[(long long)r * v + z], col[0]);
+                    else f2m_red(&P.fvo_bar[(long long)z * o + r], col[0]);
                 }
             }
         }
         if (!more) break;
-        cur = nxt;
+        cur = s_item[(k & 1) ^ 1];
     }
 }
 
