@@ -65,6 +65,14 @@ struct PermBlock {
     long long swoff;       // offset of Wbar_tau (values) in the Wbar buffer
 };
 
+// *p += v in global memory.  atomicAdd through a pointer that the compiler does not
+// know to be global (one read from a job table or from shared memory) first tests for
+// shared memory and carries the code for it: 265 to 242 ms of the mixed epilogue at
+// nocc 20 nvir 180.
+__device__ __forceinline__ void red_add(double *p, double v) {
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
+}
+
 // 16-bit Wbar_tau: blocks of at least 8 x values are stored as 8 x 8 tiles
 // [h][y][q][p][x / 8][rz / 8][x % 8][rz % 8] (rz = r Tz + z), smaller ones as rows
 // [h][y][p][x][q][rz].  A tile is one 128-byte line, the 8 z runs of eight x that

@@ -202,8 +202,8 @@ __device__ __forceinline__ void f2_dd_add(double (*s_part)[12], const F2mSub &R,
     tot += __shfl_xor_sync(0x00ffffffu, tot, 4);
     const int slot = 2 - (lane >> 3);
     if (l < sel3(R.len[0], R.len[1], R.len[2], slot))
-        atomicAdd(&mo_bar[o + sel3(R.st[0], R.st[1], R.st[2], slot) + l], -acc);
-    if (lane < 3) atomicAdd(&mo_bar[sel3(i0, i1, i2, lane)], tot);
+        red_add(&mo_bar[o + sel3(R.st[0], R.st[1], R.st[2], slot) + l], -acc);
+    if (lane < 3) red_add(&mo_bar[sel3(i0, i1, i2, lane)], tot);
 }
 
 // Write-back of the element results sW, sV (planes of 512 in f2m_res order): the
@@ -296,16 +296,16 @@ __device__ __forceinline__ void f2_writeback(const ARGS &A, const F2mSub &R, int
                 col[8 + z] += vb * ot.y;
             }
             if (in) {
-                atomicAdd(&A.ovov_bar[(((long long)p * v + x) * o + q) * v + y0 + yy], r1);
-                atomicAdd(&A.t2_bar[(((long long)q * o + p) * v + y0 + yy) * v + x], r2);
+                red_add(&A.ovov_bar[(((long long)p * v + x) * o + q) * v + y0 + yy], r1);
+                red_add(&A.t2_bar[(((long long)q * o + p) * v + y0 + yy) * v + x], r2);
             }
         }
         // column sums t1_bar[r, z] (values 0-7), fvo_bar[z, r] (8-15) over the region's runs
         const double cv = group_reduce_scatter<16, 32>(col, lane);
         if (lane < 16 && (lane & 7) < lz) {
             const int z = sel3(R.st[0], R.st[1], R.st[2], pp[2]) + (lane & 7);
-            if (lane < 8) atomicAdd(&A.t1_bar[(long long)r * v + z], cv);
-            else atomicAdd(&A.fvo_bar[(long long)z * o + r], cv);
+            if (lane < 8) red_add(&A.t1_bar[(long long)r * v + z], cv);
+            else red_add(&A.fvo_bar[(long long)z * o + r], cv);
         }
     }
 }

@@ -264,10 +264,6 @@ __device__ __noinline__ void f2m_issue(const F2mLoad *L, int rho, int n, float *
     if (lane == 0) mbar_arrive(&full[st]);
 }
 
-__device__ __forceinline__ void f2m_red(double *p, float v) {
-    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"((double)v) : "memory");
-}
-
 __device__ __forceinline__ void f2m_bar(int id) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kF2mThreads) : "memory");
 }
@@ -687,8 +683,8 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
             if (P.want_grad) {
                 const int slot = 2 - (lane >> 3), l = lane & 7;
                 if (lane < 24 && l < sel3(l0, l1, l2, slot))
-                    atomicAdd(&P.mo_bar[o + sel3(R.st[0], R.st[1], R.st[2], slot) + l], acc);
-                if (lane >= 16 && lane < 19) atomicAdd(&P.mo_bar[sel3(i0, i1, i2, lane - 16)], -tot);
+                    red_add(&P.mo_bar[o + sel3(R.st[0], R.st[1], R.st[2], slot) + l], acc);
+                if (lane >= 16 && lane < 19) red_add(&P.mo_bar[sel3(i0, i1, i2, lane - 16)], -tot);
             }
         }
 
@@ -811,12 +807,12 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
                 double *ob = T.ob + (long long)(xx * o) * v;
                 double *tb2 = T.tb + xx;
                 if (xx < lx && yr0 < ly) {
-                    f2m_red(ob + yr0, rs1[0]);
-                    f2m_red(tb2 + (long long)yr0 * v, rs2[0]);
+                    red_add(ob + yr0, rs1[0]);
+                    red_add(tb2 + (long long)yr0 * v, rs2[0]);
                 }
                 if (xx < lx && yr1 < ly) {
-                    f2m_red(ob + yr1, rs1[1]);
-                    f2m_red(tb2 + (long long)yr1 * v, rs2[1]);
+                    red_add(ob + yr1, rs1[1]);
+                    red_add(tb2 + (long long)yr1 * v, rs2[1]);
                 }
                 // column sums t1_bar[r, z] (values 0-7), fvo_bar[z, r] (8-15); every
                 // level adds lane pairs in the order bit 3, 2, 1, 0, 4 of the run
@@ -847,8 +843,8 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
                 }
                 if (act && (ci & 7) < lz) {
                     const int r = T.rz & 0xffffu, z = (int)(T.rz >> 16) + (ci & 7);
-                    if (ci < 8) f2m_red(&P.t1_bar[(long long)r * v + z], col[0]);
-                    else f2m_red(&P.fvo_bar[(long long)z * o + r], col[0]);
+                    if (ci < 8) red_add(&P.t1_bar[(long long)r * v + z], col[0]);
+                    else red_add(&P.fvo_bar[(long long)z * o + r], col[0]);
                 }
             }
         }

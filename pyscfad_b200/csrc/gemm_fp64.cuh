@@ -197,7 +197,7 @@ __device__ __forceinline__ void gemm_fp64_tile(const GemmArgs &g, int m0, int n0
                 const int nl = wn0 + 8 * j + 2 * ft + c;
                 if (n0 + nl >= g.N) continue;
                 const double val = g.alpha * acc[i][j][c];
-                if (g.atomic) atomicAdd(row + outN[nl], val);
+                if (g.atomic) red_add(row + outN[nl], val);
                 else row[outN[nl]] = val;
             }
     }

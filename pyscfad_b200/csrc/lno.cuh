@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
             for (int h = 0; h < 2; h++) {
                 const int i = (gt % o8) * 8 + 2 * ft + h;
                 const double gv = h ? acc[k][1] : acc[k][0];
-                if (l < o && i < o && gv != 0.0) atomicAdd(&A.mat_bar[l * o + i], gy * gv);
+                if (l < o && i < o && gv != 0.0) red_add(&A.mat_bar[l * o + i], gy * gv);
             }
         }
     }

@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
 #pragma unroll
                     for (int j = 0; j < HC; j++) {
                         const int col = (j >> 3) * 16 + (j & 7);
-                        if (col < lim) atomicAdd(g + col, sc * (double)acc[j]);
+                        if (col < lim) red_add(g + col, sc * (double)acc[j]);
                     }
                 }
 #pragma unroll
