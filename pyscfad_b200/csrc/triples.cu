@@ -557,19 +557,73 @@ __global__ void k_lno_mat_norms(const double *__restrict__ mat, int o, Ctrl *ctr
     }
 }
 
+// Tile (row block fb >= column block yb) of a triangle of nb x nb blocks, for each px
+__device__ __forceinline__ void tri_tile(long long t, int nb, long long &px, int &fb, int &yb) {
+    const int per = nb * (nb + 1) / 2;
+    px = t / per;
+    const int e = (int)(t - px * per);
+    fb = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+    while (fb * (fb + 1) / 2 > e) fb--;
+    while ((fb + 1) * (fb + 2) / 2 <= e) fb++;
+    yb = e - fb * (fb + 1) / 2;
+}
+
+// The same operand from the packed layout: a block reads a 64 x 64 tile f0 >= y0 of
+// the triangle of one (p, x) once, rows of 512 bytes, and writes it both ways.
+// Bound by HBM (nocc 40 nvir 360: 5.9 to 4.9 ms;
+// with 32 x 32 tiles of both triangles half of the reads ran down columns).
 template <typename H>
-__global__ void k_prep_A1h(const double *__restrict__ ovvv, int packed, Dims d, int Kp8,
-                           const Ctrl *ctrl, H *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_prep_A1h_packed(const double *__restrict__ ovvv, Dims d, int Kp8,
+                                                         const Ctrl *ctrl, H *__restrict__ out) {
+    __shared__ double tile[64][65];
+    int fb, yb;
+    long long px;
+    tri_tile(blockIdx.x, (Kp8 + 63) / 64, px, fb, yb);
+    const int f0 = fb * 64, y0 = yb * 64, lane = threadIdx.x & 63, row = threadIdx.x >> 6;
+    const double sA = ctrl->scale[0];
+    const double *src = ovvv + px * ((long long)d.v * (d.v + 1) / 2);
+#pragma unroll 4
+    for (int r = row; r < 64; r += 4) {
+        const int f = f0 + r, y = y0 + lane;
+        double val = 0.0;
+        if (f < d.v && y <= f) {
+            val = src[(long long)f * (f + 1) / 2 + y] * sA;
+            if (fb == yb) tile[lane][r] = val;   // the diagonal tile holds both triangles
+        }
+        if (fb != yb || y <= f || f >= d.v) tile[r][lane] = val;
+    }
+    __syncthreads();
+    const long long half = (long long)d.v * d.o * d.v * Kp8;
+    for (int pass = 0; pass < (fb == yb ? 1 : 2); pass++) {
+        // rows of the first pass are y with f along the lanes, of the second f with y along them
+        const int a0 = pass ? f0 : y0, b0 = pass ? y0 : f0;
+        const int b = b0 + lane;
+#pragma unroll 4
+        for (int r = row; r < 64; r += 4) {
+            const int a = a0 + r;
+            if (a < d.v && b < Kp8) {
+                H hi, lo;
+                split16<H>(pass ? tile[r][lane] : tile[lane][r], hi, lo);
+                const long long e = ((long long)a * d.o * d.v + px) * Kp8 + b;
+                out[e] = hi;
+                out[half + e] = lo;
+            }
+        }
+    }
+}
+
+template <typename H>
+__global__ void k_prep_A1h(const double *__restrict__ ovvv, Dims d, int Kp8, const Ctrl *ctrl,
+                           H *__restrict__ out) {
     __shared__ double tile[32][33];
     const long long px = blockIdx.z;
     const int f0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-    const long long npair = (long long)d.v * (d.v + 1) / 2;
     const double sA = ctrl->scale[0];
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         int f = f0 + r, y = y0 + threadIdx.x;
         double val = 0.0;
         if (f < d.v && y < d.v)
-            val = packed ? ovvv[px * npair + tri_index(f, y)] : ovvv[(px * d.v + f) * d.v + y];
+            val = ovvv[(px * d.v + f) * d.v + y];
         tile[r][threadIdx.x] = val;
     }
     __syncthreads();
@@ -627,25 +681,43 @@ __global__ void k_prep_A2h(const double *__restrict__ ovoo, Dims d, int Op8, con
     }
 }
 
-// B2h[h][y][r][z][m] = split(t2[r,m,z,y] * sB), m < Op8
+// The tile of a block in an (m, y) transposition for each (r, z): 64 m by 64 y
+__device__ __forceinline__ void rz_tile(const Dims &d, int nm, int &r, int &z, int &m0, int &y0) {
+    const int nmb = (nm + 63) / 64, nyb = (d.v + 63) / 64;
+    long long t = blockIdx.x;
+    m0 = (int)(t % nmb) * 64;
+    t /= nmb;
+    y0 = (int)(t % nyb) * 64;
+    t /= nyb;
+    z = (int)(t % d.v);
+    r = (int)(t / d.v);
+}
+
+// B2h[h][y][r][z][m] = split(t2[r,m,z,y] * sB), m < Op8.  Through a tile in shared
+// memory, so that reads run along y and writes along m: bound by HBM (a thread per
+// output element read sectors for one value each, nocc 40 nvir 360: 4.5 ms; now 0.8).
 template <typename H>
-__global__ void k_prep_B2h(const double *__restrict__ t2, Dims d, int Op8, const Ctrl *ctrl,
-                           H *__restrict__ out) {
-    const long long total = (long long)d.v * d.o * d.v * Op8;
+__global__ void __launch_bounds__(256) k_prep_B2h(const double *__restrict__ t2, Dims d, int Op8, const Ctrl *ctrl,
+                                                  H *__restrict__ out) {
+    __shared__ double tile[64][65];
+    int r, z, m0, y0;
+    rz_tile(d, Op8, r, z, m0, y0);
+    const int lane = threadIdx.x & 63, row = threadIdx.x >> 6;
     const double sB = ctrl->scale[1];
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        int m = e % Op8;
-        long long t = e / Op8;
-        int z = t % d.v;
-        t /= d.v;
-        int r = t % d.o;
-        int y = t / d.o;
-        double val = m < d.o ? t2[(((long long)r * d.o + m) * d.v + z) * d.v + y] * sB : 0.0;
+    const int mn = min(64, Op8 - m0), yn = min(64, d.v - y0);
+    for (int k = row; k < mn; k += 4) {
+        const int m = m0 + k;
+        tile[k][lane] = (m < d.o && lane < yn) ? t2[(((long long)r * d.o + m) * d.v + z) * d.v + y0 + lane] * sB : 0.0;
+    }
+    __syncthreads();
+    const long long half = (long long)d.v * d.o * d.v * Op8;
+    for (int e = threadIdx.x; e < yn * mn; e += 256) {
+        const int k = e % mn, yl = e / mn;
         H hi, lo;
-        split16<H>(val, hi, lo);
-        out[e] = hi;
-        out[total + e] = lo;
+        split16<H>(tile[k][yl], hi, lo);
+        const long long at = (((long long)(y0 + yl) * d.o + r) * d.v + z) * Op8 + m0 + k;
+        out[at] = hi;
+        out[half + at] = lo;
     }
 }
 
@@ -777,40 +849,55 @@ __global__ void k_fold_ovvv_full(const double *__restrict__ GA1, Dims d, double 
 }
 
 // packed ovvv_bar[p,x,tri(f,y)] = G[f,y] + G[y,f] (f != y), G[f,f]; G[f,y] = G_A1[y][p][x][f]
-// (pyscfad/cc/ccsd_t.py:184-191)
-__global__ void k_fold_ovvv_packed(const double *__restrict__ GA1, Dims d, double *__restrict__ out) {
-    const long long npair = (long long)d.v * (d.v + 1) / 2;
-    const long long total = (long long)d.o * d.v * npair;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const long long px = e / npair;
-        const long long ij = e % npair;
-        int f = (int)((sqrt(8.0 * (double)ij + 1.0) - 1.0) * 0.5);
-        while ((long long)f * (f + 1) / 2 > ij) f--;
-        while ((long long)(f + 1) * (f + 2) / 2 <= ij) f++;
-        const int y = (int)(ij - (long long)f * (f + 1) / 2);
-        const long long sy = (long long)d.o * d.v * d.Kp;
-        double val = GA1[y * sy + px * d.Kp + f];
-        if (f != y) val += GA1[(long long)f * sy + px * d.Kp + y];
-        out[e] = val;
+// (pyscfad/cc/ccsd_t.py:184-191).  A block takes a 64 x 64 tile f0 >= y0 of one
+// (p, x): rows of 512 bytes of both triangles, G[f,y] transposed in shared
+// memory.  Bound by HBM.  One element per thread, without tiles, read G[f,y]
+// with a lane per y (nocc 40 nvir 360: 22 to 4.8 ms).
+__global__ void __launch_bounds__(256) k_fold_ovvv_packed(const double *__restrict__ GA1, Dims d,
+                                                          double *__restrict__ out) {
+    __shared__ double tile[64][65];
+    int fb, yb;
+    long long px;
+    tri_tile(blockIdx.x, (d.v + 63) / 64, px, fb, yb);
+    const int f0 = fb * 64, y0 = yb * 64, lane = threadIdx.x & 63, row = threadIdx.x >> 6;
+    const long long sy = (long long)d.o * d.v * d.Kp, npair = (long long)d.v * (d.v + 1) / 2;
+    const double *src = GA1 + px * d.Kp;
+#pragma unroll 4
+    for (int r = row; r < 64; r += 4) {
+        const int y = y0 + r, f = f0 + lane;
+        tile[r][lane] = (y < d.v && f < d.v) ? src[y * sy + f] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int r = row; r < 64; r += 4) {
+        const int f = f0 + r, y = y0 + lane;
+        if (f < d.v && y <= f) {
+            const double val = tile[lane][r] + (f != y ? src[f * sy + y] : 0.0);
+            out[px * npair + (long long)f * (f + 1) / 2 + y] = val;
+        }
     }
 }
 
-// t2_bar[r,q,z,f] += G_B1[q][r][z][f] + G_B2[f][r][z][q]
-__global__ void k_fold_t2(const double *__restrict__ GB1, const double *__restrict__ GB2, Dims d,
-                          double *__restrict__ t2_bar) {
-    const long long total = (long long)d.o * d.o * d.v * d.v;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int f = e % d.v;
-        long long t = e / d.v;
-        const int z = t % d.v;
-        t /= d.v;
-        const int q = t % d.o;
-        const int r = t / d.o;
-        t2_bar[e] += GB1[(((long long)q * d.o + r) * d.v + z) * d.Kp + f] +
-                     GB2[(((long long)f * d.o + r) * d.v + z) * d.o + q];
+// t2_bar[r,q,z,f] += G_B1[q][r][z][f] + G_B2[f][r][z][q].  G_B2 through a tile in
+// shared memory: read along q, added along f (nocc 40 nvir 360: 5.1 to 1.5 ms).
+__global__ void __launch_bounds__(256) k_fold_t2(const double *__restrict__ GB1, const double *__restrict__ GB2, Dims d,
+                                                 double *__restrict__ t2_bar) {
+    __shared__ double tile[64][65];
+    int r, z, q0, f0;
+    rz_tile(d, d.o, r, z, q0, f0);
+    const int lane = threadIdx.x & 63, row = threadIdx.x >> 6;
+    const int qn = min(64, d.o - q0), fn = min(64, d.v - f0);
+    for (int e = threadIdx.x; e < fn * qn; e += 256) {
+        const int k = e % qn, fl = e / qn;
+        tile[k][fl] = GB2[(((long long)(f0 + fl) * d.o + r) * d.v + z) * d.o + q0 + k];
     }
+    __syncthreads();
+    if (lane < fn)
+        for (int k = row; k < qn; k += 4) {
+            const int q = q0 + k, f = f0 + lane;
+            t2_bar[(((long long)r * d.o + q) * d.v + z) * d.v + f] +=
+                GB1[(((long long)q * d.o + r) * d.v + z) * d.Kp + f] + tile[k][lane];
+        }
 }
 
 // ovoo_bar[p,x,m,q] = G_A2[q][p][x][m]
@@ -833,6 +920,17 @@ __global__ void k_copy_scalar(const double *src, double *dst) { dst[0] = src[0];
 // ---------------------------------------------------------------------------
 // driver
 // ---------------------------------------------------------------------------
+// 64 x 64 tiles of the triangle of an n x n block, for each of `count` (p, x)
+static inline unsigned tri_grid(int n, size_t count) {
+    const int nb = (n + 63) / 64;
+    return (unsigned)((size_t)nb * (nb + 1) / 2 * count);
+}
+
+// 64 x 64 tiles of (m < nm, y < nvir) for each (r, z)
+static inline unsigned rz_grid(const Dims &d, int nm) {
+    return (unsigned)((size_t)((nm + 63) / 64) * ((d.v + 63) / 64) * d.o * d.v);
+}
+
 static inline unsigned grid1d(long long n, int threads) {
     long long b = (n + threads - 1) / threads;
     if (b > 148 * 64) b = 148 * 64;
@@ -1557,22 +1655,30 @@ static int prep_launches(const Plan &P, cudaStream_t st, const TriplesIO &io) {
         TB_KLAUNCH(P_PREP, k_absmax<<<grid1d((long long)o * v, 256), 256, 0, st>>>(io.fvo, (long long)o * v, &ctrl->absmax[5]));
         TB_KLAUNCH(P_PREP, k_make_scales<<<1, 1, 0, st>>>(ctrl, bf16 ? 0 : 1));
         if (bf16) {
-            TB_KLAUNCH(P_PREP, k_prep_A1h<__nv_bfloat16><<<dim3((P.Kp8 + 31) / 32, (d.v + 31) / 32, (unsigned)(o * v)), dim3(32, 8), 0, st>>>(
-                io.ovvv, P.packed, d, P.Kp8, ctrl, (__nv_bfloat16 *)(ws + P.off_A1h)));
+            if (P.packed)
+                TB_KLAUNCH(P_PREP, k_prep_A1h_packed<__nv_bfloat16><<<tri_grid(P.Kp8, o * v), 256, 0, st>>>(
+                    io.ovvv, d, P.Kp8, ctrl, (__nv_bfloat16 *)(ws + P.off_A1h)));
+            else
+                TB_KLAUNCH(P_PREP, k_prep_A1h<__nv_bfloat16><<<dim3((P.Kp8 + 31) / 32, (d.v + 31) / 32, (unsigned)(o * v)), dim3(32, 8), 0, st>>>(
+                    io.ovvv, d, P.Kp8, ctrl, (__nv_bfloat16 *)(ws + P.off_A1h)));
             TB_KLAUNCH(P_PREP, k_prep_B1h<__nv_bfloat16><<<(unsigned)(o * o * v), 128, 0, st>>>(io.t2, d, P.Kp8, ctrl,
                                                                             (__nv_bfloat16 *)(ws + P.off_B1h)));
             TB_KLAUNCH(P_PREP, k_prep_A2h<__nv_bfloat16><<<grid1d((long long)o * o * v * P.Op8, 256), 256, 0, st>>>(
                 io.ovoo, d, P.Op8, ctrl, (__nv_bfloat16 *)(ws + P.off_A2h)));
-            TB_KLAUNCH(P_PREP, k_prep_B2h<__nv_bfloat16><<<grid1d((long long)v * o * v * P.Op8, 256), 256, 0, st>>>(
+            TB_KLAUNCH(P_PREP, k_prep_B2h<__nv_bfloat16><<<rz_grid(d, P.Op8), 256, 0, st>>>(
                 io.t2, d, P.Op8, ctrl, (__nv_bfloat16 *)(ws + P.off_B2h)));
         } else {
-            TB_KLAUNCH(P_PREP, k_prep_A1h<__half><<<dim3((P.Kp8 + 31) / 32, (d.v + 31) / 32, (unsigned)(o * v)), dim3(32, 8), 0, st>>>(
-                io.ovvv, P.packed, d, P.Kp8, ctrl, (__half *)(ws + P.off_A1h)));
+            if (P.packed)
+                TB_KLAUNCH(P_PREP, k_prep_A1h_packed<__half><<<tri_grid(P.Kp8, o * v), 256, 0, st>>>(
+                    io.ovvv, d, P.Kp8, ctrl, (__half *)(ws + P.off_A1h)));
+            else
+                TB_KLAUNCH(P_PREP, k_prep_A1h<__half><<<dim3((P.Kp8 + 31) / 32, (d.v + 31) / 32, (unsigned)(o * v)), dim3(32, 8), 0, st>>>(
+                    io.ovvv, d, P.Kp8, ctrl, (__half *)(ws + P.off_A1h)));
             TB_KLAUNCH(P_PREP, k_prep_B1h<__half><<<(unsigned)(o * o * v), 128, 0, st>>>(io.t2, d, P.Kp8, ctrl,
                                                                      (__half *)(ws + P.off_B1h)));
             TB_KLAUNCH(P_PREP, k_prep_A2h<__half><<<grid1d((long long)o * o * v * P.Op8, 256), 256, 0, st>>>(
                 io.ovoo, d, P.Op8, ctrl, (__half *)(ws + P.off_A2h)));
-            TB_KLAUNCH(P_PREP, k_prep_B2h<__half><<<grid1d((long long)v * o * v * P.Op8, 256), 256, 0, st>>>(
+            TB_KLAUNCH(P_PREP, k_prep_B2h<__half><<<rz_grid(d, P.Op8), 256, 0, st>>>(
                 io.t2, d, P.Op8, ctrl, (__half *)(ws + P.off_B2h)));
         }
         if (P.vtables) {
@@ -1597,14 +1703,13 @@ static int fold_launches(const Plan &P, cudaStream_t st, const TriplesIO &io) {
     const size_t o = d.o, v = d.v;
     if (P.want_grad) {
         if (P.packed) {
-            TB_KLAUNCH(P_FOLD, k_fold_ovvv_packed<<<grid1d((long long)o * v * (v * (v + 1) / 2), 256), 256, 0, st>>>(
-                GA1, d, io.ovvv_bar));
+            TB_KLAUNCH(P_FOLD, k_fold_ovvv_packed<<<tri_grid(d.v, o * v), 256, 0, st>>>(GA1, d, io.ovvv_bar));
         } else {
             TB_KLAUNCH(P_FOLD, k_fold_ovvv_full<<<dim3((d.v + 31) / 32, (d.v + 31) / 32, (unsigned)(o * v)), dim3(32, 8), 0, st>>>(
                 GA1, d, io.ovvv_bar));
         }
         TB_LAUNCH_CHECK();
-        TB_KLAUNCH(P_FOLD, k_fold_t2<<<grid1d((long long)o * o * v * v, 256), 256, 0, st>>>(GB1, GB2, d, io.t2_bar));
+        TB_KLAUNCH(P_FOLD, k_fold_t2<<<rz_grid(d, d.o), 256, 0, st>>>(GB1, GB2, d, io.t2_bar));
         TB_KLAUNCH(P_FOLD, k_fold_ovoo<<<grid1d((long long)o * v * o * o, 256), 256, 0, st>>>(GA2, d, io.ovoo_bar));
     }
     TB_KLAUNCH(P_FOLD, k_copy_scalar<<<1, 1, 0, st>>>(&ctrl->e_acc, io.e_out));

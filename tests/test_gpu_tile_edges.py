@@ -107,3 +107,24 @@ def test_adjoint_tiles(o, v, tv, precision):
     assert abs(float(e) - float(e0)) <= e_tol * abs(float(e0))
     for k in G.KEYS:
         assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < g_tol, k
+
+
+# The 64 x 64 tiles in which a packed ovvv is split and its gradient folded, and in
+# which t2 is transposed and its gradient folded (nocc 66: a second tile): one short
+# of a tile, exact, one past, several.  The packed and the full ovvv hold the same
+# values, so the results differ by the order of FP64 sums.
+@pytest.mark.parametrize("o,v", [(2, 63), (2, 64), (3, 65), (2, 130), (66, 2)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed_bf16"])
+def test_packed_layout_tiles(o, v, precision):
+    inp = make_inputs(o, v, 40, seed=v, fvo_sigma=1e-3)
+    ins = {k: getattr(inp, k) for k in G.KEYS}
+    e0, g0 = triples.energy_vjp(**ins, precision=precision, device="cuda")
+    e, g = triples.energy_vjp(**dict(ins, ovvv=inp.ovvv_tril()), precision=precision, device="cuda")
+    assert abs(float(e) - float(e0)) <= 1e-12 * abs(float(e0))
+    full = g0["ovvv"].cpu().numpy()
+    il, jl = np.tril_indices(v)
+    fold = full[:, :, il, jl] + np.where(il != jl, full[:, :, jl, il], 0.0)
+    assert _relerr(g["ovvv"].cpu().numpy(), fold) < 1e-11
+    for k in G.KEYS:
+        if k != "ovvv":
+            assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-11, k
