@@ -56,10 +56,10 @@ constexpr int kB1Threads = 320;   // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 // K <= 512 * 64 keep the rounding of the sum well below the fp16 split error
 constexpr int kB1RunSegments = 512;
 
-// N tiles are nw = 16 n columns wide: nvir (kinds 0, 1) or nocc (2, 3) split
-// evenly over the fewest tiles of at most BN and rounded up to 16, so that nvir
-// 180 takes two tiles of 96 where fixed 128-wide tiles padded it to 256.  K
-// blocks issue only the 16-wide steps that hold values.
+// N tiles are nw = 16 n columns wide: nvir (kinds 0, 1) or nocc (2, 3) rounded up
+// to 16, or BN and a narrower last tile (nvir 180: 128 + 64; two of 96 took a
+// 64-column load more per K block: ovvv and t2 kinds 197 to 183 ms at nocc 20).
+// K blocks issue only the 16-wide steps that hold values.
 template <bool A_MN, int BN>
 struct TcB1Cfg {
     static constexpr int A_BYTES = kTcBM * kTcBK * 2;
@@ -150,6 +150,9 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
         rem %= per_batch;
         mt = rem / P.ntile_n;
         nt = rem % P.ntile_n;
+        // the column tiles of a row block are neighbours; their order turns with every round of
+        // the grid, or a CTA could meet the last, narrower one each time
+        if (P.ntile_n > 1) nt = (nt + t / P.ntile_n / max((int)gridDim.x / P.ntile_n, 1)) % P.ntile_n;
     };
 
     if (warp == 0) {

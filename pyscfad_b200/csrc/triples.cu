@@ -1541,8 +1541,7 @@ static int b1_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, con
         const int most = kind <= 1 ? 128 : 64;
         B.ncol = kind <= 1 ? d.v : d.o;
         B.ntile_n = (B.ncol + most - 1) / most;
-        B.nw = ((B.ncol + B.ntile_n - 1) / B.ntile_n + 15) / 16 * 16;
-        B.ntile_n = (B.ncol + B.nw - 1) / B.nw;
+        B.nw = B.ntile_n > 1 ? most : (B.ncol + 15) / 16 * 16;
     }
     B.G = (double *)(ws + (kind == 0 ? P.off_GA1 : kind == 1 ? P.off_GB1 : kind == 2 ? P.off_GA2 : P.off_GB2));
     B.oscale = &ctrl->scale[(kind == 0 || kind == 2) ? 1 : 0];
