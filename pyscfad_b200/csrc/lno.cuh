@@ -136,24 +136,29 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_fwd(const __grid_constan
 // ---------------------------------------------------------------------------
 // Rows: all o values of the slot, a row stride apart; columns: the other two
 // occupied indices and e, COLS at a time (consecutive e).  Per tile
-//   PW[i] = sum_l mat[l,i] WW[l],  energy += PW Q,  PQ[l] = sum_i mat[l,i] Q[i],
-//   Gram += WW Q^T
+//   PW[i] = sum_l mat[l,i] WW[l],  PQ[l] = sum_i mat[l,i] Q[i],  Gram += WW Q^T
+// and at the end energy = <mat, Gram> (= sum PW Q)
 // on the FP64 tensor cores (per 8x8 output tile a thread holds D[g][2t],
 // D[g][2t+1], A[g][t] and B[t][g] of each k-step, g = lane / 4, t = lane % 4).
 // FIRST: PW and PQ are stored, else added to; slot 0 runs last and forms Zbar
 // and f PQ.  Streams WW, Q and the running sums: HBM; wide tiles at small o and the
 // running sums loaded before the tile's copies are waited for keep enough bytes
-// in flight.  The Gram tiles belong to warps; every CTA adds its o x o sums to
-// mat_bar once, so the grid is what is resident (those atomics all meet on o^2
-// addresses: with the columns of four Gram tiles split over eight warps the
-// kernel took twice as long).
+// in flight.  The running sums are the accumulators, and a warp's fragments serve
+// all its rows and columns.  Up to four Gram tiles are shared by the eight warps
+// by columns, in two chains each; the shares are added in shared memory, since
+// every CTA adds its o x o sums to mat_bar and those atomics all meet on o^2
+// addresses (added there share by share the kernel took twice as long; the grid
+// is what is resident for the same reason).  Nocc 14 nvir 96: 20.7 to 17.3 ms of
+// a call against a tile at a time, energies from PW and a Gram tile per warp.
 template <int COLS>
 struct LnoProj {
     static constexpr int LD = COLS + 4;   // conflict-free fragment loads
     static constexpr int MAXO = 2048 / COLS;                      // 16, 32, 64
     static constexpr int NG = (MAXO / 8) * (MAXO / 8);            // Gram tiles
     static constexpr int GW = NG < kLnoThreads / 32 ? 1 : NG / (kLnoThreads / 32);   // Gram tiles per warp
-    static constexpr int TW = (MAXO / 8) * (COLS / 8) / (kLnoThreads / 32);   // output tiles per warp
+    // output tiles per warp: IT of 8 rows (every one, or every second), JT of 8 columns
+    static constexpr int JT = COLS >= 64 ? COLS / 64 : 1, IT = COLS >= 64 ? MAXO / 8 : MAXO / 16;
+    static constexpr int TW = IT * JT;
     static size_t smem(int o) {
         const int rows = (o + 7) / 8 * 8;
         return (size_t)(4 * rows * LD + o * o + kLnoMaxO + 2 * COLS) * sizeof(double);
@@ -163,7 +168,7 @@ struct LnoProj {
 template <int COLS>
 __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_constant__ LnoArgs A, int slot, int first) {
     using C = LnoProj<COLS>;
-    constexpr int LD = C::LD, CT = COLS / 8;
+    constexpr int LD = C::LD;
     extern __shared__ __align__(16) uint8_t lno_raw[];
     const int o = A.o, o4 = (o + 3) & ~3, o8 = (o + 7) / 8, rows = 8 * o8;
     double *sw_b = reinterpret_cast<double *>(lno_raw), *sq_b = sw_b + 2 * rows * LD, *sM = sq_b + 2 * rows * LD;
@@ -179,10 +184,16 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
     for (int k = threadIdx.x; k < o * o; k += blockDim.x) sM[k] = A.mat[k];
     for (int k = threadIdx.x; k < o; k += blockDim.x) s_eo[k] = A.mo_e[k];
     const int ngram = o8 * o8;
-    double acc[C::GW][2];
+    // few Gram tiles: the warps share them by columns
+    const int nks = ngram == 1 ? 8 : ngram <= 4 ? 2 : 1, ks = nks > 1 ? warp / ngram : 0;
+    const int gram0 = nks > 1 ? (warp < ngram * nks ? warp % ngram : ngram) : warp;
+    const int gc0 = ks * (COLS / nks), gc1 = gc0 + COLS / nks;
+    double acc[C::GW][2], alt[C::GW][2];   // two chains
 #pragma unroll
-    for (int k = 0; k < C::GW; k++) acc[k][0] = acc[k][1] = 0.0;
-    double en = 0.0;
+    for (int k = 0; k < C::GW; k++) acc[k][0] = acc[k][1] = alt[k][0] = alt[k][1] = 0.0;
+    // this warp's output tile k = m JT + j: rows and columns
+    auto row0 = [&](int m) -> int { return (COLS >= 64 ? m : (warp >> 2) + 2 * m) * 8; };
+    auto col0 = [&](int j) -> int { return (COLS >= 64 ? warp + 8 * j : warp & 3) * 8; };
     // first element of tile t (row 0)
     auto tile_base = [&](int t) -> long long {
         const int oth = t / per;
@@ -227,10 +238,10 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
         double2 pw[C::TW], pq[C::TW];   // running sums of this thread's output positions
 #pragma unroll
         for (int k = 0; k < C::TW; k++) {
-            const int tile = warp + k * (kLnoThreads / 32), i = tile / CT * 8 + fg;
+            const int i = row0(k / C::JT) + fg;
             pw[k] = pq[k] = double2{0.0, 0.0};
             if (grad && !first && i < o) {
-                const long long at = base + i * rstride + tile % CT * 8 + 2 * ft;
+                const long long at = base + i * rstride + col0(k % C::JT) + 2 * ft;
                 pw[k] = *reinterpret_cast<const double2 *>(A.PW + at);
                 pq[k] = *reinterpret_cast<const double2 *>(A.PQ + at);
             }
@@ -239,27 +250,35 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
         __syncthreads();
         const double *sw = sw_b + buf * rows * LD, *sq = sq_b + buf * rows * LD;
         const double *s_ecol = s_ecol_b + buf * COLS;
-#pragma unroll
-        for (int k = 0; k < C::TW; k++) {
-            const int tile = warp + k * (kLnoThreads / 32);
-            if (tile >= o8 * CT) break;
-            const int nt = tile % CT, i = tile / CT * 8 + fg, cl = nt * 8 + 2 * ft;
-            const long long at = base + i * rstride + cl;
-            double u0 = 0.0, u1 = 0.0, p0 = 0.0, p1 = 0.0;
+        if (grad) {
+#pragma unroll 1
             for (int k0 = 0; k0 < o4; k0 += 4) {
                 const int l = k0 + ft;
-                const bool in = i < o && l < o;
-                dmma_884(u0, u1, in ? sM[l * o + i] : 0.0, sw[l * LD + nt * 8 + fg]);
-                if (grad) dmma_884(p0, p1, in ? sM[i * o + l] : 0.0, sq[l * LD + nt * 8 + fg]);
+                double bw[C::JT], bq[C::JT];
+#pragma unroll
+                for (int j = 0; j < C::JT; j++) {
+                    bw[j] = sw[l * LD + col0(j) + fg];
+                    bq[j] = sq[l * LD + col0(j) + fg];
+                }
+#pragma unroll
+                for (int m = 0; m < C::IT; m++) {
+                    if (row0(m) >= o) continue;
+                    const int i = row0(m) + fg;
+                    const bool in = i < o && l < o;
+                    const double aw = in ? sM[l * o + i] : 0.0, aq = in ? sM[i * o + l] : 0.0;
+#pragma unroll
+                    for (int j = 0; j < C::JT; j++) {
+                        dmma_884(pw[m * C::JT + j].x, pw[m * C::JT + j].y, aw, bw[j]);
+                        dmma_884(pq[m * C::JT + j].x, pq[m * C::JT + j].y, aq, bq[j]);
+                    }
+                }
             }
-            if (i < o) {
-                en += u0 * sq[i * LD + cl] + u1 * sq[i * LD + cl + 1];
-                if (grad) {
+#pragma unroll
+            for (int k = 0; k < C::TW; k++) {
+                const int i = row0(k / C::JT) + fg, cl = col0(k % C::JT) + 2 * ft;
+                if (i < o) {
+                    const long long at = base + i * rstride + cl;
                     double2 w = pw[k], r = pq[k];
-                    w.x += u0;
-                    w.y += u1;
-                    r.x += p0;
-                    r.y += p1;
                     if (last) {
                         w.x = A.f * w.x / (s_eo[i] + s_ecol[cl]);
                         w.y = A.f * w.y / (s_eo[i] + s_ecol[cl + 1]);
@@ -271,21 +290,40 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
                 }
             }
         }
-        if (grad) {
-            // Gram[l, i] += sum_c WW[l, c] Q[i, c]
+        // Gram[l, i] += sum_c WW[l, c] Q[i, c]
 #pragma unroll
-            for (int k = 0; k < C::GW; k++) {
-                const int gt = warp + k * (kLnoThreads / 32);
-                if (gt < ngram) {
-                    const int mt = gt / o8, nt = gt % o8;
-#pragma unroll 8
-                    for (int k0 = 0; k0 < COLS; k0 += 4)
-                        dmma_884(acc[k][0], acc[k][1], sw[(mt * 8 + fg) * LD + k0 + ft], sq[(nt * 8 + fg) * LD + k0 + ft]);
+        for (int k = 0; k < C::GW; k++) {
+            const int gt = gram0 + k * (kLnoThreads / 32);
+            if (gt < ngram) {
+                const double *gw = sw + (gt / o8 * 8 + fg) * LD + ft, *gq = sq + (gt % o8 * 8 + fg) * LD + ft;
+#pragma unroll 4
+                for (int c = gc0; c < gc1; c += 8) {
+                    dmma_884(acc[k][0], acc[k][1], gw[c], gq[c]);
+                    dmma_884(alt[k][0], alt[k][1], gw[c + 4], gq[c + 4]);
                 }
             }
         }
         __syncthreads();   // buffer buf is refilled two tiles from now
         buf ^= 1;
+    }
+    // The energy is <mat, Gram>.  Shares of a Gram tile are added in shared memory: the blocks
+    // of all SMs meet on the o^2 addresses of mat_bar.
+    double *share = reinterpret_cast<double *>(lno_raw);   // (the loop's last barrier is behind)
+    if (nks > 1) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+    }
+    double en = 0.0;
+#pragma unroll
+    for (int k = 0; k < C::GW; k++) {
+        const int gt = gram0 + k * (kLnoThreads / 32);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            acc[k][h] += alt[k][h];
+            const int l = gt / o8 * 8 + fg, i = gt % o8 * 8 + 2 * ft + h;
+            if (gt < ngram && l < o && i < o) en += sM[l * o + i] * acc[k][h];
+            if (nks > 1) share[(warp * 32 + lane) * 2 + h] = acc[k][h];
+        }
     }
     for (int off = 16; off > 0; off >>= 1) en += __shfl_xor_sync(0xffffffffu, en, off);
     if (lane == 0) red[warp] = en;
@@ -295,16 +333,17 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
         for (int w = 0; w < kLnoThreads / 32; w++) s += red[w];
         A.part[slot * gridDim.x + blockIdx.x] = A.g * s;
     }
-    if (!grad) return;
+    if (!grad || ks > 0) return;
 #pragma unroll
     for (int k = 0; k < C::GW; k++) {
-        const int gt = warp + k * (kLnoThreads / 32);
+        const int gt = gram0 + k * (kLnoThreads / 32);
         if (gt < ngram) {
-            const int l = (gt / o8) * 8 + fg;
+            const int l = gt / o8 * 8 + fg;
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const int i = (gt % o8) * 8 + 2 * ft + h;
-                const double gv = h ? acc[k][1] : acc[k][0];
+                const int i = gt % o8 * 8 + 2 * ft + h;
+                double gv = acc[k][h];
+                for (int w = 1; w < nks; w++) gv += share[((warp + w * ngram) * 32 + lane) * 2 + h];
                 if (l < o && i < o && gv != 0.0) red_add(&A.mat_bar[l * o + i], gy * gv);
             }
         }
