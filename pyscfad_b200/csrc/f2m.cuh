@@ -58,8 +58,8 @@
 //   this kernel, Wbar in rows                                 266  198  396   91
 //   Wbar in 8 x 8 tiles: whole lines per warp, where rows
 //   were 16-byte halves of sectors from two items             213  165  324   89
-//   short code, records, preparation in the write-back              132  265   60
-//   global reductions                                               119  242   56
+//   short code, records, preparation in the write-back          -  132  265   60
+//   global reductions                                         156  119  242   56
 // (In rows, items in fixed strides instead of by the counter: 454 ms in the first.)
 //
 // The FP32 sums keep a fixed order: rows run over z; columns over

@@ -1,5 +1,5 @@
-// Tensor-core (tcgen05) form of the adjoint contractions, one launch per
-// ordering tau of a chunk.  Wbar_tau is staged by the epilogue as fp16/bf16
+// Tensor-core (tcgen05) form of the adjoint contractions, one launch per kind for
+// every ordering tau of the chunks of a group.  Wbar_tau is staged by the epilogue as fp16/bf16
 // hi/lo splits (scaled by a per-chunk power of two), as rows
 // [h][y][p][x][q][r][z] or, for x blocks of 8 and 16, as 8 x 8 tiles of (x, rz)
 // (wbar_tiled); either serves all four products through TMA boxes, 128B-swizzled
