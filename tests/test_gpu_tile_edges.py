@@ -128,3 +128,21 @@ def test_packed_layout_tiles(o, v, precision):
     for k in G.KEYS:
         if k != "ovvv":
             assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-11, k
+
+
+# The LNO projection's kernels for up to 16, 32 and 64 occupied orbitals, at and past
+# the 8-row tiles: Gram tiles shared by eight warps (nocc 8), by two (9-16), one or
+# more per warp (17-64); the energy of an energy-only call comes from them as well.
+@pytest.mark.parametrize("o,v", [(8, 5), (9, 4), (12, 17), (16, 3), (17, 3), (24, 3), (32, 2), (33, 2), (40, 2), (64, 2)])
+def test_lno_projection_tiles(o, v):
+    inp = make_inputs(o, v, 40, seed=o, fvo_sigma=1e-3)
+    mat = np.random.default_rng(o).normal(size=(o, o))
+    e_ref, g_ref = O.np_lno_energy_vjp(inp, mat)
+    ins = [getattr(inp, k) for k in G.KEYS]
+    e, g = triples.lno_energy_vjp(mat, *ins, precision="fp64", device="cuda")
+    e1 = triples.lno_energy(mat, *ins, precision="fp64", device="cuda")
+    # FP64 sums of up to nocc^3 nvir^3 terms of both signs in another order, and the parity bounds
+    assert abs(float(e) - e_ref) <= 1e-11 * abs(e_ref)
+    assert abs(float(e1) - float(e)) <= 1e-12 * abs(e_ref)
+    for k in ("mat",) + G.KEYS:
+        assert _relerr(g[k].cpu().numpy(), g_ref[k]) < 1e-10, k
