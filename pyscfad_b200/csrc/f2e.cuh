@@ -1,0 +1,186 @@
+// FP64 element kernels: the epilogue of chunks whose sub-ranges are short (a
+// remainder block, or blocks of 4 and less), for the FP64 and the LNO calls.
+//
+// A short item has 1 to 256 elements a, b, c where the orbit kernels (f2.cuh) give
+// every item a CTA with the tables and slots of 512.  Here a thread takes one
+// element of one item, items lie one behind the other (l0 l1 l2 consecutive
+// threads, c fastest), and everything is gathered straight from memory: the
+// entries of an item are a few lines that its lanes meet in L1.  Sums over one of
+// the three coordinates are butterflies over the lane bits that hold it; a
+// coordinate that reaches into the next warp leaves a partial sum per warp.  Each
+// thread keeps its six results of W and V in its own shared-memory column, which
+// lets the loop over the regions run rolled.
+// What bounds it: latency and issue of the gathers (126 loads per element).
+// Measured against the orbit kernels and 512-slot boxes for every item, LNO E + VJP in
+// FP64: nocc 64 nvir 3 57.5 to 2.3 ms, nocc 49 nvir 17 (16 + 1) 122 to 81, nocc 49 nvir 31
+// 612 to 352, nocc 9 nvir 45 10.8 to 10.1 ms.
+#pragma once
+#include "common.cuh"
+#include "f2.cuh"
+
+namespace tb {
+
+constexpr int kElemThreads = 256;
+
+// The element of this thread.
+struct Elem {
+    int rep, sub, loc[3];   // item, coordinates
+    int el, warps;          // slot in the item (row-major a, b, c), warps that share the item
+    unsigned m[3], all;     // lane bits of each coordinate, of the item
+    bool ok;                // false: beyond the last item
+};
+
+template <typename ARGS>
+__device__ __forceinline__ Elem elem_of(const ARGS &A, int g) {
+    const F2mSub &R = A.sub[0];   // the sub-ranges of a chunk have the same lengths
+    const int k2 = 31 - __clz(R.len[2]), k1 = 31 - __clz(R.len[1]), k0 = 31 - __clz(R.len[0]), kn = k0 + k1 + k2;
+    Elem E;
+    const int item = g >> kn;
+    E.el = g & ((1 << kn) - 1);
+    E.rep = item / A.nsub;
+    E.sub = item - E.rep * A.nsub;
+    E.ok = E.rep < A.n_ijk;
+    if (!E.ok) E.rep = A.n_ijk - 1;
+    E.loc[2] = E.el & (R.len[2] - 1);
+    E.loc[1] = (E.el >> k2) & (R.len[1] - 1);
+    E.loc[0] = E.el >> (k1 + k2);
+    E.warps = kn > 5 ? 1 << (kn - 5) : 1;
+    E.m[2] = (unsigned)(R.len[2] - 1) & 31u;
+    E.m[1] = ((unsigned)(R.len[1] - 1) << k2) & 31u;
+    E.m[0] = ((unsigned)(R.len[0] - 1) << (k1 + k2)) & 31u;
+    E.all = E.m[0] | E.m[1] | E.m[2];
+    return E;
+}
+
+// Sum over the lanes that differ in the bits of `mask` (the same for all lanes).
+__device__ __forceinline__ double elem_sum(double v, unsigned mask) {
+#pragma unroll
+    for (unsigned b = 1; b < 32; b <<= 1)
+        if (mask & b) v += __shfl_xor_sync(0xffffffffu, v, b);
+    return v;
+}
+
+// WW and VV of the element, six orderings each
+template <typename StageT, typename ARGS>
+__device__ __forceinline__ void elem_amplitudes(const ARGS &A, const F2mSub &R, const int (&ids)[3], const int (&loc)[3],
+                                                double (&WW)[6], double (&VV)[6]) {
+    const int o = A.o, v = A.v;
+    const StageT *S[6];
+#pragma unroll
+    for (int pi = 0; pi < 6; pi++) {
+        int pp[3] = {0, 0, 0};
+        perm_of(pi, pp);
+        const int x = loc[pp[0]], y = loc[pp[1]], z = loc[pp[2]], ex = R.len[pp[0]], ez = R.len[pp[2]];
+        const int swz = sizeof(StageT) == 4 && ex == 8 && ez == 8 ? f2m_row_swizzle(y) : 0;
+        S[pi] = static_cast<const StageT *>(A.S) + R.pi[pi].s0 + y * ex * ez + ((x * ez + z) ^ swz);
+    }
+    double tz[3][3], fz[3][3];   // t1[r, z], fvo[z, r]
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int s = 0; s < 3; s++) {
+            const int z = R.st[s] + loc[s];
+            tz[r][s] = __ldg(&A.t1[(long long)ids[r] * v + z]);
+            fz[r][s] = __ldg(&A.fvo[(long long)z * o + ids[r]]);
+        }
+#pragma unroll
+    for (int s = 0; s < 6; s++) WW[s] = VV[s] = 0.0;
+#pragma unroll
+    for (int rho = 0; rho < 6; rho++) {
+        int pr[3] = {0, 0, 0};
+        perm_of(rho, pr);
+        const int p = ids[pr[0]], q = ids[pr[1]];
+        const long long idx = ((long long)p * o + q) * o + ids[pr[2]];
+#pragma unroll
+        for (int pi = 0; pi < 6; pi++) {
+            const int s = f2m_sof(pi, rho);
+            int pp[3] = {0, 0, 0};
+            perm_of(pi, pp);
+            const int x = R.st[pp[0]] + loc[pp[0]], y = R.st[pp[1]] + loc[pp[1]];
+            WW[s] += (double)__ldg(S[pi] + idx * R.pi[pi].rs);
+            VV[s] += __ldg(&A.ovov[(((long long)p * v + x) * o + q) * v + y]) * tz[pr[2]][pp[2]] +
+                     __ldg(&A.t2[(((long long)q * o + p) * v + y) * v + x]) * fz[pr[2]][pp[2]];
+        }
+    }
+}
+
+// Orbital-energy gradient of dd = dE/dD
+template <typename ARGS>
+__device__ __forceinline__ void elem_dd(const ARGS &A, const F2mSub &R, const Elem &E, const int (&ids)[3], double dd) {
+    const int lane = threadIdx.x & 31;
+    const double tot = elem_sum(dd, E.all);
+    if (E.ok && (lane & E.all) == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) red_add(&A.mo_bar[ids[k]], tot);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const unsigned others = E.all & ~E.m[k];
+        const double acc = elem_sum(dd, others);
+        if (E.ok && (lane & others) == 0) red_add(&A.mo_bar[A.o + R.st[k] + E.loc[k]], -acc);
+    }
+}
+
+// Write-back of the element's results, column threadIdx.x of sW and sV [6][kElemThreads]:
+// Wbar, and the V-term gradients v = ovov[p,x,q,y] t1[r,z] + t2[q,p,y,x] fvo[z,r], over the leading
+// regions (pi, rho).  Regions that share r and z share the column sums.
+template <int SPLIT, typename ARGS>
+__device__ __forceinline__ void elem_writeback(const ARGS &A, const F2mSub &R, const Elem &E, const int (&ids)[3], int opat,
+                                               int vpat, const typename F2Smem<SPLIT>::W *sW, const double *sV) {
+    const int o = A.o, v = A.v, lane = threadIdx.x & 31;
+    const unsigned lead = opat == 0 ? 63u : opat == 1 ? 19u : opat == 2 ? 13u : 1u;    // orderings of f2m_lead
+    const unsigned vlead = vpat == 0 ? 63u : vpat == 1 ? 19u : vpat == 2 ? 13u : 1u;
+#pragma unroll 1
+    for (int rz = 0; rz < 9; rz++) {
+        const int rs = rz / 3, zs = rz % 3;   // slots of r and z
+        const int zl = sel3(E.loc[0], E.loc[1], E.loc[2], zs), z = sel3(R.st[0], R.st[1], R.st[2], zs) + zl;
+        const unsigned mz = zs == 0 ? E.m[0] : zs == 1 ? E.m[1] : E.m[2], others = E.all & ~mz;
+        const int r = sel3(ids[0], ids[1], ids[2], rs);
+        const double tv = __ldg(&A.t1[(long long)r * v + z]), fv = __ldg(&A.fvo[(long long)z * o + r]);
+        double ct = 0.0, cf = 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {   // (unrolled: the loads of four regions in flight)
+            // the two other slots in either order: u & 1 for rho, u >> 1 for pi
+            const int ra = rs == 0 ? 1 : 0, rb = rs == 2 ? 1 : 2, za = zs == 0 ? 1 : 0, zb = zs == 2 ? 1 : 2;
+            const int pr0 = u & 1 ? rb : ra, pr1 = u & 1 ? ra : rb, pp0 = u >> 1 ? zb : za, pp1 = u >> 1 ? za : zb;
+            const int rho = perm_index(pr0, pr1), pi = perm_index(pp0, pp1);
+            const bool vl = (vlead >> pi) & 1u;
+            if (!__any_sync(0xffffffffu, vl)) continue;
+            const bool in = E.ok && vl && ((lead >> rho) & 1u);
+            // s with s o rho = pi: its slots are the virtual ones paired with occupied slots 0 and 1
+            const int s0 = pr0 == 0 ? pp0 : (pr1 == 0 ? pp1 : zs), s1 = pr0 == 1 ? pp0 : (pr1 == 1 ? pp1 : zs);
+            const int at = perm_index(s0, s1) * kElemThreads + threadIdx.x;
+            const int p = sel3(ids[0], ids[1], ids[2], pr0), q = sel3(ids[0], ids[1], ids[2], pr1);
+            const int xl = sel3(E.loc[0], E.loc[1], E.loc[2], pp0), yl = sel3(E.loc[0], E.loc[1], E.loc[2], pp1);
+            const int x = sel3(R.st[0], R.st[1], R.st[2], pp0) + xl, y = sel3(R.st[0], R.st[1], R.st[2], pp1) + yl;
+            const long long ov = (((long long)p * v + x) * o + q) * v + y, tt = (((long long)q * o + p) * v + y) * v + x;
+            const double vb = in ? sV[at] : 0.0;
+            if (in) {
+                const F2mPi &D = R.pi[pi];
+                const long long w = f2m_wbar(D, p, q, r) + (long long)xl * D.wx + (long long)yl * D.wy + zl;
+                if constexpr (SPLIT == 0) {
+                    static_cast<double *>(A.SW)[w] = sW[at];
+                } else {
+                    const uint32_t pk = sW[at];
+                    static_cast<uint16_t *>(A.SW)[w] = (uint16_t)pk;
+                    static_cast<uint16_t *>(A.SW)[w + D.half] = (uint16_t)(pk >> 16);
+                }
+                ct += vb * __ldg(&A.ovov[ov]);
+                cf += vb * __ldg(&A.t2[tt]);
+            }
+            const double r1 = elem_sum(vb * tv, mz), r2 = elem_sum(vb * fv, mz);
+            if (in && (lane & mz) == 0) {
+                red_add(&A.ovov_bar[ov], r1);
+                red_add(&A.t2_bar[tt], r2);
+            }
+        }
+        ct = elem_sum(ct, others);
+        cf = elem_sum(cf, others);
+        if (E.ok && (lane & others) == 0) {
+            red_add(&A.t1_bar[(long long)r * v + z], ct);
+            red_add(&A.fvo_bar[(long long)z * o + r], cf);
+        }
+    }
+}
+
+}  // namespace tb

@@ -21,8 +21,8 @@
 // each value once per permutation, hence g.
 //
 // Three kernels over FP64 arrays [i][j][k][e] of the box (e: 512 slots per
-// triple of 8-wide sub-ranges, in the thread order of the orbit kernels; slots
-// beyond a short sub-range hold zeros):
+// triple of 8-wide sub-ranges, in the thread order of the orbit kernels; l0 l1 l2
+// slots, row-major, where a sub-range is short):
 //   k_lno_fwd   an occupied representative and a sub-range triple per CTA: six
 //               orderings of two elements per thread, WW and Q of the six
 //               occupied orders out as whole lines
@@ -31,6 +31,8 @@
 //               one forms Zbar
 //   k_lno_adj   as k_lno_fwd: r3, Wbar and V-term gradients (FP64 sums) written
 //               back over the leading regions, orbital-energy gradients
+// and k_lno_fwd_e, k_lno_adj_e with a thread per element for the chunks of short
+// sub-ranges.
 // Bytes per raw amplitude: 4 or 8 + 16/6, 128/6, 24/6 + 4 or 8: a third of what
 // the four passes over arrays of all orderings took (104 and 120), which were
 // bound by shared-memory gathers and memory latency.  Measured, nocc 14 nvir 96
@@ -42,6 +44,7 @@
 
 #include "common.cuh"
 #include "f2.cuh"
+#include "f2e.cuh"
 #include "f2m.cuh"
 #include "gemm_fp64.cuh"
 
@@ -53,6 +56,7 @@ constexpr int kLnoThreads = kF2Threads;
 struct LnoArgs {
     int o, v;
     int nsub;                   // sub-range triples of the box (all of them)
+    int kn, ne;                 // log2 of the slots of one, slots of an occupied triple (even)
     F2mSub sub[kF2mMaxSub];     // pat: equal blocks; regions as in the canonical epilogue
     int n_ijk;
     const int *ijk;             // occupied representatives i >= j >= k
@@ -112,7 +116,7 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_fwd(const __grid_constan
     const double *ev = A.mo_e + o;
     const double e_occ = A.mo_e[i0] + A.mo_e[i1] + A.mo_e[i2];
     const double e_bc = ok0 ? ev[R.st[1] + cb] + ev[R.st[2] + cc] : 0.0;
-    const long long ne = (long long)A.nsub * 512;
+    const long long ne = A.ne;
 #pragma unroll
     for (int e = 0; e < 2; e++) {
         const bool ok = e == 0 ? ok0 : ok1;
@@ -129,6 +133,32 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_fwd(const __grid_constan
             A.Q[at] = ok ? Z[s] * rD : 0.0;
         });
     }
+}
+
+// k_lno_fwd of a chunk with a short sub-range: a thread per element (f2e.cuh)
+template <typename StageT>
+__global__ void __launch_bounds__(kElemThreads, 2) k_lno_fwd_e(const __grid_constant__ LnoArgs A) {
+    const int o = A.o;
+    const Elem E = elem_of(A, blockIdx.x * kElemThreads + threadIdx.x);
+    const F2mSub &R = A.sub[E.sub];
+    const int ids[3] = {A.ijk[3 * E.rep], A.ijk[3 * E.rep + 1], A.ijk[3 * E.rep + 2]};
+    double WW[6], VV[6], X[6], Z[6];
+    elem_amplitudes<StageT>(A, R, ids, E.loc, WW, VV);
+#pragma unroll
+    for (int s = 0; s < 6; s++) X[s] = WW[s] + 0.5 * VV[s];
+    f2_r3(X, Z);
+    const double *ev = A.mo_e + o;
+    const double rD = 1.0 / (A.mo_e[ids[0]] + A.mo_e[ids[1]] + A.mo_e[ids[2]] - ev[R.st[0] + E.loc[0]] -
+                             ev[R.st[1] + E.loc[1]] - ev[R.st[2] + E.loc[2]]);
+    if (!E.ok) return;
+    const int slot = (E.sub << A.kn) + E.el;
+    lno_for_s([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        const long long at = lno_box<s>(o, A.ne, ids[0], ids[1], ids[2]) + slot;
+        A.WW[at] = WW[s];
+        A.Q[at] = Z[s] * rD;
+        if (A.ne > A.nsub << A.kn && slot == 0) A.WW[at + 1] = A.Q[at + 1] = 0.0;   // a single element: the unused slot
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -165,7 +195,9 @@ struct LnoProj {
     }
 };
 
-template <int COLS>
+// FULL: three full sub-ranges, 512 slots a triple: a tile of columns is consecutive (with the general
+// form's divisions per thread and column, nocc 14 nvir 96 takes 2 % more of a call).
+template <int COLS, bool FULL>
 __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_constant__ LnoArgs A, int slot, int first) {
     using C = LnoProj<COLS>;
     constexpr int LD = C::LD;
@@ -174,9 +206,11 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
     double *sw_b = reinterpret_cast<double *>(lno_raw), *sq_b = sw_b + 2 * rows * LD, *sM = sq_b + 2 * rows * LD;
     double *s_eo = sM + o * o, *s_ecol_b = s_eo + kLnoMaxO;
     __shared__ double red[kLnoThreads / 32];
-    const long long ne = (long long)A.nsub * 512;
-    const long long rstride = slot == 0 ? o * o * ne : (slot == 1 ? o * ne : ne);
-    const int per = (int)(ne / COLS), ntile = o * o * per;
+    // columns: the other two occupied indices and e, `ncol` of them; the first `run` are consecutive, and
+    // so on from o run on
+    const int ne = A.ne, ncol = o * o * ne, ntile = (ncol + COLS - 1) / COLS;
+    const int run = slot == 0 ? ncol : (slot == 1 ? o * ne : ne);
+    const long long rstride = run;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int fg = lane >> 2, ft = lane & 3;
     const bool grad = A.want_grad != 0, last = slot == 0;
@@ -194,37 +228,39 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
     // this warp's output tile k = m JT + j: rows and columns
     auto row0 = [&](int m) -> int { return (COLS >= 64 ? m : (warp >> 2) + 2 * m) * 8; };
     auto col0 = [&](int j) -> int { return (COLS >= 64 ? warp + 8 * j : warp & 3) * 8; };
-    // first element of tile t (row 0)
-    auto tile_base = [&](int t) -> long long {
-        const int oth = t / per;
-        const long long e0 = (long long)(t - oth * per) * COLS;
-        return slot == 1 ? (long long)(oth / o) * o * o * ne + (oth % o) * ne + e0
-                         : (slot == 0 ? oth * ne : oth * o * ne) + e0;
-    };
+    // column c of row 0
+    auto column = [&](int c) -> long long { return c + (long long)(c / run) * run * (o - 1); };
     auto issue = [&](int t, int b) {
-        const long long base = tile_base(t);
         double *sw = sw_b + b * rows * LD, *sq = sq_b + b * rows * LD;
-        for (int e = threadIdx.x; e < rows * (COLS / 2); e += blockDim.x) {
-            const int l = e / (COLS / 2), j = e % (COLS / 2) * 2;
-            const long long at = base + (l < o ? l * rstride + j : 0);
-            const int bytes = l < o ? 16 : 0;
+        const int j = threadIdx.x % (COLS / 2) * 2;   // (this thread's columns in every turn)
+        const bool in = FULL || t * COLS + j < ncol;
+        const long long base = FULL ? column(t * COLS) + j : (in ? column(t * COLS + j) : 0);
+        for (int l = threadIdx.x / (COLS / 2); l < rows; l += kLnoThreads / (COLS / 2)) {
+            const bool ok = in && l < o;
+            const long long at = base + (ok ? l * rstride : 0);
+            const int bytes = ok ? 16 : 0;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sw + l * LD + j)), "l"(A.WW + at), "r"(bytes) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sq + l * LD + j)), "l"(A.Q + at), "r"(bytes) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (grad && last && threadIdx.x < COLS) {
             // energies of the column: the other two occupied indices, a, b and c
-            const int oth = t / per, e = (t - oth * per) * COLS + threadIdx.x;
-            const F2mSub &R = A.sub[e >> 9];
-            int a, b2, c;
-            f2_element(e & 255, a, b2, c);
-            a += 4 * ((e >> 8) & 1);
-            double ec = -1.0;   // a slot beyond a short range: any non-zero value
-            if (a < R.len[0] && b2 < R.len[1] && c < R.len[2]) {
+            const int col = t * COLS + threadIdx.x, oth = col / ne, e = col - oth * ne, sub = e >> A.kn;
+            double ec = -1e30;   // an unused slot: any non-zero value
+            if (col < ncol && sub < A.nsub) {
+                const F2mSub &R = A.sub[sub];
+                const int pos = e & ((1 << A.kn) - 1);
+                int a, b2, c;
+                if (FULL) {   // the orbit kernels' order, else row-major
+                    f2_element(pos & 255, a, b2, c);
+                    a += 4 * (pos >> 8);
+                } else {
+                    c = pos % R.len[2];
+                    b2 = pos / R.len[2] % R.len[1];
+                    a = pos / (R.len[2] * R.len[1]);
+                }
                 const double *ev = A.mo_e + o;
                 ec = A.mo_e[oth / o] + A.mo_e[oth % o] - ev[R.st[0] + a] - ev[R.st[1] + b2] - ev[R.st[2] + c];
-            } else {
-                ec = -1e30;
             }
             s_ecol_b[b * COLS + threadIdx.x] = ec;
         }
@@ -234,14 +270,23 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
     for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
         if (t + (int)gridDim.x < ntile) issue(t + gridDim.x, buf ^ 1);
         else asm volatile("cp.async.commit_group;" ::: "memory");   // keeps the wait count uniform
-        const long long base = tile_base(t);
+        const long long tile0 = FULL ? column(t * COLS) : 0;
+        long long colat[C::JT];   // this thread's output columns (negative: beyond the last)
+        if constexpr (!FULL) {
+#pragma unroll
+            for (int j = 0; j < C::JT; j++) {
+                const int c = t * COLS + col0(j) + 2 * ft;
+                colat[j] = c < ncol ? column(c) : -1;
+            }
+        }
+        auto output = [&](int i, int j) -> long long { return (FULL ? tile0 + col0(j) + 2 * ft : colat[j]) + i * rstride; };
         double2 pw[C::TW], pq[C::TW];   // running sums of this thread's output positions
 #pragma unroll
         for (int k = 0; k < C::TW; k++) {
             const int i = row0(k / C::JT) + fg;
             pw[k] = pq[k] = double2{0.0, 0.0};
-            if (grad && !first && i < o) {
-                const long long at = base + i * rstride + col0(k % C::JT) + 2 * ft;
+            if (grad && !first && i < o && (FULL || colat[k % C::JT] >= 0)) {
+                const long long at = output(i, k % C::JT);
                 pw[k] = *reinterpret_cast<const double2 *>(A.PW + at);
                 pq[k] = *reinterpret_cast<const double2 *>(A.PQ + at);
             }
@@ -276,8 +321,8 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
 #pragma unroll
             for (int k = 0; k < C::TW; k++) {
                 const int i = row0(k / C::JT) + fg, cl = col0(k % C::JT) + 2 * ft;
-                if (i < o) {
-                    const long long at = base + i * rstride + cl;
+                if (i < o && (FULL || colat[k % C::JT] >= 0)) {
+                    const long long at = output(i, k % C::JT);
                     double2 w = pw[k], r = pq[k];
                     if (last) {
                         w.x = A.f * w.x / (s_eo[i] + s_ecol[cl]);
@@ -374,7 +419,7 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_adj(const __grid_constan
     int ca, cb, cc;
     f2_element(tid, ca, cb, cc);
     const int gidx = f2m_res(0, ca) ^ f2m_res(1, cb) ^ f2m_res(2, cc);
-    const long long ne = (long long)A.nsub * 512;
+    const long long ne = A.ne;
     const float wsc = SPLIT == 1 ? (float)*A.wscale : 1.0f;
     // Dbar = -(g ybar / f) Zbar Q, each occupied order once
     const double dfac = -(A.g * A.ybar / A.f) / (opat == 0 ? 1.0 : (opat == 3 ? 6.0 : 2.0));
@@ -407,6 +452,40 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_adj(const __grid_constan
     __syncthreads();
     f2_dd_add(s_part, R, o, i0, i1, i2, A.mo_bar);
     f2_writeback<SPLIT>(A, R, i0, i1, i2, opat, vpat, tab, tf, s_res, sW, sV);
+}
+
+// k_lno_adj of a chunk with a short sub-range: a thread per element
+template <int SPLIT>
+__global__ void __launch_bounds__(kElemThreads, 2) k_lno_adj_e(const __grid_constant__ LnoArgs A) {
+    using WT = typename F2Smem<SPLIT>::W;
+    __shared__ double sV[6 * kElemThreads];
+    __shared__ WT sW[6 * kElemThreads];
+    const int o = A.o;
+    const Elem E = elem_of(A, blockIdx.x * kElemThreads + threadIdx.x);
+    const F2mSub &R = A.sub[E.sub];
+    const int ids[3] = {A.ijk[3 * E.rep], A.ijk[3 * E.rep + 1], A.ijk[3 * E.rep + 2]};
+    const int opat = (ids[0] == ids[2]) ? 3 : (ids[0] == ids[1] ? 1 : (ids[1] == ids[2] ? 2 : 0));
+    const float wsc = SPLIT == 1 ? (float)*A.wscale : 1.0f;
+    const double dfac = -(A.g * A.ybar / A.f) / (opat == 0 ? 1.0 : (opat == 3 ? 6.0 : 2.0));
+    const int slot = (E.sub << A.kn) + E.el;
+    double Z[6], P[6], X[6], ds = 0.0;
+    lno_for_s([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        const long long at = lno_box<s>(o, A.ne, ids[0], ids[1], ids[2]) + slot;
+        Z[s] = __ldg(&A.PW[at]);
+        P[s] = __ldg(&A.PQ[at]);
+        ds += Z[s] * __ldg(&A.Q[at]);
+    });
+    f2_r3(Z, X);
+#pragma unroll
+    for (int s = 0; s < 6; s++) {
+        const double wb = P[s] + X[s];
+        sV[s * kElemThreads + threadIdx.x] = 0.5 * X[s];
+        if constexpr (SPLIT == 0) sW[s * kElemThreads + threadIdx.x] = wb;
+        else sW[s * kElemThreads + threadIdx.x] = f2m_split<SPLIT>((float)wb, wsc);
+    }
+    elem_dd(A, R, E, ids, E.ok && A.f != 0.0 ? dfac * ds : 0.0);
+    elem_writeback<SPLIT>(A, R, E, ids, opat, R.pat, sW, sV);
 }
 
 // ---------------------------------------------------------------------------

@@ -152,6 +152,9 @@ static long long chunk_stage_elems(const ChunkDesc &ch, const Dims &d) {
     return s;
 }
 
+// LNO box slots of an occupied triple: every virtual triple of the chunk's blocks once, an even number
+static int box_slots(const ChunkDesc &ch) { return (ch.nabc[0] * ch.nabc[1] * ch.nabc[2] + 1) / 2 * 2; }
+
 static int plan_once(int precision, int nocc, int nvir, int packed, int want_grad, Plan &P, int lno,
                      const triples_options *opt, bool vtables, int most_group) {
     if (nocc < 1 || nvir < 1 || nocc > kMaxCols || nvir > 32767) return TRIPLES_ERR_INVALID_ARGUMENT;
@@ -199,7 +202,7 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
     P.nb = num_blocks(d);
     P.n_ijk = nocc * (nocc + 1) * (nocc + 2) / 6;
     long long maxst = 0, maxwb = 0;
-    int maxitems = 0, maxsub = 1;
+    int maxitems = 0, maxbox = 1;
     for (int A = 0; A < P.nb; A++)
         for (int B = 0; B <= A; B++)
             for (int C = 0; C <= B; C++) {
@@ -211,7 +214,7 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
                 if (w > maxwb) maxwb = w;
                 int it = ch.nabc[0] * ch.nabc[1] * ch.nabc[2];
                 if (it > maxitems) maxitems = it;
-                maxsub = std::max(maxsub, ((ch.nabc[0] + 7) / 8) * ((ch.nabc[1] + 7) / 8) * ((ch.nabc[2] + 7) / 8));
+                maxbox = std::max(maxbox, box_slots(ch));
             }
     P.stage_elems = (size_t)maxst;
     P.wbar_elems = (size_t)maxwb;
@@ -272,7 +275,7 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
     P.off_epart = take((size_t)P.group * P.n_ijk * P.f2_gy * el);
     if (P.lno) {
         // FP64 box arrays: WW (0), PQ (1), Q (2), PW / Zbar (3); the energy alone needs only 0 and 2
-        const size_t box = o * o * o * 512 * (size_t)maxsub;
+        const size_t box = o * o * o * (size_t)maxbox;
         P.off_L[0] = take(box * el);
         P.off_L[2] = take(box * el);
         if (want_grad) {
@@ -1433,15 +1436,15 @@ static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, c
 // LNO chunk epilogue: energy of the projected amplitudes and, with want_grad,
 // mat_bar, the orbital-energy and V-term gradients and the Wbar staging that
 // the adjoint contractions read next (lno.cuh).
-template <int COLS>
+template <int COLS, bool FULL>
 static int lno_projections(const LnoArgs &A, cudaStream_t st, unsigned &grid) {
-    const long long tiles = (long long)A.o * A.o * A.nsub * (512 / COLS);
+    const long long tiles = ((long long)A.o * A.o * A.ne + COLS - 1) / COLS;   // (a CTA has one tile at least)
     grid = (unsigned)std::min(tiles, (long long)2 * num_sms());
     const size_t smem = LnoProj<COLS>::smem(A.o);
-    const int rc = smem_optin(k_lno_proj<COLS>, smem);
+    const int rc = smem_optin(k_lno_proj<COLS, FULL>, smem);
     if (rc != TRIPLES_OK) return rc;
     for (int slot = 2; slot >= 0; slot--)
-        TB_KLAUNCH(P_LNO_PROJ, (k_lno_proj<COLS><<<grid, kLnoThreads, smem, st>>>(A, slot, slot == 2 ? 1 : 0)));
+        TB_KLAUNCH(P_LNO_PROJ, (k_lno_proj<COLS, FULL><<<grid, kLnoThreads, smem, st>>>(A, slot, slot == 2 ? 1 : 0)));
     return TRIPLES_OK;
 }
 
@@ -1477,6 +1480,9 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
         sub_regions(ch, o, sst, len, mixed ? 2 : 1, (int)sizeof(StageT), u);
         u.pat = ch.blk[0] == ch.blk[2] ? 3 : (ch.blk[0] == ch.blk[1] ? 1 : (ch.blk[1] == ch.blk[2] ? 2 : 0));
     }
+    A.kn = 0;
+    while ((1 << A.kn) < A.sub[0].len[0] * A.sub[0].len[1] * A.sub[0].len[2]) A.kn++;
+    A.ne = box_slots(ch);
     A.n_ijk = P.n_ijk;
     A.ijk = (int *)(ws + P.off_ijk);
     A.S = ws + P.off_S;
@@ -1495,12 +1501,15 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     A.want_grad = P.want_grad;
     A.part = (double *)(ws + P.off_lpart);
     const unsigned items = (unsigned)(P.n_ijk * A.nsub);
-    TB_KLAUNCH(P_LNO, (k_lno_fwd<StageT><<<items, kLnoThreads, F2Smem<0>::TABLES, st>>>(A)));
+    const bool full = A.kn == 9;
+    const unsigned elems = (unsigned)((((long long)items << A.kn) + kElemThreads - 1) / kElemThreads);   // element kernels
+    if (full) TB_KLAUNCH(P_LNO, (k_lno_fwd<StageT><<<items, kLnoThreads, F2Smem<0>::TABLES, st>>>(A)));
+    else TB_KLAUNCH(P_LNO, (k_lno_fwd_e<StageT><<<elems, kElemThreads, 0, st>>>(A)));
     // columns per tile: 128 while two buffers of all rows leave room for two CTAs per SM
     unsigned parts = 0;
-    const int prc = o <= 16   ? lno_projections<128>(A, st, parts)
-                    : o <= 32 ? lno_projections<64>(A, st, parts)
-                              : lno_projections<32>(A, st, parts);
+    const int prc = o <= 16   ? (full ? lno_projections<128, true>(A, st, parts) : lno_projections<128, false>(A, st, parts))
+                    : o <= 32 ? (full ? lno_projections<64, true>(A, st, parts) : lno_projections<64, false>(A, st, parts))
+                              : (full ? lno_projections<32, true>(A, st, parts) : lno_projections<32, false>(A, st, parts));
     if (prc != TRIPLES_OK) return prc;
     Group<ChunkAux, 1> G;
     G.n = 1;
@@ -1509,12 +1518,15 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     TB_KLAUNCH(P_PREP, (k_energy_sum<<<1, 256, 0, st>>>(G, 1)));
     if (!P.want_grad) return TRIPLES_OK;
     if (!mixed) {
-        TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<0><<<items, kLnoThreads, F2Smem<0>::BYTES, st>>>(A)));
+        if (full) TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<0><<<items, kLnoThreads, F2Smem<0>::BYTES, st>>>(A)));
+        else TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj_e<0><<<elems, kElemThreads, 0, st>>>(A)));
         return TRIPLES_OK;
     }
     // fp16: power-of-two scale of the split Wbar; bf16: scale 1 (both read by the contractions)
     TB_KLAUNCH(P_PREP, (k_chunk_scale<<<1, 32, 0, st>>>(G)));
-    if (bf16) TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<2><<<items, kLnoThreads, F2Smem<2>::BYTES, st>>>(A)));
+    if (!full && bf16) TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj_e<2><<<elems, kElemThreads, 0, st>>>(A)));
+    else if (!full) TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj_e<1><<<elems, kElemThreads, 0, st>>>(A)));
+    else if (bf16) TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<2><<<items, kLnoThreads, F2Smem<2>::BYTES, st>>>(A)));
     else TB_KLAUNCH(P_LNO_ADJ, (k_lno_adj<1><<<items, kLnoThreads, F2Smem<1>::BYTES, st>>>(A)));
     return TRIPLES_OK;
 }

@@ -1,0 +1,69 @@
+"""Chunks with a short virtual sub-range (remainder blocks, blocks of 4 and
+less): their kernels take a thread per element, so items share warps and CTAs
+and an LNO box has as many slots as the blocks have virtual triples."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from pyscfad_b200 import triples
+from pyscfad_b200.synthetic import make_inputs
+from tests import golden_util as G
+
+
+def _relerr(a, b):
+    return float(np.abs(a - b).max() / max(np.abs(b).max(), 1e-7))
+
+
+@pytest.mark.parametrize("o,v", [(64, 1), (64, 2), (64, 3), (49, 5), (30, 7), (20, 12)])
+def test_lno_scratch_follows_the_blocks(o, v):
+    """Four FP64 box arrays over (i, j, k, virtual triple of the largest chunk) and what a canonical call needs;
+    512 slots whatever the blocks were 4.4 GB at nocc 64 nvir 2."""
+    largest = 1 << (v.bit_length() - 1)                   # nvir below 16: the largest block is its leading bit
+    slots = max(2, largest ** 3)
+    for precision in ("fp64", "mixed"):
+        box = 4 * 8 * o ** 3 * slots
+        canonical = triples.workspace_size(o, v, True, True, precision)
+        assert triples.lno_workspace_size(o, v, True, True, precision) <= canonical + box + (1 << 20)
+
+
+# Element kernels of every item size and warp layout: 1 to 256 elements (blocks 1, 2, 4, 8, 16 in
+# every combination of nvir 31 = 16 + 8 + 4 + 2 + 1), equal occupied and equal virtual ranges,
+# against the oracle; FP64 sums in another order.
+@pytest.mark.gpu
+@pytest.mark.parametrize("o,v,tv", [(2, 31, 0), (5, 23, 0), (4, 21, 4), (3, 9, 1), (6, 6, 2), (9, 19, 0)])
+def test_lno_short_ranges_match_the_oracle(o, v, tv):
+    inp = make_inputs(o, v, 40, seed=v, fvo_sigma=1e-3)
+    mat = np.random.default_rng(o).normal(size=(o, o))
+    e_ref, g_ref = O.np_lno_energy_vjp(inp, mat)
+    ins = [getattr(inp, k) for k in G.KEYS]
+    e, g = triples.lno_energy_vjp(mat, *ins, precision="fp64", device="cuda", block_size=tv)
+    e1 = triples.lno_energy(mat, *ins, precision="fp64", device="cuda", block_size=tv)
+    assert abs(float(e) - e_ref) <= 1e-11 * abs(e_ref)
+    assert abs(float(e1) - float(e)) <= 1e-12 * abs(e_ref)
+    for k in ("mat",) + G.KEYS:
+        assert _relerr(g[k].cpu().numpy(), g_ref[k]) < 1e-10, k
+    # the mixed modes' parity bounds
+    for precision, e_tol, g_tol in (("mixed", 1e-6, 1e-5), ("mixed_bf16", 1e-4, 1e-3)):
+        e, g = triples.lno_energy_vjp(mat, *ins, precision=precision, device="cuda", block_size=tv)
+        assert abs(float(e) - e_ref) <= e_tol * abs(e_ref)
+        for k in ("mat",) + G.KEYS:
+            assert _relerr(g[k].cpu().numpy(), g_ref[k]) < g_tol, (precision, k)
+
+
+# The projection's forms for up to 16, 32 and 64 occupied orbitals over boxes of several sub-range
+# triples, many tiles a CTA, full and short: the identity projector is the canonical energy
+# (another path and another order of FP64 sums).
+@pytest.mark.gpu
+@pytest.mark.parametrize("o,v", [(14, 33), (17, 17), (20, 33), (33, 17), (33, 20), (40, 16)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed_bf16"])
+def test_lno_projection_over_several_ranges(o, v, precision):
+    inp = make_inputs(o, v, 40, seed=o, fvo_sigma=1e-3)
+    ins = [getattr(inp, k) for k in G.KEYS]
+    e0, g0 = triples.energy_vjp(*ins, precision="fp64", device="cuda")
+    e, g = triples.lno_energy_vjp(np.eye(o), *ins, precision=precision, device="cuda")
+    e_tol, g_tol = {"fp64": (1e-12, 1e-10), "mixed": (1e-6, 1e-5), "mixed_bf16": (1e-4, 1e-3)}[precision]
+    assert abs(float(e) - float(e0)) <= e_tol * abs(float(e0))
+    for k in G.KEYS:
+        assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < g_tol, k
+    torch.cuda.synchronize()
