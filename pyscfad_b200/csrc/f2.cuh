@@ -23,8 +23,8 @@ struct F2P {
     int nsub, n_ijk;
     const int *ijk;
     const double *mo_e, *t1, *t2, *ovov, *fvo;
-    const double *S;    // W per ordering tau, blocked staging (no row exchange)
-    double *SW;         // Wbar out, per tau at ch.pb[tau].swoff: [y][p][x][q][r][z]
+    const void *S;      // W per ordering tau, blocked staging (FP64 rows are not exchanged)
+    void *SW;           // Wbar out, per tau at ch.pb[tau].swoff: [y][p][x][q][r][z]
     double ybar;
     int want_grad;
     double *e_part;     // energy partial of each item, at sub * n_ijk + rep
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kF2Threads, 2) k_f2t(const __grid_constant__ J
     const double e_occ = A.mo_e[i0] + A.mo_e[i1] + A.mo_e[i2];
     const double e_bc = ok0 ? ev[R.st[1] + cb] + ev[R.st[2] + cc] : 0.0;
     double WW[2][6], VV[2][6];
-    f2_amplitudes(A.S, R, o, i0, i1, i2, ca, cb, cc, ok0, ok1, tab, tf, WW, VV);
+    f2_amplitudes(static_cast<const double *>(A.S), R, o, i0, i1, i2, ca, cb, cc, ok0, ok1, tab, tf, WW, VV);
     // orbit weights: n_ijk n_abc / 18 for three distinct virtuals; the energy
     // counts each orbit once per ordering of equal sub-ranges
     const double cocc = opat == 0 ? 2.0 : (opat == 3 ? 6.0 / 18.0 : 1.0);

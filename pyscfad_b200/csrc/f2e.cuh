@@ -1,5 +1,6 @@
 // FP64 element kernels: the epilogue of chunks whose sub-ranges are short (a
-// remainder block, or blocks of 4 and less), for the FP64 and the LNO calls.
+// remainder block, or blocks of 4 and less), for the FP64 calls (by_element in
+// triples.cu) and the LNO calls.
 //
 // A short item has 1 to 256 elements a, b, c where the orbit kernels (f2.cuh) give
 // every item a CTA with the tables and slots of 512.  Here a thread takes one
@@ -13,7 +14,8 @@
 // What bounds it: latency and issue of the gathers (126 loads per element).
 // Measured against the orbit kernels and 512-slot boxes for every item, LNO E + VJP in
 // FP64: nocc 64 nvir 3 57.5 to 2.3 ms, nocc 49 nvir 17 (16 + 1) 122 to 81, nocc 49 nvir 31
-// 612 to 352, nocc 9 nvir 45 10.8 to 10.1 ms.
+// 612 to 352, nocc 9 nvir 45 10.8 to 10.1 ms; FP64 energy: nocc 64 nvir 3 6.7 to 0.46 ms,
+// nocc 160 nvir 9 324 to 94, nocc 32 nvir 17 4.4 to 3.2; FP64 E + VJP nocc 257 nvir 3 608 to 141 ms.
 #pragma once
 #include "common.cuh"
 #include "f2.cuh"
@@ -181,6 +183,58 @@ __device__ __forceinline__ void elem_writeback(const ARGS &A, const F2mSub &R, c
             red_add(&A.fvo_bar[(long long)z * o + r], cf);
         }
     }
+}
+
+// The items of the jobs (chunks) of a launch; a job starts with a new CTA.
+template <typename JOBS>
+__global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__ JOBS J) {
+    __shared__ double sV[6 * kElemThreads], sW[6 * kElemThreads];
+    JobCursor jcur;
+    int blk;
+    const int jb = jcur.at(J, (int)blockIdx.x, blk);
+    const F2P &A = J.job[JOBS::kOne ? 0 : jb];
+    const Elem E = elem_of(A, blk * kElemThreads + threadIdx.x);
+    const F2mSub &R = A.sub[E.sub];
+    const int ids[3] = {A.ijk[3 * E.rep], A.ijk[3 * E.rep + 1], A.ijk[3 * E.rep + 2]};
+    const int opat = (ids[0] == ids[2]) ? 3 : (ids[0] == ids[1] ? 1 : (ids[1] == ids[2] ? 2 : 0));
+    const int vpat = R.pat, lane = threadIdx.x & 31;
+    double WW[6], VV[6], X[6], Z[6], RW[6];
+    elem_amplitudes<double>(A, R, ids, E.loc, WW, VV);
+    // orbit weights as in k_f2t
+    const double cocc = opat == 0 ? 2.0 : (opat == 3 ? 6.0 / 18.0 : 1.0);
+    const double cen = vpat == 0 ? cocc : (vpat == 3 ? cocc / 6.0 : cocc * 0.5);
+#pragma unroll
+    for (int s = 0; s < 6; s++) X[s] = WW[s] + 0.5 * VV[s];
+    f2_r3(X, Z);
+    f2_r3(WW, RW);
+    const double *ev = A.mo_e + A.o;
+    const double rD = 1.0 / (A.mo_e[ids[0]] + A.mo_e[ids[1]] + A.mo_e[ids[2]] - ev[R.st[0] + E.loc[0]] -
+                             ev[R.st[1] + E.loc[1]] - ev[R.st[2] + E.loc[2]]);
+    double esum = 0.0;
+#pragma unroll
+    for (int s = 0; s < 6; s++) esum += WW[s] * Z[s];
+    // one partial per item, or per warp of it
+    const double en = elem_sum(E.ok ? cen * esum * rD : 0.0, E.all);
+    if (E.ok && (lane & E.all) == 0) A.e_part[(long long)(E.sub * E.warps + (E.el >> 5)) * A.n_ijk + E.rep] = en;
+    if (!A.want_grad) return;
+    const double g0 = cocc * A.ybar * rD;
+    double wb[6], vb[6], w3 = 0.0, v3 = 0.0;
+#pragma unroll
+    for (int s = 0; s < 6; s++) {
+        wb[s] = g0 * (Z[s] + RW[s]);
+        vb[s] = g0 * 0.5 * RW[s];
+        w3 += wb[s];
+        v3 += vb[s];
+    }
+    // equal occupied indices: the orderings that name the same raw amplitudes add up
+#pragma unroll
+    for (int s = 0; s < 6; s++) {
+        const int s1 = perm_compose(s, 2), s2 = perm_compose(s, 1), at = s * kElemThreads + threadIdx.x;
+        sW[at] = opat == 0 ? wb[s] : opat == 1 ? wb[s] + wb[s1] : opat == 2 ? wb[s] + wb[s2] : w3;
+        sV[at] = opat == 0 ? vb[s] : opat == 1 ? vb[s] + vb[s1] : opat == 2 ? vb[s] + vb[s2] : v3;
+    }
+    elem_dd(A, R, E, ids, E.ok ? -cen * A.ybar * esum * rD * rD : 0.0);
+    elem_writeback<0>(A, R, E, ids, opat, vpat, sW, sV);
 }
 
 }  // namespace tb

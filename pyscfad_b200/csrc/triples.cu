@@ -21,6 +21,7 @@
 #include "tc_f1.cuh"
 #include "f2m.cuh"
 #include "f2.cuh"
+#include "f2e.cuh"
 #include "tc_b1.cuh"
 #include "lno.cuh"
 #include "pyscfad_b200.h"
@@ -1332,6 +1333,30 @@ static void for_sub_ranges(const ChunkDesc &ch, F &&f) {
         }
 }
 
+// Elements of one sub-range triple of a chunk (all of them have the same lengths), 512 if they are full
+static int chunk_elems(const ChunkDesc &ch) {
+    return std::min(8, ch.nabc[0]) * std::min(8, ch.nabc[1]) * std::min(8, ch.nabc[2]);
+}
+// CTAs of an element kernel over a chunk, warps (energy partials) of one of its items
+template <typename ARGS>
+static int elem_ctas(const Plan &P, const ARGS &A) {
+    const long long n = (long long)P.n_ijk * A.nsub * A.sub[0].len[0] * A.sub[0].len[1] * A.sub[0].len[2];
+    return (int)((n + kElemThreads - 1) / kElemThreads);
+}
+static int elem_warps(int elems) { return elems > 32 ? elems / 32 : 1; }
+
+// FP64 chunks that go to the element kernel (k_f2e) instead of the orbit kernel (k_f2t): a short
+// sub-range, and enough items that the orbit kernel's CTAs would not run side by side (n_ijk 56 is nocc 6;
+// E + VJP in blocks of 2, nvir 30, element against orbit kernel: nocc 5 7.43 / 7.14 ms, nocc 7 8.2 / 10.1).
+// With the adjoint, items of 256 elements fill the orbit kernel's CTA well enough (nocc 16 nvir 36 =
+// 2 x 16 + 4: 8.5 / 8.35 ms; the energy alone 3.12 / 3.29) and those of 128 need more of them (nvir 34:
+// nocc 7 1.10 / 1.10 ms, nocc 12 3.76 / 3.86, nocc 16 7.64 / 7.95).
+static bool by_element(const Plan &P, const ChunkDesc &ch) {
+    const int e = chunk_elems(ch);
+    if (!P.want_grad) return e < 512 && P.n_ijk >= 56;
+    return e <= 64 ? P.n_ijk >= 56 : e <= 128 && P.n_ijk >= 300;
+}
+
 // Where the regions of a sub-range triple lie in the (blocked) staging and in
 // Wbar (wmul: 2 for the 16-bit hi and lo planes, 1 for FP64).
 static void sub_regions(const ChunkDesc &ch, int o, const int *st, const int *len, int wmul, int elem, F2mSub &u) {
@@ -1393,8 +1418,8 @@ static void f2_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, co
     F.n_ijk = P.n_ijk;
     F.ijk = (int *)(ws + P.off_ijk);
     F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
-    F.S = (const double *)(ws + P.off_S) + (size_t)slot * P.stage_slot;
-    F.SW = P.want_grad ? (double *)(ws + P.off_SW) + (size_t)slot * P.wbar_slot : nullptr;
+    F.S = ws + P.off_S + (size_t)slot * P.stage_slot * sizeof(double);
+    F.SW = P.want_grad ? ws + P.off_SW + (size_t)slot * P.wbar_slot * sizeof(double) : nullptr;
     F.ybar = io.ybar;
     F.want_grad = P.want_grad;
     F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
@@ -1481,7 +1506,7 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
         u.pat = ch.blk[0] == ch.blk[2] ? 3 : (ch.blk[0] == ch.blk[1] ? 1 : (ch.blk[1] == ch.blk[2] ? 2 : 0));
     }
     A.kn = 0;
-    while ((1 << A.kn) < A.sub[0].len[0] * A.sub[0].len[1] * A.sub[0].len[2]) A.kn++;
+    while ((1 << A.kn) < chunk_elems(ch)) A.kn++;
     A.ne = box_slots(ch);
     A.n_ijk = P.n_ijk;
     A.ijk = (int *)(ws + P.off_ijk);
@@ -1502,7 +1527,7 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     A.part = (double *)(ws + P.off_lpart);
     const unsigned items = (unsigned)(P.n_ijk * A.nsub);
     const bool full = A.kn == 9;
-    const unsigned elems = (unsigned)((((long long)items << A.kn) + kElemThreads - 1) / kElemThreads);   // element kernels
+    const unsigned elems = (unsigned)elem_ctas(P, A);
     if (full) TB_KLAUNCH(P_LNO, (k_lno_fwd<StageT><<<items, kLnoThreads, F2Smem<0>::TABLES, st>>>(A)));
     else TB_KLAUNCH(P_LNO, (k_lno_fwd_e<StageT><<<elems, kElemThreads, 0, st>>>(A)));
     // columns per tile: 128 while two buffers of all rows leave room for two CTAs per SM
@@ -1833,15 +1858,25 @@ static int fp64_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t s
         rc = lno_chunk<double>(P, ch[0], st, io, ws);
         if (rc != TRIPLES_OK) return rc;
     } else {
-        Group<F2P, NG> G;
+        // chunks for the orbit kernel and for the element kernel
+        Group<F2P, NG> G, H;
         Group<ChunkAux, NG> X;
+        int norb = 0, nelem = 0;
         for (int c = 0; c < n; c++) {
-            f2_params(P, ch[c], c, ws, io, G.job[c]);
-            X.job[c] = chunk_aux(P, ch[c], c, io, P.n_ijk * G.job[c].nsub);
+            const bool elem = by_element(P, ch[c]);
+            F2P &j = elem ? H.job[nelem++] : G.job[norb++];
+            f2_params(P, ch[c], c, ws, io, j);
+            X.job[c] = chunk_aux(P, ch[c], c, io, P.n_ijk * j.nsub * (elem ? elem_warps(chunk_elems(ch[c])) : 1));
         }
         X.n = n;
-        const int items = group_starts(G, n, [&](const F2P &j) { return P.n_ijk * j.nsub; });
-        TB_KLAUNCH(P_F2, (k_f2t<<<(unsigned)items, kF2Threads, F2Smem<0>::BYTES, st>>>(G)));
+        if (norb > 0) {
+            const int items = group_starts(G, norb, [&](const F2P &j) { return P.n_ijk * j.nsub; });
+            TB_KLAUNCH(P_F2, (k_f2t<<<(unsigned)items, kF2Threads, F2Smem<0>::BYTES, st>>>(G)));
+        }
+        if (nelem > 0) {
+            const int ctas = group_starts(H, nelem, [&](const F2P &j) { return elem_ctas(P, j); });
+            TB_KLAUNCH(P_F2, (k_f2e<<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
+        }
         TB_KLAUNCH(P_F2, (k_energy_sum<<<1, 256, 0, st>>>(X, n)));
     }
     if (!P.want_grad) return TRIPLES_OK;

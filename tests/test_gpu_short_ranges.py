@@ -67,3 +67,35 @@ def test_lno_projection_over_several_ranges(o, v, precision):
     for k in G.KEYS:
         assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < g_tol, k
     torch.cuda.synchronize()
+
+
+# FP64 items of 1 to 256 elements in both kernels that take them (nocc 5 and 6 lie on either
+# side of the rule), chunks of both kinds in one group, several warps to an item (energy partials
+# of nvir 36: 8 warps), nocc above 128; against the oracle or, where that is slow, against the same
+# problem cut into 16-wide blocks.  FP64 sums in another order.
+@pytest.mark.gpu
+@pytest.mark.parametrize("o,v,tv", [(5, 31, 0), (6, 31, 0), (7, 20, 4), (6, 9, 1), (8, 13, 2), (6, 36, 0), (9, 23, 0)])
+def test_fp64_short_ranges_match_the_oracle(o, v, tv):
+    inp = make_inputs(o, v, 40, seed=v, fvo_sigma=1e-3)
+    e_ref, g_ref = O.oracle_energy_vjp(inp)
+    ins = [getattr(inp, k) for k in G.KEYS]
+    e, g = triples.energy_vjp(*ins, precision="fp64", device="cuda", block_size=tv)
+    e1 = triples.energy(*ins, precision="fp64", device="cuda", block_size=tv)
+    assert abs(float(e) - e_ref) <= 1e-12 * abs(e_ref)
+    assert abs(float(e1) - e_ref) <= 1e-12 * abs(e_ref)
+    for k in G.KEYS:
+        assert _relerr(g[k].cpu().numpy(), g_ref[k]) < 1e-10, k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("o,v,tv", [(20, 33, 2), (33, 19, 4), (130, 3, 0), (40, 17, 8)])
+def test_fp64_short_ranges_against_other_blocks(o, v, tv):
+    inp = make_inputs(o, v, 40, seed=v, fvo_sigma=1e-3)
+    ins = [getattr(inp, k) for k in G.KEYS]
+    e0, g0 = triples.energy_vjp(*ins, precision="fp64", device="cuda", block_size=1 if o > 128 else 16)
+    e, g = triples.energy_vjp(*ins, precision="fp64", device="cuda", block_size=tv)
+    e1 = triples.energy(*ins, precision="fp64", device="cuda", block_size=tv)
+    assert abs(float(e) - float(e0)) <= 1e-12 * abs(float(e0))
+    assert abs(float(e1) - float(e0)) <= 1e-12 * abs(float(e0))
+    for k in G.KEYS:
+        assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-10, k
