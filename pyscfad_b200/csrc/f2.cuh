@@ -25,6 +25,7 @@ struct F2P {
     const double *mo_e, *t1, *t2, *ovov, *fvo;
     const void *S;      // W per ordering tau, blocked staging (FP64 rows are not exchanged)
     void *SW;           // Wbar out, per tau at ch.pb[tau].swoff: [y][p][x][q][r][z]
+    const double *wscale;   // power-of-two scale of the fp16 split (element kernel of the mixed modes)
     double ybar;
     int want_grad;
     double *e_part;     // energy partial of each item, at sub * n_ijk + rep

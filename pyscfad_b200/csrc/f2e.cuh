@@ -1,6 +1,6 @@
 // FP64 element kernels: the epilogue of chunks whose sub-ranges are short (a
-// remainder block, or blocks of 4 and less), for the FP64 calls (by_element in
-// triples.cu) and the LNO calls.
+// remainder block, or blocks of 4 and less): the LNO calls, and the canonical ones
+// that by_element (triples.cu) names, the mixed modes' among them.
 //
 // A short item has 1 to 256 elements a, b, c where the orbit kernels (f2.cuh) give
 // every item a CTA with the tables and slots of 512.  Here a thread takes one
@@ -185,10 +185,13 @@ __device__ __forceinline__ void elem_writeback(const ARGS &A, const F2mSub &R, c
     }
 }
 
-// The items of the jobs (chunks) of a launch; a job starts with a new CTA.
-template <typename JOBS>
+// The items of the jobs (chunks) of a launch; a job starts with a new CTA.  SPLIT 0: FP64 staging and
+// Wbar; 1 and 2: FP32 staging, fp16 and bf16 hi/lo Wbar (the mixed modes).
+template <int SPLIT, typename JOBS>
 __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__ JOBS J) {
-    __shared__ double sV[6 * kElemThreads], sW[6 * kElemThreads];
+    using StageT = typename std::conditional<SPLIT == 0, double, float>::type;
+    __shared__ double sV[6 * kElemThreads];
+    __shared__ typename F2Smem<SPLIT>::W sW[6 * kElemThreads];
     JobCursor jcur;
     int blk;
     const int jb = jcur.at(J, (int)blockIdx.x, blk);
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__
     const int opat = (ids[0] == ids[2]) ? 3 : (ids[0] == ids[1] ? 1 : (ids[1] == ids[2] ? 2 : 0));
     const int vpat = R.pat, lane = threadIdx.x & 31;
     double WW[6], VV[6], X[6], Z[6], RW[6];
-    elem_amplitudes<double>(A, R, ids, E.loc, WW, VV);
+    elem_amplitudes<StageT>(A, R, ids, E.loc, WW, VV);
     // orbit weights as in k_f2t
     const double cocc = opat == 0 ? 2.0 : (opat == 3 ? 6.0 / 18.0 : 1.0);
     const double cen = vpat == 0 ? cocc : (vpat == 3 ? cocc / 6.0 : cocc * 0.5);
@@ -217,6 +220,7 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__
     const double en = elem_sum(E.ok ? cen * esum * rD : 0.0, E.all);
     if (E.ok && (lane & E.all) == 0) A.e_part[(long long)(E.sub * E.warps + (E.el >> 5)) * A.n_ijk + E.rep] = en;
     if (!A.want_grad) return;
+    const float wsc = SPLIT > 0 ? (float)*A.wscale : 1.0f;
     const double g0 = cocc * A.ybar * rD;
     double wb[6], vb[6], w3 = 0.0, v3 = 0.0;
 #pragma unroll
@@ -230,11 +234,13 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__
 #pragma unroll
     for (int s = 0; s < 6; s++) {
         const int s1 = perm_compose(s, 2), s2 = perm_compose(s, 1), at = s * kElemThreads + threadIdx.x;
-        sW[at] = opat == 0 ? wb[s] : opat == 1 ? wb[s] + wb[s1] : opat == 2 ? wb[s] + wb[s2] : w3;
+        const double w = opat == 0 ? wb[s] : opat == 1 ? wb[s] + wb[s1] : opat == 2 ? wb[s] + wb[s2] : w3;
+        if constexpr (SPLIT == 0) sW[at] = w;
+        else sW[at] = f2m_split<SPLIT>((float)w, wsc);
         sV[at] = opat == 0 ? vb[s] : opat == 1 ? vb[s] + vb[s1] : opat == 2 ? vb[s] + vb[s2] : v3;
     }
     elem_dd(A, R, E, ids, E.ok ? -cen * A.ybar * esum * rD * rD : 0.0);
-    elem_writeback<0>(A, R, E, ids, opat, vpat, sW, sV);
+    elem_writeback<SPLIT>(A, R, E, ids, opat, vpat, sW, sV);
 }
 
 }  // namespace tb

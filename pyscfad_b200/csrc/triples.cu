@@ -1345,14 +1345,18 @@ static int elem_ctas(const Plan &P, const ARGS &A) {
 }
 static int elem_warps(int elems) { return elems > 32 ? elems / 32 : 1; }
 
-// FP64 chunks that go to the element kernel (k_f2e) instead of the orbit kernel (k_f2t): a short
+// Chunks that go to the element kernel (k_f2e).  FP64, instead of the orbit kernel (k_f2t): a short
 // sub-range, and enough items that the orbit kernel's CTAs would not run side by side (n_ijk 56 is nocc 6;
 // E + VJP in blocks of 2, nvir 30, element against orbit kernel: nocc 5 7.43 / 7.14 ms, nocc 7 8.2 / 10.1).
 // With the adjoint, items of 256 elements fill the orbit kernel's CTA well enough (nocc 16 nvir 36 =
 // 2 x 16 + 4: 8.5 / 8.35 ms; the energy alone 3.12 / 3.29) and those of 128 need more of them (nvir 34:
 // nocc 7 1.10 / 1.10 ms, nocc 12 3.76 / 3.86, nocc 16 7.64 / 7.95).
+// Mixed modes: items of up to 32 elements, in place of k_f2m, which evaluates 512 slots of every item
+// (energy nocc 64 nvir 3 0.84 / 7.4 ms, nocc 32 nvir 7 0.79 / 2.6; E + VJP nocc 16 nvir 17 0.94 / 1.03,
+// nocc 300 nvir 2 73 / 275).  Larger items and fewer of them stay with k_f2m and its FP32 sums.
 static bool by_element(const Plan &P, const ChunkDesc &ch) {
     const int e = chunk_elems(ch);
+    if (P.prec != TRIPLES_PRECISION_FP64) return e <= 32 && P.n_ijk >= 500;
     if (!P.want_grad) return e < 512 && P.n_ijk >= 56;
     return e <= 64 ? P.n_ijk >= 56 : e <= 128 && P.n_ijk >= 300;
 }
@@ -1405,21 +1409,24 @@ static void sub_regions(const ChunkDesc &ch, int o, const int *st, const int *le
     }
 }
 
-// FP64 epilogue parameters of one chunk.
+// Parameters of one chunk for the FP64 epilogue and for the element kernel of any mode.
 static void f2_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, const TriplesIO &io, F2P &F) {
+    const bool mixed = P.prec != TRIPLES_PRECISION_FP64;
+    const size_t el = mixed ? 4 : 8;   // bytes of a staged value, of a Wbar value (hi and lo)
     F.o = P.d.o;
     F.v = P.d.v;
     F.nsub = 0;
     for_sub_ranges(ch, [&](const int *st, const int *len) {
         F2mSub &u = F.sub[F.nsub++];
-        sub_regions(ch, F.o, st, len, 1, 8, u);
+        sub_regions(ch, F.o, st, len, mixed ? 2 : 1, (int)el, u);
         u.pat = st[0] == st[2] ? 3 : (st[0] == st[1] ? 1 : (st[1] == st[2] ? 2 : 0));
     });
     F.n_ijk = P.n_ijk;
     F.ijk = (int *)(ws + P.off_ijk);
     F.mo_e = io.mo_energy; F.t1 = io.t1; F.t2 = io.t2; F.ovov = io.ovov; F.fvo = io.fvo;
-    F.S = ws + P.off_S + (size_t)slot * P.stage_slot * sizeof(double);
-    F.SW = P.want_grad ? ws + P.off_SW + (size_t)slot * P.wbar_slot * sizeof(double) : nullptr;
+    F.S = ws + P.off_S + (size_t)slot * P.stage_slot * el;
+    F.SW = P.want_grad ? ws + P.off_SW + (size_t)slot * P.wbar_slot * el : nullptr;
+    F.wscale = &((Ctrl *)(ws + P.off_ctrl))->slot[slot].wscale;
     F.ybar = io.ybar;
     F.want_grad = P.want_grad;
     F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
@@ -1810,16 +1817,33 @@ static int mixed_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t 
         const int rc = lno_chunk<float>(P, ch[0], st, io, ws);
         if (rc != TRIPLES_OK) return rc;
     } else {
+        // chunks for the persistent epilogue and for the element kernel
         Group<F2M, NG> G;
+        Group<F2P, NG> H;
         Group<ChunkAux, NG> X;
+        int nf2m = 0, nelem = 0;
         for (int c = 0; c < n; c++) {
-            f2m_params(P, ch[c], c, ws, io, false, G.job[c]);
-            X.job[c] = chunk_aux(P, ch[c], c, io, P.n_ijk * G.job[c].nsub);
+            if (by_element(P, ch[c])) {
+                F2P &j = H.job[nelem++];
+                f2_params(P, ch[c], c, ws, io, j);
+                X.job[c] = chunk_aux(P, ch[c], c, io, P.n_ijk * j.nsub * elem_warps(chunk_elems(ch[c])));
+            } else {
+                F2M &j = G.job[nf2m++];
+                f2m_params(P, ch[c], c, ws, io, false, j);
+                X.job[c] = chunk_aux(P, ch[c], c, io, P.n_ijk * j.nsub);
+            }
         }
         X.n = n;
         if (P.want_grad) TB_KLAUNCH(P_PREP, (k_chunk_scale<<<n, 32, 0, st>>>(X)));
-        const int items = group_starts(G, n, [&](const F2M &j) { return P.n_ijk * j.nsub; });
-        TB_KLAUNCH(P_F2, launch_f2m(bf16, st, items, G));
+        if (nf2m > 0) {
+            const int items = group_starts(G, nf2m, [&](const F2M &j) { return P.n_ijk * j.nsub; });
+            TB_KLAUNCH(P_F2, launch_f2m(bf16, st, items, G));
+        }
+        if (nelem > 0) {
+            const int ctas = group_starts(H, nelem, [&](const F2P &j) { return elem_ctas(P, j); });
+            if (bf16) TB_KLAUNCH(P_F2, (k_f2e<2><<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
+            else TB_KLAUNCH(P_F2, (k_f2e<1><<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
+        }
         TB_KLAUNCH(P_F2, (k_energy_sum<<<1, 256, 0, st>>>(X, n)));
     }
     if (!P.want_grad) return TRIPLES_OK;
@@ -1875,7 +1899,7 @@ static int fp64_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t s
         }
         if (nelem > 0) {
             const int ctas = group_starts(H, nelem, [&](const F2P &j) { return elem_ctas(P, j); });
-            TB_KLAUNCH(P_F2, (k_f2e<<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
+            TB_KLAUNCH(P_F2, (k_f2e<0><<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
         }
         TB_KLAUNCH(P_F2, (k_energy_sum<<<1, 256, 0, st>>>(X, n)));
     }

@@ -99,3 +99,23 @@ def test_fp64_short_ranges_against_other_blocks(o, v, tv):
     assert abs(float(e1) - float(e0)) <= 1e-12 * abs(float(e0))
     for k in G.KEYS:
         assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-10, k
+
+
+# The mixed modes' items of up to 32 elements (nocc 14 on: the rule's number of items), in calls that also
+# hold larger ones (nvir 17, 19, 23), with the parity bounds of these modes against FP64.
+@pytest.mark.gpu
+@pytest.mark.parametrize("o,v,tv", [(13, 7, 0), (14, 7, 0), (14, 1, 0), (15, 19, 0), (16, 23, 0), (14, 9, 2), (20, 6, 1)])
+@pytest.mark.parametrize("precision", ["mixed", "mixed_bf16"])
+def test_mixed_short_ranges(o, v, tv, precision):
+    inp = make_inputs(o, v, 40, seed=v, fvo_sigma=1e-3)
+    ins = [getattr(inp, k) for k in G.KEYS]
+    e0, g0 = triples.energy_vjp(*ins, precision="fp64", device="cuda", block_size=tv)
+    e, g = triples.energy_vjp(*ins, precision=precision, device="cuda", block_size=tv)
+    e1 = triples.energy(*ins, precision=precision, device="cuda", block_size=tv)
+    e_tol, g_tol = (1e-6, 1e-5) if precision == "mixed" else (1e-4, 1e-3)
+    scale = 1e-14 if v == 1 else 0.0   # one virtual orbital has no triples: both are rounding noise
+    assert abs(float(e) - float(e0)) <= e_tol * abs(float(e0)) + scale
+    assert abs(float(e1) - float(e0)) <= e_tol * abs(float(e0)) + scale
+    if v > 1:
+        for k in G.KEYS:
+            assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < g_tol, k
