@@ -1064,7 +1064,8 @@ static int gemm_dispatch(const GemmTile &t, F &&f) {
 }
 
 // Shared memory above the default 48 KB needs an opt-in per kernel and device
-// (the attribute call is idempotent and cheap next to a launch).
+// (the attribute call is idempotent and cheap next to a launch).  `bytes` is the same
+// in every call for a kernel: host threads share the limit.
 template <typename K>
 static int smem_optin(K kernel, size_t bytes) {
     TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
@@ -1473,8 +1474,6 @@ static int lno_projections(const LnoArgs &A, cudaStream_t st, unsigned &grid) {
     const long long tiles = ((long long)A.o * A.o * A.ne + COLS - 1) / COLS;   // (a CTA has one tile at least)
     grid = (unsigned)std::min(tiles, (long long)2 * num_sms());
     const size_t smem = LnoProj<COLS>::smem(A.o);
-    const int rc = smem_optin(k_lno_proj<COLS, FULL>, smem);
-    if (rc != TRIPLES_OK) return rc;
     for (int slot = 2; slot >= 0; slot--)
         TB_KLAUNCH(P_LNO_PROJ, (k_lno_proj<COLS, FULL><<<grid, kLnoThreads, smem, st>>>(A, slot, slot == 2 ? 1 : 0)));
     return TRIPLES_OK;
@@ -1486,6 +1485,16 @@ static int lno_chunk(const Plan &P, const ChunkDesc &ch, cudaStream_t st, const 
     {
         const int rc = once_per_device(mixed ? INIT_LNO : INIT_LNO64, [&]() -> int {
             int rc = smem_optin(k_lno_fwd<StageT>, F2Smem<0>::TABLES);
+            // the projections for the largest nocc of each: a limit set per call would be changed
+            // by another host thread between that and the launch
+            auto proj = [&](auto cols) {
+                using C = LnoProj<decltype(cols)::value>;
+                if (rc == TRIPLES_OK) rc = smem_optin(k_lno_proj<decltype(cols)::value, true>, C::smem(C::MAXO));
+                if (rc == TRIPLES_OK) rc = smem_optin(k_lno_proj<decltype(cols)::value, false>, C::smem(C::MAXO));
+            };
+            proj(std::integral_constant<int, 128>{});
+            proj(std::integral_constant<int, 64>{});
+            proj(std::integral_constant<int, 32>{});
             if (rc != TRIPLES_OK) return rc;
             if (!mixed) return smem_optin(k_lno_adj<0>, F2Smem<0>::BYTES);
             if ((rc = smem_optin(k_lno_adj<1>, F2Smem<1>::BYTES)) != TRIPLES_OK) return rc;

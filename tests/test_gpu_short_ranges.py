@@ -119,3 +119,29 @@ def test_mixed_short_ranges(o, v, tv, precision):
     if v > 1:
         for k in G.KEYS:
             assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < g_tol, k
+
+
+# Host threads with different nocc share the projection kernel of their range; each call must find the shared
+# memory that it asks for, whatever another thread is launching.
+@pytest.mark.gpu
+def test_lno_calls_of_host_threads_do_not_disturb_each_other():
+    from concurrent.futures import ThreadPoolExecutor
+
+    sizes = (9, 10, 12, 14, 16, 9, 13, 16)
+    problems = []
+    for t, o in enumerate(sizes):
+        inp = make_inputs(o, 3, 20, seed=t, fvo_sigma=1e-3)
+        ins = [torch.as_tensor(np.ascontiguousarray(getattr(inp, k)), device="cuda") for k in G.KEYS]
+        problems.append((torch.eye(o, dtype=torch.float64, device="cuda"), ins, torch.cuda.Stream()))
+    e_ref = [float(triples.lno_energy(m, *ins)) for m, ins, _ in problems]
+    torch.cuda.synchronize()
+
+    def work(t):
+        m, ins, st = problems[t]
+        with torch.cuda.stream(st):
+            return [float(triples.lno_energy(m, *ins)) for _ in range(300)]
+
+    with ThreadPoolExecutor(len(sizes)) as pool:
+        results = list(pool.map(work, range(len(sizes))))
+    for t in range(len(sizes)):
+        assert max(abs(e - e_ref[t]) for e in results[t]) <= 1e-12 * abs(e_ref[t])
