@@ -45,7 +45,7 @@ extern "C" {
 enum triples_status {
     TRIPLES_OK = 0,
     TRIPLES_ERR_INVALID_ARGUMENT = 1,  /* bad size, null pointer, bad enum */
-    TRIPLES_ERR_WORKSPACE = 2,         /* workspace smaller than triples_workspace_size() */
+    TRIPLES_ERR_WORKSPACE = 2,         /* workspace smaller than triples_workspace_least() */
     TRIPLES_ERR_CUDA = 3,              /* a CUDA call failed; see triples_last_cuda_error() */
     TRIPLES_ERR_UNSUPPORTED = 4,       /* precision / device not supported */
     TRIPLES_ERR_DEVICE_TIMEOUT = 5     /* a bounded device-side wait gave up */
@@ -96,6 +96,14 @@ size_t triples_workspace_size_ex(int precision, int nocc, int nvir, int ovvv_pac
  * most about 2 GiB).  A workspace of triples_workspace_size_ex() bytes, or of
  * triples_df_workspace_size() for the DF calls, is always enough. */
 size_t triples_workspace_extra(int precision, int nocc, int nvir, int ovvv_packed, int want_grad,
+                               const triples_options *opt);
+
+/* What the same call cannot do without, where memory is short: at most
+ * triples_workspace_size_ex() bytes.  The mixed modes then gather the V-term
+ * entries for every work item instead of preparing tables (up to 12 % of the
+ * workspace; the same values).  For the DF calls take the difference off
+ * triples_df_workspace_size(). */
+size_t triples_workspace_least(int precision, int nocc, int nvir, int ovvv_packed, int want_grad,
                                const triples_options *opt);
 
 /* E(T) into *e_out (device FP64 scalar).
@@ -298,6 +306,10 @@ typedef struct triples_batch triples_batch;   /* opaque */
 /* Bytes of device workspace a batch of these problems needs (0 on invalid
  * arguments): every problem's workspace plus the batch's job tables. */
 size_t triples_batch_workspace_size(int precision, int nprob, const triples_problem *probs);
+
+/* The same with triples_workspace_least() for every problem: the least that
+ * triples_batch_create takes. */
+size_t triples_batch_workspace_least(int precision, int nprob, const triples_problem *probs);
 
 /* Plans the batch over `workspace` and writes its job tables there (a
  * blocking host-to-device copy: not for stream capture).  The problems'

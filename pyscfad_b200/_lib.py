@@ -77,6 +77,8 @@ def load():
                                           [_c_double, _c_int, _opt, _vp, _c_size, _vp] + [_vp] * 7)
     lib.triples_workspace_extra.restype = _c_size
     lib.triples_workspace_extra.argtypes = [_c_int] * 5 + [_opt]
+    lib.triples_workspace_least.restype = _c_size
+    lib.triples_workspace_least.argtypes = [_c_int] * 5 + [_opt]
     lib.triples_lno_workspace_size_ex.restype = _c_size
     lib.triples_lno_workspace_size_ex.argtypes = [_c_int] * 5 + [_opt]
     lib.triples_lno_energy_vjp_ex.restype = _c_int
@@ -103,6 +105,8 @@ def load():
     _prob = ctypes.POINTER(Problem)
     lib.triples_batch_workspace_size.restype = _c_size
     lib.triples_batch_workspace_size.argtypes = [_c_int, _c_int, _prob]
+    lib.triples_batch_workspace_least.restype = _c_size
+    lib.triples_batch_workspace_least.argtypes = [_c_int, _c_int, _prob]
     lib.triples_batch_create.restype = _c_int
     lib.triples_batch_create.argtypes = [_c_int, _c_int, _prob, _c_double, _vp, _c_size, ctypes.POINTER(_vp)]
     lib.triples_batch_run.restype = _c_int

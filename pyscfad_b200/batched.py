@@ -168,7 +168,11 @@ class BatchedTriples:
         nbytes = int(self.lib.triples_batch_workspace_size(self.prec, n, arr))
         if nbytes == 0:
             raise _lib.TriplesError(1, "triples_batch_workspace_size")
-        self.batch_workspace = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+        try:
+            self.batch_workspace = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+        except torch.cuda.OutOfMemoryError:
+            nbytes = int(self.lib.triples_batch_workspace_least(self.prec, n, arr))
+            self.batch_workspace = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         handle = ctypes.c_void_p()
         torch.cuda.synchronize(self.device)
         _lib.check(self.lib.triples_batch_create(self.prec, n, arr, 1.0, self.batch_workspace.data_ptr(), nbytes,

@@ -83,9 +83,9 @@ def _check_memory(mycc, t1, ovvv, precision):
     workspace."""
     nocc, nvir = t1.shape
     packed = len(ovvv.shape) == 3
-    need = triples.workspace_size(nocc, nvir, packed, True, precision)
+    need = triples.workspace_least(nocc, nvir, packed, True, precision)
     if torch.cuda.is_available() and not triples.holds_workspace(need):
-        free, _ = torch.cuda.mem_get_info()
+        free = triples.free_memory(need)
         if need > free:
             raise RuntimeError(f"_ccsd_t_energy_vjp: at least {need / 1e6:.0f} MB of device memory "
                                f"needed, {free / 1e6:.0f} MB free.")

@@ -2007,7 +2007,7 @@ static void batch_chunks(const Plan &P, std::vector<ChunkDesc> &out) {
 // Plans, workspace offsets and (with image != nullptr) the job tables of a
 // batch; B.ws must then be the device workspace the tables point into.
 static int batch_build(Batch &B, int prec, int nprob, const triples_problem *probs, double ybar,
-                       std::vector<char> *image) {
+                       std::vector<char> *image, bool vtables) {
     if (nprob < 1 || !probs) return TRIPLES_ERR_INVALID_ARGUMENT;
     B.prec = prec;
     B.nprob = nprob;
@@ -2020,7 +2020,7 @@ static int batch_build(Batch &B, int prec, int nprob, const triples_problem *pro
         triples_options opt{};
         opt.block_size = q.block_size;
         opt.tile_n = q.tile_n;
-        const int rc = make_plan(prec, q.nocc, q.nvir, q.ovvv_packed, 1, B.plans[p], 0, &opt);
+        const int rc = make_plan(prec, q.nocc, q.nvir, q.ovvv_packed, 1, B.plans[p], 0, &opt, vtables);
         if (rc != TRIPLES_OK) return rc;
         B.ws_off[p] = off;
         off = align256(off + B.plans[p].total);
@@ -2226,6 +2226,13 @@ size_t triples_workspace_extra(int precision, int nocc, int nvir, int ovvv_packe
     if (tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, P, 0, opt) != TRIPLES_OK) return 0;
     if (tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, Q, 0, opt, true, tb::kMaxGroup) != TRIPLES_OK) return 0;
     return Q.total > P.total ? Q.total - P.total : 0;
+}
+
+size_t triples_workspace_least(int precision, int nocc, int nvir, int ovvv_packed, int want_grad,
+                               const triples_options *opt) {
+    tb::Plan P;
+    if (tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, P, 0, opt, false) != TRIPLES_OK) return 0;
+    return P.total;
 }
 
 static int triples_call(void *stream, int precision, int nocc, int nvir, int ovvv_packed, int want_grad,
@@ -2540,7 +2547,13 @@ struct triples_batch {
 
 size_t triples_batch_workspace_size(int precision, int nprob, const triples_problem *probs) {
     tb::Batch B;
-    if (tb::batch_build(B, precision, nprob, probs, 1.0, nullptr) != TRIPLES_OK) return 0;
+    if (tb::batch_build(B, precision, nprob, probs, 1.0, nullptr, true) != TRIPLES_OK) return 0;
+    return B.total;
+}
+
+size_t triples_batch_workspace_least(int precision, int nprob, const triples_problem *probs) {
+    tb::Batch B;
+    if (tb::batch_build(B, precision, nprob, probs, 1.0, nullptr, false) != TRIPLES_OK) return 0;
     return B.total;
 }
 
@@ -2549,18 +2562,20 @@ int triples_batch_create(int precision, int nprob, const triples_problem *probs,
     if (!batch) return TRIPLES_ERR_INVALID_ARGUMENT;
     *batch = nullptr;
     if (!workspace) return TRIPLES_ERR_WORKSPACE;
-    {
-        // the workspace must hold the batch before any table points into it
+    // the workspace must hold the batch before any table points into it
+    bool vtables = true;
+    for (;; vtables = false) {
         tb::Batch sizing;
-        const int rc = tb::batch_build(sizing, precision, nprob, probs, ybar, nullptr);
+        const int rc = tb::batch_build(sizing, precision, nprob, probs, ybar, nullptr, vtables);
         if (rc != TRIPLES_OK) return rc;
-        if (workspace_bytes < sizing.total) return TRIPLES_ERR_WORKSPACE;
+        if (workspace_bytes >= sizing.total) break;
+        if (!vtables) return TRIPLES_ERR_WORKSPACE;
     }
     triples_batch *h = new (std::nothrow) triples_batch;
     if (!h) return TRIPLES_ERR_INVALID_ARGUMENT;
     h->b.ws = (char *)workspace;
     std::vector<char> image;
-    int rc = tb::batch_build(h->b, precision, nprob, probs, ybar, &image);
+    int rc = tb::batch_build(h->b, precision, nprob, probs, ybar, &image, vtables);
     if (rc == TRIPLES_OK && !image.empty()) {
         const cudaError_t e = cudaMemcpy(h->b.ws + h->b.tables_off, image.data(), image.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {

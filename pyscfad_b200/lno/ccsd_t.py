@@ -59,7 +59,7 @@ def _check_memory(nocc, nvir, packed, want_grad, precision="fp64"):
     cannot hold the workspace."""
     need = triples.lno_workspace_size(nocc, nvir, packed, want_grad, precision)
     if torch.cuda.is_available() and not triples.holds_workspace(need):
-        free, _ = torch.cuda.mem_get_info()
+        free = triples.free_memory(need)
         if need > free:
             raise RuntimeError(f"{need / 1e6:.0f} MB more memory is needed "
                                f"({free / 1e6:.0f} MB of device memory free).")

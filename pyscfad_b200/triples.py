@@ -18,29 +18,72 @@ KEYS = ("mo_energy", "t1", "t2", "ovoo", "ovov", "ovvv", "fvo")
 # share scratch, so they may run concurrently.
 _workspaces: dict = {}
 
+# How much of their optional scratch streams do without because device memory was short: 1 the
+# chunk groups, 2 the V-term tables as well (until release_workspace).
+_without: dict = {}
 
-# Streams on which the extra bytes once did not fit: their calls do without.
-_no_extra: set = set()
+
+def _key(device, stream):
+    return (device.type, device.index, int(stream.cuda_stream))
 
 
-def _workspace(nbytes: int, device: torch.device, stream, extra: int = 0) -> torch.Tensor:
-    """At least nbytes of scratch, and `extra` more (triples_workspace_extra) while the device has room."""
-    key = (device.type, device.index, int(stream.cuda_stream))
-    if key in _no_extra:
-        extra = 0
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes + extra:
+def _alloc(nbytes: int, device: torch.device, stream) -> torch.Tensor:
+    # allocated on its own stream: given back, the memory is reused behind that stream's work
+    with torch.cuda.stream(stream):
+        return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+
+
+def _workspace(nbytes: int, device: torch.device, stream, extra: int = 0, least=None) -> torch.Tensor:
+    """Scratch of nbytes, with `extra` more while the device has room for it (triples_workspace_extra); where
+    it has not even room for nbytes, of least() bytes (triples_workspace_least)."""
+    key = _key(device, stream)
+    while True:
+        level = _without.get(key, 0)
+        want = nbytes + extra if level == 0 else nbytes if level == 1 or least is None else least()
+        buf = _workspaces.get(key)
+        if buf is not None and buf.numel() >= want:
+            return buf
         _workspaces.pop(key, None)
         del buf
         try:
-            buf = torch.empty(max(nbytes + extra, 256), dtype=torch.uint8, device=device)
+            buf = _workspaces[key] = _alloc(want, device, stream)
+            return buf
         except torch.cuda.OutOfMemoryError:
-            if extra == 0:
+            if level >= 2 or least is None:
                 raise
-            _no_extra.add(key)
-            buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
+            _without[key] = level + 1
+
+
+def _give_back(device: torch.device) -> bool:
+    """Drop the scratch of the device's streams that may hold more than their calls need; these calls
+    take less from now on.  False if there was none."""
+    index = torch.cuda.current_device() if device.index is None else device.index
+    keys = [k for k in list(_workspaces) if k[0] == device.type and k[1] in (index, None) and _without.get(k, 0) < 2]
+    for k in keys:
+        _without[k] = _without.get(k, 0) + 1
+        _workspaces.pop(k, None)
+    return bool(keys)
+
+
+def _with_room(device: torch.device, call):
+    """call(), and again with optional scratch given back while the device memory does not suffice (for
+    the scratch, the outputs or the inputs' copies)."""
+    while True:
+        try:
+            return call()
+        except torch.cuda.OutOfMemoryError:
+            if not _give_back(device):
+                raise
+
+
+def free_memory(need: int) -> int:
+    """Free bytes of the current device, with the optional scratch given back first where they are
+    fewer than need."""
+    free, _ = torch.cuda.mem_get_info()
+    if need > free and _give_back(torch.device("cuda", torch.cuda.current_device())):
+        torch.cuda.empty_cache()
+        free, _ = torch.cuda.mem_get_info()
+    return free
 
 
 def holds_workspace(nbytes: int) -> bool:
@@ -54,7 +97,7 @@ def holds_workspace(nbytes: int) -> bool:
 
 def release_workspace():
     _workspaces.clear()
-    _no_extra.clear()
+    _without.clear()
 
 
 def _as_dev(x, device) -> torch.Tensor:
@@ -113,12 +156,28 @@ def workspace_size(nocc, nvir, packed=True, want_grad=True, precision="fp64", bl
                                                      int(want_grad), ctypes.byref(opt)))
 
 
+def workspace_least(nocc, nvir, packed=True, want_grad=True, precision="fp64") -> int:
+    """Scratch below which a call is refused: workspace_size without what only makes it faster."""
+    return int(_lib.load().triples_workspace_least(_lib.PRECISION[precision], nocc, nvir, int(packed), int(want_grad),
+                                                   None))
+
+
+def _optional(prec, o, v, packed, want_grad, opt):
+    """The extra and least arguments of _workspace for a canonical plan."""
+    lib, args = _lib.load(), (prec, o, v, int(packed), int(want_grad), ctypes.byref(opt) if opt is not None else None)
+    return lib.triples_workspace_extra(*args), lambda: lib.triples_workspace_least(*args)
+
+
 def _device_of(device, t1):
     return torch.device(device or (t1.device if isinstance(t1, torch.Tensor) and t1.is_cuda else "cuda"))
 
 
-def _run(mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, device, stream, check,
-         block_size, chunk_range, accumulation_segment, tile_n=0):
+def _run(*args):
+    return _with_room(_device_of(args[10], args[1]), lambda: _run_once(*args))
+
+
+def _run_once(mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, device, stream, check,
+              block_size, chunk_range, accumulation_segment, tile_n=0):
     lib = _lib.load()
     device = _device_of(device, t1)
     args = [_as_dev(a, device) for a in (mo_energy, t1, t2, ovoo, ovov, ovvv, fvo)]
@@ -129,10 +188,9 @@ def _run(mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, d
     if nbytes == 0:
         raise _lib.TriplesError(1, "triples_workspace_size_ex")
     st = stream if stream is not None else torch.cuda.current_stream(device)
-    ws = _workspace(nbytes, device, st,
-                    lib.triples_workspace_extra(prec, o, v, int(packed), int(want_grad), ctypes.byref(opt)))
     e = torch.zeros((), dtype=torch.float64, device=device)
     grads = {k: torch.empty_like(a) for k, a in zip(KEYS, args)} if want_grad else {}
+    ws = _workspace(nbytes, device, st, *_optional(prec, o, v, packed, want_grad, opt))   # the outputs must fit first
     gptr = [grads[k].data_ptr() for k in KEYS] if want_grad else [None] * len(KEYS)
     rc = lib.triples_energy_vjp_ex(st.cuda_stream, prec, o, v, int(packed), *[a.data_ptr() for a in args],
                                    float(ybar), int(want_grad), ctypes.byref(opt), ws.data_ptr(), ws.numel(),
@@ -175,8 +233,12 @@ def lno_workspace_size(nocc, nvir, packed=True, want_grad=True, precision="fp64"
                                                          int(want_grad), ctypes.byref(opt)))
 
 
-def _run_lno(mat, mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, device, stream, check,
-             block_size):
+def _run_lno(*args):
+    return _with_room(_device_of(args[11], args[2]), lambda: _run_lno_once(*args))
+
+
+def _run_lno_once(mat, mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, device, stream, check,
+                  block_size):
     lib = _lib.load()
     device = _device_of(device, t1)
     args = [_as_dev(a, device) for a in (mat, mo_energy, t1, t2, ovoo, ovov, ovvv, fvo)]
@@ -188,10 +250,10 @@ def _run_lno(mat, mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, pre
     if nbytes == 0:
         raise _lib.TriplesError(4 if o > 64 else 1, "triples_lno_workspace_size_ex")
     st = stream if stream is not None else torch.cuda.current_stream(device)
-    ws = _workspace(nbytes, device, st)
     e = torch.zeros((), dtype=torch.float64, device=device)
     keys = ("mat",) + KEYS
     grads = {k: torch.empty_like(a) for k, a in zip(keys, args)} if want_grad else {}
+    ws = _workspace(nbytes, device, st)
     gptr = [grads[k].data_ptr() for k in keys] if want_grad else [None] * len(keys)
     rc = lib.triples_lno_energy_vjp_ex(st.cuda_stream, prec, o, v, int(packed), *[a.data_ptr() for a in args],
                                        float(ybar), int(want_grad), ctypes.byref(opt), ws.data_ptr(), ws.numel(),
@@ -238,21 +300,7 @@ def energy_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, precision="fp64", de
               check=True) -> torch.Tensor:
     """E(T) with ovvv built on the device from the DF factors as pyscfad's DF
     ERIs build it (dfccsd.py:77-88): Lov[naux, o*v], Lvv[naux, v(v+1)/2] packed."""
-    lib = _lib.load()
-    device = torch.device(device or (t1.device if isinstance(t1, torch.Tensor) and t1.is_cuda else "cuda"))
-    args, o, v, naux = _df_args(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, device)
-    prec = _lib.PRECISION[precision]
-    nbytes = lib.triples_df_workspace_size(prec, o, v, naux, 0)
-    if nbytes == 0:
-        raise _lib.TriplesError(1, "triples_df_workspace_size")
-    st = stream if stream is not None else torch.cuda.current_stream(device)
-    ws = _workspace(nbytes, device, st, lib.triples_workspace_extra(prec, o, v, 1, 0, None))
-    e = torch.zeros((), dtype=torch.float64, device=device)
-    rc = lib.triples_energy_df(st.cuda_stream, prec, o, v, naux, *[a.data_ptr() for a in args], ws.data_ptr(),
-                               ws.numel(), e.data_ptr())
-    _lib.check(rc, "triples_energy_df")
-    if check:
-        _lib.check(lib.triples_check_device_status(st.cuda_stream, ws.data_ptr()), "triples_energy_df (device)")
+    e, _ = _run_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, 1.0, False, precision, device, stream, check)
     return e
 
 
@@ -261,22 +309,39 @@ def energy_vjp_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar=1.0, precis
     """E(T) and its VJP with respect to the DF factors instead of ovvv: the
     dict holds "Lov" [naux, o*v] and "Lvv" [naux, v(v+1)/2] (one entry per
     packed pair) next to the other inputs' cotangents."""
+    return _run_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, True, precision, device, stream, check)
+
+
+def _run_df(*args):
+    return _with_room(_device_of(args[11], args[1]), lambda: _run_df_once(*args))
+
+
+def _run_df_once(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, want_grad, precision, device, stream, check):
     lib = _lib.load()
-    device = torch.device(device or (t1.device if isinstance(t1, torch.Tensor) and t1.is_cuda else "cuda"))
+    device = _device_of(device, t1)
     args, o, v, naux = _df_args(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, device)
     prec = _lib.PRECISION[precision]
-    nbytes = lib.triples_df_workspace_size(prec, o, v, naux, 1)
+    nbytes = lib.triples_df_workspace_size(prec, o, v, naux, int(want_grad))
     if nbytes == 0:
         raise _lib.TriplesError(1, "triples_df_workspace_size")
     st = stream if stream is not None else torch.cuda.current_stream(device)
-    ws = _workspace(nbytes, device, st, lib.triples_workspace_extra(prec, o, v, 1, 1, None))
     e = torch.zeros((), dtype=torch.float64, device=device)
-    grads = {k: torch.empty_like(a) for k, a in zip(DF_KEYS, args)}
-    rc = lib.triples_energy_vjp_df(st.cuda_stream, prec, o, v, naux, *[a.data_ptr() for a in args], float(ybar),
-                                   ws.data_ptr(), ws.numel(), e.data_ptr(), *[grads[k].data_ptr() for k in DF_KEYS])
-    _lib.check(rc, "triples_energy_vjp_df")
+    grads = {k: torch.empty_like(a) for k, a in zip(DF_KEYS, args)} if want_grad else {}
+    extra, least = _optional(prec, o, v, True, want_grad, None)
+    # (the plan's optional part is that of a canonical call; ovvv and its cotangent lie behind it)
+    ws = _workspace(nbytes, device, st, extra,
+                    lambda: nbytes - lib.triples_workspace_size(prec, o, v, 1, int(want_grad)) + least())
+    ins = [a.data_ptr() for a in args]
+    if want_grad:
+        name = "triples_energy_vjp_df"
+        rc = lib.triples_energy_vjp_df(st.cuda_stream, prec, o, v, naux, *ins, float(ybar), ws.data_ptr(), ws.numel(),
+                                       e.data_ptr(), *[grads[k].data_ptr() for k in DF_KEYS])
+    else:
+        name = "triples_energy_df"
+        rc = lib.triples_energy_df(st.cuda_stream, prec, o, v, naux, *ins, ws.data_ptr(), ws.numel(), e.data_ptr())
+    _lib.check(rc, name)
     if check:
-        _lib.check(lib.triples_check_device_status(st.cuda_stream, ws.data_ptr()), "triples_energy_vjp_df (device)")
+        _lib.check(lib.triples_check_device_status(st.cuda_stream, ws.data_ptr()), name + " (device)")
     return e, grads
 
 
