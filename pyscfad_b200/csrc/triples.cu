@@ -1937,24 +1937,23 @@ static int run_impl(const Plan &P, cudaStream_t st, const TriplesIO &io) {
         if ((prc = setup_tensor_cores()) != TRIPLES_OK) return prc;
     }
 
-    std::vector<ChunkDesc> chunks;
+    // the chunks of a group (P.group at most) run in one launch per kernel
+    ChunkDesc ch[kMaxGroup];
+    int n = 0;
+    auto run_group = [&]() -> int {
+        if (n == 0) return TRIPLES_OK;
+        const int rc = mixed ? (n == 1 ? mixed_chunks<1>(P, ch, n, st, io, M) : mixed_chunks<kMaxGroup>(P, ch, n, st, io, M))
+                             : (n == 1 ? fp64_chunks<1>(P, ch, n, st, io) : fp64_chunks<kMaxGroup>(P, ch, n, st, io));
+        n = 0;
+        return rc;
+    };
     for (int A = P.a0; A < P.nb && (P.a1 <= 0 || A < P.a1); A++)
         for (int B = 0; B <= A; B++)
             for (int C = 0; C <= B; C++) {
-                chunks.emplace_back();
-                make_chunk(d, A, B, C, chunks.back());
+                make_chunk(d, A, B, C, ch[n++]);
+                if (n == P.group && (prc = run_group()) != TRIPLES_OK) return prc;
             }
-    // the chunks of a group (P.group at most) run in one launch per kernel
-    for (size_t c0 = 0; c0 < chunks.size(); c0 += P.group) {
-        const int n = (int)std::min((size_t)P.group, chunks.size() - c0);
-        const ChunkDesc *ch = &chunks[c0];
-        if (mixed) {
-            prc = n == 1 ? mixed_chunks<1>(P, ch, n, st, io, M) : mixed_chunks<kMaxGroup>(P, ch, n, st, io, M);
-        } else {
-            prc = n == 1 ? fp64_chunks<1>(P, ch, n, st, io) : fp64_chunks<kMaxGroup>(P, ch, n, st, io);
-        }
-        if (prc != TRIPLES_OK) return prc;
-    }
+    if ((prc = run_group()) != TRIPLES_OK) return prc;
     return fold_launches(P, st, io);
 }
 
