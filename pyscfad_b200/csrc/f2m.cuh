@@ -236,10 +236,23 @@ struct F2mLoad {
 // Out of line: the instruction cache holds the code of an item only if its
 // rare paths are short.
 __device__ __noinline__ void f2m_wait_slow(uint64_t *bar, uint32_t parity, volatile int *abortp, int *err) {
-    if (!mbar_wait(bar, parity, abortp)) {
+    if (*abortp == 0 && !mbar_wait(bar, parity, abortp)) {
         *abortp = 1;
+        // no stage reaches its count of readers any more, so none is refilled
+        for (int s = 1; s <= kF2mStages; s++) atomicAdd((int *)abortp - s, 1 << 16);
         atomicOr(err, 64);
     }
+}
+
+// After a wait that gave up no further copy is issued, and those in flight land before the CTA ends: each of
+// the threads 0 to kF2mStages + 1 waits (with the same limit) for the phase that its barrier is in.  A
+// stage or table buffer has at most one load outstanding, because its next one is issued only after every
+// warp has waited for it, or not at all.  (A barrier without one waits to the limit.)
+__device__ __noinline__ void f2m_drain(uint64_t *bar) {
+    const uint32_t phase = mbar_try_wait(bar, 0) ? 1u : 0u;
+#pragma unroll 1
+    for (uint32_t i = 0; i < kSpinLimit && !mbar_try_wait(bar, phase); i++)
+        if ((i & 255u) == 255u) __nanosleep(32);
 }
 
 // W stage n of the CTA (one warp): the regions of (item, rho) of a load record;
@@ -282,12 +295,14 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
     uint2 *sRes = reinterpret_cast<uint2 *>(smem + C::OFF_RES);
     F2mTask *s_rec = reinterpret_cast<F2mTask *>(smem + C::OFF_REC);
     __shared__ uint64_t full[kF2mStages], tfull[2];
-    __shared__ unsigned s_read[kF2mStages];        // warps that have read the stage
+    // warps that have read the stage, abort flag, next item of the CTA by parity of the current one
+    // (one array: the flag follows the counts, and the static arrays stay within 2048 bytes)
+    __shared__ unsigned s_read[kF2mStages + 3];
     __shared__ unsigned s_task[36];                // per (pi, rho): slots of pi, of rho, and s with s o rho = pi
     __shared__ __align__(16) double s_en[2][32];   // energies of the item: 8 per slot, then i, j, k
     __shared__ __align__(16) int s_res[3][8];      // byte offsets of f2m_res
     __shared__ double s_part[8][14];               // per-warp partials: c, b, a sums (4 each), energy
-    __shared__ int s_abort, s_next[2];             // next item of the CTA, by parity of the current one
+    int *const s_next = reinterpret_cast<int *>(&s_read[kF2mStages + 1]);
     __shared__ __align__(16) F2mLoad s_load[2];    // of the current and the next item
     __shared__ F2mItem s_item[2];
     __shared__ unsigned s_tasks[2];                // regions handed out for write-back
@@ -295,7 +310,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned *ticket = J.job[0].ticket;
     if (tid == 0) {
-        s_abort = 0;
+        s_read[kF2mStages] = 0u;
         s_next[0] = (int)(gridDim.x + atomicAdd(ticket, 1u));
         for (int s = 0; s < kF2mStages; s++) {
             mbar_init(&full[s], 2);
@@ -315,7 +330,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
         s_task[tid] = (unsigned)(pp[0] | (pp[1] << 2) | (pp[2] << 4) | (pr[0] << 6) | (pr[1] << 8) | (pr[2] << 10) | (s << 12));
     }
     __syncthreads();
-    volatile int *abortp = &s_abort;
+    volatile int *abortp = reinterpret_cast<volatile int *>(&s_read[kF2mStages]);
     // Job of global item w and the item in it (w only grows).
     using Item = F2mItem;
     JobCursor jcur;
@@ -332,8 +347,8 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
         I.wscale = P.want_grad ? (float)*P.wscale : 1.0f;
         return I;
     };
-    // every wait is bounded; after a timeout the remaining items run through
-    // without waiting (no address depends on the data) and the status bit is set
+    // every wait is bounded; after a timeout the status bit is set, nothing more is loaded and the
+    // remaining items run through without waiting (no address depends on the data)
     auto wait = [&](uint64_t *bar, uint32_t parity) {
         if (!mbar_try_wait(bar, parity)) f2m_wait_slow(bar, parity, abortp, J.job[0].err);
     };
@@ -659,7 +674,7 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
         }
         f2m_bar(2);   // results and partials visible
         // (these warps take fewer regions below)
-        if (warp == 1 && more) issue_tables(s_item[(k & 1) ^ 1], tb_ ^ 1);
+        if (warp == 1 && more && s_read[kF2mStages] == 0u) issue_tables(s_item[(k & 1) ^ 1], tb_ ^ 1);
         if (warp == 2 && s_next[(k & 1) ^ 1] < nitems) announce(s_next[(k & 1) ^ 1], k & 1);
         if (warp == 0) {
             // warps with bit 0, 1, 2 = bit 2 of c, bit 2 of b, bit 1 of a
@@ -851,6 +866,8 @@ __global__ void __launch_bounds__(kF2mThreads, 2) k_f2m(const __grid_constant__ 
         if (!more) break;
         cur = s_item[(k & 1) ^ 1];
     }
+    __syncthreads();   // (every warp's waits are behind)
+    if (*abortp && tid < kF2mStages + 2) f2m_drain(tid < kF2mStages ? &full[tid] : &tfull[tid - kF2mStages]);
 }
 
 }  // namespace tb

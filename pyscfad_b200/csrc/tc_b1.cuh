@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kB1Threads, 1) k_b1_tc(const __grid_constant__
     const TcB1Params &Pfirst = J.job[0];
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     if ((smem_u32(smem_raw) & 1023u) != 0) {   // the swizzle's pattern counts from 1024 B boundaries
-        if (threadIdx.x == 0) atomicOr(Pfirst.err, 64);
+        if (threadIdx.x == 0) atomicOr(Pfirst.err, 128);
         return;
     }
     uint8_t *smem = smem_raw + 1024;

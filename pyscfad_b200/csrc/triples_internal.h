@@ -31,7 +31,9 @@ struct ChunkSlot {
 
 // Control block (workspace offset 0)
 struct Ctrl {
-    int err;                      // device-side error bits (bounded waits that gave up)
+    int err;                      // device-side error bits: bounded waits that gave up (1, 2, 4: W contraction's
+                                  // producer, MMA, epilogue; 8, 16, 32: adjoint contractions'; 64: mixed
+                                  // epilogue), 128: misaligned shared memory of the adjoint contractions
     double e_acc;                 // E(T) accumulator
     double scale[2];              // operand scales (A: ovvv/ovoo, B: t2), powers of two
     float out_scale;              // 1 / (scale[0] * scale[1])
