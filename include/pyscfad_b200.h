@@ -44,7 +44,7 @@ extern "C" {
 
 enum triples_status {
     TRIPLES_OK = 0,
-    TRIPLES_ERR_INVALID_ARGUMENT = 1,  /* bad size, null pointer, bad enum */
+    TRIPLES_ERR_INVALID_ARGUMENT = 1,  /* bad size, null pointer, bad enum, workspace not 16-byte aligned */
     TRIPLES_ERR_WORKSPACE = 2,         /* workspace smaller than triples_workspace_least() */
     TRIPLES_ERR_CUDA = 3,              /* a CUDA call failed; see triples_last_cuda_error() */
     TRIPLES_ERR_UNSUPPORTED = 4,       /* precision / device not supported */
@@ -84,7 +84,9 @@ typedef struct triples_options {
     int tile_n;
 } triples_options;
 
-/* Bytes of device workspace the calls below need for this problem.
+/* Bytes of device workspace the calls below need for this problem.  A workspace
+ * starts on a 16-byte boundary (TRIPLES_ERR_INVALID_ARGUMENT otherwise; device
+ * allocators give 256).
  * want_grad = 0 sizes triples_energy, 1 sizes triples_energy_vjp. */
 size_t triples_workspace_size(int precision, int nocc, int nvir, int ovvv_packed,
                               int want_grad);

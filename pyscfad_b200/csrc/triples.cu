@@ -2234,12 +2234,16 @@ size_t triples_workspace_least(int precision, int nocc, int nvir, int ovvv_packe
     return P.total;
 }
 
+// The kernels read and write the workspace in 16-byte pieces (vectors, bulk and tensor copies).
+static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
 static int triples_call(void *stream, int precision, int nocc, int nvir, int ovvv_packed, int want_grad,
                         const triples_options *opt, const tb::TriplesIO &io, size_t workspace_bytes) {
     tb::Plan P;
     int rc = tb::make_plan_for(precision, nocc, nvir, ovvv_packed, want_grad, P, opt, workspace_bytes);
     if (rc != TRIPLES_OK) return rc;
     if (!io.workspace || workspace_bytes < P.total) return TRIPLES_ERR_WORKSPACE;
+    if (!aligned16(io.workspace)) return TRIPLES_ERR_INVALID_ARGUMENT;
     if (!io.mo_energy || !io.t1 || !io.t2 || !io.ovoo || !io.ovov || !io.ovvv || !io.fvo || !io.e_out)
         return TRIPLES_ERR_INVALID_ARGUMENT;
     if (want_grad && (!io.mo_energy_bar || !io.t1_bar || !io.t2_bar || !io.ovoo_bar || !io.ovov_bar ||
@@ -2303,6 +2307,7 @@ static int triples_lno_call(void *stream, int precision, int nocc, int nvir, int
     int rc = tb::make_plan(precision, nocc, nvir, ovvv_packed, want_grad, P, 1, opt);
     if (rc != TRIPLES_OK) return rc;
     if (!io.workspace || workspace_bytes < P.total) return TRIPLES_ERR_WORKSPACE;
+    if (!aligned16(io.workspace)) return TRIPLES_ERR_INVALID_ARGUMENT;
     if (!io.mat || !io.mo_energy || !io.t1 || !io.t2 || !io.ovoo || !io.ovov || !io.ovvv || !io.fvo || !io.e_out)
         return TRIPLES_ERR_INVALID_ARGUMENT;
     if (want_grad && (!io.mat_bar || !io.mo_energy_bar || !io.t1_bar || !io.t2_bar || !io.ovoo_bar ||
@@ -2410,6 +2415,7 @@ static int triples_df_call(void *stream, int precision, int nocc, int nvir, int 
     int rc = df_layout(precision, nocc, nvir, naux, want_grad, L, workspace_bytes);
     if (rc != TRIPLES_OK) return rc;
     if (!io.workspace || workspace_bytes < L.total) return TRIPLES_ERR_WORKSPACE;
+    if (!aligned16(io.workspace)) return TRIPLES_ERR_INVALID_ARGUMENT;
     if (!Lov || !Lvv || !io.mo_energy || !io.t1 || !io.t2 || !io.ovoo || !io.ovov || !io.fvo || !io.e_out)
         return TRIPLES_ERR_INVALID_ARGUMENT;
     if (want_grad && (!Lov_bar || !Lvv_bar || !io.mo_energy_bar || !io.t1_bar || !io.t2_bar || !io.ovoo_bar ||
@@ -2561,6 +2567,7 @@ int triples_batch_create(int precision, int nprob, const triples_problem *probs,
     if (!batch) return TRIPLES_ERR_INVALID_ARGUMENT;
     *batch = nullptr;
     if (!workspace) return TRIPLES_ERR_WORKSPACE;
+    if (!aligned16(workspace)) return TRIPLES_ERR_INVALID_ARGUMENT;
     // the workspace must hold the batch before any table points into it
     bool vtables = true;
     for (;; vtables = false) {
