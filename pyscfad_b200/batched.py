@@ -105,12 +105,30 @@ def _choice(entry):
     return int(entry), 0
 
 
+def _scratch(lib, prec, prob: _Problem, tv: int):
+    """Scratch of one call: (what it needs, with room for its chunk groups)."""
+    args = (prec, prob.nocc, prob.nvir, int(prob.packed), 1, ctypes.byref(_lib.options(block_size=tv)))
+    need = int(lib.triples_workspace_size_ex(*args))
+    return need, need + int(lib.triples_workspace_extra(*args))
+
+
 def _call(lib, prec, prob: _Problem, ws: torch.Tensor, stream: torch.cuda.Stream, tv: int, tile_n: int = 0):
     opt = _lib.options(block_size=tv, tile_n=tile_n)
+    # its own scratch, whatever larger problem or candidate ws is sized for: a call runs the same
+    # chunk groups in the tuner and in a lane
+    nbytes = min(ws.numel(), _scratch(lib, prec, prob, tv)[1])
     rc = lib.triples_energy_vjp_ex(stream.cuda_stream, prec, prob.nocc, prob.nvir, int(prob.packed),
                                    *[a.data_ptr() for a in prob.inputs], 1.0, 1, ctypes.byref(opt), ws.data_ptr(),
-                                   ws.numel(), prob.energy.data_ptr(), *[prob.grads[k].data_ptr() for k in KEYS])
+                                   nbytes, prob.energy.data_ptr(), *[prob.grads[k].data_ptr() for k in KEYS])
     _lib.check(rc, "triples_energy_vjp_ex")
+
+
+def _alloc(need: int, more: int, device) -> torch.Tensor:
+    """`more` bytes where the device has room for them, else `need`."""
+    try:
+        return torch.empty(max(more, 256), dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return torch.empty(max(need, 256), dtype=torch.uint8, device=device)
 
 
 class BatchedTriples:
@@ -149,8 +167,7 @@ class BatchedTriples:
             self._create_batch()
             self.workspaces = []
         else:
-            self.workspaces = [torch.empty(max(self._ws_bytes(l), 256), dtype=torch.uint8, device=self.device)
-                               for l in range(self.lanes)]
+            self.workspaces = [_alloc(*self._ws_bytes(l), self.device) for l in range(self.lanes)]
 
     def _create_batch(self):
         n = len(self.problems)
@@ -186,11 +203,6 @@ class BatchedTriples:
             self.handle = None
 
     # -- set-up ---------------------------------------------------------------
-    def _size(self, prob: _Problem, tv: int) -> int:
-        opt = _lib.options(block_size=tv)
-        return int(self.lib.triples_workspace_size_ex(self.prec, prob.nocc, prob.nvir, int(prob.packed), 1,
-                                                      ctypes.byref(opt)))
-
     def _tune(self, tune: bool):
         stream = self.streams[0]
         scratch = None
@@ -201,9 +213,11 @@ class BatchedTriples:
                 continue
             key = (prob.nocc, prob.nvir, self.precision, int(prob.packed))
             if key not in self.autotuner.table:
-                need = max(self._size(prob, tv) for tv in TV_CANDIDATES if prob.nocc * tv <= 1024)
-                if scratch is None or scratch.numel() < need:
-                    scratch = torch.empty(need, dtype=torch.uint8, device=self.device)
+                sizes = [_scratch(self.lib, self.prec, prob, tv) for tv in TV_CANDIDATES if prob.nocc * tv <= 1024]
+                need, more = (max(column) for column in zip(*sizes))
+                if scratch is None or scratch.numel() < more:
+                    scratch = None
+                    scratch = _alloc(need, more, self.device)
                 with torch.cuda.stream(stream):
                     self.autotuner.best(prob, self.precision, scratch, stream)
             prob.tv, prob.tile_n = _choice(self.autotuner.table[key])
@@ -219,8 +233,9 @@ class BatchedTriples:
             self.problems[i].lane = lane
             load[lane] += self._cost(self.problems[i])
 
-    def _ws_bytes(self, lane: int) -> int:
-        return max([self._size(p, p.tv) for p in self.problems if p.lane == lane] or [0])
+    def _ws_bytes(self, lane: int):
+        sizes = [_scratch(self.lib, self.prec, p, p.tv) for p in self.problems if p.lane == lane]
+        return tuple(max(column) for column in zip(*sizes)) if sizes else (0, 0)
 
     def _enqueue(self):
         """The whole batch on the current stream (batch engine), or all calls of all
