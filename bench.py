@@ -401,7 +401,8 @@ LNO_METRIC = "LNO (T) E+VJP TFLOP/s (projected first occupied index), B200 vs re
 # ordering of a chunk: the forward pass reads w and writes WW and Q; the
 # projection reads them and writes Zbar, Dbar and P^T(Wtbar); the adjoint pass
 # reads the last two and writes vbar and the Wbar operand (FP64, or two 16-bit
-# halves); the V gradients read vbar and Dbar.
+# halves); the V gradients read vbar and Dbar.  (The form to compare with; the
+# library works on the box below.)
 def lno_pass_bytes(sz):
     return {"lno_tile_fwd": sz + 16, "lno_projection": 40, "lno_tile_adj": 16 + 8 + (8 if sz == 8 else 4),
             "lno_vgrad": 16}

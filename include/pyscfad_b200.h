@@ -9,7 +9,7 @@
  * call arrives with it (arguments, triples_options), so host threads may
  * call it concurrently on different streams and workspaces (the reference's
  * C kernels are likewise re-entrant).  The first call on a device does a
- * one-time set-up (kernel attributes, constant tables) under a lock; make it
+ * one-time set-up (kernel attributes) under a lock; make it
  * before any stream capture.
  *
  * Array layouts are the reference's canonical ones (C order, FP64), i.e. the
@@ -185,9 +185,11 @@ int triples_lno_energy_vjp(void *stream, int precision, int nocc, int nvir, int 
                            double *ovoo_bar, double *ovov_bar, double *ovvv_bar,
                            double *fvo_bar);
 
-/* Introspection (host only, no GPU): the gather tables and de-duplication
- * patterns of the LNO orbit tiles, as the library builds them, copied into
- * `out` when `bytes` suffices; returns the size needed.  Layout: six
+/* Introspection (host only, no GPU): gather tables and de-duplication patterns
+ * of orbit tiles over 4-wide virtual sub-ranges, copied into `out` when `bytes`
+ * suffices; returns the size needed.  They describe no kernel of this library
+ * (the LNO kernels work on 8-wide sub-ranges without tables) and stay for callers
+ * that read them.  Layout: six
  * sigma-permuted slot maps [6][64], two r3 slot maps [2][6][64] (slots padded
  * as s + 3 (s / 16)), candidate maps [36][6] and [2][36][6] (a 16-byte aligned
  * block of 1808 bytes), then 16 patterns of {nslab, cand[36], prim[36]}. */

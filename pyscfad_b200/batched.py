@@ -10,8 +10,8 @@ and its VJP for all of them with one of two engines:
   chunk step c launches every kernel kind (W contraction, Wbar scale,
   epilogue, energy sum, the four adjoint contractions) ONCE over the c-th
   chunk of every problem, the persistent kernels pulling tiles from a job
-  table built when the batch is created.  A batch of 256 small problems is
-  a few hundred launches instead of tens of thousands.
+  table built when the batch is created.  256 problems of nocc 4-12 and nvir
+  20-80 are 5432 launches.
 * ``engine="lanes"``: one ``triples_energy_vjp_ex`` call per problem, spread
   over ``lanes`` CUDA streams (largest first, each to the least-loaded
   lane), one workspace per lane.

@@ -40,11 +40,6 @@ __host__ __device__ inline Map4 map2(int e0, long long s0, long long s1) {
 __host__ __device__ inline Map4 map3(int e0, int e1, long long s0, long long s1, long long s2) {
     return Map4{e0, e1, kBig, s0, s1, s2, 0};
 }
-__host__ __device__ inline Map4 map4(int e0, int e1, int e2, long long s0, long long s1,
-                                     long long s2, long long s3) {
-    return Map4{e0, e1, e2, s0, s1, s2, s3};
-}
-
 __device__ __forceinline__ long long apply(const Map4 &m, int idx) {
     int i0 = idx % m.e0;
     int t = idx / m.e0;

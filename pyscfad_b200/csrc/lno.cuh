@@ -108,29 +108,26 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_fwd(const __grid_constan
     const int i0 = A.ijk[3 * rep], i1 = A.ijk[3 * rep + 1], i2 = A.ijk[3 * rep + 2];
     int ca, cb, cc;
     f2_element(threadIdx.x, ca, cb, cc);
-    const bool ok0 = ca < R.len[0] && cb < R.len[1] && cc < R.len[2];
-    const bool ok1 = ok0 && ca + 4 < R.len[0];
     f2_load_tables(A, R, i0, i1, i2, tab, tf);
     double WW[2][6], VV[2][6];
-    f2_amplitudes(reinterpret_cast<const StageT *>(A.S), R, o, i0, i1, i2, ca, cb, cc, ok0, ok1, tab, tf, WW, VV);
+    f2_amplitudes(reinterpret_cast<const StageT *>(A.S), R, o, i0, i1, i2, ca, cb, cc, true, true, tab, tf, WW, VV);
     const double *ev = A.mo_e + o;
     const double e_occ = A.mo_e[i0] + A.mo_e[i1] + A.mo_e[i2];
-    const double e_bc = ok0 ? ev[R.st[1] + cb] + ev[R.st[2] + cc] : 0.0;
+    const double e_bc = ev[R.st[1] + cb] + ev[R.st[2] + cc];
     const long long ne = A.ne;
 #pragma unroll
     for (int e = 0; e < 2; e++) {
-        const bool ok = e == 0 ? ok0 : ok1;
         double X[6], Z[6];
 #pragma unroll
         for (int s = 0; s < 6; s++) X[s] = WW[e][s] + 0.5 * VV[e][s];
         f2_r3(X, Z);
-        const double rD = ok ? 1.0 / (e_occ - ev[R.st[0] + ca + 4 * e] - e_bc) : 0.0;
+        const double rD = 1.0 / (e_occ - ev[R.st[0] + ca + 4 * e] - e_bc);
         const int slot = sub * 512 + e * 256 + threadIdx.x;
         lno_for_s([&](auto sc) {
             constexpr int s = decltype(sc)::value;
             const long long at = lno_box<s>(o, ne, i0, i1, i2) + slot;
-            A.WW[at] = ok ? WW[e][s] : 0.0;
-            A.Q[at] = ok ? Z[s] * rD : 0.0;
+            A.WW[at] = WW[e][s];
+            A.Q[at] = Z[s] * rD;
         });
     }
 }
@@ -489,16 +486,16 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_lno_adj_e(const __grid_cons
 }
 
 // ---------------------------------------------------------------------------
-// orbit bookkeeping as host tables (introspection only): candidate region
-// c = 6 pi + rho holds occupied triple (ijk[pi0], ijk[pi1], ijk[pi2]) over the
-// 4-wide virtual sub-ranges (U[rho0], U[rho1], U[rho2])
+// orbit bookkeeping of 4-wide sub-ranges as host tables (triples_lno_tables; no
+// kernel reads them): candidate region c = 6 pi + rho holds occupied triple
+// (ijk[pi0], ijk[pi1], ijk[pi2]) over the virtual sub-ranges (U[rho0], U[rho1], U[rho2])
 // ---------------------------------------------------------------------------
 constexpr int kLnoSB = 4;
 constexpr int kLnoRegion = kLnoSB * kLnoSB * kLnoSB;
 __host__ __device__ constexpr int lno_pad(int slot) { return slot + 3 * (slot >> 4); }
 
 struct alignas(16) LnoTables {
-    unsigned char symsl[6][kLnoRegion];      // 16-byte multiples first: copied as uint4
+    unsigned char symsl[6][kLnoRegion];      // 16-byte multiples first
     unsigned char r3sl[2][6][kLnoRegion];
     unsigned char symc[36][6];
     unsigned char r3c[2][36][6];

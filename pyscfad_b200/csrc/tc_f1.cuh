@@ -10,10 +10,10 @@
 //
 // Tile: 128 rows = 8 p x 16 x, 16 rt columns = rt r x 16 z (rt even, at most
 // BN / 16), K blocks of 64 (the last of each term issues only the 16-wide steps
-// it holds).  rt divides nocc as evenly as the widest tile allows (f1_tile in
+// it holds).  rt divides nocc as evenly as the widest tile allows (plan_once in
 // triples.cu): nocc 20 takes two tiles of 10 r where fixed 8-wide tiles padded
 // it to 24 and 16-wide ones to 32.  Persistent CTAs (one per SM), warp roles: 0 TMA producer, 1 MMA issuer and
-// TMEM owner, 2-5 epilogue (TMEM -> registers -> staging, FP32).
+// TMEM owner, 2-9 epilogue (TMEM -> registers -> staging, FP32).
 #pragma once
 #include "common.cuh"
 #include "tc_ptx.cuh"

@@ -47,12 +47,11 @@ static thread_local int g_last_cuda_error = 0;
 // ---------------------------------------------------------------------------
 // optional per-kernel-class timing with CUDA events (on the launch stream)
 // ---------------------------------------------------------------------------
-enum ProfCat { P_PREP = 0, P_F1, P_F2, P_B1A, P_B1B, P_B1C, P_B1D, P_FOLD, P_LNO, P_LNO_PROJ, P_LNO_ADJ, P_LNO_VG,
-               P_NCAT };
+enum ProfCat { P_PREP = 0, P_F1, P_F2, P_B1A, P_B1B, P_B1C, P_B1D, P_FOLD, P_LNO, P_LNO_PROJ, P_LNO_ADJ, P_NCAT };
 static const char *kProfNames[P_NCAT] = {"prep", "f1_contract", "f2_epilogue",
                                          "b1a_ovvv_grad", "b1b_t2_grad", "b1c_ovoo_grad",
                                          "b1d_t2_ooov_grad", "fold", "lno_tile_fwd", "lno_projection",
-                                         "lno_tile_adj", "lno_vgrad"};
+                                         "lno_tile_adj"};
 struct ProfRec {
     int cat;
     cudaEvent_t a, b;
@@ -192,8 +191,9 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
     d.n = nocc + nvir;
     d.Tv = choose_tv(nocc, opt ? opt->block_size : 0);
     if (lno) {
-        // halve the block until four FP64 arrays of a chunk's raw amplitudes fit the
-        // budget (the box arrays take a sixth; the rule fixes the decomposition)
+        // halve the block until four FP64 arrays of six times a chunk's box would fit the budget (from
+        // nocc 50 on).  The box arrays take a sixth of that; the rule stays because it decides
+        // the decomposition, and with it the order of the FP32 sums of the mixed modes.
         const double o3 = (double)nocc * nocc * nocc;
         while (d.Tv > 4 && kLnoArrays * 6.0 * o3 * d.Tv * d.Tv * d.Tv * sizeof(double) > kLnoBudgetBytes) d.Tv >>= 1;
     }
@@ -203,7 +203,7 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
     P.nb = num_blocks(d);
     P.n_ijk = nocc * (nocc + 1) * (nocc + 2) / 6;
     long long maxst = 0, maxwb = 0;
-    int maxitems = 0, maxbox = 1;
+    int maxbox = 1;
     for (int A = 0; A < P.nb; A++)
         for (int B = 0; B <= A; B++)
             for (int C = 0; C <= B; C++) {
@@ -213,16 +213,12 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
                 if (s > maxst) maxst = s;
                 long long w = chunk_wbar_elems(ch, d);
                 if (w > maxwb) maxwb = w;
-                int it = ch.nabc[0] * ch.nabc[1] * ch.nabc[2];
-                if (it > maxitems) maxitems = it;
                 maxbox = std::max(maxbox, box_slots(ch));
             }
     P.stage_elems = (size_t)maxst;
     P.wbar_elems = (size_t)maxwb;
     P.stage_slot = (P.stage_elems + 63) / 64 * 64;   // slots start 256-byte aligned
     P.wbar_slot = (P.wbar_elems + 63) / 64 * 64;
-    P.max_items = maxitems;
-    P.f2_gy = kMaxSub;
     const bool mixed = precision != TRIPLES_PRECISION_FP64;
     P.stage_bytes = mixed ? sizeof(float) : sizeof(double);
 
@@ -273,7 +269,7 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
         P.off_tf = take(o * nb8 * 8 * sizeof(float2));
     }
     P.off_ijk = take((size_t)P.n_ijk * 3 * sizeof(int));
-    P.off_epart = take((size_t)P.group * P.n_ijk * P.f2_gy * el);
+    P.off_epart = take((size_t)P.group * P.n_ijk * kMaxPartials * el);
     if (P.lno) {
         // FP64 box arrays: WW (0), PQ (1), Q (2), PW / Zbar (3); the energy alone needs only 0 and 2
         const size_t box = o * o * o * (size_t)maxbox;
@@ -286,7 +282,7 @@ static int plan_once(int precision, int nocc, int nvir, int packed, int want_gra
             P.off_L[1] = P.off_L[0];
             P.off_L[3] = P.off_L[2];
         }
-        P.off_lpart = take((size_t)6 * kLnoGrid * el);
+        P.off_lpart = take((size_t)3 * kLnoGrid * el);
     }
     P.total = off;
     return TRIPLES_OK;
@@ -392,9 +388,9 @@ __global__ void k_prep_B2(const double *__restrict__ t2, Dims d, double *__restr
 // 16-bit split operands for the tensor-core path
 // ---------------------------------------------------------------------------
 // Occupied representatives i >= j >= k: first the o(o-1)(o-2)/6 with
-// i > j > k (combinatorial order), then the o(o-1)/2 with i == j > k, as
-// many with i > j == k, and the o with i == j == k, so that each pattern the
-// persistent epilogue takes (the first three) is one contiguous range.
+// i > j > k (combinatorial order: neighbours share i and j, and so the tables and
+// lines that they read), then the o(o-1)/2 with i == j > k, as many with
+// i > j == k, and the o with i == j == k.
 __host__ __device__ inline int n_distinct_ijk(int o) { return o * (o - 1) * (o - 2) / 6; }
 
 __global__ void k_ijk_table(int o, int *ijk) {
@@ -1148,8 +1144,8 @@ static int gemm_plain(cudaStream_t st, int M, int N, int K, const double *A, lon
     return TRIPLES_OK;
 }
 
-// One-time set-up per device and kind of work (shared-memory opt-ins and
-// constant tables), under a lock so that host threads making their first
+// One-time set-up per device and kind of work (shared-memory opt-ins), under a
+// lock so that host threads making their first
 // call at the same time do it once.  Assumes the device's primary context
 // lives as long as the process (a cudaDeviceReset would need it again).
 enum InitKind { INIT_F2_F32 = 0, INIT_F2_F64, INIT_TC, INIT_LNO, INIT_LNO64, INIT_NKINDS };
@@ -1174,7 +1170,7 @@ static ChunkAux chunk_aux(const Plan &P, const ChunkDesc &ch, int slot, const Tr
     A.ctrl = (Ctrl *)(ws + P.off_ctrl);
     A.slot = &A.ctrl->slot[slot];
     A.mo_e = io.mo_energy;
-    A.e_part = (const double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
+    A.e_part = (const double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * kMaxPartials;
     A.ybar = io.ybar;
     A.o = P.d.o;
     A.a0 = ch.base[0]; A.na = ch.nabc[0];
@@ -1198,8 +1194,7 @@ static void for_job_kinds(F &&f) {
     f(Table<T>{});
 }
 
-// once per device and precision: shared-memory opt-ins and the constant tables
-// of the FP64 epilogue's region patterns
+// once per device and precision: shared-memory opt-ins
 static int setup_epilogue(bool mixed) {
     return once_per_device(mixed ? INIT_F2_F32 : INIT_F2_F64, [&]() -> int {
         if (mixed) {
@@ -1430,7 +1425,7 @@ static void f2_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, co
     F.wscale = &((Ctrl *)(ws + P.off_ctrl))->slot[slot].wscale;
     F.ybar = io.ybar;
     F.want_grad = P.want_grad;
-    F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
+    F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * kMaxPartials;
     F.mo_bar = io.mo_energy_bar;
     F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
 }
@@ -1459,7 +1454,7 @@ static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, c
     F.wscale = &ctrl->slot[slot].wscale;
     F.ybar = io.ybar;
     F.want_grad = P.want_grad;
-    F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * P.f2_gy;
+    F.e_part = (double *)(ws + P.off_epart) + (size_t)slot * P.n_ijk * kMaxPartials;
     F.mo_bar = io.mo_energy_bar;
     F.t1_bar = io.t1_bar; F.fvo_bar = io.fvo_bar; F.ovov_bar = io.ovov_bar; F.t2_bar = io.t2_bar;
     F.err = &ctrl->err;
@@ -1472,7 +1467,7 @@ static void f2m_params(const Plan &P, const ChunkDesc &ch, int slot, char *ws, c
 template <int COLS, bool FULL>
 static int lno_projections(const LnoArgs &A, cudaStream_t st, unsigned &grid) {
     const long long tiles = ((long long)A.o * A.o * A.ne + COLS - 1) / COLS;   // (a CTA has one tile at least)
-    grid = (unsigned)std::min(tiles, (long long)2 * num_sms());
+    grid = (unsigned)std::min({tiles, (long long)2 * num_sms(), (long long)kLnoGrid});
     const size_t smem = LnoProj<COLS>::smem(A.o);
     for (int slot = 2; slot >= 0; slot--)
         TB_KLAUNCH(P_LNO_PROJ, (k_lno_proj<COLS, FULL><<<grid, kLnoThreads, smem, st>>>(A, slot, slot == 2 ? 1 : 0)));

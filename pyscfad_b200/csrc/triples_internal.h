@@ -8,7 +8,7 @@
 namespace tb {
 
 constexpr int kMaxTv = 16;        // largest virtual block
-constexpr int kMaxSub = 64;       // energy partials per occupied representative
+constexpr int kMaxPartials = 32;  // energy partials per occupied representative: 8 sub-range triples, or 4 of 8 warps
 constexpr int kMaxCols = 1024;    // largest nocc * Tv (one staged (r, z) row)
 constexpr int kCtrlBytes = 256;   // control block at workspace offset 0
 // Chunk slots of a call: most bytes of staging and Wbar.  A chunk of nocc 5 has
@@ -18,9 +18,9 @@ constexpr int kCtrlBytes = 256;   // control block at workspace offset 0
 // 5 nvir 19 mixed 1.26 / 0.45 / 0.45 ms, FP64 kernels 0.95 / 0.45 / 0.45 ms, nocc
 // 13 nvir 83 bf16 41.4 / 35.2 / 33.0 ms, nocc 12 nvir 100 FP64 112 / 112 / 104 ms.
 constexpr size_t kGroupBytes = (size_t)2 << 30;
-constexpr int kLnoGrid = 1184;    // LNO streaming kernels: most blocks per ordering (energy partials)
-constexpr int kLnoArrays = 4;     // LNO whole-chunk FP64 work arrays (with the adjoint)
-constexpr double kLnoBudgetBytes = 96e9;   // their largest total before the block size is halved
+constexpr int kLnoGrid = 1024;    // LNO projection: most blocks (an energy partial each and slot)
+constexpr int kLnoArrays = 4;     // LNO box arrays (with the adjoint)
+constexpr double kLnoBudgetBytes = 96e9;   // block size rule of the LNO plan (plan_once)
 
 // State of one chunk slot
 struct ChunkSlot {
@@ -52,11 +52,9 @@ struct Plan {
     int f1_bn;       // widest N tile of the tensor-core W contraction (128 or 256)
     int f1_rt;       // occupied r values of its N tiles (16 columns each)
     int prec, want_grad, packed;
-    int lno;         // projected (LNO) energy: whole-chunk work arrays off_L
+    int lno;         // projected (LNO) energy: box arrays off_L
     int nb;          // number of virtual blocks
     int n_ijk;       // occupied triplet representatives i >= j >= k
-    int max_items;   // largest |A||B||C| over chunks
-    int f2_gy;       // epilogue grid.y upper bound
     int Kp8, Op8;    // 16-byte padded contraction lengths of the 16-bit operands
     size_t stage_elems, stage_bytes, wbar_elems;
     size_t stage_slot, wbar_slot;   // elements from one chunk slot to the next
