@@ -1,4 +1,4 @@
-// FP64 element kernels: the epilogue of chunks whose sub-ranges are short (a
+// Element kernels: the epilogue of chunks whose sub-ranges are short (a
 // remainder block, or blocks of 4 and less): the LNO calls, and the canonical ones
 // that by_element (triples.cu) names, the mixed modes' among them.
 //
@@ -185,13 +185,10 @@ __device__ __forceinline__ void elem_writeback(const ARGS &A, const F2mSub &R, c
     }
 }
 
-// The items of the jobs (chunks) of a launch; a job starts with a new CTA.  SPLIT 0: FP64 staging and
-// Wbar; 1 and 2: FP32 staging, fp16 and bf16 hi/lo Wbar (the mixed modes).
-template <int SPLIT, typename JOBS>
+// The items of the jobs (chunks) of a launch, FP64; a job starts with a new CTA.
+template <typename JOBS>
 __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__ JOBS J) {
-    using StageT = typename std::conditional<SPLIT == 0, double, float>::type;
-    __shared__ double sV[6 * kElemThreads];
-    __shared__ typename F2Smem<SPLIT>::W sW[6 * kElemThreads];
+    __shared__ double sV[6 * kElemThreads], sW[6 * kElemThreads];
     JobCursor jcur;
     int blk;
     const int jb = jcur.at(J, (int)blockIdx.x, blk);
@@ -202,7 +199,7 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__
     const int opat = (ids[0] == ids[2]) ? 3 : (ids[0] == ids[1] ? 1 : (ids[1] == ids[2] ? 2 : 0));
     const int vpat = R.pat, lane = threadIdx.x & 31;
     double WW[6], VV[6], X[6], Z[6], RW[6];
-    elem_amplitudes<StageT>(A, R, ids, E.loc, WW, VV);
+    elem_amplitudes<double>(A, R, ids, E.loc, WW, VV);
     // orbit weights as in k_f2t
     const double cocc = opat == 0 ? 2.0 : (opat == 3 ? 6.0 / 18.0 : 1.0);
     const double cen = vpat == 0 ? cocc : (vpat == 3 ? cocc / 6.0 : cocc * 0.5);
@@ -220,7 +217,6 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__
     const double en = elem_sum(E.ok ? cen * esum * rD : 0.0, E.all);
     if (E.ok && (lane & E.all) == 0) A.e_part[(long long)(E.sub * E.warps + (E.el >> 5)) * A.n_ijk + E.rep] = en;
     if (!A.want_grad) return;
-    const float wsc = SPLIT > 0 ? (float)*A.wscale : 1.0f;
     const double g0 = cocc * A.ybar * rD;
     double wb[6], vb[6], w3 = 0.0, v3 = 0.0;
 #pragma unroll
@@ -234,13 +230,195 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__
 #pragma unroll
     for (int s = 0; s < 6; s++) {
         const int s1 = perm_compose(s, 2), s2 = perm_compose(s, 1), at = s * kElemThreads + threadIdx.x;
-        const double w = opat == 0 ? wb[s] : opat == 1 ? wb[s] + wb[s1] : opat == 2 ? wb[s] + wb[s2] : w3;
-        if constexpr (SPLIT == 0) sW[at] = w;
-        else sW[at] = f2m_split<SPLIT>((float)w, wsc);
+        sW[at] = opat == 0 ? wb[s] : opat == 1 ? wb[s] + wb[s1] : opat == 2 ? wb[s] + wb[s2] : w3;
         sV[at] = opat == 0 ? vb[s] : opat == 1 ? vb[s] + vb[s1] : opat == 2 ? vb[s] + vb[s2] : v3;
     }
     elem_dd(A, R, E, ids, E.ok ? -cen * A.ybar * esum * rD * rD : 0.0);
-    elem_writeback<SPLIT>(A, R, E, ids, opat, vpat, sW, sV);
+    elem_writeback<0>(A, R, E, ids, opat, vpat, sW, sV);
+}
+
+// ---------------------------------------------------------------------------
+// The mixed modes: items within a warp (at most 32 elements).  FP32 where k_f2m is, and the same
+// FP32 operations in the same order, so that a chunk gives the same values in either kernel: V terms
+// summed over rho, rows along z, columns over y + 4, then bit 0 of y, bits 2, 1 and 0 of x, bit 1 of y.
+// (What k_f2m adds for coordinates beyond a short range are zeros.)
+// ---------------------------------------------------------------------------
+struct ElemBits {         // lane bit of bit `b` of coordinate t, 0 where the range is shorter
+    int k[3], at[3];
+    __device__ __forceinline__ unsigned operator()(int t, int b) const {
+        return b < sel3(k[0], k[1], k[2], t) ? 1u << (sel3(at[0], at[1], at[2], t) + b) : 0u;
+    }
+};
+
+// Column sum of vb * table over the item's (x, y), x and y in coordinates tx, ty
+__device__ __forceinline__ float elem_column(float vb, float table, const ElemBits &bit, int tx, int ty) {
+    float v = __fmul_rn(vb, table);
+    const unsigned y2 = bit(ty, 2);
+    if (y2) {   // (bits are the same for all lanes)
+        const float low = __shfl_xor_sync(0xffffffffu, v, y2), both = fmaf(vb, table, low);
+        const float other = __shfl_xor_sync(0xffffffffu, both, y2);
+        v = threadIdx.x & y2 ? both : other;
+    }
+    const unsigned order[5] = {bit(ty, 0), bit(tx, 2), bit(tx, 1), bit(tx, 0), bit(ty, 1)};
+#pragma unroll
+    for (int i = 0; i < 5; i++)
+        if (order[i]) v += __shfl_xor_sync(0xffffffffu, v, order[i]);
+    return v;
+}
+
+template <int H, typename JOBS>
+__global__ void __launch_bounds__(kElemThreads, 2) k_f2em(const __grid_constant__ JOBS J) {
+    __shared__ float sV[6 * kElemThreads];
+    __shared__ uint32_t sW[6 * kElemThreads];
+    JobCursor jcur;
+    int blk;
+    const int jb = jcur.at(J, (int)blockIdx.x, blk);
+    const F2P &A = J.job[JOBS::kOne ? 0 : jb];
+    const Elem E = elem_of(A, blk * kElemThreads + threadIdx.x);
+    const F2mSub &R = A.sub[E.sub];
+    const int o = A.o, v = A.v, lane = threadIdx.x & 31;
+    const int ids[3] = {A.ijk[3 * E.rep], A.ijk[3 * E.rep + 1], A.ijk[3 * E.rep + 2]};
+    const int opat = (ids[0] == ids[2]) ? 3 : (ids[0] == ids[1] ? 1 : (ids[1] == ids[2] ? 2 : 0));
+    const int vpat = R.pat;
+    const float *S[6];
+#pragma unroll
+    for (int pi = 0; pi < 6; pi++) {
+        int pp[3] = {0, 0, 0};
+        perm_of(pi, pp);
+        S[pi] = static_cast<const float *>(A.S) + R.pi[pi].s0 +
+                (E.loc[pp[1]] * R.len[pp[0]] + E.loc[pp[0]]) * R.len[pp[2]] + E.loc[pp[2]];   // (not two ranges of 8: no row exchange)
+    }
+    float tz[3][3], fz[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int s = 0; s < 3; s++) {
+            const int z = R.st[s] + E.loc[s];
+            tz[r][s] = (float)__ldg(&A.t1[(long long)ids[r] * v + z]);
+            fz[r][s] = (float)__ldg(&A.fvo[(long long)z * o + ids[r]]);
+        }
+    double WW[6], X[6], Z[6], RW[6];
+    float VV[6];
+#pragma unroll
+    for (int s = 0; s < 6; s++) {
+        WW[s] = 0.0;
+        VV[s] = 0.f;
+    }
+#pragma unroll
+    for (int rho = 0; rho < 6; rho++) {
+        int pr[3] = {0, 0, 0};
+        perm_of(rho, pr);
+        const int p = ids[pr[0]], q = ids[pr[1]];
+        const long long idx = ((long long)p * o + q) * o + ids[pr[2]];
+#pragma unroll
+        for (int pi = 0; pi < 6; pi++) {
+            const int s = f2m_sof(pi, rho);
+            int pp[3] = {0, 0, 0};
+            perm_of(pi, pp);
+            const int x = R.st[pp[0]] + E.loc[pp[0]], y = R.st[pp[1]] + E.loc[pp[1]];
+            WW[s] += (double)__ldg(S[pi] + idx * R.pi[pi].rs);
+            const float ov = (float)__ldg(&A.ovov[(((long long)p * v + x) * o + q) * v + y]);
+            const float tt = (float)__ldg(&A.t2[(((long long)q * o + p) * v + y) * v + x]);
+            VV[s] = __fadd_rn(VV[s], fmaf(ov, tz[pr[2]][pp[2]], __fmul_rn(tt, fz[pr[2]][pp[2]])));
+        }
+    }
+    const double cocc = opat == 0 ? 2.0 : (opat == 3 ? 6.0 / 18.0 : 1.0);
+    const double cen = vpat == 0 ? cocc : (vpat == 3 ? cocc / 6.0 : cocc * 0.5);
+#pragma unroll
+    for (int s = 0; s < 6; s++) X[s] = WW[s] + 0.5 * (double)VV[s];
+    f2_r3(X, Z);
+    f2_r3(WW, RW);
+    const double *ev = A.mo_e + o;
+    const double rD = 1.0 / (A.mo_e[ids[0]] + A.mo_e[ids[1]] + A.mo_e[ids[2]] - ev[R.st[0] + E.loc[0]] -
+                             ev[R.st[1] + E.loc[1]] - ev[R.st[2] + E.loc[2]]);
+    double esum = 0.0;
+#pragma unroll
+    for (int s = 0; s < 6; s++) esum += WW[s] * Z[s];
+    const double en = elem_sum(E.ok ? cen * esum * rD : 0.0, E.all);
+    if (E.ok && (lane & E.all) == 0) A.e_part[(long long)E.sub * A.n_ijk + E.rep] = en;
+    if (!A.want_grad) return;
+    const float wsc = (float)*A.wscale;
+    const double g0 = cocc * A.ybar * rD;
+    float wb[6], vb[6];
+    double w3 = 0.0, v3 = 0.0;
+#pragma unroll
+    for (int s = 0; s < 6; s++) {
+        wb[s] = (float)(g0 * (Z[s] + RW[s]));
+        vb[s] = (float)(g0 * 0.5 * RW[s]);
+        w3 += (double)wb[s];
+        v3 += (double)vb[s];
+    }
+#pragma unroll
+    for (int s = 0; s < 6; s++) {
+        const int s1 = perm_compose(s, 2), s2 = perm_compose(s, 1), at = s * kElemThreads + threadIdx.x;
+        const float w = opat == 0 ? wb[s] : opat == 1 ? wb[s] + wb[s1] : opat == 2 ? wb[s] + wb[s2] : (float)w3;
+        sV[at] = opat == 0 ? vb[s] : opat == 1 ? vb[s] + vb[s1] : opat == 2 ? vb[s] + vb[s2] : (float)v3;
+        sW[at] = f2m_split<H>(w, wsc);
+    }
+    elem_dd(A, R, E, ids, E.ok ? -cen * A.ybar * esum * rD * rD : 0.0);
+    // write-back as in elem_writeback
+    ElemBits bit;
+#pragma unroll
+    for (int t = 0; t < 3; t++) bit.k[t] = 31 - __clz(R.len[t]);
+    bit.at[2] = 0;
+    bit.at[1] = bit.k[2];
+    bit.at[0] = bit.k[2] + bit.k[1];
+    const unsigned lead = opat == 0 ? 63u : opat == 1 ? 19u : opat == 2 ? 13u : 1u;
+    const unsigned vlead = vpat == 0 ? 63u : vpat == 1 ? 19u : vpat == 2 ? 13u : 1u;
+#pragma unroll 1
+    for (int rz = 0; rz < 9; rz++) {
+        const int rs = rz / 3, zs = rz % 3;
+        const int zl = sel3(E.loc[0], E.loc[1], E.loc[2], zs), z = sel3(R.st[0], R.st[1], R.st[2], zs) + zl;
+        const unsigned mz = zs == 0 ? E.m[0] : zs == 1 ? E.m[1] : E.m[2], others = E.all & ~mz;
+        const int r = sel3(ids[0], ids[1], ids[2], rs), lz = sel3(R.len[0], R.len[1], R.len[2], zs);
+        const int zat = sel3(bit.at[0], bit.at[1], bit.at[2], zs);
+        const float tv = (float)__ldg(&A.t1[(long long)r * v + z]), fv = (float)__ldg(&A.fvo[(long long)z * o + r]);
+        double ct = 0.0, cf = 0.0;
+#pragma unroll 1
+        for (int u = 0; u < 4; u++) {
+            const int ra = rs == 0 ? 1 : 0, rb = rs == 2 ? 1 : 2, za = zs == 0 ? 1 : 0, zb = zs == 2 ? 1 : 2;
+            const int pr0 = u & 1 ? rb : ra, pr1 = u & 1 ? ra : rb, pp0 = u >> 1 ? zb : za, pp1 = u >> 1 ? za : zb;
+            const int rho = perm_index(pr0, pr1), pi = perm_index(pp0, pp1);
+            const bool vl = (vlead >> pi) & 1u;
+            if (!__any_sync(0xffffffffu, vl)) continue;
+            const bool in = E.ok && vl && ((lead >> rho) & 1u);
+            const int s0 = pr0 == 0 ? pp0 : (pr1 == 0 ? pp1 : zs), s1 = pr0 == 1 ? pp0 : (pr1 == 1 ? pp1 : zs);
+            const int at = perm_index(s0, s1) * kElemThreads + threadIdx.x;
+            const int p = sel3(ids[0], ids[1], ids[2], pr0), q = sel3(ids[0], ids[1], ids[2], pr1);
+            const int xl = sel3(E.loc[0], E.loc[1], E.loc[2], pp0), yl = sel3(E.loc[0], E.loc[1], E.loc[2], pp1);
+            const int x = sel3(R.st[0], R.st[1], R.st[2], pp0) + xl, y = sel3(R.st[0], R.st[1], R.st[2], pp1) + yl;
+            const long long ov = (((long long)p * v + x) * o + q) * v + y, tt = (((long long)q * o + p) * v + y) * v + x;
+            const float vbe = in ? sV[at] : 0.f;
+            float ox = 0.f, oy = 0.f;
+            if (in) {
+                const F2mPi &D = R.pi[pi];
+                const long long w = f2m_wbar(D, p, q, r) + (long long)xl * D.wx + (long long)yl * D.wy + zl;
+                const uint32_t pk = sW[at];
+                static_cast<uint16_t *>(A.SW)[w] = (uint16_t)pk;
+                static_cast<uint16_t *>(A.SW)[w + D.half] = (uint16_t)(pk >> 16);
+                ox = (float)__ldg(&A.ovov[ov]);
+                oy = (float)__ldg(&A.t2[tt]);
+            }
+            float r1 = 0.f, r2 = 0.f;
+#pragma unroll 1
+            for (int c = 0; c < lz; c++) {   // along z
+                const int src = (int)(lane & ~mz) | (c << zat);
+                const float vc = __shfl_sync(0xffffffffu, vbe, src);
+                r1 = fmaf(vc, __shfl_sync(0xffffffffu, tv, src), r1);
+                r2 = fmaf(vc, __shfl_sync(0xffffffffu, fv, src), r2);
+            }
+            if (in && (lane & mz) == 0) {
+                red_add(&A.ovov_bar[ov], (double)r1);
+                red_add(&A.t2_bar[tt], (double)r2);
+            }
+            ct += (double)elem_column(vbe, ox, bit, pp0, pp1);
+            cf += (double)elem_column(vbe, oy, bit, pp0, pp1);
+        }
+        if (E.ok && (lane & others) == 0) {
+            red_add(&A.t1_bar[(long long)r * v + z], ct);
+            red_add(&A.fvo_bar[(long long)z * o + r], cf);
+        }
+    }
 }
 
 }  // namespace tb

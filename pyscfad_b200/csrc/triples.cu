@@ -1347,9 +1347,9 @@ static int elem_warps(int elems) { return elems > 32 ? elems / 32 : 1; }
 // With the adjoint, items of 256 elements fill the orbit kernel's CTA well enough (nocc 16 nvir 36 =
 // 2 x 16 + 4: 8.5 / 8.35 ms; the energy alone 3.12 / 3.29) and those of 128 need more of them (nvir 34:
 // nocc 7 1.10 / 1.10 ms, nocc 12 3.76 / 3.86, nocc 16 7.64 / 7.95).
-// Mixed modes: items of up to 32 elements, in place of k_f2m, which evaluates 512 slots of every item
-// (energy nocc 64 nvir 3 0.84 / 7.4 ms, nocc 32 nvir 7 0.79 / 2.6; E + VJP nocc 16 nvir 17 0.94 / 1.03,
-// nocc 300 nvir 2 73 / 275).  Larger items and fewer of them stay with k_f2m and its FP32 sums.
+// Mixed modes (k_f2em): items of up to 32 elements, in place of k_f2m, which evaluates 512 slots of
+// every item; its FP32 values are the same (energy nocc 64 nvir 3 0.84 / 7.4 ms, nocc 32 nvir 7 0.78 / 2.6;
+// E + VJP nocc 16 nvir 17 0.95 / 1.03, nocc 300 nvir 2 72 / 275).
 static bool by_element(const Plan &P, const ChunkDesc &ch) {
     const int e = chunk_elems(ch);
     if (P.prec != TRIPLES_PRECISION_FP64) return e <= 32 && P.n_ijk >= 500;
@@ -1845,8 +1845,8 @@ static int mixed_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t 
         }
         if (nelem > 0) {
             const int ctas = group_starts(H, nelem, [&](const F2P &j) { return elem_ctas(P, j); });
-            if (bf16) TB_KLAUNCH(P_F2, (k_f2e<2><<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
-            else TB_KLAUNCH(P_F2, (k_f2e<1><<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
+            if (bf16) TB_KLAUNCH(P_F2, (k_f2em<2><<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
+            else TB_KLAUNCH(P_F2, (k_f2em<1><<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
         }
         TB_KLAUNCH(P_F2, (k_energy_sum<<<1, 256, 0, st>>>(X, n)));
     }
@@ -1903,7 +1903,7 @@ static int fp64_chunks(const Plan &P, const ChunkDesc *ch, int n, cudaStream_t s
         }
         if (nelem > 0) {
             const int ctas = group_starts(H, nelem, [&](const F2P &j) { return elem_ctas(P, j); });
-            TB_KLAUNCH(P_F2, (k_f2e<0><<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
+            TB_KLAUNCH(P_F2, (k_f2e<<<(unsigned)ctas, kElemThreads, 0, st>>>(H)));
         }
         TB_KLAUNCH(P_F2, (k_energy_sum<<<1, 256, 0, st>>>(X, n)));
     }

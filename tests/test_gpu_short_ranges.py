@@ -121,6 +121,29 @@ def test_mixed_short_ranges(o, v, tv, precision):
             assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < g_tol, k
 
 
+# An item of up to 32 elements gives the same FP32 values in its element kernel as in the persistent epilogue,
+# which the batch engine uses for every chunk (nvir below 8: all items short, of 1 to 64 elements, with
+# equal occupied and virtual ranges); only FP64 sums are ordered differently.
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["mixed", "mixed_bf16"])
+def test_mixed_short_ranges_have_the_values_of_the_persistent_epilogue(precision):
+    from pyscfad_b200.batched import BatchedTriples
+
+    problems = []
+    for o, v in ((14, 2), (14, 3), (15, 5), (16, 7), (17, 6), (20, 1)):
+        inp = make_inputs(o, v, 40, seed=o + v, fvo_sigma=1e-3)
+        problems.append({k: getattr(inp, k) for k in G.KEYS})
+    batch = BatchedTriples(problems, precision=precision, engine="batch", tune=False)
+    batch.run()
+    for prob, (e0, g0) in zip(problems, batch.results()):
+        e, g = triples.energy_vjp(*(prob[k] for k in G.KEYS), precision=precision, device="cuda")
+        if prob["t1"].shape[1] == 1:
+            continue   # one virtual orbital has no triples: both are rounding noise
+        assert abs(float(e) - e0) <= 1e-12 * abs(e0)
+        for k in G.KEYS:
+            assert _relerr(g[k].cpu().numpy(), g0[k].cpu().numpy()) < 1e-11, k
+
+
 # Host threads with different nocc share the projection kernel of their range; each call must find the shared
 # memory that it asks for, whatever another thread is launching.
 @pytest.mark.gpu
