@@ -7,6 +7,7 @@ ovvv[o,v,v(v+1)/2] (packed, DF ERIs) or ovvv[o,v,v,v], fvo[v,o].
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -33,13 +34,13 @@ def _alloc(nbytes: int, device: torch.device, stream) -> torch.Tensor:
         return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
 
 
-def _workspace(nbytes: int, device: torch.device, stream, extra: int = 0, least=None) -> torch.Tensor:
+def _workspace(nbytes: int, device: torch.device, stream, extra: int = 0, least: int = 0) -> torch.Tensor:
     """Scratch of nbytes, with `extra` more while the device has room for it (triples_workspace_extra); where
-    it has not even room for nbytes, of least() bytes (triples_workspace_least)."""
+    it has not even room for nbytes, of `least` bytes if given (triples_workspace_least)."""
     key = _key(device, stream)
     while True:
         level = _without.get(key, 0)
-        want = nbytes + extra if level == 0 else nbytes if level == 1 or least is None else least()
+        want = nbytes + extra if level == 0 else nbytes if level == 1 else least or nbytes
         buf = _workspaces.get(key)
         if buf is not None and buf.numel() >= want:
             return buf
@@ -49,7 +50,7 @@ def _workspace(nbytes: int, device: torch.device, stream, extra: int = 0, least=
             buf = _workspaces[key] = _alloc(want, device, stream)
             return buf
         except torch.cuda.OutOfMemoryError:
-            if level >= 2 or least is None:
+            if level >= 2 or (not extra and not least):
                 raise
             _without[key] = level + 1
 
@@ -65,14 +66,14 @@ def _give_back(device: torch.device) -> bool:
     return bool(keys)
 
 
-def _with_room(device: torch.device, call):
-    """call(), and again with optional scratch given back while the device memory does not suffice (for
+def _with_room(call, device, t1, *args):
+    """call(...), and again with optional scratch given back while the device memory does not suffice (for
     the scratch, the outputs or the inputs' copies)."""
     while True:
         try:
-            return call()
+            return call(device, t1, *args)
         except torch.cuda.OutOfMemoryError:
-            if not _give_back(device):
+            if not _give_back(_device_of(device, t1)):
                 raise
 
 
@@ -162,35 +163,39 @@ def workspace_least(nocc, nvir, packed=True, want_grad=True, precision="fp64") -
                                                    None))
 
 
-def _optional(prec, o, v, packed, want_grad, opt):
-    """The extra and least arguments of _workspace for a canonical plan."""
-    lib, args = _lib.load(), (prec, o, v, int(packed), int(want_grad), ctypes.byref(opt) if opt is not None else None)
-    return lib.triples_workspace_extra(*args), lambda: lib.triples_workspace_least(*args)
+@functools.lru_cache(maxsize=256)
+def _plan_bytes(prec, o, v, packed, want_grad, *opt):
+    """Scratch of a call by its sizes and options alone: (what it takes, triples_workspace_extra beyond that,
+    triples_workspace_least)."""
+    lib, args = _lib.load(), (prec, o, v, packed, want_grad, ctypes.byref(_lib.Options(*opt)))
+    return (lib.triples_workspace_size_ex(*args), lib.triples_workspace_extra(*args),
+            lib.triples_workspace_least(*args))
 
 
 def _device_of(device, t1):
     return torch.device(device or (t1.device if isinstance(t1, torch.Tensor) and t1.is_cuda else "cuda"))
 
 
-def _run(*args):
-    return _with_room(_device_of(args[10], args[1]), lambda: _run_once(*args))
+def _run(mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, device, stream, check,
+         block_size, chunk_range, accumulation_segment, tile_n=0):
+    return _with_room(_run_once, device, t1, mo_energy, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, stream,
+                      check, _lib.options(block_size, chunk_range, accumulation_segment, tile_n))
 
 
-def _run_once(mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, device, stream, check,
-              block_size, chunk_range, accumulation_segment, tile_n=0):
+def _run_once(device, t1, mo_energy, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, stream, check, opt):
     lib = _lib.load()
     device = _device_of(device, t1)
     args = [_as_dev(a, device) for a in (mo_energy, t1, t2, ovoo, ovov, ovvv, fvo)]
     o, v, packed = _shapes(*args[1:], args[0])
     prec = _lib.PRECISION[precision]
-    opt = _lib.options(block_size, chunk_range, accumulation_segment, tile_n)
-    nbytes = lib.triples_workspace_size_ex(prec, o, v, int(packed), int(want_grad), ctypes.byref(opt))
+    nbytes, extra, least = _plan_bytes(prec, o, v, int(packed), int(want_grad), opt.block_size, opt.chunk_a0, opt.chunk_a1,
+                                       opt.accumulation_segment, opt.tile_n)
     if nbytes == 0:
         raise _lib.TriplesError(1, "triples_workspace_size_ex")
     st = stream if stream is not None else torch.cuda.current_stream(device)
     e = torch.zeros((), dtype=torch.float64, device=device)
     grads = {k: torch.empty_like(a) for k, a in zip(KEYS, args)} if want_grad else {}
-    ws = _workspace(nbytes, device, st, *_optional(prec, o, v, packed, want_grad, opt))   # the outputs must fit first
+    ws = _workspace(nbytes, device, st, extra, least)   # (the outputs must fit first)
     gptr = [grads[k].data_ptr() for k in KEYS] if want_grad else [None] * len(KEYS)
     rc = lib.triples_energy_vjp_ex(st.cuda_stream, prec, o, v, int(packed), *[a.data_ptr() for a in args],
                                    float(ybar), int(want_grad), ctypes.byref(opt), ws.data_ptr(), ws.numel(),
@@ -233,11 +238,13 @@ def lno_workspace_size(nocc, nvir, packed=True, want_grad=True, precision="fp64"
                                                          int(want_grad), ctypes.byref(opt)))
 
 
-def _run_lno(*args):
-    return _with_room(_device_of(args[11], args[2]), lambda: _run_lno_once(*args))
+def _run_lno(mat, mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, device, stream, check,
+             block_size):
+    return _with_room(_run_lno_once, device, t1, mat, mo_energy, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision,
+                      stream, check, block_size)
 
 
-def _run_lno_once(mat, mo_energy, t1, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, device, stream, check,
+def _run_lno_once(device, t1, mat, mo_energy, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad, precision, stream, check,
                   block_size):
     lib = _lib.load()
     device = _device_of(device, t1)
@@ -312,11 +319,12 @@ def energy_vjp_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar=1.0, precis
     return _run_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, True, precision, device, stream, check)
 
 
-def _run_df(*args):
-    return _with_room(_device_of(args[11], args[1]), lambda: _run_df_once(*args))
+def _run_df(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, want_grad, precision, device, stream, check):
+    return _with_room(_run_df_once, device, t1, mo_energy, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, want_grad, precision,
+                      stream, check)
 
 
-def _run_df_once(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, want_grad, precision, device, stream, check):
+def _run_df_once(device, t1, mo_energy, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, want_grad, precision, stream, check):
     lib = _lib.load()
     device = _device_of(device, t1)
     args, o, v, naux = _df_args(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, device)
@@ -327,10 +335,9 @@ def _run_df_once(mo_energy, t1, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, want_grad, 
     st = stream if stream is not None else torch.cuda.current_stream(device)
     e = torch.zeros((), dtype=torch.float64, device=device)
     grads = {k: torch.empty_like(a) for k, a in zip(DF_KEYS, args)} if want_grad else {}
-    extra, least = _optional(prec, o, v, True, want_grad, None)
-    # (the plan's optional part is that of a canonical call; ovvv and its cotangent lie behind it)
-    ws = _workspace(nbytes, device, st, extra,
-                    lambda: nbytes - lib.triples_workspace_size(prec, o, v, 1, int(want_grad)) + least())
+    # the plan is that of a canonical call with packed ovvv; ovvv and its cotangent lie behind it
+    plan, extra, least = _plan_bytes(prec, o, v, 1, int(want_grad), 0, 0, 0, 0, 0)
+    ws = _workspace(nbytes, device, st, extra, nbytes - plan + least)
     ins = [a.data_ptr() for a in args]
     if want_grad:
         name = "triples_energy_vjp_df"

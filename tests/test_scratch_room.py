@@ -33,21 +33,21 @@ def room(monkeypatch):
 def test_scratch_falls_back_to_what_the_call_needs(room):
     limit, log = room
     cpu = torch.device("cpu")
-    assert triples._workspace(1000, cpu, _Stream, 500, lambda: 900).numel() == 1500
-    assert triples._workspace(1000, cpu, _Stream, 500, lambda: 900).numel() == 1500    # kept
+    assert triples._workspace(1000, cpu, _Stream, 500, 900).numel() == 1500
+    assert triples._workspace(1000, cpu, _Stream, 500, 900).numel() == 1500    # kept
     triples.release_workspace()
     limit[0] = 1200
-    assert triples._workspace(1000, cpu, _Stream, 500, lambda: 900).numel() == 1000
+    assert triples._workspace(1000, cpu, _Stream, 500, 900).numel() == 1000
     triples.release_workspace()
     limit[0] = 950
-    assert triples._workspace(1000, cpu, _Stream, 500, lambda: 900).numel() == 900
+    assert triples._workspace(1000, cpu, _Stream, 500, 900).numel() == 900
     del log[:]
-    assert triples._workspace(1000, cpu, _Stream, 500, lambda: 900).numel() == 900     # no further attempt at more
+    assert triples._workspace(1000, cpu, _Stream, 500, 900).numel() == 900     # no further attempt at more
     assert log == []
     triples.release_workspace()
     limit[0] = 800
     with pytest.raises(torch.cuda.OutOfMemoryError):
-        triples._workspace(1000, cpu, _Stream, 500, lambda: 900)
+        triples._workspace(1000, cpu, _Stream, 500, 900)
     assert triples._workspaces == {}
 
 
@@ -55,21 +55,21 @@ def test_outputs_get_the_room_of_the_optional_scratch(room):
     """An allocation beside the scratch that fails: the scratch is given back and the call tried once more."""
     cpu, tries = torch.device("cpu", 0), []
 
-    def call():
-        ws = triples._workspace(1000, cpu, _Stream, 500, lambda: 900)
+    def call(device, t1):
+        ws = triples._workspace(1000, cpu, _Stream, 500, 900)
         tries.append(ws.numel())
         if ws.numel() > 900:
             raise torch.cuda.OutOfMemoryError("no room for the outputs")
         return "done"
 
-    assert triples._with_room(cpu, call) == "done" and tries == [1500, 1000, 900]
+    assert triples._with_room(call, cpu, None) == "done" and tries == [1500, 1000, 900]
     # nothing optional left to give back: the error reaches the caller
 
-    def never():
+    def never(device, t1):
         raise torch.cuda.OutOfMemoryError("no room")
 
     with pytest.raises(torch.cuda.OutOfMemoryError):
-        triples._with_room(cpu, never)
+        triples._with_room(never, cpu, None)
 
 
 @pytest.mark.parametrize("o,v", [(5, 19), (20, 180), (40, 360), (50, 450)])
