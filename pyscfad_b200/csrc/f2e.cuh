@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2e(const __grid_constant__
 }
 
 // ---------------------------------------------------------------------------
-// The mixed modes: items within a warp (at most 32 elements).  FP32 where k_f2m is, and the same
+// The mixed modes.  With the adjoint, items within a warp (at most 32 elements).  FP32 where k_f2m is, and the same
 // FP32 operations in the same order, so that a chunk gives the same values in either kernel: V terms
 // summed over rho, rows along z, columns over y + 4, then bit 0 of y, bits 2, 1 and 0 of x, bit 1 of y.
 // (What k_f2m adds for coordinates beyond a short range are zeros.)
@@ -285,8 +285,9 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2em(const __grid_constant_
     for (int pi = 0; pi < 6; pi++) {
         int pp[3] = {0, 0, 0};
         perm_of(pi, pp);
-        S[pi] = static_cast<const float *>(A.S) + R.pi[pi].s0 +
-                (E.loc[pp[1]] * R.len[pp[0]] + E.loc[pp[0]]) * R.len[pp[2]] + E.loc[pp[2]];   // (not two ranges of 8: no row exchange)
+        const int ex = R.len[pp[0]], ez = R.len[pp[2]], y = E.loc[pp[1]];
+        const int swz = ex == 8 && ez == 8 ? f2m_row_swizzle(y) : 0;
+        S[pi] = static_cast<const float *>(A.S) + R.pi[pi].s0 + y * ex * ez + ((E.loc[pp[0]] * ez + E.loc[pp[2]]) ^ swz);
     }
     float tz[3][3], fz[3][3];
 #pragma unroll
@@ -335,7 +336,7 @@ __global__ void __launch_bounds__(kElemThreads, 2) k_f2em(const __grid_constant_
 #pragma unroll
     for (int s = 0; s < 6; s++) esum += WW[s] * Z[s];
     const double en = elem_sum(E.ok ? cen * esum * rD : 0.0, E.all);
-    if (E.ok && (lane & E.all) == 0) A.e_part[(long long)E.sub * A.n_ijk + E.rep] = en;
+    if (E.ok && (lane & E.all) == 0) A.e_part[(long long)(E.sub * E.warps + (E.el >> 5)) * A.n_ijk + E.rep] = en;
     if (!A.want_grad) return;
     const float wsc = (float)*A.wscale;
     const double g0 = cocc * A.ybar * rD;

@@ -192,8 +192,9 @@ struct LnoProj {
     }
 };
 
-// FULL: three full sub-ranges, 512 slots a triple: a tile of columns is consecutive (with the general
-// form's divisions per thread and column, nocc 14 nvir 96 takes 2 % more of a call).
+// FULL: three full sub-ranges, 512 slots a triple: a tile of columns is consecutive (the general form, with
+// a division per thread and column, took 2 % more of a call at nocc 14 nvir 96, 6 % of this kernel at
+// nocc 49 nvir 24).
 template <int COLS, bool FULL>
 __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_constant__ LnoArgs A, int slot, int first) {
     using C = LnoProj<COLS>;
@@ -229,15 +230,24 @@ __global__ void __launch_bounds__(kLnoThreads, 2) k_lno_proj(const __grid_consta
     auto column = [&](int c) -> long long { return c + (long long)(c / run) * run * (o - 1); };
     auto issue = [&](int t, int b) {
         double *sw = sw_b + b * rows * LD, *sq = sq_b + b * rows * LD;
-        const int j = threadIdx.x % (COLS / 2) * 2;   // (this thread's columns in every turn)
-        const bool in = FULL || t * COLS + j < ncol;
-        const long long base = FULL ? column(t * COLS) + j : (in ? column(t * COLS + j) : 0);
-        for (int l = threadIdx.x / (COLS / 2); l < rows; l += kLnoThreads / (COLS / 2)) {
-            const bool ok = in && l < o;
-            const long long at = base + (ok ? l * rstride : 0);
-            const int bytes = ok ? 16 : 0;
+        auto copy = [&](int l, int j, long long at, int bytes) {
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sw + l * LD + j)), "l"(A.WW + at), "r"(bytes) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sq + l * LD + j)), "l"(A.Q + at), "r"(bytes) : "memory");
+        };
+        if constexpr (FULL) {
+            const long long base = column(t * COLS);
+            for (int e = threadIdx.x; e < rows * (COLS / 2); e += blockDim.x) {
+                const int l = e / (COLS / 2), j = e % (COLS / 2) * 2;
+                copy(l, j, base + (l < o ? l * rstride + j : 0), l < o ? 16 : 0);
+            }
+        } else {
+            const int j = threadIdx.x % (COLS / 2) * 2;   // (this thread's columns in every turn)
+            const bool in = t * COLS + j < ncol;
+            const long long base = in ? column(t * COLS + j) : 0;
+            for (int l = threadIdx.x / (COLS / 2); l < rows; l += kLnoThreads / (COLS / 2)) {
+                const bool ok = in && l < o;
+                copy(l, j, base + (ok ? l * rstride : 0), ok ? 16 : 0);
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (grad && last && threadIdx.x < COLS) {

@@ -1347,12 +1347,13 @@ static int elem_warps(int elems) { return elems > 32 ? elems / 32 : 1; }
 // With the adjoint, items of 256 elements fill the orbit kernel's CTA well enough (nocc 16 nvir 36 =
 // 2 x 16 + 4: 8.5 / 8.35 ms; the energy alone 3.12 / 3.29) and those of 128 need more of them (nvir 34:
 // nocc 7 1.10 / 1.10 ms, nocc 12 3.76 / 3.86, nocc 16 7.64 / 7.95).
-// Mixed modes (k_f2em): items of up to 32 elements, in place of k_f2m, which evaluates 512 slots of
-// every item; its FP32 values are the same (energy nocc 64 nvir 3 0.84 / 7.4 ms, nocc 32 nvir 7 0.78 / 2.6;
-// E + VJP nocc 16 nvir 17 0.95 / 1.03, nocc 300 nvir 2 72 / 275).
+// Mixed modes (k_f2em): items of up to 32 elements, 64 without the adjoint, in place of k_f2m, which
+// evaluates 512 slots of every item; its FP32 values are the same (energy nocc 64 nvir 3 0.84 / 7.4 ms,
+// nocc 200 nvir 4 23 / 59, nocc 20 nvir 17 0.59 / 0.87; E + VJP nocc 16 nvir 17 0.95 / 1.03, nocc 300 nvir 2
+// 72 / 275).
 static bool by_element(const Plan &P, const ChunkDesc &ch) {
     const int e = chunk_elems(ch);
-    if (P.prec != TRIPLES_PRECISION_FP64) return e <= 32 && P.n_ijk >= 500;
+    if (P.prec != TRIPLES_PRECISION_FP64) return e <= (P.want_grad ? 32 : 64) && P.n_ijk >= 500;
     if (!P.want_grad) return e < 512 && P.n_ijk >= 56;
     return e <= 64 ? P.n_ijk >= 56 : e <= 128 && P.n_ijk >= 300;
 }
