@@ -97,6 +97,8 @@ def holds_workspace(nbytes: int) -> bool:
 
 
 def release_workspace():
+    """Give all cached scratch back to torch's allocator: per stream that of its largest call, up to 2 GiB
+    of it optional (the library's own calls give that part back when memory is short)."""
     _workspaces.clear()
     _without.clear()
 
