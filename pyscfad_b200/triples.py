@@ -23,6 +23,9 @@ _workspaces: dict = {}
 # chunk groups, 2 the V-term tables as well (until release_workspace).
 _without: dict = {}
 
+# Streams with calls recorded in a CUDA graph: its replays use their scratch, which is not given back.
+_captured: set = set()
+
 
 def _key(device, stream):
     return (device.type, device.index, int(stream.cuda_stream))
@@ -55,11 +58,20 @@ def _workspace(nbytes: int, device: torch.device, stream, extra: int = 0, least:
             _without[key] = level + 1
 
 
+def _stream_of(stream, device):
+    """The stream of a call, noted if the call is being captured."""
+    st = stream if stream is not None else torch.cuda.current_stream(device)
+    if torch.cuda.is_current_stream_capturing():
+        _captured.add(_key(device, st))
+    return st
+
+
 def _give_back(device: torch.device) -> bool:
     """Drop the scratch of the device's streams that may hold more than their calls need; these calls
     take less from now on.  False if there was none."""
     index = torch.cuda.current_device() if device.index is None else device.index
-    keys = [k for k in list(_workspaces) if k[0] == device.type and k[1] in (index, None) and _without.get(k, 0) < 2]
+    keys = [k for k in list(_workspaces) if k[0] == device.type and k[1] in (index, None) and
+            _without.get(k, 0) < 2 and k not in _captured]
     for k in keys:
         _without[k] = _without.get(k, 0) + 1
         _workspaces.pop(k, None)
@@ -101,6 +113,7 @@ def release_workspace():
     of it optional (the library's own calls give that part back when memory is short)."""
     _workspaces.clear()
     _without.clear()
+    _captured.clear()
 
 
 def _as_dev(x, device) -> torch.Tensor:
@@ -194,7 +207,7 @@ def _run_once(device, t1, mo_energy, t2, ovoo, ovov, ovvv, fvo, ybar, want_grad,
                                        opt.accumulation_segment, opt.tile_n)
     if nbytes == 0:
         raise _lib.TriplesError(1, "triples_workspace_size_ex")
-    st = stream if stream is not None else torch.cuda.current_stream(device)
+    st = _stream_of(stream, device)
     e = torch.zeros((), dtype=torch.float64, device=device)
     grads = {k: torch.empty_like(a) for k, a in zip(KEYS, args)} if want_grad else {}
     ws = _workspace(nbytes, device, st, extra, least)   # (the outputs must fit first)
@@ -258,7 +271,7 @@ def _run_lno_once(device, t1, mat, mo_energy, t2, ovoo, ovov, ovvv, fvo, ybar, w
     nbytes = lib.triples_lno_workspace_size_ex(prec, o, v, int(packed), int(want_grad), ctypes.byref(opt))
     if nbytes == 0:
         raise _lib.TriplesError(4 if o > 64 else 1, "triples_lno_workspace_size_ex")
-    st = stream if stream is not None else torch.cuda.current_stream(device)
+    st = _stream_of(stream, device)
     e = torch.zeros((), dtype=torch.float64, device=device)
     keys = ("mat",) + KEYS
     grads = {k: torch.empty_like(a) for k, a in zip(keys, args)} if want_grad else {}
@@ -334,7 +347,7 @@ def _run_df_once(device, t1, mo_energy, t2, ovoo, ovov, Lov, Lvv, fvo, ybar, wan
     nbytes = lib.triples_df_workspace_size(prec, o, v, naux, int(want_grad))
     if nbytes == 0:
         raise _lib.TriplesError(1, "triples_df_workspace_size")
-    st = stream if stream is not None else torch.cuda.current_stream(device)
+    st = _stream_of(stream, device)
     e = torch.zeros((), dtype=torch.float64, device=device)
     grads = {k: torch.empty_like(a) for k, a in zip(DF_KEYS, args)} if want_grad else {}
     # the plan is that of a canonical call with packed ovvv; ovvv and its cotangent lie behind it

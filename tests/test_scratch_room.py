@@ -72,6 +72,21 @@ def test_outputs_get_the_room_of_the_optional_scratch(room):
         triples._with_room(never, cpu, None)
 
 
+def test_scratch_of_captured_calls_stays(room):
+    """A recorded graph holds its scratch's address: it is not given back for another stream's sake."""
+    cpu = torch.device("cpu", 0)
+
+    class Other:
+        cuda_stream = 1
+
+    kept = triples._workspace(1000, cpu, _Stream, 500, 900)
+    triples._captured.add(triples._key(cpu, _Stream))
+    triples._workspace(1000, cpu, Other, 500, 900)
+    assert triples._give_back(cpu)
+    assert list(triples._workspaces.values()) == [kept] and triples._workspaces[triples._key(cpu, _Stream)] is kept
+    assert not triples._give_back(cpu)
+
+
 @pytest.mark.parametrize("o,v", [(5, 19), (20, 180), (40, 360), (50, 450)])
 def test_least_scratch_is_without_the_tables(o, v):
     lib = _lib.load()
@@ -87,6 +102,26 @@ def test_least_scratch_is_without_the_tables(o, v):
     for prec in (0, 1):
         n = lib.triples_batch_workspace_size(prec, 2, arr) - lib.triples_batch_workspace_least(prec, 2, arr)
         assert n == 2 * (lib.triples_workspace_size(prec, o, v, 1, 1) - lib.triples_workspace_least(prec, o, v, 1, 1, None))
+
+
+@pytest.mark.gpu
+def test_captured_call_is_noted_and_replays():
+    inp = make_inputs(4, 20, 30, seed=3, fvo_sigma=1e-3)
+    ins = [torch.as_tensor(np.ascontiguousarray(getattr(inp, k)), device="cuda") for k in G.KEYS]
+    e0, g0 = triples.energy_vjp(*ins, precision="mixed")
+    triples.release_workspace()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        e, g = triples.energy_vjp(*ins, precision="mixed", check=False)
+    assert len(triples._captured) == 1 and triples._captured <= set(triples._workspaces)
+    assert not triples._give_back(torch.device("cuda"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert abs(float(e) - float(e0)) <= 1e-12 * abs(float(e0))
+    for k in G.KEYS:
+        ref = g0[k].cpu().numpy()
+        assert float(np.abs(g[k].cpu().numpy() - ref).max()) <= 1e-11 * max(float(np.abs(ref).max()), 1e-7), k
+    triples.release_workspace()
 
 
 @pytest.mark.gpu
